@@ -666,13 +666,32 @@ __global__ void k_read_ints(IntReads r, volatile int *dst)
 
 // One mapped pinned buffer per host thread and device (256 bytes each, kept
 // until the process exits).
-int read_ints(const IntReads &r, int *out, cudaStream_t st)
+int pinned_ints(int **host, int **dptr)
 {
     static thread_local int *host_buf[64] = {nullptr};
+    static thread_local int *dev_buf[64] = {nullptr};
     int dev = 0;
     PFF_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || r.k > 8) {
-        set_error("read_ints: device %d or %d reads out of range", dev, r.k);
+    if (dev < 0 || dev >= 64) {
+        set_error("pinned_ints: device %d out of range", dev);
+        return PFF_ERR_ARG;
+    }
+    if (!host_buf[dev]) {
+        void *p = nullptr, *d = nullptr;
+        PFF_CUDA(cudaHostAlloc(&p, 64 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        PFF_CUDA(cudaHostGetDevicePointer(&d, p, 0));
+        host_buf[dev] = (int *)p;
+        dev_buf[dev] = (int *)d;
+    }
+    *host = host_buf[dev];
+    *dptr = dev_buf[dev];
+    return PFF_OK;
+}
+
+int read_ints(const IntReads &r, int *out, cudaStream_t st)
+{
+    if (r.k > 8) {
+        set_error("read_ints: %d reads out of range", r.k);
         return PFF_ERR_ARG;
     }
     int total = 0;
@@ -681,17 +700,12 @@ int read_ints(const IntReads &r, int *out, cudaStream_t st)
         set_error("read_ints: %d ints exceed 64", total);
         return PFF_ERR_ARG;
     }
-    if (!host_buf[dev]) {
-        void *p = nullptr;
-        PFF_CUDA(cudaHostAlloc(&p, 64 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-        host_buf[dev] = (int *)p;
-    }
-    int *dptr = nullptr;
-    PFF_CUDA(cudaHostGetDevicePointer((void **)&dptr, host_buf[dev], 0));
+    int *host = nullptr, *dptr = nullptr;
+    PFF_TRY(pinned_ints(&host, &dptr));
     { k_read_ints<<<1, 1, 0, st>>>(r, dptr); count_launch(); }
     PFF_CUDA(cudaStreamSynchronize(st));
     PFF_TRY(check_cuda("read_ints"));
-    const volatile int *h = host_buf[dev];
+    const volatile int *h = host;
     for (int q = 0; q < total; ++q) out[q] = h[q];
     return PFF_OK;
 }

@@ -72,6 +72,9 @@ struct IntReads {
 };
 int read_ints(const IntReads &r, int *out, cudaStream_t st);
 
+// The calling thread's 64 pinned ints on the current device: host and device address.
+int pinned_ints(int **host, int **dptr);
+
 
 // Bump allocator over a caller-provided device workspace (256-byte aligned slices).
 struct Carver {

@@ -46,10 +46,10 @@ __global__ void k_count_pits(const int32_t *__restrict__ rec, Grid g, int *count
 
 // basin_id_init (:47-61)
 template <int MODE>
-__global__ void k_basin_init(int32_t *bid, Grid g, const int *guard)
+__global__ void k_basin_init(int32_t *bid, Grid g)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.N() || (guard && *guard == 0)) return;
+    if (i >= g.N()) return;
     bid[i] = can_leave_i<MODE>(g, i) ? 0 : i + 1;
 }
 
@@ -312,82 +312,77 @@ __device__ __forceinline__ void block_append(bool pred, int val, int *list, int 
     __syncthreads();
 }
 
-// info[0] pits, info[2] set if some exit target is not a tile-border cell
-// (receivers that are not D4 neighbours)
-// tiles: optional list of tile ids -- recompute only those tiles; pits:
-// optional (nullptr: no pit list).
-template <int MODE>
-__device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, int32_t *R, int *pits, int *info,
-                                  const Grid &g, int tx, int ty, int *p, int *ext);
-
-// Tile terminals of the tiles listed in tiles[0 .. *ntiles) (one block per tile,
-// the grid strides over the list; the count is read on the device), or of every
-// tile (tiles == NULL, a 2-D grid of tiles).
-template <int MODE>
-__global__ void __launch_bounds__(TILE_THREADS) k_tile_terminal(const int32_t *__restrict__ rec, int32_t *J, int32_t *R,
-                                                                int *pits, int *info, Grid g, const int *tiles,
-                                                                const int *ntiles)
+// Exact quotient and remainder of n / d for 0 <= n < 2^31 and d >= 2 without the
+// integer divide sequence: with m = floor(2^32 / d) or m = floor((2^32 - 1) / d) (one
+// less only when d divides 2^32), q = umulhi(n, m) is floor(n / d) or one less
+// (n m / 2^32 > n / d - 2 n / 2^32 > n / d - 1), and one correction of the remainder
+// fixes it.
+__device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int &r)
 {
-    __shared__ int p[TILE_CELLS];
-    __shared__ int ext[TILE_CELLS];
-    if (!tiles) {
-        tile_terminal_one<MODE>(rec, J, R, pits, info, g, blockIdx.x, blockIdx.y, p, ext);
-        return;
-    }
-    const int ntx = (g.nx + TILE_W - 1) / TILE_W, n = *ntiles;
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
-        const int t = tiles[k];
-        tile_terminal_one<MODE>(rec, J, R, pits, info, g, t % ntx, t / ntx, p, ext);
-        __syncthreads();  // p and ext are reused by the next tile
-    }
+    q = (int)__umulhi((unsigned)n, m);
+    r = n - q * d;
+    if (r >= d) { ++q; r -= d; }
 }
 
+// Tile-local index of the receiver r of cell i = (row0 + ly, col0 + lx) (local index c), or
+// c itself when the cell is a root or its receiver lies outside the w x h tile.
+__device__ __forceinline__ int tile_local(int r, int i, int c, int lx, int ly, int row0, int col0, int w, int h, int nx,
+                                          unsigned mnx)
+{
+    if (r == i) return c;
+    if (r == i - 1) return lx > 0 ? c - 1 : c;
+    if (r == i + 1) return lx < w - 1 ? c + 1 : c;
+    if (r == i - nx) return ly > 0 ? c - TILE_W : c;
+    if (r == i + nx) return ly < h - 1 ? c + TILE_W : c;
+    int rr, rc;
+    divmod_nx(r, nx, mnx, rr, rc);
+    rr -= row0;
+    rc -= col0;
+    return rr >= 0 && rr < h && rc >= 0 && rc < w ? rr * TILE_W + rc : c;
+}
+
+// Tile terminals of one tile by one block: J[i] = the receiver of the last in-tile cell of
+// i's path (the root itself, or the first cell past the tile).  info[0] pits (pits ==
+// nullptr: no pit list), info[2] set if some exit target is not a tile-border cell
+// (receivers that are not D4 neighbours).  copy: also rec_copy = rec.
+//
+// Bound by the latency of the jump rounds' shared-memory chains.  Each thread keeps its 8
+// cells' pointers in registers and issues their 8 loads together; pointers are 16-bit.
 template <int MODE>
 __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, int32_t *R, int *pits, int *info,
-                                  const Grid &g, int tx, int ty, int *p, int *ext)
+                                  const Grid &g, int tx, int ty, uint16_t *p, int *rv, int32_t *rec_copy)
 {
     const int nx = g.nx, ny = g.ny;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
     const int col0 = tx * TILE_W, row0 = ty * TILE_H;
     const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
+    static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
+    const int lx = threadIdx.x & (TILE_W - 1), ly0 = threadIdx.x / TILE_W;
+    const int i0 = (row0 + ly0) * nx + col0 + lx;
+    int r[TILE_PER_THREAD], q[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) r[k] = (lx < w && ly0 + 4 * k < h) ? rec[i0 + 4 * k * nx] : -1;
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = threadIdx.x + k * TILE_THREADS;
-        const int lx = c % TILE_W, ly = c / TILE_W;
-        int pc = c, e = -2;
-        if (lx < w && ly < h) {
-            const int i = (row0 + ly) * nx + col0 + lx;
-            const int r = rec[i];
-            if (r == i) {
-                e = -1;
-            } else {
-                int rly, rlx;
-                if (r == i - 1) { rly = ly; rlx = lx - 1; }
-                else if (r == i + 1) { rly = ly; rlx = lx + 1; }
-                else if (r == i - nx) { rly = ly - 1; rlx = lx; }
-                else if (r == i + nx) { rly = ly + 1; rlx = lx; }
-                else { const int rr = r / nx; rly = rr - row0; rlx = r - rr * nx - col0; }
-                if (rly >= 0 && rly < h && rlx >= 0 && rlx < w) pc = rly * TILE_W + rlx;
-                else e = r;
-            }
-        }
-        p[c] = pc;
-        ext[c] = e;
+        const int c = threadIdx.x + k * TILE_THREADS, i = i0 + 4 * k * nx;
+        q[k] = r[k] < 0 ? c : tile_local(r[k], i, c, lx, ly0 + 4 * k, row0, col0, w, h, nx, mnx);
+        p[c] = (uint16_t)q[k];
+        rv[c] = r[k];
+        if (rec_copy && r[k] >= 0) rec_copy[i] = r[k];
     }
     __syncthreads();
-    // at most ceil(log2 2048) = 11 rounds for any acyclic in-tile path.  A thread reads
-    // all its cells' pointers, then all the pointers they point to, then stores: the
-    // shared-memory round trips overlap (one interleaving of the same concurrent updates)
+    // at most ceil(log2 2048) = 11 rounds for any acyclic in-tile path (one interleaving
+    // of concurrent pointer jumps: a pointer always holds some later cell of the path)
     for (int round = 0; round < 12; ++round) {
         bool ch = false;
-        int q[TILE_PER_THREAD], qq[TILE_PER_THREAD];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) q[k] = p[threadIdx.x + k * TILE_THREADS];
+        int qq[TILE_PER_THREAD];
 #pragma unroll
         for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
 #pragma unroll
         for (int k = 0; k < TILE_PER_THREAD; ++k)
             if (qq[k] != q[k]) {
-                p[threadIdx.x + k * TILE_THREADS] = qq[k];
+                p[threadIdx.x + k * TILE_THREADS] = (uint16_t)qq[k];
+                q[k] = qq[k];
                 ch = true;
             }
         if (!__syncthreads_or(ch)) break;
@@ -395,19 +390,18 @@ __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, i
     bool nonlocal = false;
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = threadIdx.x + k * TILE_THREADS;
-        const int lx = c % TILE_W, ly = c / TILE_W;
+        const int c = threadIdx.x + k * TILE_THREADS, ly = ly0 + 4 * k, i = i0 + 4 * k * nx;
         bool pit = false;
-        int i = -1;
-        if (lx < w && ly < h) {
-            i = (row0 + ly) * nx + col0 + lx;
-            const int t = p[c];
-            const int e = ext[t];
-            const int j = (e == -1) ? (row0 + t / TILE_W) * nx + col0 + (t % TILE_W) : e;
+        if (r[k] >= 0) {
+            const int j = rv[q[k]];
             J[i] = j;
-            if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || ext[c] == -1) R[i] = j;
-            if (ext[c] >= 0 && !is_tile_border_i(nx, ny, ext[c])) nonlocal = true;
-            pit = pits && ext[c] == -1 && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
+            if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || r[k] == i) R[i] = j;
+            if (q[k] == c && r[k] != i) {  // an exit
+                int rr, rc;
+                divmod_nx(r[k], nx, mnx, rr, rc);
+                if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
+            }
+            pit = pits && r[k] == i && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pit);
         if (m) {
@@ -419,6 +413,28 @@ __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, i
         }
     }
     if (nonlocal) info[2] = 1;
+}
+
+// Tile terminals of the tiles listed in tiles[0 .. *ntiles) (one block per tile,
+// the grid strides over the list; the count is read on the device), or of every
+// tile (tiles == NULL, a 2-D grid of tiles).
+template <int MODE>
+__global__ void __launch_bounds__(TILE_THREADS) k_tile_terminal(const int32_t *__restrict__ rec, int32_t *J, int32_t *R,
+                                                                int *pits, int *info, Grid g, const int *tiles,
+                                                                const int *ntiles, int32_t *rec_copy)
+{
+    __shared__ uint16_t p[TILE_CELLS];
+    __shared__ int rv[TILE_CELLS];
+    if (!tiles) {
+        tile_terminal_one<MODE>(rec, J, R, pits, info, g, blockIdx.x, blockIdx.y, p, rv, rec_copy);
+        return;
+    }
+    const int ntx = (g.nx + TILE_W - 1) / TILE_W, n = *ntiles;
+    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+        const int t = tiles[k];
+        tile_terminal_one<MODE>(rec, J, R, pits, info, g, t % ntx, t / ntx, p, rv, nullptr);
+        __syncthreads();  // p and rv are reused by the next tile
+    }
 }
 
 // Pointer jumping on R over all border cells, every round in one cooperative
@@ -455,18 +471,6 @@ __global__ void __launch_bounds__(256) k_labels_final(const int32_t *__restrict_
     bid[i] = can_leave_i<MODE>(g, root) ? 0 : root + 1;
 }
 
-// Exact quotient and remainder of n / d for 0 <= n < 2^31 and d >= 2 without the
-// integer divide sequence: with m = floor(2^32 / d) or m = floor((2^32 - 1) / d) (one
-// less only when d divides 2^32), q = umulhi(n, m) is floor(n / d) or one less
-// (n m / 2^32 > n / d - 2 n / 2^32 > n / d - 1), and one correction of the remainder
-// fixes it.
-__device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int &r)
-{
-    q = (int)__umulhi((unsigned)n, m);
-    r = n - q * d;
-    if (r >= d) { ++q; r -= d; }
-}
-
 // k_labels_final on 4 cells per thread (modes 0-2, nx % 4 == 0): 16-byte loads and
 // stores, the gathers of the 4 cells in flight together, and the roots' rows and
 // columns without integer division.
@@ -495,11 +499,11 @@ __global__ void __launch_bounds__(256) k_labels_final4(const int32_t *__restrict
 
 // k_basin_init on 4 cells of one row per thread (modes 0-2, nx % 4 == 0)
 template <int MODE>
-__global__ void k_basin_init4(int32_t *bid, Grid g, const int *guard, unsigned mnx)
+__global__ void k_basin_init4(int32_t *bid, Grid g, unsigned mnx)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int i0 = 4 * q;
-    if (i0 >= g.N() || (guard && *guard == 0)) return;
+    if (i0 >= g.N()) return;
     int row, col;
     divmod_nx(i0, g.nx, mnx, row, col);
     int lab[4];
@@ -554,13 +558,11 @@ __device__ __forceinline__ void saddle_min_warp(long long *saddle, int bi, long 
         atomicMin(saddle + bi, (long long)((((unsigned long long)mh << 32) | ml) ^ 0x8000000000000000ull));
 }
 
-// Passes 1-2 for one cell; the saddle candidate (if any) is returned in key/has.
-// Returns 0 for a cell off every border, 1 for a border cell of the outlet
-// basin 0, 2 for a border cell of a pit basin.
-template <int MODE>
-__device__ __forceinline__ int saddle_cell(int i, int row, int col, const Grid &g, int bi, float zi, const int (&jn)[4],
-                                           const int (&bn)[4], const float (&zn)[4], uint8_t *is_border, float *zp,
-                                           long long &key, bool &has)
+// Passes 1-2 for one cell; key: the lowest (z', neighbour basin) of a border cell (a
+// saddle candidate if below the invalid key).  Returns 0 for a cell off every
+// border, 1 for a border cell of the outlet basin 0, 2 for a border cell of a pit basin.
+__device__ __forceinline__ int saddle_cell(int i, int bi, float zi, const int (&jn)[4], const int (&bn)[4],
+                                           const float (&zn)[4], uint8_t *is_border, float *zp, long long &key)
 {
     bool border = false;
     float zmin = 1e9f;
@@ -571,8 +573,7 @@ __device__ __forceinline__ int saddle_cell(int i, int row, int col, const Grid &
     const float zpi = border ? fmaxf(zi, zmin) : 1e9f;
     zp[i] = zpi;
     if (!border) return 0;
-    const long long iv = invalid_key();
-    long long res = iv;
+    long long res = 0x7fffffffffffffffll;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (jn[k] == -1 || bn[k] == bi) continue;
@@ -580,15 +581,16 @@ __device__ __forceinline__ int saddle_cell(int i, int row, int col, const Grid &
         res = c < res ? c : res;
     }
     key = res;
-    has = res != iv;
     return bi != 0 ? 2 : 1;
 }
 
 template <int MODE>
 __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restrict__ bid, uint8_t *is_border,
                                                           float *zp, long long *saddle, const float *__restrict__ z,
-                                                          Grid g, int *blist, int *nblist, int *alist, int *nalist)
+                                                          Grid g, int *blist, int *nblist, int *alist, int *nalist,
+                                                          const int *info)
 {
+    if (info && (info[0] == 0 || info[2] || info[4])) return;  // nothing to do, or the host's steps
     __shared__ int buf[4][32 * SAD_ROWS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int warp = blockIdx.x * 4 + wib;
@@ -641,7 +643,6 @@ __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restr
             float zl = __shfl_up_sync(0xffffffffu, zc, 1), zr = __shfl_down_sync(0xffffffffu, zc, 1);
             int listed = 0;  // saddle_cell's code
             long long key = 0;
-            bool has = false;
             if (incol) {
                 const bool interior =
                     MODE != 3 && rw > 0 && rw < ny - 1 && (MODE == 1 || (col > 0 && col < nx - 1));
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restr
                                        i + nx};
                     const int bn[4] = {ba, bl, br, bb};
                     const float zn[4] = {za, zl, zr, zb};
-                    listed = saddle_cell<MODE>(i, rw, col, g, bc, zc, jn, bn, zn, is_border, zp, key, has);
+                    listed = saddle_cell(i, bc, zc, jn, bn, zn, is_border, zp, key);
                 } else if (can_leave<MODE>(g, i, rw, col)) {
                     zp[i] = zc;
                 } else {
@@ -665,10 +666,10 @@ __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restr
                         bn[k] = jn[k] != -1 ? bid[jn[k]] : 0;
                         zn[k] = jn[k] != -1 ? z[jn[k]] : 0.f;
                     }
-                    listed = saddle_cell<MODE>(i, rw, col, g, bc, zc, jn, bn, zn, is_border, zp, key, has);
+                    listed = saddle_cell(i, bc, zc, jn, bn, zn, is_border, zp, key);
                 }
             }
-            if (has) atomicMin(saddle + bc, key);
+            if (listed && key < invalid_key()) atomicMin(saddle + bc, key);
             // every border cell, the pit-basin ones marked by the sign bit
             const unsigned m = __ballot_sync(0xffffffffu, listed != 0);
             if (listed) buf[wib][nb + __popc(m & ((1u << lane) - 1u))] = listed == 2 ? (i | (int)0x80000000) : i;
@@ -678,6 +679,13 @@ __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restr
         }
     }
     __syncwarp();
+    if (!blist) {  // one list, pit-basin cells marked by the sign bit
+        int base = 0;
+        if (lane == 0 && nb) base = atomicAdd(nalist, nb);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int k = lane; k < nb; k += 32) alist[base + k] = buf[wib][k];
+        return;
+    }
     int npit = 0;
     for (int k = lane; k < nb; k += 32) npit += buf[wib][k] < 0;
     npit = __reduce_add_sync(0xffffffffu, npit);
@@ -711,9 +719,11 @@ constexpr int SAD4_ROWS = 8;
 template <int MODE>
 __global__ void __launch_bounds__(128, 4) k_saddle_p12_strip4(const int32_t *__restrict__ bid, uint8_t *is_border,
                                                               float *zp, long long *saddle, const float *__restrict__ z,
-                                                              Grid g, int *blist, int *nblist, int *alist, int *nalist)
+                                                              Grid g, int *blist, int *nblist, int *alist, int *nalist,
+                                                              const int *info)
 {
     static_assert(MODE >= 0 && MODE <= 2, "custom codes take k_saddle_p12_strip");
+    if (info && (info[0] == 0 || info[2] || info[4])) return;  // nothing to do, or the host's steps
     __shared__ int buf[4][128 * SAD4_ROWS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int warp = blockIdx.x * 4 + wib;
@@ -860,6 +870,13 @@ __global__ void __launch_bounds__(128, 4) k_saddle_p12_strip4(const int32_t *__r
         }
     }
     __syncwarp();
+    if (!blist) {  // one list, pit-basin cells marked by the sign bit
+        int base = 0;
+        if (lane == 0 && nb) base = atomicAdd(nalist, nb);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int k = lane; k < nb; k += 32) alist[base + k] = buf[wib][k];
+        return;
+    }
     int npit = 0;
     for (int k = lane; k < nb; k += 32) npit += buf[wib][k] < 0;
     npit = __reduce_add_sync(0xffffffffu, npit);
@@ -902,7 +919,6 @@ __global__ void __launch_bounds__(256) k_saddle_p12_border(const int32_t *__rest
         const int idx = k * stride + blockIdx.x * 256 + threadIdx.x;
         int code = 0, i = -1, bi = 0;
         long long key = 0;
-        bool has = false;
         if (idx < n) {
             i = aprev[idx];
             int row, col;
@@ -917,9 +933,9 @@ __global__ void __launch_bounds__(256) k_saddle_p12_border(const int32_t *__rest
             }
             // an outlet is never listed (its z' is z and it has no border status)
             bi = bid[i];
-            code = saddle_cell<MODE>(i, row, col, g, bi, z[i], jn, bn, zn, is_border, zp, key, has);
+            code = saddle_cell(i, bi, z[i], jn, bn, zn, is_border, zp, key);
         }
-        saddle_min_warp(saddle, bi, key, has);
+        saddle_min_warp(saddle, bi, key, code != 0 && key < invalid_key());
         block_append<256>(code != 0, i, anext, nanext);
         block_append<256>(code == 2, i, blist, nblist);
     }
@@ -1237,14 +1253,10 @@ __global__ void k_relabel_init(int32_t *fin, const int32_t *__restrict__ bid, co
 // round, with block barriers (its own global writes are visible to it after each);
 // longer lists take the cooperative launch with grid-wide barriers.  Each kernel
 // reads the count on the device and leaves the other's lists.
-// Inside the reroute graph the block kernel also sets a conditional handle, so the
-// cooperative launch (whose launch alone costs about 10 us) runs only for long lists.
 constexpr int RJ_BLOCK = 16384;
-__global__ void __launch_bounds__(1024) k_relabel_jump_block(int32_t *fin, const int *__restrict__ pits, const int *np,
-                                                            cudaGraphConditionalHandle hj, int set)
+__global__ void __launch_bounds__(1024) k_relabel_jump_block(int32_t *fin, const int *__restrict__ pits, const int *np)
 {
     const int n = *np;
-    if (set && threadIdx.x == 0) cudaGraphSetConditional(hj, n > RJ_BLOCK ? 1u : 0u);
     if (n > RJ_BLOCK) return;
     for (int r = 0; r < 32; ++r) {
         bool ch = false;
@@ -1257,10 +1269,9 @@ __global__ void __launch_bounds__(1024) k_relabel_jump_block(int32_t *fin, const
         if (!__syncthreads_or(ch)) break;
     }
 }
-static void launch_relabel_jump_block(int32_t *fin, const int *pits, const int *np, cudaGraphConditionalHandle hj,
-                                      int set, cudaStream_t st)
+static void launch_relabel_jump_block(int32_t *fin, const int *pits, const int *np, cudaStream_t st)
 {
-    PFF_PROBED("k_relabel_jump_block", st, k_relabel_jump_block<<<1, 1024, 0, st>>>(fin, pits, np, hj, set));
+    PFF_PROBED("k_relabel_jump_block", st, k_relabel_jump_block<<<1, 1024, 0, st>>>(fin, pits, np));
     count_launch();
 }
 
@@ -1341,10 +1352,8 @@ __global__ void k_dirty_list(uint8_t *dirty, int ntiles, int *list, int *count)
 // rec_ = rec on the carved cells: every write of the carve (reversed links and
 // saddle links) is at a tagged cell, and rec == rec_ everywhere else.
 __global__ void __launch_bounds__(256) k_sync_tagged(int32_t *rec_, const int32_t *__restrict__ rec,
-                                                     const uint8_t *__restrict__ tag, int N, int vec,
-                                                     const int *guard)
+                                                     const uint8_t *__restrict__ tag, int N, int vec)
 {
-    if (guard && *guard == 0) return;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = 4 * q;
     if (vec && i + 3 < N) {
@@ -1483,6 +1492,12 @@ __global__ void k_relabel_check(const int32_t *__restrict__ fin, const long long
     }
 }
 
+}  // namespace pff
+
+#include "pff_lake_loop.cuh"
+
+namespace pff {
+
 // ---- launchers ---------------------------------------------------------------
 
 template <int MODE>
@@ -1495,10 +1510,10 @@ static void l_basin_init(int32_t *bid, const Grid &g, cudaStream_t st)
 {
     if (MODE != 3 && g.nx % 4 == 0 && ((uintptr_t)bid % 16) == 0) {
         const unsigned m = (unsigned)(0x100000000ull / (unsigned long long)g.nx);
-        { k_basin_init4<MODE == 3 ? 0 : MODE><<<div_up(g.N() / 4, 256), 256, 0, st>>>(bid, g, nullptr, m); count_launch(); }
+        { k_basin_init4<MODE == 3 ? 0 : MODE><<<div_up(g.N() / 4, 256), 256, 0, st>>>(bid, g, m); count_launch(); }
         return;
     }
-    { k_basin_init<MODE><<<div_up(g.N(), 256), 256, 0, st>>>(bid, g, nullptr); count_launch(); }
+    { k_basin_init<MODE><<<div_up(g.N(), 256), 256, 0, st>>>(bid, g); count_launch(); }
 }
 template <int MODE>
 static void l_saddle(const int32_t *bid, uint8_t *isb, float *zp, long long *saddle, int32_t *snode,
@@ -1517,11 +1532,12 @@ static void l_saddle(const int32_t *bid, uint8_t *isb, float *zp, long long *sad
 
 template <int MODE>
 static void l_tile_terminal(const int32_t *rec, int32_t *J, int32_t *R, int *pits, int *info, const Grid &g,
-                            cudaStream_t st)
+                            int32_t *rec_copy, cudaStream_t st)
 {
     dim3 gr(div_up(g.nx, TILE_W), div_up(g.ny, TILE_H));
     PFF_PROBED("k_tile_terminal<grid>", st,
-               k_tile_terminal<MODE><<<gr, TILE_THREADS, 0, st>>>(rec, J, R, pits, info, g, nullptr, nullptr));
+               k_tile_terminal<MODE><<<gr, TILE_THREADS, 0, st>>>(rec, J, R, pits, info, g, nullptr, nullptr,
+                                                                  rec_copy));
     count_launch();
 }
 template <int MODE>
@@ -1542,7 +1558,8 @@ static void l_tile_terminal_list(const int32_t *rec, int32_t *J, int32_t *R, int
         if (resident[dev] > 0) grid = std::min(grid, resident[dev]);
     }
     PFF_PROBED("k_tile_terminal<list>", st,
-               k_tile_terminal<MODE><<<grid, TILE_THREADS, 0, st>>>(rec, J, R, nullptr, info, g, tiles, ntiles));
+               k_tile_terminal<MODE><<<grid, TILE_THREADS, 0, st>>>(rec, J, R, nullptr, info, g, tiles, ntiles,
+                                                                    nullptr));
     count_launch();
 }
 template <int MODE>
@@ -1577,14 +1594,14 @@ static void l_saddle_lists(const int32_t *bid, uint8_t *isb, float *zp, long lon
             const long long warps = (long long)((g.nx + 127) / 128) * ((g.ny + SAD4_ROWS - 1) / SAD4_ROWS);
             PFF_PROBED("k_saddle_p12_strip", st,
                        k_saddle_p12_strip4<MODE><<<div_up(warps, 4), 128, 0, st>>>(bid, isb, zp, saddle, z, g, blist,
-                                                                                   nblist, anext, nanext));
+                                                                                   nblist, anext, nanext, nullptr));
             count_launch();
         }
     } else if (!aprev) {
         const long long warps = (long long)((g.nx + 31) / 32) * ((g.ny + SAD_ROWS - 1) / SAD_ROWS);
         PFF_PROBED("k_saddle_p12_strip", st,
                    k_saddle_p12_strip<MODE><<<div_up(warps, 4), 128, 0, st>>>(bid, isb, zp, saddle, z, g, blist,
-                                                                              nblist, anext, nanext));
+                                                                              nblist, anext, nanext, nullptr));
         count_launch();
     } else {
         { k_saddle_p12_border<MODE><<<grid, 256, 0, st>>>(bid, isb, zp, saddle, z, g, aprev, naprev, anext, nanext,
@@ -1595,17 +1612,6 @@ static void l_saddle_lists(const int32_t *bid, uint8_t *isb, float *zp, long lon
     { k_saddle_p5_decide_list<<<grid, 256, 0, st>>>(bid, outlet, inv, N, pits, np); count_launch(); }
     { k_saddle_p5_serial_fix<<<1, 32, 0, st>>>(bid, outlet, inv, N); count_launch(); }
     { k_saddle_p5_apply_list<<<grid, 256, 0, st>>>(saddle, outlet, snode, inv, N, pits, np); count_launch(); }
-}
-
-template <int MODE>
-static void l_basin_init_if(int32_t *bid, const Grid &g, const int *guard, cudaStream_t st)
-{
-    if (MODE != 3 && g.nx % 4 == 0 && ((uintptr_t)bid % 16) == 0) {
-        const unsigned m = (unsigned)(0x100000000ull / (unsigned long long)g.nx);
-        { k_basin_init4<MODE == 3 ? 0 : MODE><<<div_up(g.N() / 4, 256), 256, 0, st>>>(bid, g, guard, m); count_launch(); }
-        return;
-    }
-    { k_basin_init<MODE><<<div_up(g.N(), 256), 256, 0, st>>>(bid, g, guard); count_launch(); }
 }
 
 int launch_basin_init(int32_t *bid, const Grid &g, cudaStream_t st)
@@ -1693,14 +1699,10 @@ extern "C" int pff_saddlesort(const int32_t *bid, uint8_t *is_border, float *z_p
     return check_cuda("pff_saddlesort");
 }
 
-extern "C" size_t pff_reroute_workspace_bytes(int N)
-{
-    const size_t n = (size_t)N;
-    return Carver::round(n + 1) * 2 + Carver::round(4 * (n + 1)) + Carver::round(4 * n) * 8 + Carver::round(8 * n) +
-           Carver::round(sizeof(int) * 512) + 8192;
-}
-
 namespace pff {
+
+constexpr int RR_CTR = 512;           // counters of the host-driven loop (see RerouteWs::ctr)
+constexpr int RR_SYNC = 64;           // the device loop's final state, barriers and prologue counters
 
 struct RerouteWs {
     uint8_t *inv;
@@ -1714,26 +1716,50 @@ struct RerouteWs {
                // [43] error; [44] dirty tiles; [45] odd carve; [50 + p] alist[p] count;
                // [64..127] border-jump round flags;
                // [128..191] label round flags; [192..255] carve round flags; [256..319] relabel flags
+    // the device-driven loop (pff_lake_loop.cuh); nf is blist's memory, abid that of tiles
+    int32_t *nf;
+    int *pit0, *abid, *dtiles;
+    long long *akey;
+    int *loop;  // RR_SYNC ints, LOOP_ITS x LOOP_CTR counters, then the dirty flags, contiguous
 };
 
-static RerouteWs carve_ws(void *workspace, size_t bytes, int N)
+static RerouteWs carve_ws(void *workspace, size_t bytes, int N, size_t *used = nullptr)
 {
     Carver cv(workspace, bytes);
     RerouteWs w;
-    w.inv = cv.take<uint8_t>((size_t)N + 1);
-    w.R = cv.take<int32_t>(N);
-    w.fin = cv.take<int32_t>((size_t)N + 1);
-    w.dirty = cv.take<uint8_t>((size_t)N);  // one byte per tile needed; N bytes bounds it
-    w.tiles = cv.take<int>(N);
-    w.pits[0] = cv.take<int>(N);
-    w.pits[1] = cv.take<int>(N);
-    w.blist = cv.take<int>(N);
-    w.segs = cv.take<int>(N);
-    w.alist[0] = cv.take<int>(N);
-    w.alist[1] = cv.take<int>(N);
-    w.ctr = cv.take<int>(512);
+    const size_t n = (size_t)N;
+    w.inv = cv.take<uint8_t>(n + 1);
+    w.R = cv.take<int32_t>(n);
+    w.fin = cv.take<int32_t>(n + 1);
+    w.dirty = cv.take<uint8_t>(n);  // one byte per tile needed; N bytes bounds it
+    w.tiles = cv.take<int>(n);
+    w.pits[0] = cv.take<int>(n);
+    w.pits[1] = cv.take<int>(n);
+    w.blist = cv.take<int>(n + 1);
+    w.segs = cv.take<int>(n);
+    w.alist[0] = cv.take<int>(n);
+    w.alist[1] = cv.take<int>(n);
+    w.ctr = cv.take<int>(RR_CTR);
+    w.nf = w.blist;
+    w.abid = w.tiles;
+    w.pit0 = cv.take<int>(n);
+    w.akey = cv.take<long long>(n);
+    w.dtiles = cv.take<int>(n / 4 + 1);  // a 64 x 32 tiling of a grid of 2 x 2 or more has at most N / 4 tiles
+    w.loop = cv.take<int>(RR_SYNC + LOOP_ITS * LOOP_CTR + n / 4 + 1);
+    if (used) *used = cv.off;
     return w;
 }
+
+}  // namespace pff
+
+extern "C" size_t pff_reroute_workspace_bytes(int N)
+{
+    size_t used = 0;
+    carve_ws(nullptr, 0, N, &used);
+    return used + 256;
+}
+
+namespace pff {
 
 // Tile pass over the receivers `rec`: tile terminals J into Jbuf, pit list and
 // count (read back), border list.  *nonlocal_host is set if some receiver is not
@@ -1743,7 +1769,7 @@ static int tile_pass(const int32_t *rec, int32_t *Jbuf, const Grid &g, RerouteWs
 {
     int *info = w.ctr + 16 * parity;
     PFF_CUDA(cudaMemsetAsync(info, 0, 4 * sizeof(int), st));
-    PFF_MODE_DISPATCH(g.mode, l_tile_terminal, rec, Jbuf, w.R, w.pits[parity], info, g, st);
+    PFF_MODE_DISPATCH(g.mode, l_tile_terminal, rec, Jbuf, w.R, w.pits[parity], info, g, nullptr, st);
     int h[4];
     PFF_TRY(read_ints(IntReads().add(info, 4), h, st));
     *npits_host = h[0];
@@ -1800,451 +1826,136 @@ static int general_labels(const int32_t *rec, int32_t *work, int32_t *bid, const
 }  // namespace pff
 
 namespace pff {
+
 // ---- the outer loop of reroute_flow driven on the device (carve rerouting) -------------
-// The host-driven loop reads pit counts and flags once per outer iteration to
-// decide whether to go on.  Here the decisions are made by one-thread kernels
-// that set CUDA-graph conditional handles, so a whole call is one graph launch:
-//
-//   prologue: rec_ = rec, counters zeroed, tile terminals + pit list
-//   plan0 (IF pits and D4 receivers):
-//     labels by border pointer jumping; plan1 (IF no receiver cycle):
-//       iteration 0 (strip saddle pass, carve, relabel preparation); decide
-//       WHILE (go on): iteration (parity 1); decide; IF (go on): iteration (parity 0); decide
-//   basin_id_init (:537) when the loop ended normally
-//
-// Two iterations per WHILE body keep every kernel argument fixed (the list
-// buffers alternate with the iteration's parity).  decide mirrors the host loop's
-// tests in its order (:500, :512-514 and the carve checks) and stops the loop
-// after at most outer <= 32 iterations.  The rare cases that need the
-// reference's N-wide steps (non-D4 receivers, receiver cycles) stop the graph in
-// a recorded state; the host then runs those steps from there.
-//
-// ctl = w.ctr + RR_CTL: [0] iteration, [1] outer, [2] n_outer, [3] state,
-// [4] sync_tagged needed, [5] basin_init needed, [6] plan0 passed, [7] plan1
-// passed, [8] iterations run.
-enum { RR_RUN = 0, RR_NOPITS = 1, RR_DONE = 2, RR_GENERAL = 3, RR_RESUME = 4, RR_WALKERR = 5, RR_BOUND = 6 };
-constexpr int RR_CTL = 400;
+// Four launches per call: the tile pass (with rec_ = rec and the pit list), the labels
+// and the strip saddle pass of iteration 0, then the loop kernel, which goes on to
+// the end (pff_lake_loop.cuh).  The rare cases that need the reference's N-wide steps
+// (non-D4 receivers, receiver cycles) stop it in a recorded state; the host then runs
+// those steps from there.
 
-__device__ __forceinline__ int d_ceil_log2(long long n)
+// Whether pff_reroute_flow runs its outer loop on the device (default) or from the host;
+// PFF_REROUTE_NO_GRAPH in the environment turns the default off,
+// pff_reroute_use_graphs changes it at run time.
+static std::atomic<int> g_rr_device{-1};
+static bool rr_device_on()
 {
-    int r = 0;
-    long long p = 1;
-    while (p < n) { p <<= 1; ++r; }
-    return r;
-}
-
-__global__ void k_rr_plan0(int *ctl, const int *info, cudaGraphConditionalHandle ha)
-{
-    if (threadIdx.x) return;
-    const int npits = info[0], nonlocal = info[2];
-    for (int k = 0; k < 9; ++k) ctl[k] = 0;
-    int go = 0;
-    if (npits == 0) ctl[3] = RR_NOPITS;                 // :496-497
-    else {
-        ctl[1] = d_ceil_log2(npits) + 1;                // :500
-        if (nonlocal) ctl[3] = RR_GENERAL;
-        else { ctl[3] = RR_RUN; go = 1; }
-    }
-    ctl[6] = go;
-    cudaGraphSetConditional(ha, go);
-}
-
-__global__ void k_rr_plan1(int *ctl, const int *unresolved, cudaGraphConditionalHandle hb)
-{
-    if (threadIdx.x) return;
-    const int go = *unresolved ? 0 : 1;
-    if (!go) ctl[3] = RR_GENERAL;  // the input receivers hold a cycle
-    ctl[7] = go;
-    cudaGraphSetConditional(hb, go);
-}
-
-__global__ void k_rr_decide(int *ctl, const int *ctr, const int *np_next, cudaGraphConditionalHandle hc,
-                            cudaGraphConditionalHandle hm, int set_hm)
-{
-    if (threadIdx.x) return;
-    const int it = ctl[0], outer = ctl[1];
-    int n_outer = ctl[2] + 1;
-    const int walk_err = ctr[43], odd = ctr[45], cycle = ctr[49], nd_next = *np_next;
-    int state = RR_RUN;
-    if (walk_err) state = RR_WALKERR;
-    else if (odd) state = RR_RESUME;              // a reversed path without an outlet link
-    else if (it + 1 >= outer) state = RR_DONE;    // :500
-    else if (cycle) state = RR_RESUME;            // the carve closed a receiver cycle
-    else if (nd_next == 0) { ++n_outer; state = RR_DONE; }  // the next count is 0 (:512-514)
-    else if (it + 1 >= 64) state = RR_BOUND;
-    ctl[2] = n_outer;
-    ctl[3] = state;
-    ctl[4] = state != RR_RUN;                     // rec_ = rec on the carved cells before stopping
-    ctl[5] = state == RR_DONE || state == RR_WALKERR;
-    ctl[8] += 1;
-    if (state == RR_RUN) ctl[0] = it + 1;
-    cudaGraphSetConditional(hc, state == RR_RUN);
-    if (set_hm) cudaGraphSetConditional(hm, state == RR_RUN);
-}
-
-struct RRBufs {
-    int32_t *bid, *rec, *rec_, *rec__;
-    const float *z;
-    float *zp;
-    uint8_t *isb;
-    long long *out, *sad;
-    int32_t *snode;
-    uint8_t *tag, *tag_;
-    Grid g;
-    RerouteWs w;
-};
-
-static int coop_blocks_for(const void *fn)
-{
-    int dev = 0, nsm = 148, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, 0);
-    return nsm * (per < 4 ? per : 4);
-}
-
-// One fast outer iteration with list parity par, enqueued on s (captured).  first:
-// iteration 0 (labels come from the prologue); otherwise it starts with the basin
-// relabelling and the dirty tiles' terminals that the previous iteration's
-// decision asked for.
-static int rr_cond(cudaStream_t s, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, cudaGraph_t *body);
-static int rr_handle(cudaStream_t s, cudaGraphConditionalHandle *h);
-
-// One outer iteration, captured on s (inside the reroute graph); aux captures the
-// body of the conditional cooperative relabel launch.
-static int rr_iteration(const RRBufs &A, int par, bool first, cudaStream_t s, cudaStream_t aux)
-{
-    const Grid &g = A.g;
-    const RerouteWs &w = A.w;
-    const int N = g.N(), nx = g.nx, B = 256;
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = nsm * 8;
-    const int ntx = div_up(nx, TILE_W), ntiles = ntx * div_up(g.ny, TILE_H);
-    int *np = w.ctr + 16 * par, *np_next = w.ctr + 16 * (par ^ 1);
-    if (!first) {
-        { k_relabel<<<div_up(div_up(N, 4), B), B, 0, s>>>(A.bid, w.fin, A.rec_, A.rec, A.tag, A.tag_, N,
-                                                         ((uintptr_t)A.bid & 15) == 0 && ((uintptr_t)A.tag & 3) == 0); count_launch(); }
-        PFF_MODE_DISPATCH(g.mode, l_tile_terminal_list, A.rec_, A.rec__, w.R, np_next, g, w.tiles, w.ctr + 44,
-                          std::min(ntiles, grid), s);
-        { k_basin_reset_list<<<grid, B, 0, s>>>(A.sad, A.out, A.snode, w.inv, w.pits[par ^ 1], np_next); count_launch(); }
-    } else {
-        { k_basin_arrays_init<<<div_up(N + 1, B), B, 0, s>>>(A.sad, A.out, A.snode, w.inv, N + 1); count_launch(); }
-    }
-    PFF_CUDA(cudaMemsetAsync(w.ctr + 40, 0, 6 * sizeof(int), s));
-    PFF_CUDA(cudaMemsetAsync(w.ctr + 50 + par, 0, sizeof(int), s));
-    PFF_MODE_DISPATCH(g.mode, l_saddle_lists, A.bid, A.isb, A.zp, A.sad, A.snode, A.out, w.inv, A.z, g, w.pits[par],
-                      np, w.blist, w.ctr + 40, first ? nullptr : w.alist[par ^ 1], w.ctr + 50 + (par ^ 1),
-                      w.alist[par], w.ctr + 50 + par, grid, s);
-    if (first) {  // later iterations: k_relabel cleared the previous carve's tags
-        PFF_CUDA(cudaMemsetAsync(A.tag, 0, (size_t)N, s));
-        PFF_CUDA(cudaMemsetAsync(A.tag_, 0, (size_t)N, s));
-    }
-    { k_carve_segments<<<nsm * 4, 32 * SEG_WARPS, 0, s>>>(A.snode, A.rec_, A.rec__, w.pits[par], np, N, w.segs,
-                                                           w.ctr + 41, N, w.ctr + 43); count_launch(); }
-    { k_carve_walk<<<nsm * 4, WALK_THREADS, 0, s>>>(A.rec_, A.rec, A.tag, A.tag_, w.segs, w.ctr + 41, N, nx, g.ny,
-                                                     w.dirty); count_launch(); }
-    { k_carve_link_list<<<grid, B, 0, s>>>(A.rec, A.snode, A.out, w.pits[par], np, N, w.dirty, nx); count_launch(); }
-    PFF_CUDA(cudaMemsetAsync(np_next, 0, 4 * sizeof(int), s));
-    { k_relabel_init<<<grid, B, 0, s>>>(w.fin, A.bid, A.snode, A.out, w.pits[par], np, N, w.pits[par ^ 1], np_next,
-                                        w.ctr + 45); count_launch(); }
-    { k_dirty_list<<<div_up(ntiles, B), B, 0, s>>>(w.dirty, ntiles, w.tiles, w.ctr + 44); count_launch(); }
-    int *flags = w.ctr + 256;
-    PFF_CUDA(cudaMemsetAsync(flags, 0, 64 * sizeof(int), s));
-    static int coop_relabel = 0;
-    if (!coop_relabel) coop_relabel = coop_blocks_for((const void *)k_relabel_jump_coop);
-    int *plist = w.pits[par];
-    int32_t *fin = w.fin;
-    cudaGraphConditionalHandle hj;
-    PFF_TRY(rr_handle(s, &hj));
-    launch_relabel_jump_block(fin, plist, np, hj, 1, s);
-    cudaGraph_t jbody = nullptr;
-    PFF_TRY(rr_cond(s, hj, cudaGraphCondTypeIf, &jbody));
-    PFF_CUDA(cudaStreamBeginCaptureToGraph(aux, jbody, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    void *args[] = {&fin, &plist, &np, &flags};
-    // not counted: the graph's launch tally counts it once per replay, and it runs
-    // only for pit lists longer than RJ_BLOCK
-    const cudaError_t le = cudaLaunchCooperativeKernel((void *)k_relabel_jump_coop, coop_relabel, 256, args, 0, aux);
-    cudaGraph_t captured = nullptr;
-    const cudaError_t ee = cudaStreamEndCapture(aux, &captured);
-    PFF_CUDA(le);
-    PFF_CUDA(ee);
-    PFF_CUDA(cudaMemsetAsync(w.ctr + 49, 0, sizeof(int), s));
-    { k_relabel_check<<<grid, B, 0, s>>>(w.fin, A.out, w.pits[par], np, N, w.ctr + 49); count_launch(); }
-    return check_cuda("reroute iteration");
-}
-
-// streams used to capture the graph's nested bodies (one per nesting depth)
-static cudaStream_t rr_capture_stream(int dev, int depth)
-{
-    static cudaStream_t streams[64][10];
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
-    if (!streams[dev][depth]) cudaStreamCreateWithFlags(&streams[dev][depth], cudaStreamNonBlocking);
-    return streams[dev][depth];
-}
-
-// a conditional node after the current capture frontier of s; its body graph is returned
-static int rr_cond(cudaStream_t s, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type, cudaGraph_t *body)
-{
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t gr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t nd = 0;
-    PFF_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &gr, &deps, &nd));
-    cudaGraphNodeParams p{};
-    p.type = cudaGraphNodeTypeConditional;
-    p.conditional.handle = h;
-    p.conditional.type = type;
-    p.conditional.size = 1;
-    cudaGraphNode_t node;
-    PFF_CUDA(cudaGraphAddNode(&node, gr, deps, nd, &p));
-    *body = p.conditional.phGraph_out[0];
-    PFF_CUDA(cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies));
-    return PFF_OK;
-}
-
-static int rr_handle(cudaStream_t s, cudaGraphConditionalHandle *h)
-{
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t gr;
-    PFF_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &gr, nullptr, nullptr));
-    PFF_CUDA(cudaGraphConditionalHandleCreate(h, gr, 0, cudaGraphCondAssignDefault));
-    return PFF_OK;
-}
-
-struct RRKernelCounts {
-    long long pro, a, b0, it2;  // kernels in the prologue, body A, iteration 0, a parity-1 iteration + decide
-    long long tail;             // the state copy at the end (graphs built for pff_reroute_flow_async)
-};
-
-// the final state words (RR_CTL .. +8) into the caller's device buffer
-// (out may be pinned host memory, written through its unified address)
-__global__ void k_rr_ctl_copy(const int *ctl, int *out)
-{
-    if (threadIdx.x < 9) ((volatile int *)out)[threadIdx.x] = ctl[threadIdx.x];
-}
-
-// Capture the whole graph.  Every capture begun here is ended on every path.
-static int rr_capture(const RRBufs &A, int dev, cudaGraph_t G, RRKernelCounts *kc, int *ctl_out)
-{
-    const Grid &g = A.g;
-    const RerouteWs &w = A.w;
-    const int N = g.N();
-    const size_t nb4 = sizeof(int32_t) * (size_t)N;
-    const int ntx = div_up(g.nx, TILE_W), ntiles = ntx * div_up(g.ny, TILE_H);
-    int *ctl = w.ctr + RR_CTL;
-    cudaStream_t s[5];
-    for (int d = 0; d < 5; ++d) {
-        s[d] = rr_capture_stream(dev, d);
-        if (!s[d]) { set_error("reroute graph: no capture stream"); return PFF_ERR_CUDA; }
-    }
-    int depth = 0, rc = PFF_OK;
-    cudaGraph_t body[5] = {G, nullptr, nullptr, nullptr, nullptr};
-    auto begin = [&](int d) -> int {
-        PFF_CUDA(cudaStreamBeginCaptureToGraph(s[d], body[d], nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-        depth = d + 1;
-        return PFF_OK;
-    };
-    long long l0 = g_launches.load();
-    do {
-        if ((rc = begin(0))) break;
-        // prologue (:491)
-        if (cudaMemcpyAsync(A.rec_, A.rec, nb4, cudaMemcpyDeviceToDevice, s[0]) != cudaSuccess ||
-            cudaMemsetAsync(w.ctr, 0, 512 * sizeof(int), s[0]) != cudaSuccess ||
-            cudaMemsetAsync(w.dirty, 0, (size_t)ntiles, s[0]) != cudaSuccess) { rc = check_cuda("reroute graph"); break; }
-        PFF_MODE_DISPATCH(g.mode, l_tile_terminal, A.rec_, A.rec__, w.R, w.pits[0], w.ctr, g, s[0]);
-        cudaGraphConditionalHandle ha, hb, hc, hm;
-        if ((rc = rr_handle(s[0], &ha))) break;
-        { k_rr_plan0<<<1, 32, 0, s[0]>>>(ctl, w.ctr, ha); count_launch(); }
-        kc->pro = g_launches.load() - l0;
-        l0 = g_launches.load();
-        if ((rc = rr_cond(s[0], ha, cudaGraphCondTypeIf, &body[1]))) break;
-        if ((rc = begin(1))) break;
-        // labels: pointer jumping over border cells, one gather per cell
-        if (cudaMemsetAsync(w.ctr + 64, 0, 64 * sizeof(int), s[1]) != cudaSuccess ||
-            cudaMemsetAsync(w.ctr + 48, 0, sizeof(int), s[1]) != cudaSuccess) { rc = check_cuda("reroute graph"); break; }
-        {
-            static int coop_border = 0;
-            if (!coop_border) coop_border = coop_blocks_for((const void *)k_border_jump_coop);
-            int nx = g.nx, ny = g.ny, tx = ntx;
-            long long nslots = (long long)ntx * div_up(g.ny, TILE_H) * BORDER_SLOTS;
-            int32_t *R = w.R;
-            int *flags = w.ctr + 64;
-            void *args[] = {&R, &nx, &ny, &tx, &nslots, &flags};
-            if (cudaLaunchCooperativeKernel((void *)k_border_jump_coop, coop_border, 256, args, 0, s[1]) != cudaSuccess) {
-                rc = check_cuda("reroute graph: cooperative launch");
-                break;
-            }
-            count_launch();
-        }
-        PFF_MODE_DISPATCH(g.mode, l_labels_final, A.rec__, w.R, A.bid, g, A.rec_, w.ctr + 48, s[1]);
-        if ((rc = rr_handle(s[1], &hb))) break;
-        { k_rr_plan1<<<1, 32, 0, s[1]>>>(ctl, w.ctr + 48, hb); count_launch(); }
-        kc->a = g_launches.load() - l0;
-        l0 = g_launches.load();
-        if ((rc = rr_cond(s[1], hb, cudaGraphCondTypeIf, &body[2]))) break;
-        if ((rc = begin(2))) break;
-        if ((rc = rr_iteration(A, 0, true, s[2], rr_capture_stream(dev, 7)))) break;
-        if ((rc = rr_handle(s[2], &hc))) break;
-        { k_rr_decide<<<1, 32, 0, s[2]>>>(ctl, w.ctr, w.ctr + 16, hc, hc, 0); count_launch(); }
-        { k_sync_tagged<<<div_up(div_up(N, 4), 256), 256, 0, s[2]>>>(A.rec_, A.rec, A.tag, N,
-                                                                   ((uintptr_t)A.tag & 3) == 0, ctl + 4); count_launch(); }
-        kc->b0 = g_launches.load() - l0;
-        l0 = g_launches.load();
-        if ((rc = rr_cond(s[2], hc, cudaGraphCondTypeWhile, &body[3]))) break;
-        if ((rc = begin(3))) break;
-        if ((rc = rr_iteration(A, 1, false, s[3], rr_capture_stream(dev, 8)))) break;
-        if ((rc = rr_handle(s[3], &hm))) break;
-        { k_rr_decide<<<1, 32, 0, s[3]>>>(ctl, w.ctr, w.ctr, hc, hm, 1); count_launch(); }
-        { k_sync_tagged<<<div_up(div_up(N, 4), 256), 256, 0, s[3]>>>(A.rec_, A.rec, A.tag, N,
-                                                                   ((uintptr_t)A.tag & 3) == 0, ctl + 4); count_launch(); }
-        kc->it2 = g_launches.load() - l0;
-        if ((rc = rr_cond(s[3], hm, cudaGraphCondTypeIf, &body[4]))) break;
-        if ((rc = begin(4))) break;
-        if ((rc = rr_iteration(A, 0, false, s[4], rr_capture_stream(dev, 9)))) break;
-        { k_rr_decide<<<1, 32, 0, s[4]>>>(ctl, w.ctr, w.ctr + 16, hc, hc, 0); count_launch(); }
-        { k_sync_tagged<<<div_up(div_up(N, 4), 256), 256, 0, s[4]>>>(A.rec_, A.rec, A.tag, N,
-                                                                   ((uintptr_t)A.tag & 3) == 0, ctl + 4); count_launch(); }
-        // close the bodies, innermost first; then basin_id_init on the top level
-        for (int d = 4; d >= 1; --d) {
-            cudaGraph_t out_g;
-            if (cudaStreamEndCapture(s[d], &out_g) != cudaSuccess) { rc = check_cuda("reroute graph: end capture"); break; }
-            depth = d;
-        }
-        if (rc) break;
-        PFF_MODE_DISPATCH(g.mode, l_basin_init_if, A.bid, g, ctl + 5, s[0]);
-        if (ctl_out) {
-            l0 = g_launches.load();
-            { k_rr_ctl_copy<<<1, 32, 0, s[0]>>>(ctl, ctl_out); count_launch(); }
-            kc->tail = g_launches.load() - l0;
-        }
-    } while (0);
-    // end every capture still open (innermost first)
-    for (int d = depth - 1; d >= 0; --d) {
-        cudaGraph_t out_g = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(s[d], &out_g);
-        if (e != cudaSuccess && rc == PFF_OK) {
-            set_error("reroute graph: end capture: %s", cudaGetErrorString(e));
-            rc = PFF_ERR_CUDA;
-        }
-    }
-    cudaGetLastError();
-    return rc;
-}
-
-// every pointer and size the graph bakes in, as plain 64-bit words (no padding)
-struct RRKey {
-    unsigned long long v[32];
-    int n = 0;
-    void add(unsigned long long x) { v[n++] = x; }
-    void add(const void *p) { v[n++] = (unsigned long long)(uintptr_t)p; }
-    bool operator==(const RRKey &o) const { return n == o.n && std::memcmp(v, o.v, sizeof(v[0]) * n) == 0; }
-};
-struct RREntry {
-    RRKey key;
-    cudaGraphExec_t exec = nullptr;
-    RRKernelCounts kc{};
-};
-
-// Whether pff_reroute_flow runs its outer loop from a device-driven graph (default)
-// or from the host loop; PFF_REROUTE_NO_GRAPH in the environment turns the default
-// off, pff_reroute_use_graphs changes it at run time.
-static std::atomic<int> g_rr_graphs{-1};
-static bool rr_graphs_on()
-{
-    int v = g_rr_graphs.load();
+    int v = g_rr_device.load();
     if (v < 0) {
         int fresh = getenv("PFF_REROUTE_NO_GRAPH") != nullptr ? 0 : 1;
-        if (!g_rr_graphs.compare_exchange_strong(v, fresh)) return g_rr_graphs.load() != 0;
+        if (!g_rr_device.compare_exchange_strong(v, fresh)) return g_rr_device.load() != 0;
         v = fresh;
     }
     return v != 0;
 }
 
-// Launch the device-driven loop for these buffers (a graph built and kept on the
-// first call with them), then read its final state (one synchronisation).
-// Returns PFF_ERR_UNSUPPORTED when graphs cannot be built here.
-// Kernels one launch of a graph ran, from its final state words c[0..8].
-static long long rr_tally(const RRKernelCounts &kc, const int *c)
+// Blocks of the cooperative kernels: one per LOOP_CELLS cells up to one per SM (the device's
+// occupancy for them, asked once), 0 where they cannot be launched.
+constexpr int LOOP_CELLS = 4096, LOOP_ONE = 8192;
+template <int MODE>
+static void l_loop_ready(int dev, int *ready)
 {
-    long long nk = kc.pro + kc.tail;  // prologue, body A, iteration 0, then the iterations of the WHILE
-    if (c[6]) nk += kc.a;
-    if (c[7] && c[8] > 0) nk += kc.b0 + (long long)(c[8] - 1) * kc.it2;
-    return nk + (c[5] ? 1 : 0);  // + basin_id_init
+    static std::atomic<int> known[64];
+    int v = known[dev].load();
+    if (!v) {
+        int per = 0, per2 = 0, coop = 0;
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        if (cudaFuncSetAttribute(k_reroute_loop<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) == cudaSuccess) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_reroute_loop<MODE>, LOOP_THREADS, LOOP_SMEM);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_reroute_labels<MODE>, LOOP_THREADS, 0);
+        }
+        cudaGetLastError();
+        v = coop && per > 0 && per2 > 0 ? 1 : -1;
+        known[dev].store(v);
+    }
+    *ready = v;
+}
+static int loop_blocks(const Grid &g)
+{
+    int dev = 0, nsm = 0, ready = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    PFF_MODE_DISPATCH(g.mode, l_loop_ready, dev, &ready);
+    if (ready < 0) return 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return g.N() <= LOOP_ONE ? 1 : std::min(nsm, div_up(g.N(), LOOP_CELLS));
 }
 
-// ctl_out: NULL, or a device buffer of 9 ints that the graph's last node fills with its
-// final state (a separate graph variant).  launch_only: return after the launch (the
-// caller reads the state later); kc_out receives the graph's kernel counts.
-static int reroute_graph(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *rec__, const float *z, float *z_prime,
-                         uint8_t *is_border, long long *out, long long *sad, int32_t *snode, uint8_t *tag,
-                         uint8_t *tag_, const Grid &g, RerouteWs &w, void *workspace, size_t workspace_bytes,
-                         int *state, int *it, int *outer, int *n_outer, cudaStream_t st, int *ctl_out = nullptr,
-                         bool launch_only = false, RRKernelCounts *kc_out = nullptr)
+template <int MODE>
+static void l_strip(const LoopArgs &A, cudaStream_t st)
 {
-    static std::mutex mu;
-    static RREntry cache[8];
-    static int next = 0;
-    if (!rr_graphs_on()) return PFF_ERR_UNSUPPORTED;
-    (void)workspace;
-    (void)workspace_bytes;
-    int dev = 0;
-    PFF_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return PFF_ERR_UNSUPPORTED;
-    const RRBufs bufs{bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, snode, tag, tag_, g, w};
-    RRKey key;
-    for (const void *p : {(const void *)bid, (const void *)rec, (const void *)rec_, (const void *)rec__,
-                          (const void *)z, (const void *)z_prime, (const void *)is_border, (const void *)out,
-                          (const void *)sad, (const void *)snode, (const void *)tag, (const void *)tag_,
-                          (const void *)g.codes, (const void *)w.inv, (const void *)w.ctr, (const void *)ctl_out})
-        key.add(p);
-    key.add((unsigned long long)g.nx);
-    key.add((unsigned long long)g.ny);
-    key.add((unsigned long long)g.mode);
-    key.add((unsigned long long)dev);
-    cudaGraphExec_t exec = nullptr;
-    RRKernelCounts kc{};
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        for (auto &e : cache)
-            if (e.exec && e.key == key) { exec = e.exec; kc = e.kc; }
-        if (!exec) {
-            cudaGraph_t G = nullptr;
-            PFF_CUDA(cudaGraphCreate(&G, 0));
-            const long long l0 = g_launches.load();
-            int rc = rr_capture(bufs, dev, G, &kc, ctl_out);
-            g_launches.store(l0);  // captured, not launched: replays are counted below
-            if (rc == PFF_OK && cudaGraphInstantiate(&exec, G, 0) != cudaSuccess) {
-                set_error("reroute graph: instantiate: %s", cudaGetErrorString(cudaGetLastError()));
-                exec = nullptr;
-                rc = PFF_ERR_UNSUPPORTED;
-            }
-            cudaGraphDestroy(G);
-            if (rc != PFF_OK) {
-                cudaGetLastError();
-                return PFF_ERR_UNSUPPORTED;
-            }
-            RREntry &e = cache[next];
-            next = (next + 1) % 8;
-            if (e.exec) cudaGraphExecDestroy(e.exec);
-            e.key = key;
-            e.exec = exec;
-            e.kc = kc;
-        }
+    const Grid &g = A.g;
+    const bool vec = g.nx % 4 == 0 && (((uintptr_t)A.bid | (uintptr_t)A.z | (uintptr_t)A.zp) & 15) == 0 &&
+                     ((uintptr_t)A.isb & 3) == 0;
+    int *na = A.it_ctr + LC_NA;
+    if (MODE != 3 && vec) {
+        const long long warps = (long long)((g.nx + 127) / 128) * ((g.ny + SAD4_ROWS - 1) / SAD4_ROWS);
+        k_saddle_p12_strip4<MODE == 3 ? 0 : MODE><<<div_up(warps, 4), 128, 0, st>>>(
+            A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr, A.alist[0], na, A.info);
+    } else {
+        const long long warps = (long long)((g.nx + 31) / 32) * ((g.ny + SAD_ROWS - 1) / SAD_ROWS);
+        k_saddle_p12_strip<MODE><<<div_up(warps, 4), 128, 0, st>>>(A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr,
+                                                                   A.alist[0], na, A.info);
     }
-    PFF_CUDA(cudaGraphLaunch(exec, st));
-    if (kc_out) *kc_out = kc;
-    if (launch_only) return check_cuda("reroute graph launch");
-    int c[9];
-    PFF_TRY(read_ints(IntReads().add(w.ctr + RR_CTL, 9), c, st));
-    *it = c[0];
-    *outer = c[1];
-    *n_outer = c[2];
-    *state = c[3];
-    g_launches.fetch_add(rr_tally(kc, c));
-    return check_cuda("reroute graph launch");
+    count_launch();
+}
+
+template <int MODE>
+static void l_loop(const LoopArgs &A, int32_t *R, int blocks, int *rc, cudaStream_t st)
+{
+    LoopArgs a = A;
+    const int ntx = div_up(a.g.nx, TILE_W);
+    long long nslots = (long long)ntx * div_up(a.g.ny, TILE_H) * BORDER_SLOTS;
+    int *flags = a.bar + 16;
+    void *largs[] = {&a, &R, &nslots, &flags};
+    cudaError_t e = cudaLaunchCooperativeKernel((void *)k_reroute_labels<MODE>, blocks, LOOP_THREADS, largs, 0, st);
+    if (e == cudaSuccess) {
+        count_launch();
+        l_strip<MODE>(a, st);
+        void *args[] = {&a};
+        e = cudaLaunchCooperativeKernel((void *)k_reroute_loop<MODE>, blocks, LOOP_THREADS, args, LOOP_SMEM, st);
+        count_launch();
+    }
+    if (e != cudaSuccess) {
+        set_error("pff_reroute_flow: cooperative launch: %s", cudaGetErrorString(e));
+        cudaGetLastError();
+        *rc = PFF_ERR_CUDA;
+    }
+}
+
+// Enqueue the whole reroute; its final state words (it, outer, n_outer, state, ...) land in
+// ctl_out, a buffer of 9 ints the device can write.  PFF_ERR_UNSUPPORTED where the
+// device loop is switched off or cannot be launched.
+static int reroute_device(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *rec__, const float *z, float *z_prime,
+                          uint8_t *is_border, long long *out, long long *sad, int32_t *snode, uint8_t *tag,
+                          uint8_t *tag_, const Grid &g, RerouteWs &w, int *ctl_out, cudaStream_t st)
+{
+    if (!rr_device_on()) return PFF_ERR_UNSUPPORTED;
+    const int blocks = loop_blocks(g);
+    if (blocks < 1) return PFF_ERR_UNSUPPORTED;
+    const int ntiles = div_up(g.nx, TILE_W) * div_up(g.ny, TILE_H);
+    LoopArgs A{};
+    A.bid = bid; A.rec = rec; A.rec_ = rec_; A.J = rec__;
+    A.z = z; A.zp = z_prime; A.isb = is_border;
+    A.sad = sad; A.out = out; A.snode = snode;
+    A.tag = tag; A.tag_ = tag_; A.inv = w.inv;
+    A.fin = w.fin; A.nf = w.nf;
+    A.pit0 = w.pit0; A.pits[0] = w.pits[0]; A.pits[1] = w.pits[1];
+    A.alist[0] = w.alist[0]; A.alist[1] = w.alist[1];
+    A.abid = w.abid; A.akey = w.akey;
+    A.segs = w.segs; A.dtiles = w.dtiles;
+    A.ctl = w.loop;
+    A.info = w.loop + 16;
+    A.bar = w.loop + 24;  // [0..1] the loop's, [8..9] the labels', [16..31] the labels' round flags
+    A.it_ctr = w.loop + RR_SYNC;
+    A.dirty = A.it_ctr + LOOP_ITS * LOOP_CTR;
+    A.ctl_out = ctl_out;
+    A.g = g;
+    PFF_CUDA(cudaMemsetAsync(w.loop, 0, sizeof(int) * ((size_t)RR_SYNC + LOOP_ITS * LOOP_CTR + ntiles), st));
+    PFF_MODE_DISPATCH(g.mode, l_tile_terminal, rec, rec__, w.R, w.pit0, A.info, g, rec_, st);  // :491, :493
+    int rc = PFF_OK;
+    PFF_MODE_DISPATCH(g.mode, l_loop, A, w.R, blocks, &rc, st);
+    PFF_TRY(rc);
+    return check_cuda("pff_reroute_flow");
 }
 
 // The outer loop of reroute_flow driven from the host, from iteration it_start
@@ -2383,7 +2094,7 @@ static int reroute_host_loop(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t 
             coop_relabel = nsm * (per < 4 ? per : 4);
         }
         int *plist = w.pits[par];
-        launch_relabel_jump_block(w.fin, plist, np, cudaGraphConditionalHandle{}, 0, st);
+        launch_relabel_jump_block(w.fin, plist, np, st);
         void *args[] = {&w.fin, &plist, &np, &flags};
         PFF_CUDA(cudaLaunchCooperativeKernel((void *)k_relabel_jump_coop, coop_relabel, 256, args, 0, st));
         count_launch();
@@ -2397,7 +2108,7 @@ static int reroute_host_loop(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t 
         // rec_ = rec on the carved cells (:526): inside the relabelling pass when
         // the loop goes on, else here
         if (h[0] || h[2] || it + 1 >= outer || hc || nd_next == 0) {
-            { k_sync_tagged<<<div_up(div_up(N, 4), B), B, 0, st>>>(rec_, rec, tag, N, ((uintptr_t)tag & 3) == 0, nullptr); count_launch(); }
+            { k_sync_tagged<<<div_up(div_up(N, 4), B), B, 0, st>>>(rec_, rec, tag, N, ((uintptr_t)tag & 3) == 0); count_launch(); }
         }
         if (h[0]) break;  // walk bounds exceeded: reported below
         const int ndirty = h[1];
@@ -2445,12 +2156,14 @@ static int reroute_host_loop(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t 
 // What the host does after the device-driven loop stopped in `state` (iteration it,
 // bound outer, n_outer iterations counted): nothing for a finished loop, the
 // reference's steps on the host for the general cases, an error otherwise.
-static int reroute_after_graph(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *rec__, const float *z,
+static int reroute_after_device(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *rec__, const float *z,
                                float *z_prime, uint8_t *is_border, long long *out, long long *sad,
                                int32_t *basin_saddlenode, uint8_t *tag, uint8_t *tag_, const Grid &g, RerouteWs &w,
                                int state, int it, int outer, int n_outer, int *n_outer_out, cudaStream_t st)
 {
     if (state == RR_NOPITS) return check_cuda("pff_reroute_flow");  // :496-497, bid untouched
+    if (state == RR_GENERAL || state == RR_RESUME)
+        PFF_CUDA(cudaMemsetAsync(w.ctr, 0, RR_CTR * sizeof(int), st));  // the host loop's counters
     if (state == RR_GENERAL)  // non-D4 receivers or a receiver cycle in the input: the reference's steps
         return reroute_host_loop(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag, tag_,
                                  1, g, w, 0, 0, true, 0, n_outer_out, st);
@@ -2495,16 +2208,26 @@ extern "C" int pff_reroute_flow(int32_t *bid, int32_t *rec, int32_t *rec_, int32
     if (n_outer_out) *n_outer_out = 0;
     if (carve) {
         int state = 0, it = 0, outer = 0, n_outer = 0;
-        const int rc = reroute_graph(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag,
-                                     tag_, g, w, workspace, workspace_bytes, &state, &it, &outer, &n_outer, st);
-        if (rc == PFF_OK)
-            return reroute_after_graph(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag,
+        int *host = nullptr, *dptr = nullptr;
+        PFF_TRY(pinned_ints(&host, &dptr));
+        host[3] = RR_BOUND;
+        const int rc = reroute_device(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag,
+                                      tag_, g, w, dptr, st);
+        if (rc == PFF_OK) {
+            PFF_CUDA(cudaStreamSynchronize(st));
+            const volatile int *c = host;
+            it = c[0];
+            outer = c[1];
+            n_outer = c[2];
+            state = c[3];
+            return reroute_after_device(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag,
                                        tag_, g, w, state, it, outer, n_outer, n_outer_out, st);
+        }
         if (rc != PFF_ERR_UNSUPPORTED) return rc;
-        clear_error();  // graphs unavailable: the host-driven loop below
+        clear_error();  // not available here: the host-driven loop below
     }
     PFF_CUDA(cudaMemcpyAsync(rec_, rec, nb4, cudaMemcpyDeviceToDevice, st));  // :491
-    PFF_CUDA(cudaMemsetAsync(w.ctr, 0, 512 * sizeof(int), st));
+    PFF_CUDA(cudaMemsetAsync(w.ctr, 0, RR_CTR * sizeof(int), st));
     const int ntx = div_up(nx, TILE_W), ntiles = ntx * div_up(ny, TILE_H);
     PFF_CUDA(cudaMemsetAsync(w.dirty, 0, (size_t)ntiles, st));
     return reroute_host_loop(bid, rec, rec_, rec__, z, z_prime, is_border, out, sad, basin_saddlenode, tag, tag_,
@@ -2514,14 +2237,14 @@ extern "C" int pff_reroute_flow(int32_t *bid, int32_t *rec, int32_t *rec_, int32
 extern "C" int pff_reroute_use_graphs(int on)
 {
     clear_error();
-    const int prev = rr_graphs_on() ? 1 : 0;
-    g_rr_graphs.store(on != 0 ? 1 : 0);
+    const int prev = rr_device_on() ? 1 : 0;
+    g_rr_device.store(on != 0 ? 1 : 0);
     return prev;
 }
 
 // ---- asynchronous reroute ----------------------------------------------------------
-// pff_reroute_flow split at its one synchronisation: the graph launch, whose last node
-// copies the final state words into ctl_out, and the host's continuation from a host
+// pff_reroute_flow split at its one synchronisation: the launches, the last of which
+// writes the final state words into ctl_out, and the host's continuation from a host
 // copy of those words.
 
 #define PFF_REROUTE_ARGS                                                                                        \
@@ -2544,9 +2267,6 @@ static int reroute_args_ok(const char *who, PFF_REROUTE_ARGS)
     return PFF_OK;
 }
 
-// kernel counts of the last asynchronous launch per device (for the launch tally)
-static RRKernelCounts g_async_kc[64];
-
 extern "C" int pff_reroute_flow_async(PFF_REROUTE_ARGS, int *ctl_out, void *stream)
 {
     clear_error();
@@ -2559,20 +2279,14 @@ extern "C" int pff_reroute_flow_async(PFF_REROUTE_ARGS, int *ctl_out, void *stre
     }
     Grid g{nx, ny, bound_mode, codes};
     RerouteWs w = carve_ws(workspace, workspace_bytes, nx * ny);
-    int dev = 0;
-    PFF_CUDA(cudaGetDevice(&dev));
-    int state = 0, it = 0, outer = 0, n_outer = 0;
-    RRKernelCounts kc{};
-    const int rc = reroute_graph(bid, rec, rec_, rec__, z, z_prime, is_border, (long long *)outlet,
-                                 (long long *)basin_saddle, basin_saddlenode, tag, tag_, g, w, workspace,
-                                 workspace_bytes, &state, &it, &outer, &n_outer, S(stream), ctl_out, true, &kc);
+    const int rc = reroute_device(bid, rec, rec_, rec__, z, z_prime, is_border, (long long *)outlet,
+                                  (long long *)basin_saddle, basin_saddlenode, tag, tag_, g, w, ctl_out, S(stream));
     if (rc == PFF_ERR_UNSUPPORTED) {
-        set_error("pff_reroute_flow_async: the device-driven loop is not available (graphs switched off or "
-                  "not supported here); use pff_reroute_flow");
+        set_error("pff_reroute_flow_async: the device-driven loop is not available (switched off or not supported "
+                  "here); use pff_reroute_flow");
         return PFF_ERR_UNAVAILABLE;
     }
     PFF_TRY(rc);
-    if (dev >= 0 && dev < 64) g_async_kc[dev] = kc;
     return PFF_OK;
 }
 
@@ -2587,12 +2301,9 @@ extern "C" int pff_reroute_flow_finish(PFF_REROUTE_ARGS, const int *ctl_host, in
         return PFF_ERR_ARG;
     }
     if (n_outer_out) *n_outer_out = 0;
-    int dev = 0;
-    PFF_CUDA(cudaGetDevice(&dev));
-    if (dev >= 0 && dev < 64) g_launches.fetch_add(rr_tally(g_async_kc[dev], ctl_host));
     Grid g{nx, ny, bound_mode, codes};
     RerouteWs w = carve_ws(workspace, workspace_bytes, nx * ny);
-    return reroute_after_graph(bid, rec, rec_, rec__, z, z_prime, is_border, (long long *)outlet,
+    return reroute_after_device(bid, rec, rec_, rec__, z, z_prime, is_border, (long long *)outlet,
                                (long long *)basin_saddle, basin_saddlenode, tag, tag_, g, w, ctl_host[3], ctl_host[0],
                                ctl_host[1], ctl_host[2], n_outer_out, S(stream));
 }

@@ -1,0 +1,693 @@
+// The carve reroute's outer loop (lakeflow.py:498-538) as one persistent cooperative
+// kernel.  Included by pff_lake.cu, whose helpers it uses.
+//
+// What bounds it: latency.  One outer iteration is about ten dependent steps over
+// lists (border cells, pits, path segments, touched tiles) that shrink by 2-3x per
+// iteration.  As separate kernels in a device-driven graph an iteration cost about 27
+// launches of 2 us and their gaps (135-140 us per iteration at 1001 x 777, of which
+// the work was a third).  Here a step ends with a grid barrier (about 1 us over 148
+// blocks; __syncthreads alone when one block is enough) and every block takes the loop's
+// decisions itself from counters it reads after the barrier.
+//
+// Nothing is N-wide after the first saddle pass:
+//   - labels are not rewritten between iterations: the current label of a cell is
+//     fin[bid[i]], with fin brought up to date once per iteration over the first pit list;
+//   - the receivers' second copy rec_, the carve tags and the tile terminals J are
+//     brought up to date over the tiles the carve touched.
+// One block of 1024 threads per SM: the barrier's cost grows with the number of
+// blocks, and 32 warps hide the gathers of the list steps.
+#pragma once
+
+namespace pff {
+
+// how the loop ended (final state words: [0] iteration, [1] outer, [2] n_outer, [3] state)
+enum { RR_RUN = 0, RR_NOPITS = 1, RR_DONE = 2, RR_GENERAL = 3, RR_RESUME = 4, RR_WALKERR = 5, RR_BOUND = 6 };
+
+__device__ __forceinline__ int d_ceil_log2(long long n)
+{
+    int r = 0;
+    long long p = 1;
+    while (p < n) { p <<= 1; ++r; }
+    return r;
+}
+
+constexpr int LOOP_THREADS = 1024, LOOP_GROUPS = LOOP_THREADS / TILE_THREADS;
+constexpr int LOOP_SEG_CAP = 128;               // segment starts buffered per warp
+constexpr int LOOP_ITS = 33, LOOP_CTR = 40;     // per-iteration counter slots (outer <= 32)
+constexpr int LOOP_JUMPS = 16;                  // label jump rounds (8 links each: chains up to 9^16)
+enum { LC_NP = 0, LC_NA = 1, LC_NSEG = 2, LC_NDIRTY = 3, LC_ODD = 4, LC_FLAG = 8 };  // in an iteration's slots
+constexpr int LOOP_GROUP_BYTES = TILE_CELLS * 6;  // per 256-thread group: 12 KB
+constexpr int LOOP_SMEM = LOOP_GROUPS * LOOP_GROUP_BYTES;
+static_assert(LOOP_SMEM >= LOOP_THREADS / 32 * LOOP_SEG_CAP * 4, "segment buffers share the group buffers");
+
+struct LoopArgs {
+    int32_t *bid, *rec, *rec_, *J;
+    const float *z;
+    float *zp;
+    uint8_t *isb;
+    long long *sad, *out;
+    int32_t *snode;
+    uint8_t *tag, *tag_;
+    uint8_t *inv;
+    int32_t *fin, *nf;
+    int *pit0, *pits[2];   // the first pit list; those of odd and even later iterations: [it & 1]
+    int *alist[2];         // border cells (the first list marks pit-basin cells by the sign bit)
+    int *abid;             // later lists: a border cell's label,
+    long long *akey;       // and its lowest (z', neighbour basin) key
+    int *segs, *dirty, *dtiles;
+    int *it_ctr;           // LOOP_ITS x LOOP_CTR counters, zeroed before the prologue
+    int *info;             // prologue: [0] pits, [2] non-D4 receivers, [4] unresolved labels
+    int *ctl, *ctl_out;    // final state words (RR_*), and the caller's copy
+    int *bar;              // [0] barrier arrivals, [1] error
+    Grid g;
+};
+
+// Barrier over the launch's blocks.  The launch is cooperative, so every block is
+// resident; a wait that has not ended after about two seconds gives up, records it
+// and makes the kernel return.
+struct LoopBar {
+    int *ctr;
+    int target;
+    __device__ __forceinline__ bool sync(int *dead)
+    {
+        __syncthreads();
+        if (gridDim.x > 1) {
+            target += gridDim.x;
+            if (threadIdx.x == 0) {
+                __threadfence();
+                atomicAdd(ctr, 1);
+                unsigned long long t0;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+                int spin = 0, seen;
+                for (;;) {
+                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
+                    if (seen >= target) break;
+                    if ((++spin & 1023) == 0) {
+                        unsigned long long t;
+                        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                        if (t - t0 > 2000000000ull) {
+                            *dead = 1;
+                            atomicExch(ctr + 1, 1);
+                            break;
+                        }
+                    }
+                }
+                __threadfence();
+            }
+            __syncthreads();
+        }
+        return *dead == 0;
+    }
+};
+
+__device__ __forceinline__ int vload(const int *p) { return *(const volatile int *)p; }
+
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(TILE_THREADS) : "memory"); }
+__device__ __forceinline__ bool group_or(int id, bool p)
+{
+    int r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, %2, %3, p;\n selp.s32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r)
+                 : "r"((int)p), "r"(id), "n"(TILE_THREADS)
+                 : "memory");
+    return r != 0;
+}
+
+__device__ __forceinline__ void loop_mark(const LoopArgs &A, int *nd, int tile)
+{
+    if (vload(A.dirty + tile) == 0 && atomicExch(A.dirty + tile, 1) == 0) A.dtiles[atomicAdd(nd, 1)] = tile;
+}
+
+struct TileXY {
+    int ntx;
+    unsigned mnx;
+    int nx;
+    __device__ __forceinline__ int of(int i) const
+    {
+        int row, col;
+        divmod_nx(i, nx, mnx, row, col);
+        return row / TILE_H * ntx + col / TILE_W;
+    }
+};
+
+// Bring a touched tile up to date: rec_ = rec (and, going on, the tags cleared: the
+// tagged cells are those whose receiver the carve changed), and its tile terminals.
+__device__ __forceinline__ void loop_tile(const LoopArgs &A, int tile, int ntx, unsigned mnx, int t, int bar_id,
+                                          unsigned char *smem, bool go_on)
+{
+    uint16_t *p = reinterpret_cast<uint16_t *>(smem);
+    int *rv = reinterpret_cast<int *>(smem + 2 * TILE_CELLS);
+    const int nx = A.g.nx, ny = A.g.ny;
+    const int ty = tile / ntx, tx = tile - ty * ntx;
+    const int row0 = ty * TILE_H, col0 = tx * TILE_W;
+    const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
+    const int lx = t & (TILE_W - 1), ly0 = t / TILE_W;
+    const int i0 = (row0 + ly0) * nx + col0 + lx;
+    int r[TILE_PER_THREAD], o[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const bool in = lx < w && ly0 + 4 * k < h;
+        r[k] = in ? A.rec[i0 + 4 * k * nx] : -1;
+        o[k] = in ? A.rec_[i0 + 4 * k * nx] : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k)
+        if (r[k] != o[k]) {
+            const int i = i0 + 4 * k * nx;
+            A.rec_[i] = r[k];
+            if (go_on) A.tag[i] = A.tag_[i] = 0;
+        }
+    if (!go_on) return;
+    int q[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k;
+        q[k] = r[k] < 0 ? c : tile_local(r[k], i0 + 4 * k * nx, c, lx, ly, row0, col0, w, h, nx, mnx);
+        p[c] = (uint16_t)q[k];
+        rv[c] = r[k];
+    }
+    group_sync(bar_id);
+    for (int round = 0; round < 12; ++round) {
+        bool ch = false;
+        int qq[TILE_PER_THREAD];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (qq[k] != q[k]) {
+                p[t + k * TILE_THREADS] = (uint16_t)qq[k];
+                q[k] = qq[k];
+                ch = true;
+            }
+        if (!group_or(bar_id, ch)) break;
+    }
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k)
+        if (r[k] >= 0) A.J[i0 + 4 * k * nx] = rv[q[k]];
+    group_sync(bar_id);  // the buffers are reused by the group's next tile
+}
+
+// One path segment: tag the cells of start's path inside its tile by pointer doubling
+// (after round r every cell within 2^(r+1) - 1 steps is on), until the start's own
+// doubled pointer has left the tile, then reverse the links (rec[receiver] = cell).
+__device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, unsigned mnx, int t, int bar_id,
+                                          unsigned char *smem, int *nd, const TileXY &txy)
+{
+    constexpr uint16_t NONE = 0xffff;
+    uint16_t *jmp = reinterpret_cast<uint16_t *>(smem);  // two buffers
+    uint8_t *on = smem + 4 * TILE_CELLS;
+    const int nx = A.g.nx, ny = A.g.ny;
+    int srow, scol;
+    divmod_nx(s0, nx, mnx, srow, scol);
+    const int ty = srow / TILE_H, tx = scol / TILE_W;
+    const int row0 = ty * TILE_H, col0 = tx * TILE_W;
+    const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
+    const int start = (srow - row0) * TILE_W + scol - col0;
+    const int lx = t & (TILE_W - 1), ly0 = t / TILE_W;
+    const int i0 = (row0 + ly0) * nx + col0 + lx;
+    int r[TILE_PER_THREAD], j[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k)
+        r[k] = (lx < w && ly0 + 4 * k < h) ? A.rec_[i0 + 4 * k * nx] : -1;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k;
+        const int v = r[k] < 0 ? c : tile_local(r[k], i0 + 4 * k * nx, c, lx, ly, row0, col0, w, h, nx, mnx);
+        j[k] = v == c ? NONE : v;
+        jmp[c] = (uint16_t)j[k];
+        on[c] = c == start;
+    }
+    group_sync(bar_id);
+    for (int rd = 0; rd < 11; ++rd) {  // 2^11 = TILE_CELLS
+        const uint16_t *jc = jmp + (rd & 1) * TILE_CELLS;
+        uint16_t *jn = jmp + ((rd & 1) ^ 1) * TILE_CELLS;
+        if (jc[start] == NONE) break;  // the same value for the whole group
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k) {
+            const int c = t + k * TILE_THREADS;
+            if (j[k] != NONE) {
+                if (on[c]) on[j[k]] = 1;
+                j[k] = jc[j[k]];
+            }
+            jn[c] = (uint16_t)j[k];
+        }
+        group_sync(bar_id);
+    }
+    bool local = false;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        if (!on[t + k * TILE_THREADS]) continue;
+        const int i = i0 + 4 * k * nx;
+        A.tag[i] = 1;
+        A.tag_[i] = 1;
+        if (r[k] == i) continue;  // the root
+        A.rec[r[k]] = i;
+        const int tl = txy.of(r[k]);
+        if (tl == ty * ntx + tx) local = true;
+        else loop_mark(A, nd, tl);
+    }
+    if (group_or(bar_id, local) && t == 0) loop_mark(A, nd, ty * ntx + tx);
+}
+
+// a barrier that gave up ends the kernel; the final state then says so
+#define LOOP_SYNC()                                                                  \
+    do {                                                                             \
+        if (!bar.sync(&dead)) {                                                      \
+            if (threadIdx.x == 0) A.ctl[3] = ((volatile int *)A.ctl_out)[3] = RR_BOUND; \
+            return;                                                                  \
+        }                                                                            \
+    } while (0)
+
+template <int MODE>
+__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
+{
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    __shared__ int wc[2][32];
+    __shared__ int dead;
+    const Grid &g = A.g;
+    const int nx = g.nx, N = g.N();
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const int nblk = gridDim.x, gtid = blockIdx.x * LOOP_THREADS + tid, gthreads = nblk * LOOP_THREADS;
+    const int grp = tid / TILE_THREADS, gt = tid & (TILE_THREADS - 1);
+    unsigned char *gsm = loop_smem + grp * LOOP_GROUP_BYTES;
+    const TileXY txy{(nx + TILE_W - 1) / TILE_W, mnx, nx};
+    const long long iv = invalid_key();
+    if (tid == 0) dead = 0;
+    LoopBar bar{A.bar, 0};
+    __syncthreads();
+
+    const int np0 = A.info[0];
+    int state = RR_RUN, it = 0, n_outer = 0;
+    const int outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;  // :500
+    if (np0 == 0) state = RR_NOPITS;                        // :496-497
+    else if (A.info[2] || A.info[4]) state = RR_GENERAL;    // not D4, or a receiver cycle in the input
+    if (state == RR_RUN) {
+        // clear the carve tags of an earlier call
+        if ((((uintptr_t)A.tag | (uintptr_t)A.tag_) & 15) == 0) {
+            const uint4 zero = make_uint4(0, 0, 0, 0);
+            for (int k = gtid; k < N / 16; k += gthreads) {
+                reinterpret_cast<uint4 *>(A.tag)[k] = zero;
+                reinterpret_cast<uint4 *>(A.tag_)[k] = zero;
+            }
+            for (int k = (N & ~15) + gtid; k < N; k += gthreads) A.tag[k] = A.tag_[k] = 0;
+        } else {
+            for (int k = gtid; k < N; k += gthreads) A.tag[k] = A.tag_[k] = 0;
+        }
+        if (gtid == 0) {
+            A.fin[0] = 0;
+            A.nf[0] = ~0;
+        }
+    }
+    while (state == RR_RUN) {
+        const bool first = it == 0;
+        int *C = A.it_ctr + it * LOOP_CTR, *Cn = C + LOOP_CTR;
+        const int np = first ? np0 : vload(C + LC_NP);
+        const int *pits = first ? A.pit0 : A.pits[it & 1];
+        int *pnext = A.pits[(it + 1) & 1];
+        const int *alist = A.alist[it & 1];
+        auto label = [&](int i) -> int {
+            const int b = A.bid[i];
+            return first ? b : A.fin[b];
+        };
+        // ---- passes 1-2 over the previous border cells (the first list comes from the strip pass)
+        if (!first) {
+            const int *aprev = A.alist[(it & 1) ^ 1];
+            int *anext = A.alist[it & 1];
+            const int n = vload(C - LOOP_CTR + LC_NA);
+            int trip = 0;
+            for (int k0 = blockIdx.x * LOOP_THREADS; k0 < n; k0 += gthreads, trip ^= 1) {
+                const int idx = k0 + tid;
+                int code = 0, i = -1, bi = 0;
+                long long key = 0;
+                if (idx < n) {
+                    i = aprev[idx] & 0x7FFFFFFF;
+                    int row, col;
+                    divmod_nx(i, nx, mnx, row, col);
+                    int jn[4], bn[4];
+                    float zn[4];
+                    neighbours4<MODE>(g, i, row, col, jn);
+                    bi = A.bid[i];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        bn[q] = jn[q] != -1 ? A.bid[jn[q]] : 0;
+                        zn[q] = jn[q] != -1 ? A.z[jn[q]] : 0.f;
+                    }
+                    const float zi = A.z[i];
+                    bi = A.fin[bi];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) bn[q] = A.fin[bn[q]];
+                    code = saddle_cell(i, bi, zi, jn, bn, zn, A.isb, A.zp, key);
+                }
+                saddle_min_warp(A.sad, bi, key, code != 0 && key < iv);
+                const unsigned m = __ballot_sync(0xffffffffu, code != 0);
+                if (lane == 0) wc[trip][wib] = __popc(m);
+                __syncthreads();
+                if (wib == 0) {
+                    const int c = wc[trip][lane];
+                    int s = c;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int y = __shfl_up_sync(0xffffffffu, s, o);
+                        if (lane >= o) s += y;
+                    }
+                    int base = 0;
+                    if (lane == 31 && s) base = atomicAdd(C + LC_NA, s);
+                    base = __shfl_sync(0xffffffffu, base, 31);
+                    wc[trip][lane] = base + s - c;
+                }
+                __syncthreads();
+                if (code != 0) {
+                    const int at = wc[trip][wib] + __popc(m & ((1u << lane) - 1u));
+                    anext[at] = i;
+                    A.abid[at] = bi;
+                    A.akey[at] = key;
+                }
+            }
+            LOOP_SYNC();
+        }
+        // ---- pass 3: the saddle node is the largest qualifying cell index
+        const int na = vload(C + LC_NA);
+        for (int k = gtid; k < na; k += gthreads) {
+            int i = alist[k], bi;
+            if (first) {
+                if (i >= 0) continue;  // a border cell of the outlet basin
+                i &= 0x7FFFFFFF;
+                bi = A.bid[i];
+            } else {
+                bi = A.abid[k];
+                if (bi == 0) continue;
+            }
+            const long long s = A.sad[bi];
+            const float tz = key_value(s);
+            if (!first) {
+                // the cell's lowest key is the basin's, or only the sign of a zero differs
+                const long long key = A.akey[k];
+                if (key != s && !(tz == 0.f && key_value(key) == 0.f)) continue;
+            }
+            const int tb = key_index(s);
+            bool here = A.zp[i] == tz;
+            if (here) {
+                int row, col, jn[4];
+                divmod_nx(i, nx, mnx, row, col);
+                neighbours4<MODE>(g, i, row, col, jn);
+                here = false;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (jn[q] != -1 && label(jn[q]) == tb) here = true;
+            }
+            if (here) atomicMax(A.snode + bi, i);
+        }
+        LOOP_SYNC();
+        // ---- pass 4: the outlet is the lowest foreign neighbour of the saddle node
+        for (int k = gtid; k < np; k += gthreads) {
+            const int b = pits[k] + 1;
+            if (b >= N || A.sad[b] == iv) continue;
+            const int node = A.snode[b];
+            if (node < 0) continue;
+            float tz = 1e9f;
+            int r = -1, row, col, jn[4];
+            divmod_nx(node, nx, mnx, row, col);
+            neighbours4<MODE>(g, node, row, col, jn);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (jn[q] == -1) continue;
+                const float zj = A.z[jn[q]];
+                if (label(jn[q]) != b && tz > zj) { tz = zj; r = jn[q]; }
+            }
+            if (r > -1) {
+                const long long c = pack_key(tz, r);
+                if (c < A.out[b]) A.out[b] = c;
+            }
+        }
+        LOOP_SYNC();
+        // ---- pass 5: the larger basin of each 2-cycle, decided on a snapshot
+        for (int k = gtid; k < np; k += gthreads) {
+            const int b = pits[k] + 1;
+            if (b >= N) continue;
+            const long long o = A.out[b];
+            if (o == iv) continue;
+            const int bd1 = label(key_index(o));
+            if (bd1 == 0) continue;
+            const int ro2 = key_index(A.out[bd1]);
+            const int bd2 = (ro2 >= 0 && ro2 < N) ? label(ro2) : -1;
+            if (bd2 == b && bd1 < b) A.inv[b] = 1;
+        }
+        LOOP_SYNC();
+        // ---- per basin: apply pass 5, link the saddle node, the label it merges into, the
+        //      pits left, and its path's segment starts, one tile at a time through J
+        {
+            const int D = N > 42 ? label(42) : 0;  // see k_saddle_p5_serial_fix
+            int *buf = reinterpret_cast<int *>(loop_smem) + wib * LOOP_SEG_CAP;
+            int nb = 0;  // warp-uniform
+            auto flush = [&]() {
+                __syncwarp();
+                int base = 0;
+                if (lane == 0 && nb) base = atomicAdd(C + LC_NSEG, nb);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                for (int q = lane; q < nb; q += 32)
+                    if (base + q < N) A.segs[base + q] = buf[q];
+                __syncwarp();
+                nb = 0;
+            };
+            for (int kb = (blockIdx.x * (LOOP_THREADS / 32) + wib) * 32; kb < np; kb += gthreads) {
+                const int k = kb + lane;
+                bool keep = false;
+                int x = -1, p = -1;
+                if (k < np) {
+                    p = pits[k];
+                    const int b = p + 1;
+                    if (b < N) {
+                        long long o = A.out[b];
+                        bool dead_b = A.inv[b] != 0;
+                        if (b == D && !dead_b && o != iv) {
+                            const int bd1 = label(key_index(o));
+                            dead_b = bd1 != 0 && bd1 < D && A.inv[bd1] != 0;
+                        }
+                        if (dead_b) {
+                            o = iv;
+                            A.out[b] = iv;
+                            A.sad[b] = iv;
+                            A.snode[b] = -1;
+                        }
+                        x = dead_b ? -1 : A.snode[b];
+                        if (o != iv) {
+                            const int node = key_index(o);
+                            A.rec[x] = node;
+                            loop_mark(A, C + LC_NDIRTY, txy.of(x));
+                            A.nf[b] = label(node);
+                        } else {
+                            keep = true;
+                            if (x != -1) C[LC_ODD] = 1;  // a path reversed without an outlet link
+                        }
+                    } else {
+                        keep = true;
+                    }
+                    if (keep) A.nf[b] = ~b;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (m) {
+                    int base = 0;
+                    if (lane == 0) base = atomicAdd(Cn + LC_NP, __popc(m));
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (keep) pnext[base + __popc(m & ((1u << lane) - 1u))] = p;
+                }
+                int tl = x >= 0 ? txy.of(x) : -1;
+                for (int step = 0; step <= N && __any_sync(0xffffffffu, x >= 0); ++step) {
+                    const unsigned e = __ballot_sync(0xffffffffu, x >= 0);
+                    if (x >= 0) buf[nb + __popc(e & ((1u << lane) - 1u))] = x;
+                    nb += __popc(e);
+                    if (nb > LOOP_SEG_CAP - 32) flush();
+                    if (x >= 0) {  // J[x] in x's own tile is the pit: the walk ends there
+                        x = A.J[x];
+                        const int t2 = txy.of(x);
+                        if (t2 == tl) x = -1;
+                        tl = t2;
+                    }
+                }
+            }
+            flush();
+        }
+        LOOP_SYNC();
+        // ---- walk the segments; the labels' first jump round shares the step
+        const int nseg_all = vload(C + LC_NSEG), nseg = min(nseg_all, N);
+        const bool last = it + 1 >= outer, odd = vload(C + LC_ODD) != 0, over = nseg_all > N;
+        if (nseg > WALK_BLOCK_MAX) {
+            for (int k = gtid; k < nseg; k += gthreads) {
+                const int start = A.segs[k], tl = txy.of(start);
+                int x = start;
+                bool local = false;
+                for (int step = 0; step < TILE_CELLS + 1; ++step) {
+                    A.tag[x] = 1;
+                    A.tag_[x] = 1;
+                    const int nxt = A.rec_[x];
+                    if (nxt == x) break;
+                    A.rec[nxt] = x;
+                    const int t2 = txy.of(nxt);
+                    if (t2 != tl) { loop_mark(A, C + LC_NDIRTY, t2); break; }
+                    local = true;
+                    x = nxt;
+                }
+                if (local) loop_mark(A, C + LC_NDIRTY, tl);
+            }
+        } else {
+            for (int k = grp * nblk + blockIdx.x; k < nseg; k += nblk * LOOP_GROUPS) {
+                loop_walk(A, A.segs[k], txy.ntx, mnx, gt, grp + 1, gsm, C + LC_NDIRTY, txy);
+            }
+        }
+        // nf[b]: the label basin b merges into, or ~label once known to be final.  A chain
+        // that never ends is a cycle of basins the carve closed.
+        bool settled = false;
+        for (int r = 0; r < LOOP_JUMPS; ++r) {
+            bool ch = false;
+            if (!last && !odd) {
+                for (int k = gtid; k < np; k += gthreads) {
+                    const int b = pits[k] + 1;
+                    int x = vload(A.nf + b);
+                    if (x < 0) continue;
+                    for (int s = 0; s < 8 && x >= 0; ++s) x = vload(A.nf + x);
+                    A.nf[b] = x;
+                    ch |= x >= 0;
+                }
+                if (__any_sync(0xffffffffu, ch) && lane == 0) C[LC_FLAG + r] = 1;
+            }
+            LOOP_SYNC();
+            if (last || odd || vload(C + LC_FLAG + r) == 0) { settled = true; break; }
+        }
+        // ---- the loop's decisions, in the reference's order (:500, :512-514)
+        ++n_outer;
+        if (over) state = RR_WALKERR;
+        else if (odd) state = RR_RESUME;            // the reference's N-wide steps from here on
+        else if (last) state = RR_DONE;
+        else if (!settled) state = RR_RESUME;       // the carve closed a receiver cycle
+        else if (vload(Cn + LC_NP) == 0) { ++n_outer; state = RR_DONE; }
+        else if (it + 2 >= LOOP_ITS) state = RR_BOUND;
+        const bool go_on = state == RR_RUN;
+        const int ndirty = vload(C + LC_NDIRTY);
+        for (int k = grp * nblk + blockIdx.x; k < ndirty; k += nblk * LOOP_GROUPS) {
+            const int tile = A.dtiles[k];
+            loop_tile(A, tile, txy.ntx, mnx, gt, grp + 1, gsm, go_on);
+            if (gt == 0) A.dirty[tile] = 0;
+        }
+        if (!go_on) break;
+        for (int k = gtid; k < np0; k += gthreads) {  // labels: fin[b] = final(fin[b])
+            const int b = A.pit0[k] + 1, x = first ? b : A.fin[b];
+            if (x) A.fin[b] = ~A.nf[x];
+        }
+        for (int k = gtid; k <= np; k += gthreads) {  // the basins' entries of this iteration
+            const int b = k < np ? pits[k] + 1 : 0;
+            A.sad[b] = iv;
+            A.out[b] = iv;
+            A.snode[b] = -1;
+            A.inv[b] = 0;
+        }
+        LOOP_SYNC();
+        ++it;
+    }
+    if (state == RR_DONE || state == RR_WALKERR) {  // basin_id_init (:537)
+        if (MODE != 3 && (nx & 3) == 0 && ((uintptr_t)A.bid & 15) == 0) {
+            for (int q = gtid; 4 * q < N; q += gthreads) {
+                int row, col, lab[4];
+                divmod_nx(4 * q, nx, mnx, row, col);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) lab[k] = can_leave<MODE>(g, 4 * q + k, row, col + k) ? 0 : 4 * q + k + 1;
+                reinterpret_cast<int4 *>(A.bid)[q] = make_int4(lab[0], lab[1], lab[2], lab[3]);
+            }
+        } else {
+            for (int i = gtid; i < N; i += gthreads) {
+                int row, col;
+                divmod_nx(i, nx, mnx, row, col);
+                A.bid[i] = can_leave<MODE>(g, i, row, col) ? 0 : i + 1;
+            }
+        }
+    }
+    if (gtid == 0) {
+        const int c[9] = {it, outer, n_outer, state, 0, 0, 0, 0, it + 1};
+        for (int k = 0; k < 9; ++k) {
+            A.ctl[k] = c[k];
+            ((volatile int *)A.ctl_out)[k] = c[k];
+        }
+        __threadfence_system();
+    }
+}
+
+// Labels of the first iteration: pointer jumping of R over the tile-border cells (8 links
+// per round and thread; chains of tiles up to 9^16 long), then one gather per cell and
+// the basins' initial entries (20 B per cell: the stores overlap the gathers).
+template <int MODE>
+__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, int32_t *R, long long nslots, int *flags)
+{
+    __shared__ int dead;
+    if (A.info[0] == 0 || A.info[2]) return;  // the same for every block
+    const Grid &g = A.g;
+    const int nx = g.nx, N = g.N();
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const int ntx = (nx + TILE_W - 1) / TILE_W;
+    const int gtid = blockIdx.x * LOOP_THREADS + threadIdx.x, gthreads = gridDim.x * LOOP_THREADS;
+    if (threadIdx.x == 0) dead = 0;
+    LoopBar bar{A.bar + 8, 0};
+    __syncthreads();
+    for (int r = 0; r < LOOP_JUMPS; ++r) {
+        bool ch = false;
+        for (long long k = gtid; k < nslots; k += gthreads) {
+            const int e = border_cell(nx, g.ny, ntx, k);
+            if (e < 0) continue;
+            int x = vload(R + e), y = vload(R + x);
+            if (y == x) continue;
+            for (int s = 0; s < 8 && y != x; ++s) {
+                x = y;
+                y = vload(R + x);
+            }
+            R[e] = x;
+            ch |= y != x;
+        }
+        if (__any_sync(0xffffffffu, ch) && (threadIdx.x & 31) == 0) flags[r] = 1;
+        LOOP_SYNC();
+        if (vload(flags + r) == 0) break;
+    }
+    const long long iv = invalid_key();
+    bool cyc = false;
+    if (MODE != 3 && (nx & 3) == 0 &&
+        (((uintptr_t)A.J | (uintptr_t)A.bid | (uintptr_t)A.sad | (uintptr_t)A.out | (uintptr_t)A.snode) & 15) == 0 &&
+        ((uintptr_t)A.inv & 3) == 0) {
+        for (int q = gtid; 4 * q < N; q += gthreads) {
+            const int4 j = reinterpret_cast<const int4 *>(A.J)[q];
+            const int rt[4] = {R[j.x], R[j.y], R[j.z], R[j.w]};
+            reinterpret_cast<longlong2 *>(A.sad)[2 * q] = reinterpret_cast<longlong2 *>(A.sad)[2 * q + 1] =
+                make_longlong2(iv, iv);
+            reinterpret_cast<longlong2 *>(A.out)[2 * q] = reinterpret_cast<longlong2 *>(A.out)[2 * q + 1] =
+                make_longlong2(iv, iv);
+            reinterpret_cast<int4 *>(A.snode)[q] = make_int4(-1, -1, -1, -1);
+            reinterpret_cast<uchar4 *>(A.inv)[q] = make_uchar4(0, 0, 0, 0);
+            int lab[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                cyc |= A.rec_[rt[k]] != rt[k];  // a receiver cycle: labels need the general path
+                int row, col;
+                divmod_nx(rt[k], nx, mnx, row, col);
+                lab[k] = can_leave<MODE>(g, rt[k], row, col) ? 0 : rt[k] + 1;
+            }
+            reinterpret_cast<int4 *>(A.bid)[q] = make_int4(lab[0], lab[1], lab[2], lab[3]);
+        }
+    } else {
+        for (int i = gtid; i < N; i += gthreads) {
+            const int rt = R[A.J[i]];
+            A.sad[i] = iv;
+            A.out[i] = iv;
+            A.snode[i] = -1;
+            A.inv[i] = 0;
+            cyc |= A.rec_[rt] != rt;
+            int row, col;
+            divmod_nx(rt, nx, mnx, row, col);
+            A.bid[i] = can_leave<MODE>(g, rt, row, col) ? 0 : rt + 1;
+        }
+    }
+    if (gtid == 0) {
+        A.sad[N] = iv;
+        A.out[N] = iv;
+        A.snode[N] = -1;
+        A.inv[N] = 0;
+    }
+    if (cyc) A.info[4] = 1;
+}
+
+}  // namespace pff
