@@ -324,21 +324,67 @@ __device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int 
     if (r >= d) { ++q; r -= d; }
 }
 
-// Tile-local index of the receiver r of cell i = (row0 + ly, col0 + lx) (local index c), or
-// c itself when the cell is a root or its receiver lies outside the w x h tile.
-__device__ __forceinline__ int tile_local(int r, int i, int c, int lx, int ly, int row0, int col0, int w, int h, int nx,
-                                          unsigned mnx)
+// Tile-local indices q of a thread's receivers r (its cells: rows ly0 + 4 k of column lx of
+// the w x h tile at (row0, col0), local index t + 256 k, grid index i0 + 4 k nx; r < 0: no
+// cell): the receiver's, or the cell's own where it is a root or its receiver lies outside.
+__device__ __forceinline__ void tile_locals(const int (&r)[TILE_PER_THREAD], int (&q)[TILE_PER_THREAD], int i0, int t,
+                                            int lx, int ly0, int row0, int col0, int w, int h, int nx, unsigned mnx)
 {
-    if (r == i) return c;
-    if (r == i - 1) return lx > 0 ? c - 1 : c;
-    if (r == i + 1) return lx < w - 1 ? c + 1 : c;
-    if (r == i - nx) return ly > 0 ? c - TILE_W : c;
-    if (r == i + nx) return ly < h - 1 ? c + TILE_W : c;
-    int rr, rc;
-    divmod_nx(r, nx, mnx, rr, rc);
-    rr -= row0;
-    rc -= col0;
-    return rr >= 0 && rr < h && rc >= 0 && rc < w ? rr * TILE_W + rc : c;
+    static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
+    int far = 0;  // receivers that are not the grid neighbour (wrapped edges, or no D4 link)
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS, d = r[k] - (i0 + 4 * k * nx);
+        const int sx = (d == 1) - (d == -1), sy = (d == nx) - (d == -nx);
+        const bool in = r[k] >= 0 && (unsigned)(lx + sx) < (unsigned)w && (unsigned)(ly0 + 4 * k + sy) < (unsigned)h;
+        q[k] = in ? c + sx + TILE_W * sy : c;
+        if (r[k] >= 0 && d != 0 && (sx | sy) == 0) far |= 1 << k;
+    }
+    if (!far) return;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        if (!(far >> k & 1)) continue;
+        int rr, rc;
+        divmod_nx(r[k], nx, mnx, rr, rc);
+        rr -= row0;
+        rc -= col0;
+        if (rr >= 0 && rr < h && rc >= 0 && rc < w) q[k] = rr * TILE_W + rc;
+    }
+}
+
+// A thread's 8 pointers q to their tile terminals.  Four rounds of pointer doubling in p
+// (16-bit local pointers; a pointer then spans 16 cells or ends), then every pointer is
+// followed on its own over the settled array, without barriers: most paths in a tile
+// are shorter than 64 cells.  At most 2048 / 16 steps (a cycle ends there too).
+// Bound by the shared-memory gathers' latency and bank conflicts.
+template <class Sync>
+__device__ __forceinline__ void tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD], int t, Sync sync)
+{
+    int qq[TILE_PER_THREAD];
+#pragma unroll 1
+    for (int round = 0; round < 4; ++round) {
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (qq[k] != q[k]) {
+                p[t + k * TILE_THREADS] = (uint16_t)qq[k];
+                q[k] = qq[k];
+            }
+        sync();
+    }
+#pragma unroll 1
+    for (int step = 0; step < TILE_CELLS / 16 + 1; ++step) {
+        bool ch = false;
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k) {
+            ch |= qq[k] != q[k];
+            q[k] = qq[k];
+        }
+        if (!ch) break;
+    }
 }
 
 // Tile terminals of one tile by one block: J[i] = the receiver of the last in-tile cell of
@@ -346,8 +392,6 @@ __device__ __forceinline__ int tile_local(int r, int i, int c, int lx, int ly, i
 // nullptr: no pit list), info[2] set if some exit target is not a tile-border cell
 // (receivers that are not D4 neighbours).  copy: also rec_copy = rec.
 //
-// Bound by the latency of the jump rounds' shared-memory chains.  Each thread keeps its 8
-// cells' pointers in registers and issues their 8 loads together; pointers are 16-bit.
 template <int MODE>
 __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, int32_t *R, int *pits, int *info,
                                   const Grid &g, int tx, int ty, uint16_t *p, int *rv, int32_t *rec_copy)
@@ -356,37 +400,23 @@ __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, i
     const unsigned mnx = 0xffffffffu / (unsigned)nx;
     const int col0 = tx * TILE_W, row0 = ty * TILE_H;
     const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
-    static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
     const int lx = threadIdx.x & (TILE_W - 1), ly0 = threadIdx.x / TILE_W;
     const int i0 = (row0 + ly0) * nx + col0 + lx;
     int r[TILE_PER_THREAD], q[TILE_PER_THREAD];
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) r[k] = (lx < w && ly0 + 4 * k < h) ? rec[i0 + 4 * k * nx] : -1;
+    tile_locals(r, q, i0, threadIdx.x, lx, ly0, row0, col0, w, h, nx, mnx);
+    int term = 0;  // cells that are terminals
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = threadIdx.x + k * TILE_THREADS, i = i0 + 4 * k * nx;
-        q[k] = r[k] < 0 ? c : tile_local(r[k], i, c, lx, ly0 + 4 * k, row0, col0, w, h, nx, mnx);
+        const int c = threadIdx.x + k * TILE_THREADS;
         p[c] = (uint16_t)q[k];
         rv[c] = r[k];
-        if (rec_copy && r[k] >= 0) rec_copy[i] = r[k];
+        if (q[k] == c) term |= 1 << k;
+        if (rec_copy && r[k] >= 0) rec_copy[i0 + 4 * k * nx] = r[k];
     }
     __syncthreads();
-    // at most ceil(log2 2048) = 11 rounds for any acyclic in-tile path (one interleaving
-    // of concurrent pointer jumps: a pointer always holds some later cell of the path)
-    for (int round = 0; round < 12; ++round) {
-        bool ch = false;
-        int qq[TILE_PER_THREAD];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k)
-            if (qq[k] != q[k]) {
-                p[threadIdx.x + k * TILE_THREADS] = (uint16_t)qq[k];
-                q[k] = qq[k];
-                ch = true;
-            }
-        if (!__syncthreads_or(ch)) break;
-    }
+    tile_jump(p, q, threadIdx.x, []() { __syncthreads(); });
     bool nonlocal = false;
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
@@ -396,11 +426,12 @@ __device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, i
             const int j = rv[q[k]];
             J[i] = j;
             if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || r[k] == i) R[i] = j;
-            if (q[k] == c && r[k] != i) {  // an exit
+            if ((term >> k & 1) && r[k] != i) {  // an exit
                 int rr, rc;
                 divmod_nx(r[k], nx, mnx, rr, rc);
                 if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
             }
+            if (p[q[k]] != q[k] || (q[k] == c && !(term >> k & 1))) nonlocal = true;  // a cycle in the tile
             pit = pits && r[k] == i && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pit);
@@ -1851,7 +1882,7 @@ static bool rr_device_on()
 
 // Blocks of the cooperative kernels: one per LOOP_CELLS cells up to one per SM (the device's
 // occupancy for them, asked once), 0 where they cannot be launched.
-constexpr int LOOP_CELLS = 4096, LOOP_ONE = 8192;
+constexpr int LOOP_CELLS = 2048, LOOP_ONE = 8192;
 template <int MODE>
 static void l_loop_ready(int dev, int *ready)
 {

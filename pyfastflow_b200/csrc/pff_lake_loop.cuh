@@ -32,13 +32,13 @@ __device__ __forceinline__ int d_ceil_log2(long long n)
 }
 
 constexpr int LOOP_THREADS = 1024, LOOP_GROUPS = LOOP_THREADS / TILE_THREADS;
-constexpr int LOOP_SEG_CAP = 128;               // segment starts buffered per warp
+constexpr int LOOP_CAP = 128;                   // list entries buffered per warp
 constexpr int LOOP_ITS = 33, LOOP_CTR = 40;     // per-iteration counter slots (outer <= 32)
 constexpr int LOOP_JUMPS = 16;                  // label jump rounds (8 links each: chains up to 9^16)
 enum { LC_NP = 0, LC_NA = 1, LC_NSEG = 2, LC_NDIRTY = 3, LC_ODD = 4, LC_FLAG = 8 };  // in an iteration's slots
 constexpr int LOOP_GROUP_BYTES = TILE_CELLS * 6;  // per 256-thread group: 12 KB
-constexpr int LOOP_SMEM = LOOP_GROUPS * LOOP_GROUP_BYTES;
-static_assert(LOOP_SMEM >= LOOP_THREADS / 32 * LOOP_SEG_CAP * 4, "segment buffers share the group buffers");
+constexpr int LOOP_SMEM = LOOP_THREADS / 32 * LOOP_CAP * 16;  // border-list entries of 16 B
+static_assert(LOOP_SMEM >= LOOP_GROUPS * LOOP_GROUP_BYTES, "the group buffers share that memory");
 
 struct LoopArgs {
     int32_t *bid, *rec, *rec_, *J;
@@ -159,28 +159,14 @@ __device__ __forceinline__ void loop_tile(const LoopArgs &A, int tile, int ntx, 
         }
     if (!go_on) return;
     int q[TILE_PER_THREAD];
+    tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k;
-        q[k] = r[k] < 0 ? c : tile_local(r[k], i0 + 4 * k * nx, c, lx, ly, row0, col0, w, h, nx, mnx);
-        p[c] = (uint16_t)q[k];
-        rv[c] = r[k];
+        p[t + k * TILE_THREADS] = (uint16_t)q[k];
+        rv[t + k * TILE_THREADS] = r[k];
     }
     group_sync(bar_id);
-    for (int round = 0; round < 12; ++round) {
-        bool ch = false;
-        int qq[TILE_PER_THREAD];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k)
-            if (qq[k] != q[k]) {
-                p[t + k * TILE_THREADS] = (uint16_t)qq[k];
-                q[k] = qq[k];
-                ch = true;
-            }
-        if (!group_or(bar_id, ch)) break;
-    }
+    tile_jump(p, q, t, [&]() { group_sync(bar_id); });
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k)
         if (r[k] >= 0) A.J[i0 + 4 * k * nx] = rv[q[k]];
@@ -209,11 +195,11 @@ __device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, un
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k)
         r[k] = (lx < w && ly0 + 4 * k < h) ? A.rec_[i0 + 4 * k * nx] : -1;
+    tile_locals(r, j, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k;
-        const int v = r[k] < 0 ? c : tile_local(r[k], i0 + 4 * k * nx, c, lx, ly, row0, col0, w, h, nx, mnx);
-        j[k] = v == c ? NONE : v;
+        const int c = t + k * TILE_THREADS;
+        if (j[k] == c) j[k] = NONE;
         jmp[c] = (uint16_t)j[k];
         on[c] = c == start;
     }
@@ -262,7 +248,6 @@ template <int MODE>
 __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
 {
     extern __shared__ __align__(16) unsigned char loop_smem[];
-    __shared__ int wc[2][32];
     __shared__ int dead;
     const Grid &g = A.g;
     const int nx = g.nx, N = g.N();
@@ -315,13 +300,34 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
             const int *aprev = A.alist[(it & 1) ^ 1];
             int *anext = A.alist[it & 1];
             const int n = vload(C - LOOP_CTR + LC_NA);
-            int trip = 0;
-            for (int k0 = blockIdx.x * LOOP_THREADS; k0 < n; k0 += gthreads, trip ^= 1) {
-                const int idx = k0 + tid;
-                int code = 0, i = -1, bi = 0;
+            // each warp on its own: the entries that stay on a border collect in its buffer,
+            // and the next trip's cells are loaded ahead
+            int *bufi = reinterpret_cast<int *>(loop_smem) + wib * LOOP_CAP * 4, *bufb = bufi + LOOP_CAP;
+            long long *bufk = reinterpret_cast<long long *>(bufb + LOOP_CAP);
+            int nb = 0;
+            auto flush = [&]() {
+                __syncwarp();
+                int base = 0;
+                if (lane == 0 && nb) base = atomicAdd(C + LC_NA, nb);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                for (int q = lane; q < nb; q += 32) {
+                    anext[base + q] = bufi[q];
+                    A.abid[base + q] = bufb[q];
+                    A.akey[base + q] = bufk[q];
+                }
+                __syncwarp();
+                nb = 0;
+            };
+            int k0 = (blockIdx.x * (LOOP_THREADS / 32) + wib) * 32;
+            int inext = k0 + lane < n ? aprev[k0 + lane] : -1;
+            for (; k0 < n; k0 += gthreads) {
+                const bool has = k0 + lane < n;
+                const int i = inext & 0x7FFFFFFF;
+                const int kn = k0 + gthreads + lane;
+                inext = kn < n ? aprev[kn] : -1;
+                int code = 0, bi = 0;
                 long long key = 0;
-                if (idx < n) {
-                    i = aprev[idx] & 0x7FFFFFFF;
+                if (has) {
                     int row, col;
                     divmod_nx(i, nx, mnx, row, col);
                     int jn[4], bn[4];
@@ -341,61 +347,60 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                 }
                 saddle_min_warp(A.sad, bi, key, code != 0 && key < iv);
                 const unsigned m = __ballot_sync(0xffffffffu, code != 0);
-                if (lane == 0) wc[trip][wib] = __popc(m);
-                __syncthreads();
-                if (wib == 0) {
-                    const int c = wc[trip][lane];
-                    int s = c;
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int y = __shfl_up_sync(0xffffffffu, s, o);
-                        if (lane >= o) s += y;
-                    }
-                    int base = 0;
-                    if (lane == 31 && s) base = atomicAdd(C + LC_NA, s);
-                    base = __shfl_sync(0xffffffffu, base, 31);
-                    wc[trip][lane] = base + s - c;
-                }
-                __syncthreads();
                 if (code != 0) {
-                    const int at = wc[trip][wib] + __popc(m & ((1u << lane) - 1u));
-                    anext[at] = i;
-                    A.abid[at] = bi;
-                    A.akey[at] = key;
+                    const int at = nb + __popc(m & ((1u << lane) - 1u));
+                    bufi[at] = i;
+                    bufb[at] = bi;
+                    bufk[at] = key;
                 }
+                nb += __popc(m);
+                if (nb > LOOP_CAP - 32) flush();
             }
+            flush();
             LOOP_SYNC();
         }
         // ---- pass 3: the saddle node is the largest qualifying cell index
         const int na = vload(C + LC_NA);
-        for (int k = gtid; k < na; k += gthreads) {
-            int i = alist[k], bi;
-            if (first) {
-                if (i >= 0) continue;  // a border cell of the outlet basin
-                i &= 0x7FFFFFFF;
-                bi = A.bid[i];
-            } else {
-                bi = A.abid[k];
-                if (bi == 0) continue;
-            }
-            const long long s = A.sad[bi];
-            const float tz = key_value(s);
-            if (!first) {
-                // the cell's lowest key is the basin's, or only the sign of a zero differs
-                const long long key = A.akey[k];
-                if (key != s && !(tz == 0.f && key_value(key) == 0.f)) continue;
-            }
-            const int tb = key_index(s);
-            bool here = A.zp[i] == tz;
-            if (here) {
-                int row, col, jn[4];
-                divmod_nx(i, nx, mnx, row, col);
-                neighbours4<MODE>(g, i, row, col, jn);
-                here = false;
+        // cell i of basin bi with z' equal to the saddle's: is a neighbour in its basin?
+        auto claim = [&](int i, int bi, int tb) {
+            int row, col, jn[4];
+            divmod_nx(i, nx, mnx, row, col);
+            neighbours4<MODE>(g, i, row, col, jn);
+            bool here = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (jn[q] != -1 && label(jn[q]) == tb) here = true;
+            if (here) atomicMax(A.snode + bi, i);
+        };
+        if (first) {
+            for (int k = gtid; 4 * k < na; k += gthreads) {  // the list's memory is padded to 16 bytes
+                const int4 v = reinterpret_cast<const int4 *>(alist)[k];
+                int i[4] = {v.x, v.y, v.z, v.w}, bi[4];
+                float zpi[4];
+                long long s[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const bool on = 4 * k + q < na && i[q] < 0;  // a border cell of a pit basin
+                    i[q] &= 0x7FFFFFFF;
+                    bi[q] = on ? A.bid[i[q]] : 0;
+                    zpi[q] = on ? A.zp[i[q]] : 0.f;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] = bi[q] ? A.sad[bi[q]] : iv;
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (jn[q] != -1 && label(jn[q]) == tb) here = true;
+                    if (bi[q] && zpi[q] == key_value(s[q])) claim(i[q], bi[q], key_index(s[q]));
             }
-            if (here) atomicMax(A.snode + bi, i);
+        } else {
+            for (int k = gtid; k < na; k += gthreads) {
+                const int bi = A.abid[k];
+                const long long key = A.akey[k];
+                if (bi == 0) continue;
+                const long long s = A.sad[bi];
+                // the cell's lowest key is the basin's, or only the sign of a zero differs
+                if (key == s) atomicMax(A.snode + bi, alist[k]);
+                else if (key_value(s) == 0.f && key_value(key) == 0.f) claim(alist[k], bi, key_index(s));
+            }
         }
         LOOP_SYNC();
         // ---- pass 4: the outlet is the lowest foreign neighbour of the saddle node
@@ -420,24 +425,19 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
             }
         }
         LOOP_SYNC();
-        // ---- pass 5: the larger basin of each 2-cycle, decided on a snapshot
-        for (int k = gtid; k < np; k += gthreads) {
-            const int b = pits[k] + 1;
-            if (b >= N) continue;
-            const long long o = A.out[b];
-            if (o == iv) continue;
-            const int bd1 = label(key_index(o));
-            if (bd1 == 0) continue;
-            const int ro2 = key_index(A.out[bd1]);
-            const int bd2 = (ro2 >= 0 && ro2 < N) ? label(ro2) : -1;
-            if (bd2 == b && bd1 < b) A.inv[b] = 1;
-        }
-        LOOP_SYNC();
-        // ---- per basin: apply pass 5, link the saddle node, the label it merges into, the
-        //      pits left, and its path's segment starts, one tile at a time through J
+        // ---- per basin: pass 5 (the larger basin of each 2-cycle, decided on this snapshot of
+        //      the outlets; the invalid entries are written in the next step), link the saddle
+        //      node, the label it merges into, the pits left, and its path's segment starts,
+        //      one tile at a time through J
         {
+            auto two_cycle = [&](int b, long long o) -> bool {
+                const int bd1 = label(key_index(o));
+                if (bd1 == 0 || bd1 >= b) return false;
+                const int ro2 = key_index(A.out[bd1]);
+                return ro2 >= 0 && ro2 < N && label(ro2) == b;
+            };
             const int D = N > 42 ? label(42) : 0;  // see k_saddle_p5_serial_fix
-            int *buf = reinterpret_cast<int *>(loop_smem) + wib * LOOP_SEG_CAP;
+            int *buf = reinterpret_cast<int *>(loop_smem) + wib * LOOP_CAP;
             int nb = 0;  // warp-uniform
             auto flush = [&]() {
                 __syncwarp();
@@ -458,16 +458,17 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                     const int b = p + 1;
                     if (b < N) {
                         long long o = A.out[b];
-                        bool dead_b = A.inv[b] != 0;
+                        bool dead_b = o != iv && two_cycle(b, o);
                         if (b == D && !dead_b && o != iv) {
                             const int bd1 = label(key_index(o));
-                            dead_b = bd1 != 0 && bd1 < D && A.inv[bd1] != 0;
+                            if (bd1 != 0 && bd1 < D) {
+                                const long long o1 = A.out[bd1];
+                                dead_b = o1 != iv && two_cycle(bd1, o1);
+                            }
                         }
                         if (dead_b) {
                             o = iv;
-                            A.out[b] = iv;
-                            A.sad[b] = iv;
-                            A.snode[b] = -1;
+                            A.inv[b] = 1;
                         }
                         x = dead_b ? -1 : A.snode[b];
                         if (o != iv) {
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                     const unsigned e = __ballot_sync(0xffffffffu, x >= 0);
                     if (x >= 0) buf[nb + __popc(e & ((1u << lane) - 1u))] = x;
                     nb += __popc(e);
-                    if (nb > LOOP_SEG_CAP - 32) flush();
+                    if (nb > LOOP_CAP - 32) flush();
                     if (x >= 0) {  // J[x] in x's own tile is the pit: the walk ends there
                         x = A.J[x];
                         const int t2 = txy.of(x);
@@ -511,7 +512,17 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
         // ---- walk the segments; the labels' first jump round shares the step
         const int nseg_all = vload(C + LC_NSEG), nseg = min(nseg_all, N);
         const bool last = it + 1 >= outer, odd = vload(C + LC_ODD) != 0, over = nseg_all > N;
-        if (nseg > WALK_BLOCK_MAX) {
+        for (int k = gtid; k < np; k += gthreads) {
+            const int b = pits[k] + 1;
+            if (b < N && A.inv[b]) {
+                A.out[b] = iv;
+                A.sad[b] = iv;
+                A.snode[b] = -1;
+            }
+        }
+        // a group of 256 threads takes about 5 us per segment whatever its length, a thread
+        // about 0.6 us per cell; segments are many while the paths are short
+        if (nseg > 2 * LOOP_GROUPS * nblk) {
             for (int k = gtid; k < nseg; k += gthreads) {
                 const int start = A.segs[k], tl = txy.of(start);
                 int x = start;
