@@ -11,7 +11,9 @@
 // round) does not depend on the payload, so one pass carries both the f32
 // payload p and an exact uint32 count payload c.
 #include <cub/block/block_scan.cuh>
+#include <algorithm>
 #include <type_traits>
+#include "pff_coop.cuh"
 #include "pff_internal.h"
 
 namespace pff {
@@ -154,12 +156,9 @@ struct __align__(16) Pub {
     int d0;
 };
 
-// Fallback path (receivers that are not D4 neighbours): scatter + sort.  Each
-// kernel runs only if *need is set (need == nullptr: always).
-__global__ void k_acc_init(Pub *A, Pub *B, int4 *priv, const float *__restrict__ Q, uint32_t *counts, int N,
-                           const int *need)
+// Fallback path (receivers that are not D4 neighbours, or no grid given): scatter + sort.
+__device__ __forceinline__ void acc_init(Pub *A, Pub *B, int4 *priv, const float *Q, uint32_t *counts, int N)
 {
-    if (need && !*need) return;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N; t += gridDim.x * blockDim.x) {
         const Pub s{0, Q[t], 1u, -1};
         A[t] = s;
@@ -169,10 +168,8 @@ __global__ void k_acc_init(Pub *A, Pub *B, int4 *priv, const float *__restrict__
     }
 }
 
-__global__ void k_acc_scatter(const int32_t *__restrict__ rcv, Pub *A, int4 *priv, int N, const int *need,
-                              int *overflow)
+__device__ __forceinline__ void acc_scatter(const int32_t *rcv, Pub *A, int4 *priv, int N, int *overflow)
 {
-    if (need && !*need) return;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < N; t += gridDim.x * blockDim.x) {
         const int r = rcv[t];
         if (r == t) continue;
@@ -206,33 +203,31 @@ __device__ __forceinline__ void block_append2(bool pa, bool pf, int t, int *la, 
 // Sort each node's donor slots ascending, copy its public record to the second
 // buffer, and list the nodes that have donors (round-0 active list).
 template <int BS>
-__global__ void __launch_bounds__(BS) k_acc_list0(Pub *A, Pub *B, int4 *priv, int *list, int *nlist, int N,
-                                                  const int *need)
+__device__ __forceinline__ void acc_list0(Pub *A, Pub *B, int4 *priv, int *list, int *nlist, int N)
 {
-    if (need && !*need) return;
     const int stride = gridDim.x * BS, trips = (N + stride - 1) / stride;
     for (int k = 0; k < trips; ++k) {
-    const int t = k * stride + blockIdx.x * BS + threadIdx.x;
-    int n = 0;
-    if (t < N) {
-        Pub s = A[t];
-        n = s.ndnr;
-        if (n >= 2) {
-            int4 q = priv[t];
-            int d[4] = {s.d0, q.x, q.y, q.z};
-            const int m = n < 4 ? n : 4;
-            for (int a = 1; a < m; ++a) {
-                int x = d[a], b = a - 1;
-                while (b >= 0 && d[b] > x) { d[b + 1] = d[b]; --b; }
-                d[b + 1] = x;
+        const int t = k * stride + blockIdx.x * BS + threadIdx.x;
+        int n = 0;
+        if (t < N) {
+            Pub s = A[t];
+            n = s.ndnr;
+            if (n >= 2) {
+                int4 q = priv[t];
+                int d[4] = {s.d0, q.x, q.y, q.z};
+                const int m = n < 4 ? n : 4;
+                for (int a = 1; a < m; ++a) {
+                    int x = d[a], b = a - 1;
+                    while (b >= 0 && d[b] > x) { d[b + 1] = d[b]; --b; }
+                    d[b + 1] = x;
+                }
+                s.d0 = d[0];
+                A[t].d0 = d[0];
+                priv[t] = make_int4(d[1], d[2], d[3], -1);
             }
-            s.d0 = d[0];
-            A[t].d0 = d[0];
-            priv[t] = make_int4(d[1], d[2], d[3], -1);
+            if (n > 0) B[t] = s;
         }
-        if (n > 0) B[t] = s;
-    }
-    block_append2<BS>(n > 0, false, t, list, nlist, nullptr, nullptr);
+        block_append2<BS>(n > 0, false, t, list, nlist, nullptr, nullptr);
     }
 }
 
@@ -304,14 +299,6 @@ __global__ void __launch_bounds__(BS) k_acc_gather(const int32_t *__restrict__ r
     block_append2<BS>(nd > 0, false, t, list, nlist, nullptr, nullptr);
 }
 
-__global__ void k_acc_fallback_reset(int *nlist, const int *need)
-{
-    if (*need) {
-        nlist[0] = 0;  // active and finished counts of round 0
-        nlist[1] = 0;
-    }
-}
-
 __device__ __forceinline__ int sel4(int k, int a, int b, int c, int d)
 {
     return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
@@ -328,108 +315,186 @@ __device__ __forceinline__ Pub pick4(int q, const Pub &a, const Pub &b, const Pu
     return q == 0 ? a : (q == 1 ? b : (q == 2 ? c : d));
 }
 
-// One round.  Items [0, nA) are active nodes, [nA, nA+nF) nodes that finished in
-// the previous round (copied into the buffer written this round).  In the last
-// round (it == logn) every active node reports its start-of-round value, which
-// is what the reference's fuse(.., logn) selects (downstream_propag.py:59-74).
-// With need != nullptr the round runs only if *need is set (the scatter path's
-// rounds before the tile front's first round).  With fin_q, the finished items
-// also write their Q and count (the nodes that finished inside the tile front).
-template <int BS>
-__global__ void __launch_bounds__(BS, 5) k_acc_round(const Pub *__restrict__ cur, Pub *nxt, int4 *priv,
-                                                  const int *__restrict__ la, const int *nla,
-                                                  const int *__restrict__ lf, const int *nlf, int *la2, int *nla2,
-                                                  int *lf2, int *nlf2, float *Q, uint32_t *counts, int it, int last,
-                                                  const int *need, int fin_q)
+// One active node's round: the reference's swap-remove scan (downstream_propag.py:131-162)
+// on start-of-round donor states.  Returns 0: keeps donors, 1: finished (Q and count
+// written).  last: the start-of-round value is the result (fuse(.., logn), :59-74).
+__device__ __forceinline__ int acc_node(int t, const Pub *cur, Pub *nxt, int4 *priv, float *Q, uint32_t *counts,
+                                        bool last)
 {
-    if (need && !*need) return;
-    const int nA = *nla, nF = *nlf;
-    const int total = nA + nF;
-    const int stride = gridDim.x * BS;
-    // Uniform trip count so every thread reaches the block-wide appends together.
-    // The appends keep each round's list close to ascending order, so the whole
-    // GPU works on a narrow window of cells whose donors stay in L2.
-    const int trips = (total + stride - 1) / stride;
-    for (int k = 0; k < trips; ++k) {
-        const int idx = k * stride + blockIdx.x * BS + threadIdx.x;
-        bool keep = false, fin = false;
-        int t = -1;
-        if (idx < nA) {
-            t = la[idx];
-            const Pub s = cur[t];
-            int todo = s.ndnr;
-            int own[4] = {s.d0, -1, -1, -1};
-            if (todo > 1) {
-                const int4 pq = priv[t];
-                own[1] = pq.x; own[2] = pq.y; own[3] = pq.z;
-            }
-            // Every donor state this round can need is one of the start-of-round
-            // slots: load them all up front (independent loads).  The reference's
-            // swap-remove scan (downstream_propag.py:131-162) then runs on
-            // registers: slot k holds donor w_k whose preloaded state is q_k.
-            Pub P0 = s, P1 = s, P2 = s, P3 = s;
-            if (todo > 0) P0 = cur[own[0]];
-            if (todo > 1) P1 = cur[own[1]];
-            if (todo > 2) P2 = cur[own[2]];
-            if (todo > 3) P3 = cur[own[3]];
-            int w0 = own[0], w1 = own[1], w2 = own[2], w3 = own[3];
-            int q0 = 0, q1 = 1, q2 = 2, q3 = 3;
-            bool worked = false;
-            float padd = 0.f;
-            uint32_t cadd = 0;
-            int i = 0;
+    const Pub s = cur[t];
+    if (last) {
+        Q[t] = s.p;
+        if (counts) counts[t] = s.c;
+        return 2;
+    }
+    int todo = s.ndnr;
+    int own[4] = {s.d0, -1, -1, -1};
+    if (todo > 1) {
+        const int4 pq = priv[t];
+        own[1] = pq.x; own[2] = pq.y; own[3] = pq.z;
+    }
+    // Every donor state this round can need is one of the start-of-round slots: load
+    // them all up front (independent loads).  The scan then runs on registers: slot k
+    // holds donor w_k whose preloaded state is q_k.
+    Pub P0 = s, P1 = s, P2 = s, P3 = s;
+    if (todo > 0) P0 = cur[own[0]];
+    if (todo > 1) P1 = cur[own[1]];
+    if (todo > 2) P2 = cur[own[2]];
+    if (todo > 3) P3 = cur[own[3]];
+    int w0 = own[0], w1 = own[1], w2 = own[2], w3 = own[3];
+    int q0 = 0, q1 = 1, q2 = 2, q3 = 3;
+    bool worked = false;
+    float padd = 0.f;
+    uint32_t cadd = 0;
+    int i = 0;
 #pragma unroll
-            for (int step = 0; step < 8; ++step) {  // each step advances i or removes a donor
-                if (i >= todo || i >= 4) break;
-                const int q = sel4(i, q0, q1, q2, q3);
-                const Pub ds = pick4(q, P0, P1, P2, P3);
-                if (ds.ndnr <= 1) {
-                    if (!worked) { padd = s.p; cadd = s.c; }
-                    worked = true;
-                    padd = __fadd_rn(padd, ds.p);
-                    cadd += ds.c;
-                    if (ds.ndnr == 0) {
-                        --todo;
-                        if (todo > i && todo < 4) {
-                            set4(i, sel4(todo, own[0], own[1], own[2], own[3]), w0, w1, w2, w3);
-                            set4(i, todo, q0, q1, q2, q3);
-                        }
-                    } else {
-                        set4(i, ds.d0, w0, w1, w2, w3);
-                        ++i;
-                    }
-                } else {
-                    ++i;
+    for (int step = 0; step < 8; ++step) {  // each step advances i or removes a donor
+        if (i >= todo || i >= 4) break;
+        const int q = sel4(i, q0, q1, q2, q3);
+        const Pub ds = pick4(q, P0, P1, P2, P3);
+        if (ds.ndnr <= 1) {
+            if (!worked) { padd = s.p; cadd = s.c; }
+            worked = true;
+            padd = __fadd_rn(padd, ds.p);
+            cadd += ds.c;
+            if (ds.ndnr == 0) {
+                --todo;
+                if (todo > i && todo < 4) {
+                    set4(i, sel4(todo, own[0], own[1], own[2], own[3]), w0, w1, w2, w3);
+                    set4(i, todo, q0, q1, q2, q3);
                 }
-            }
-            const int donors[4] = {w0, w1, w2, w3};
-            if (last) {
-                Q[t] = s.p;
-                if (counts) counts[t] = s.c;
-            } else if (!worked) {
-                nxt[t] = s;
-                keep = true;
             } else {
-                nxt[t] = Pub{todo, padd, cadd, todo > 0 ? donors[0] : own[0]};
-                if (todo > 1) priv[t] = make_int4(donors[1], donors[2], donors[3], -1);
-                if (todo > 0) {
-                    keep = true;
-                } else {
-                    Q[t] = padd;
-                    if (counts) counts[t] = cadd;
-                    fin = true;
+                set4(i, ds.d0, w0, w1, w2, w3);
+                ++i;
+            }
+        } else {
+            ++i;
+        }
+    }
+    if (!worked) {
+        nxt[t] = s;
+        return 0;
+    }
+    nxt[t] = Pub{todo, padd, cadd, todo > 0 ? w0 : own[0]};
+    if (todo > 1) priv[t] = make_int4(w1, w2, w3, -1);
+    if (todo > 0) return 0;
+    Q[t] = padd;
+    if (counts) counts[t] = cadd;
+    return 1;
+}
+
+// Every remaining round in one cooperative launch, a grid barrier between rounds.  Round
+// it reads cnt[2 it] active nodes (list la[it & 1]) and cnt[2 it + 1] nodes that
+// finished in round it - 1 (list lf[it & 1]; copied into the buffer written this
+// round; with fin_q, round first0 also writes their Q and count: the nodes that
+// finished inside the tile front), and ends when both are zero.
+//
+// What bounds it: the late rounds, whose lists are nearly empty.  One launch per round
+// cost 2-4 us each for about 20 of them (285 us for the 24 rounds at 2048 x 2048); a
+// barrier costs 1.3 us, and the empty ones at the end are skipped.  Each warp takes 32
+// entries and collects what it keeps in shared memory, so the lists stay in runs of
+// ascending cells whose donors share cache lines.
+constexpr int ACC_THREADS = 1024, ACC_CAP = 96;
+struct AccRounds {
+    const int32_t *rcv;
+    Pub *buf[2];
+    int4 *priv;
+    float *Q;
+    uint32_t *counts;
+    int *la[2], *lf[2];
+    int *cnt;        // 2 per round
+    int *nonlocal, *overflow;
+    int N, first, logn;
+    int *bar, *over_out;
+    // ragged batch: rounds end tile by tile (N is then the packed total, nonlocal unused)
+    const BatchTile *tiles;
+    int ntiles;
+    const int *limits;  // [0] smallest, [1] largest logn of the tiles
+};
+
+__global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
+{
+    __shared__ int sa[ACC_THREADS / 32][ACC_CAP], sf[ACC_THREADS / 32][ACC_CAP];
+    __shared__ int dead;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int gthreads = gridDim.x * ACC_THREADS;
+    if (threadIdx.x == 0) dead = 0;
+    GridBar bar{a.bar, 0};
+    __syncthreads();
+    int it = a.first, logn = a.logn, logmin = a.logn;
+    if (a.tiles) {
+        logmin = a.limits[0];
+        logn = a.limits[1];
+    } else if (*a.nonlocal) {  // the same for every block
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.cnt[0] = a.cnt[2 * it] = a.cnt[2 * it + 1] = 0;
+        acc_init(a.buf[0], a.buf[1], a.priv, a.Q, a.counts, a.N);
+        if (!bar.sync(&dead)) return;
+        acc_scatter(a.rcv, a.buf[0], a.priv, a.N, a.overflow);
+        if (!bar.sync(&dead)) return;
+        acc_list0<ACC_THREADS>(a.buf[0], a.buf[1], a.priv, a.la[0], a.cnt, a.N);
+        if (!bar.sync(&dead)) return;
+        it = 0;
+    }
+    const int it0 = it;
+    for (; it <= logn; ++it) {
+        const int p = it & 1;
+        const Pub *cur = a.buf[p];
+        Pub *nxt = a.buf[p ^ 1];
+        const int nA = vload(a.cnt + 2 * it), nF = vload(a.cnt + 2 * it + 1), total = nA + nF;
+        if (total == 0) break;
+        const int *la = a.la[p], *lf = a.lf[p];
+        int *la2 = a.la[p ^ 1], *lf2 = a.lf[p ^ 1], *c2 = a.cnt + 2 * (it + 1);
+        const bool fin_q = it == it0 && it > 0;
+        int na = 0, nf = 0;  // buffered, warp-uniform
+        auto flush = [&](int *buf, int &n, int *list, int *count) {
+            __syncwarp();
+            int base = 0;
+            if (lane == 0 && n) base = atomicAdd(count, n);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            for (int q = lane; q < n; q += 32) list[base + q] = buf[q];
+            __syncwarp();
+            n = 0;
+        };
+        for (int k0 = (blockIdx.x * (ACC_THREADS / 32) + wib) * 32; k0 < total; k0 += gthreads) {
+            const int idx = k0 + lane;
+            int t = -1, r = 2;
+            if (idx < nA) {
+                t = la[idx];
+                bool last = it == logn;
+                if (a.tiles && it >= logmin) {  // the tile's own last round
+                    int lo = 0, hi = a.ntiles - 1;  // tiles sorted by offset: see k_batch_front
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (a.tiles[mid].off <= t) lo = mid;
+                        else hi = mid - 1;
+                    }
+                    last = it == a.tiles[lo].logn;
+                }
+                r = acc_node(t, cur, nxt, a.priv, a.Q, a.counts, last);
+            } else if (idx < total) {
+                const int f = lf[idx - nA];
+                const Pub s = cur[f];
+                nxt[f] = s;
+                if (fin_q) {
+                    a.Q[f] = s.p;
+                    if (a.counts) a.counts[f] = s.c;
                 }
             }
-        } else if (idx < total) {
-            const int f = lf[idx - nA];
-            const Pub s = cur[f];
-            nxt[f] = s;
-            if (fin_q) {
-                Q[f] = s.p;
-                if (counts) counts[f] = s.c;
-            }
+            const unsigned ma = __ballot_sync(0xffffffffu, r == 0), mf = __ballot_sync(0xffffffffu, r == 1);
+            if (r == 0) sa[wib][na + __popc(ma & ((1u << lane) - 1u))] = t;
+            if (r == 1) sf[wib][nf + __popc(mf & ((1u << lane) - 1u))] = t;
+            na += __popc(ma);
+            nf += __popc(mf);
+            if (na > ACC_CAP - 32) flush(sa[wib], na, la2, c2);
+            if (nf > ACC_CAP - 32) flush(sf[wib], nf, lf2, c2 + 1);
         }
-        block_append2<BS>(keep, fin, t, la2, nla2, lf2, nlf2);
+        if (na) flush(sa[wib], na, la2, c2);
+        if (nf) flush(sf[wib], nf, lf2, c2 + 1);
+        if (!bar.sync(&dead)) return;
+    }
+    if (a.over_out && blockIdx.x == 0 && threadIdx.x == 0) {
+        ((volatile int *)a.over_out)[0] = *a.overflow;
+        __threadfence_system();
     }
 }
 
@@ -529,12 +594,12 @@ __device__ __forceinline__ FrontNode front_round(const float *pc, const uint32_t
     return FrontNode{todo, padd, cadd, w0, w1, w2, w3, worked};
 }
 
+// The pointers address the grid's own cells; idb is added to every cell id written (the
+// grid's offset in a packed batch).
 template <int MODE, int FR>
-__global__ void __launch_bounds__(Front<FR>::BS) k_acc_front(const int32_t *__restrict__ rcv,
-                                                              const float *__restrict__ seed, Pub *cur_out,
-                                                              Pub *nxt_out, int4 *priv, uint32_t *counts, int *la,
-                                                              int *nla, int *lf, int *nlf, int *nonlocal, Grid g,
-                                                              int ntx)
+__device__ __forceinline__ void front_tile(const int32_t *__restrict__ rcv, const float *__restrict__ seed,
+                                           Pub *cur_out, Pub *nxt_out, int4 *priv, uint32_t *counts, int *la, int *nla,
+                                           int *lf, int *nlf, int *nonlocal, const Grid &g, int tx, int ty, int idb)
 {
     using F = Front<FR>;
     constexpr int H = F::H, RW = F::RW, RH = F::RH, NR = F::NR, BS = F::BS, TW = F::TW, TH = F::TH;
@@ -546,7 +611,6 @@ __global__ void __launch_bounds__(Front<FR>::BS) k_acc_front(const int32_t *__re
     uint32_t *nA = cB + NR, *nB = nA + NR;  // ndnr << 16 | d0 (local id)
     uint16_t *s1 = reinterpret_cast<uint16_t *>(nB + NR), *s2 = s1 + NR, *s3 = s2 + NR;
     uint8_t *dir = reinterpret_cast<uint8_t *>(s3 + NR);
-    const int tx = blockIdx.x % ntx, ty = blockIdx.x / ntx;
     const int c0 = tx * TW - H, r0 = ty * TH - H;  // region origin, before any wrap
 
     for (int k = threadIdx.x; k < RH + RW; k += BS) {
@@ -693,7 +757,7 @@ __global__ void __launch_bounds__(Front<FR>::BS) k_acc_front(const int32_t *__re
     auto l2g = [&](int l) -> int {
         if (l == (int)NONE) return -1;
         const int lr = l / RW;
-        return gid(lr, l - lr * RW);
+        return gid(lr, l - lr * RW) + idb;
     };
 #pragma unroll 1
     for (int k = 0; k < TW * TH / BS; ++k) {
@@ -732,13 +796,48 @@ __global__ void __launch_bounds__(Front<FR>::BS) k_acc_front(const int32_t *__re
                 fin = true;
             }
         }
-        block_append2<BS>(act, fin, t, la, nla, lf, nlf);
+        block_append2<BS>(act, fin, t + idb, la, nla, lf, nlf);
     }
 }
 
-__global__ void k_acc_cond_reset(int *c, const int *need)
+template <int MODE, int FR>
+__global__ void __launch_bounds__(Front<FR>::BS) k_acc_front(const int32_t *__restrict__ rcv,
+                                                              const float *__restrict__ seed, Pub *cur_out,
+                                                              Pub *nxt_out, int4 *priv, uint32_t *counts, int *la,
+                                                              int *nla, int *lf, int *nlf, int *nonlocal, Grid g,
+                                                              int ntx)
 {
-    if (*need && threadIdx.x < 2) c[threadIdx.x] = 0;
+    front_tile<MODE, FR>(rcv, seed, cur_out, nxt_out, priv, counts, la, nla, lf, nlf, nonlocal, g, blockIdx.x % ntx,
+                         blockIdx.x / ntx, 0);
+}
+
+// The front over a ragged batch: items[k] = the batch tile of work item k, whose front
+// tile is k - (the first item of that batch tile).
+constexpr int BATCH_FR = 3;
+__global__ void __launch_bounds__(Front<BATCH_FR>::BS) k_batch_front(BatchAcc b, Pub *cur_out, Pub *nxt_out, int4 *priv,
+                                                                     int *la, int *nla, int *lf, int *nlf, int *nonlocal)
+{
+    using F = Front<BATCH_FR>;
+    const int n = b.limits[2];
+    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+        const BatchTile T = b.by_offset[b.items[k]];
+        const Grid g{T.nx, T.ny, T.mode, nullptr};
+        const int ntx = (T.nx + F::TW - 1) / F::TW, e = k - T.item0, tx = e % ntx, ty = e / ntx;
+        const int32_t *rcv = b.rcv + T.off;
+        float *Q = b.Q + T.off;
+        uint32_t *c = b.counts + T.off;
+        const int idb = (int)T.off;
+        if (T.mode == 0)
+            front_tile<0, BATCH_FR>(rcv, Q, cur_out + T.off, nxt_out + T.off, priv + T.off, c, la, nla, lf, nlf, nonlocal, g,
+                                    tx, ty, idb);
+        else if (T.mode == 1)
+            front_tile<1, BATCH_FR>(rcv, Q, cur_out + T.off, nxt_out + T.off, priv + T.off, c, la, nla, lf, nlf, nonlocal, g,
+                                    tx, ty, idb);
+        else
+            front_tile<2, BATCH_FR>(rcv, Q, cur_out + T.off, nxt_out + T.off, priv + T.off, c, la, nla, lf, nlf, nonlocal, g,
+                                    tx, ty, idb);
+        __syncthreads();  // the shared buffers are reused by the next item
+    }
 }
 
 template <int MODE, int FR>
@@ -775,18 +874,58 @@ static int front_dispatch(int mode, const int32_t *rcv, const float *seed, Pub *
     }
 }
 
-__global__ void k_acc_reset_counts(int *c, int n)
-{
-    if (threadIdx.x < n) c[threadIdx.x] = 0;
-}
-__global__ void k_acc_fill_one(int *c) { *c = 1; }
-
 template <int MODE>
 static void l_acc_gather(const int32_t *rcv, Pub *A, Pub *B, int4 *priv, const float *Q, uint32_t *counts, int *list,
                          int *nlist, int *nonlocal, int *overflow, const Grid &g, cudaStream_t st)
 {
     dim3 gr(div_up(g.nx, 32), div_up(g.ny, 8));
     { k_acc_gather<MODE, 256><<<gr, 256, 0, st>>>(rcv, A, B, priv, Q, counts, list, nlist, nonlocal, overflow, g); count_launch(); }
+}
+
+// Blocks of the cooperative rounds over n nodes: one per 8192 up to one per SM.
+static int launch_rounds(AccRounds &a, int n, cudaStream_t st)
+{
+    int dev = 0, nsm = 0;
+    PFF_CUDA(cudaGetDevice(&dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    void *args[] = {&a};
+    PFF_CUDA(cudaLaunchCooperativeKernel((void *)k_acc_rounds, std::max(1, std::min(nsm, div_up(n, 8192))), ACC_THREADS,
+                                         args, 0, st));
+    count_launch();
+    return PFF_OK;
+}
+
+bool batch_front_takes(int nx, int ny, int mode) { return mode <= 2 && nx >= 3 && ny >= 3 && ceil_log2((long long)nx * ny) + 1 > BATCH_FR; }
+int batch_front_items(int nx, int ny)
+{
+    return div_up(nx, Front<BATCH_FR>::TW) * div_up(ny, Front<BATCH_FR>::TH);
+}
+
+// Upstream sums of the batch tiles the front takes, in the reference's f32 order: the
+// first rounds tile by tile in shared memory, the others over packed lists.
+int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st)
+{
+    int dev = 0, nsm = 0;
+    PFF_CUDA(cudaGetDevice(&dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    using F = Front<BATCH_FR>;
+    PFF_CUDA(cudaFuncSetAttribute(k_batch_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::SMEM));
+    PFF_CUDA(cudaMemsetAsync(b.ctr, 0, sizeof(int) * BATCH_ACC_CTR, st));
+    int *cnt = b.ctr, *nonlocal = b.ctr + 128, *bar = b.ctr + 136;
+    constexpr int pa = BATCH_FR & 1;
+    Pub *buf[2] = {(Pub *)b.bufA, (Pub *)b.bufB};
+    { k_batch_front<<<2 * nsm, F::BS, F::SMEM, st>>>(b, buf[pa], buf[pa ^ 1], (int4 *)b.priv, b.la[pa], cnt + 2 * BATCH_FR,
+                                                     b.lf[pa], cnt + 2 * BATCH_FR + 1, nonlocal); count_launch(); }
+    AccRounds a{};
+    a.rcv = b.rcv;
+    a.buf[0] = buf[0]; a.buf[1] = buf[1];
+    a.priv = (int4 *)b.priv;
+    a.Q = b.Q; a.counts = b.counts;
+    for (int k = 0; k < 2; ++k) { a.la[k] = b.la[k]; a.lf[k] = b.lf[k]; }
+    a.cnt = cnt; a.nonlocal = nonlocal; a.overflow = nonlocal + 1;
+    a.N = (int)b.total; a.first = BATCH_FR; a.bar = bar;
+    a.tiles = b.by_offset; a.ntiles = b.ntiles; a.limits = b.limits;
+    return launch_rounds(a, (int)b.total, st);
 }
 
 }  // namespace pff
@@ -879,19 +1018,18 @@ extern "C" int pff_accumulate_grid(const int32_t *receivers, float *Q, uint32_t 
     Pub *B = cv.take<Pub>(N);
     int4 *priv = cv.take<int4>(N);
     int *lA0 = cv.take<int>(N), *lA1 = cv.take<int>(N), *lF0 = cv.take<int>(N), *lF1 = cv.take<int>(N);
-    int *ctr = cv.take<int>(64);  // [2*r] active count, [2*r+1] finished count, by round parity
-    constexpr int BS = 256;
+    int *ctr = cv.take<int>(256);  // [2*r] active, [2*r+1] finished nodes of round r; flags and the barrier past 128
     const int logn = ceil_log2(N) + 1;  // flowfields.py:272
     const int FR = g_front_rounds;
     const bool front = nx > 0 && mode >= 0 && mode <= 2 && nx >= 3 && ny >= 3 && FR > 0 && logn > FR;
-    { k_acc_reset_counts<<<1, 64, 0, st>>>(ctr, 64); count_launch(); }
-    int *nonlocal = ctr + 63, *overflow = ctr + 62;
+    PFF_CUDA(cudaMemsetAsync(ctr, 0, 256 * sizeof(int), st));
+    int *nonlocal = ctr + 128, *overflow = ctr + 129, *bar = ctr + 136;
     Pub *bufs[2] = {A, B};
     int *la[2] = {lA0, lA1}, *lf[2] = {lF0, lF1};
     if (front) {
         Grid g{nx, ny, mode, codes};
         const int pa = FR & 1;
-        int *na = ctr + 4 * pa;
+        int *na = ctr + 2 * FR;
         auto run = [&](auto fr) {
             return front_dispatch<decltype(fr)::value>(mode, receivers, Q, bufs[pa], bufs[pa ^ 1], priv, counts,
                                                        la[pa], na, lf[pa], na + 1, nonlocal, g, st);
@@ -903,42 +1041,30 @@ extern "C" int pff_accumulate_grid(const int32_t *receivers, float *Q, uint32_t 
         PFF_MODE_DISPATCH(mode, l_acc_gather, receivers, A, B, priv, Q, counts, lA0, ctr + 0, nonlocal, overflow, g,
                           st);
     } else {
-        { k_acc_fill_one<<<1, 1, 0, st>>>(nonlocal); count_launch(); }
+        PFF_CUDA(cudaMemsetAsync(nonlocal, 1, sizeof(int), st));
     }
-    // receivers that are not D4 neighbours (or no grid given): scatter path
-    { k_acc_fallback_reset<<<1, 1, 0, st>>>(ctr + 0, nonlocal); count_launch(); }
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = nsm * 8;
-    { k_acc_init<<<grid, BS, 0, st>>>(A, B, priv, Q, counts, N, nonlocal); count_launch(); }
-    { k_acc_scatter<<<grid, BS, 0, st>>>(receivers, A, priv, N, nonlocal, overflow); count_launch(); }
-    { k_acc_list0<BS><<<grid, BS, 0, st>>>(A, B, priv, lA0, ctr + 0, N, nonlocal); count_launch(); }
-    static int round_blocks = 0;
-    if (!round_blocks) {
-        int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_acc_round<BS>, BS, 0);
-        round_blocks = nsm * (per > 0 ? per : 1);
-    }
-    for (int it = 0; it <= logn; ++it) {
-        const int a = it & 1, b = a ^ 1;
-        // list counters: ctr[4*parity] = active, ctr[4*parity+1] = finished
-        int *na_in = ctr + 4 * a, *nf_in = na_in + 1;
-        int *na_out = ctr + 4 * b, *nf_out = na_out + 1;
-        // with the tile front, rounds 0..FR-1 run only on the scatter path
-        const bool cond = front && it < FR;
-        if (cond) {
-            { k_acc_cond_reset<<<1, 32, 0, st>>>(na_out, nonlocal); count_launch(); }
-        } else {
-            PFF_CUDA(cudaMemsetAsync(na_out, 0, 2 * sizeof(int), st));
-        }
-        { k_acc_round<BS><<<round_blocks, BS, 0, st>>>(bufs[a], bufs[b], priv, la[a], na_in, lf[a], nf_in, la[b], na_out,
-                                               lf[b], nf_out, Q, counts, it, it == logn, cond ? nonlocal : nullptr,
-                                               front && it == FR); count_launch(); }
-    }
+    // the remaining rounds; receivers that are not D4 neighbours (or no grid given) start
+    // again there by the scatter path
+    int *host = nullptr, *dptr = nullptr;
+    PFF_TRY(pinned_ints(&host, &dptr));
+    host[0] = -1;
+    AccRounds a{};
+    a.rcv = receivers;
+    a.buf[0] = A; a.buf[1] = B;
+    a.priv = priv;
+    a.Q = Q; a.counts = counts;
+    for (int k = 0; k < 2; ++k) { a.la[k] = la[k]; a.lf[k] = lf[k]; }
+    a.cnt = ctr; a.nonlocal = nonlocal; a.overflow = overflow;
+    a.N = N; a.first = front ? FR : 0; a.logn = logn;
+    a.bar = bar; a.over_out = dptr;
+    PFF_TRY(launch_rounds(a, N, st));
+    PFF_CUDA(cudaStreamSynchronize(st));
     PFF_TRY(check_cuda("pff_accumulate"));
-    int over = 0;
-    PFF_TRY(read_ints(IntReads().add(overflow, 1), &over, st));
+    const int over = *(volatile int *)host;
+    if (over < 0) {
+        set_error("pff_accumulate: the rounds did not end");
+        return PFF_ERR_NOCONV;
+    }
     if (over) {
         set_error("pff_accumulate: a node has more than 4 donors (possible only after jump rerouting); "
                   "the reference's donor slots overflow there and this case is not supported");

@@ -12,18 +12,10 @@
 // receiver cycles (emulated), snapshot rake-and-compress rounds with donors in
 // ascending index.  Results are bit-identical to routing each tile on its own.
 #include <algorithm>
+#include <vector>
 #include "pff_internal.h"
 
 namespace pff {
-
-struct BatchTile {
-    long long off;   // first cell of the tile in the packed arrays
-    long long boff;  // first basin entry (N+1 entries per tile)
-    int nx, ny, mode;
-    int id;          // the tile's index in the caller's order
-    float dx;
-    int pad;
-};
 
 // Packed per-cell and per-basin arrays of the batch (device pointers).
 struct BatchArrays {
@@ -60,7 +52,7 @@ struct BatchShm {
     int tgt[LB_CELLS];  // sub-block cells' receivers (tile indices)
 };
 
-__device__ __forceinline__ int bceil_log2(long long n)
+__host__ __device__ __forceinline__ int bceil_log2(long long n)
 {
     int r = 0;
     long long p = 1;
@@ -689,7 +681,9 @@ __device__ void route_tile(const BatchTile &T, const BatchArrays &A, BatchShm &s
     const float *z = A.z + o;
     tile_receivers<MODE>(g, T.dx, z, A.rcv + o, A.rec_ + o, A.grad + o);
     tile_reroute<MODE>(g, T, A, z, sh);
-    // accumulate: Q holds the seed (flowfields.py:272-292)
+    // accumulate: Q holds the seed (flowfields.py:272-292).  Tiles the front takes (modes 0-2,
+    // 3 x 3 and more) are accumulated after this launch, all together
+    if (T.item0 >= 0) return;
     tile_accumulate(N, A.rcv + o, A.Q + o, A.counts + o, A.dnr + 4 * o, A.dnr_ + 4 * o, A.ndnr + o, A.ndnr_ + o,
                     A.src + o, A.p_ + o, A.c_ + o, A.mark + o, A.rec__ + o, sh);
 }
@@ -947,12 +941,18 @@ __global__ void k_batch_reset(int *ctr)
 // Workspace layout, identical for the plan and the launches.
 struct BatchWs {
     BatchArrays A;
-    BatchTile *tiles;
+    BatchTile *tiles, *by_offset;  // largest first; in packed order
     int *ctr;
+    int *limits, *items, *acc_ctr;
+    int32_t *priv;  // 4 per cell: the memory of rec_, rec__, bid and mark
     bool ok;
 };
 
-static BatchWs carve_batch(void *ws, size_t wsb, long long total, int ntiles)
+// Work items of the accumulation front: a tile nx x ny has ceil(nx/64) ceil(ny/24) <=
+// nx ny / 3 + 1 of them (tiles of at least 3 x 3).
+static size_t batch_item_cap(long long total, int ntiles) { return (size_t)(total / 3 + ntiles); }
+
+static BatchWs carve_batch(void *ws, size_t wsb, long long total, int ntiles, size_t *used = nullptr)
 {
     Carver cv(ws, wsb);
     const size_t n = (size_t)total, nb = n + (size_t)ntiles;
@@ -960,10 +960,15 @@ static BatchWs carve_batch(void *ws, size_t wsb, long long total, int ntiles)
     BatchArrays &A = w.A;
     w.ctr = cv.take<int>(64);
     w.tiles = cv.take<BatchTile>((size_t)ntiles);
-    A.rec_ = cv.take<int32_t>(n);
-    A.rec__ = cv.take<int32_t>(n);
-    A.bid = cv.take<int32_t>(n);
-    A.mark = cv.take<int32_t>(n);
+    w.by_offset = cv.take<BatchTile>((size_t)ntiles);
+    w.limits = cv.take<int>(64);
+    w.items = cv.take<int>(batch_item_cap(total, ntiles));
+    w.acc_ctr = cv.take<int>(BATCH_ACC_CTR);
+    w.priv = cv.take<int32_t>(4 * n);
+    A.rec_ = w.priv;
+    A.rec__ = A.rec_ + n;
+    A.bid = A.rec__ + n;
+    A.mark = A.bid + n;
     A.zp = cv.take<float>(n);
     A.isb = cv.take<uint8_t>(n);
     A.tag = cv.take<uint8_t>(n);
@@ -983,6 +988,7 @@ static BatchWs carve_batch(void *ws, size_t wsb, long long total, int ntiles)
     A.queue = w.ctr;
     A.status = w.ctr + 1;
     w.ok = A.c_ != nullptr;
+    if (used) *used = cv.off;
     return w;
 }
 
@@ -993,10 +999,9 @@ using namespace pff;
 extern "C" size_t pff_batch_workspace_bytes(long long total_cells, int ntiles)
 {
     if (total_cells <= 0 || ntiles <= 0) return 0;
-    const size_t n = (size_t)total_cells, nb = n + (size_t)ntiles;
-    return Carver::round(64 * 4) + Carver::round(sizeof(BatchTile) * (size_t)ntiles) + Carver::round(4 * n) * 5 +
-           Carver::round(n) * 3 + Carver::round(8 * nb) * 2 + Carver::round(4 * nb) + Carver::round(nb) +
-           Carver::round(16 * n) * 2 + Carver::round(4 * n) * 5 + 256;
+    size_t used = 0;
+    carve_batch(nullptr, 0, total_cells, ntiles, &used);
+    return used + 256;
 }
 
 namespace pff {
@@ -1044,17 +1049,34 @@ extern "C" long long pff_batch_plan(const int32_t *tile_nx, const int32_t *tile_
     for (int t = 0; t < ntiles; ++t) ord[t] = t;
     auto cells = [&](int t) { return (long long)tile_nx[t] * tile_ny[t]; };
     std::stable_sort(ord, ord + ntiles, [&](int a, int b) { return cells(a) > cells(b); });
-    BatchTile *ht = new BatchTile[ntiles];
+    std::vector<BatchTile> hp(ntiles), ht(ntiles);  // packed order, largest first
+    std::vector<int> items;
+    int limits[3] = {64, 0, 0};
+    for (int t = 0; t < ntiles; ++t) {
+        const int nx = tile_nx[t], ny = tile_ny[t], logn = bceil_log2(cells(t)) + 1;
+        // packed cell ids of the accumulation are 32-bit
+        const bool front = batch_front_takes(nx, ny, tile_mode[t]) && total < (1LL << 31);
+        hp[t] = BatchTile{tile_offset[t], tile_offset[t] + t, nx, ny, tile_mode[t], t, tile_dx[t],
+                          front ? (int)items.size() : -1, logn, 0};
+        if (!front) continue;
+        items.insert(items.end(), (size_t)batch_front_items(nx, ny), t);
+        limits[0] = std::min(limits[0], logn);
+        limits[1] = std::max(limits[1], logn);
+    }
+    limits[2] = (int)items.size();
     for (int k = 0; k < ntiles; ++k) {
-        const int t = ord[k];
-        ht[k] = BatchTile{tile_offset[t], tile_offset[t] + t, tile_nx[t], tile_ny[t], tile_mode[t], t, tile_dx[t], 0};
-        if (order) order[k] = t;
+        ht[k] = hp[ord[k]];
+        if (order) order[k] = ord[k];
     }
     BatchWs w = carve_batch(workspace, workspace_bytes, total, ntiles);
     cudaStream_t st = S(stream);
-    const cudaError_t e1 = cudaMemcpyAsync(w.tiles, ht, sizeof(BatchTile) * ntiles, cudaMemcpyHostToDevice, st);
-    const cudaError_t e2 = cudaStreamSynchronize(st);  // the host array must outlive the copy
-    delete[] ht;
+    cudaError_t e1 = cudaMemcpyAsync(w.tiles, ht.data(), sizeof(BatchTile) * ntiles, cudaMemcpyHostToDevice, st);
+    if (e1 == cudaSuccess)
+        e1 = cudaMemcpyAsync(w.by_offset, hp.data(), sizeof(BatchTile) * ntiles, cudaMemcpyHostToDevice, st);
+    if (e1 == cudaSuccess) e1 = cudaMemcpyAsync(w.limits, limits, sizeof(limits), cudaMemcpyHostToDevice, st);
+    if (e1 == cudaSuccess && !items.empty())
+        e1 = cudaMemcpyAsync(w.items, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);  // the host arrays must outlive the copies
     delete[] ord;
     if (e1 != cudaSuccess || e2 != cudaSuccess) {
         set_error("pff_batch_plan: descriptor upload: %s", cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
@@ -1095,6 +1117,17 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
     const int grid = std::min(nsm * ctas_per_sm, ntiles);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
     { k_batch_route<<<grid, threads, 0, st>>>(ntiles, A); count_launch(); }
+    if (total_cells < (1LL << 31)) {
+        BatchAcc b{};
+        b.rcv = receivers; b.Q = Q; b.counts = counts;
+        b.bufA = A.dnr; b.bufB = A.dnr_; b.priv = w.priv;
+        b.la[0] = A.ndnr; b.la[1] = A.ndnr_;
+        b.lf[0] = A.src; b.lf[1] = reinterpret_cast<int *>(A.p_);
+        b.ctr = w.acc_ctr;
+        b.by_offset = w.by_offset; b.items = w.items; b.limits = w.limits;
+        b.total = total_cells; b.ntiles = ntiles;
+        PFF_TRY(launch_batch_accumulate(b, st));
+    }
     return check_cuda("pff_batch_route");
 }
 

@@ -91,6 +91,37 @@ struct Carver {
     static size_t round(size_t n) { return (n + 255) & ~size_t(255); }
 };
 
+// A tile of a ragged batch.
+struct BatchTile {
+    long long off;   // first cell of the tile in the packed arrays
+    long long boff;  // first basin entry (N+1 entries per tile)
+    int nx, ny, mode;
+    int id;          // the tile's index in the caller's order
+    float dx;
+    int item0;       // its first work item of the accumulation front, -1: accumulated by its own CTA
+    int logn;        // rake-and-compress rounds: ceil(log2 N) + 1
+    int pad;
+};
+
+// The accumulation of a ragged batch (pff_accum.cu), over packed arrays.
+constexpr int BATCH_ACC_CTR = 256;
+struct BatchAcc {
+    const int32_t *rcv;
+    float *Q;             // in: seeds, out: sums
+    uint32_t *counts;
+    void *bufA, *bufB, *priv;  // 16 B per cell each
+    int *la[2], *lf[2];   // 4 B per cell each
+    int *ctr;             // BATCH_ACC_CTR ints
+    const BatchTile *by_offset;  // the tiles in packed order
+    const int *items;     // work item -> tile (packed order)
+    const int *limits;    // [0] smallest and [1] largest logn of the front's tiles, [2] work items
+    long long total;
+    int ntiles;
+};
+bool batch_front_takes(int nx, int ny, int mode);
+int batch_front_items(int nx, int ny);
+int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st);
+
 inline cudaStream_t S(void *s) { return (cudaStream_t)s; }
 
 // Launch helpers implemented per translation unit (declared for cross-TU use).

@@ -17,6 +17,7 @@
 // One block of 1024 threads per SM: the barrier's cost grows with the number of
 // blocks, and 32 warps hide the gathers of the list steps.
 #pragma once
+#include "pff_coop.cuh"
 
 namespace pff {
 
@@ -61,46 +62,6 @@ struct LoopArgs {
     int *bar;              // [0] barrier arrivals, [1] error
     Grid g;
 };
-
-// Barrier over the launch's blocks.  The launch is cooperative, so every block is
-// resident; a wait that has not ended after about two seconds gives up, records it
-// and makes the kernel return.
-struct LoopBar {
-    int *ctr;
-    int target;
-    __device__ __forceinline__ bool sync(int *dead)
-    {
-        __syncthreads();
-        if (gridDim.x > 1) {
-            target += gridDim.x;
-            if (threadIdx.x == 0) {
-                __threadfence();
-                atomicAdd(ctr, 1);
-                unsigned long long t0;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-                int spin = 0, seen;
-                for (;;) {
-                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
-                    if (seen >= target) break;
-                    if ((++spin & 1023) == 0) {
-                        unsigned long long t;
-                        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                        if (t - t0 > 2000000000ull) {
-                            *dead = 1;
-                            atomicExch(ctr + 1, 1);
-                            break;
-                        }
-                    }
-                }
-                __threadfence();
-            }
-            __syncthreads();
-        }
-        return *dead == 0;
-    }
-};
-
-__device__ __forceinline__ int vload(const int *p) { return *(const volatile int *)p; }
 
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(TILE_THREADS) : "memory"); }
 __device__ __forceinline__ bool group_or(int id, bool p)
@@ -259,7 +220,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
     const TileXY txy{(nx + TILE_W - 1) / TILE_W, mnx, nx};
     const long long iv = invalid_key();
     if (tid == 0) dead = 0;
-    LoopBar bar{A.bar, 0};
+    GridBar bar{A.bar, 0};
     __syncthreads();
 
     const int np0 = A.info[0];
@@ -635,7 +596,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, 
     const int ntx = (nx + TILE_W - 1) / TILE_W;
     const int gtid = blockIdx.x * LOOP_THREADS + threadIdx.x, gthreads = gridDim.x * LOOP_THREADS;
     if (threadIdx.x == 0) dead = 0;
-    LoopBar bar{A.bar + 8, 0};
+    GridBar bar{A.bar + 8, 0};
     __syncthreads();
     for (int r = 0; r < LOOP_JUMPS; ++r) {
         bool ch = false;
