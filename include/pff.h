@@ -94,6 +94,10 @@ int pff_compute_receivers_stochastic(const float *z, int32_t *receivers, float *
 int pff_receivers_set_path(int lean);
 int pff_receivers_div_selfcheck(float dx, long long *mismatches, long long *checked);
 
+/* The Manning update's h^(5/3) against the double-precision power on every float whose bits
+ * lie in [lo, hi]; *mismatches = the floats where they differ. */
+int pff_pow53_selfcheck(uint32_t lo, uint32_t hi, long long *mismatches);
+
 /* ---- accumulation (rake and compress) ----------------------------------------
  * Kernel-level mirrors of pyfastflow/flow/downstream_propag.py with identical
  * semantics (donor slots in ascending donor index, as the reference's serial

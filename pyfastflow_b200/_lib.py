@@ -71,6 +71,7 @@ SIGNATURES = {
     "pff_conv3x3_fwd": (_i32, [_vp, _i32, _i32, _vp, _vp, _vp, _i32, _i32] + [_i32] * 7 + [_vp]),
     "pff_receivers_set_path": (_i32, [_i32]),
     "pff_receivers_div_selfcheck": (_i32, [_f32, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),
+    "pff_pow53_selfcheck": (_i32, [C.c_uint32, C.c_uint32, C.POINTER(C.c_longlong)]),
     "pff_conv_set_path": (_i32, [_i32]),
     "pff_conv_tc_status": (_i32, [C.POINTER(C.c_int)]),
     "pff_conv3x3_wflip": (_i32, [_vp, _vp, _i32, _i32, _vp]),

@@ -14,6 +14,8 @@
 #include <algorithm>
 #include <vector>
 #include "pff_internal.h"
+#include "pff_lake_loop.cuh"
+#include "pff_pow.cuh"
 
 namespace pff {
 
@@ -45,6 +47,11 @@ enum : int { BST_MODE = 1, BST_CYCLE_LABELS = 8, BST_CARVE = 16 };
 constexpr int LB_SIDE = 32, LB_CELLS = LB_SIDE * LB_SIDE;  // label sub-blocks
 
 struct BatchShm {
+    LoopArgs la;  // the current tile's reroute
+    int loop[64 + LOOP_ITS * LOOP_CTR];  // its state words, barrier flags and counters (the first block's are used)
+    int any[3];   // team_any's flags (the first block's are used)
+    int any_r;
+    int it_outer[2];
     int red;
     int cur;
     int ws[32];
@@ -602,42 +609,72 @@ __device__ void tile_accumulate(int N, const int32_t *rcv, float *p, uint32_t *c
     __syncthreads();
 }
 
-// receivers (receivers.py:31-58): strict >, first k wins ties.  Writes rec and rec_
-// (and the gradient if grad is not null).
+// ---- teams ---------------------------------------------------------------------------
+// The blocks of a cluster work on one tile together; team_at gives the address of a
+// shared variable of the team's first block.
+template <class T>
+__device__ __forceinline__ T *team_at(T *p, const ClusterTeam &Tm)
+{
+    if (Tm.n == 1) return p;
+    T *q;
+    asm("mapa.u64 %0, %1, 0;" : "=l"(q) : "l"(p));
+    return q;
+}
+#define FOR_TEAM(i, N) for (int i = Tm.r * blockDim.x + threadIdx.x; i < (N); i += Tm.n * blockDim.x)
+
+// whether any thread of the team has p (a barrier)
+__device__ __forceinline__ bool team_any(bool p, BatchShm &sh, ClusterTeam &Tm)
+{
+    if (Tm.n == 1) return __syncthreads_or(p);
+    const int r = sh.any_r;
+    int *any = team_at(sh.any, Tm);
+    if (__any_sync(0xffffffffu, p) && (threadIdx.x & 31) == 0) any[r] = 1;
+    if (Tm.r == 0 && threadIdx.x == 0) sh.any[(r + 1) % 3] = 0;  // last read two calls ago
+    Tm.sync();
+    const bool res = *(volatile int *)(any + r) != 0;
+    if (threadIdx.x == 0) sh.any_r = (r + 1) % 3;
+    __syncthreads();
+    return res;
+}
+
+// receivers (receivers.py:31-58): strict >, first k wins ties (and the gradient if
+// grad is not null).
 template <int MODE>
-__device__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, int32_t *rec_, float *grad)
+__device__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, float *grad, ClusterTeam &Tm)
 {
     const int N = g.nx * g.ny;
-    FOR_CELLS(i, N) {
-        const int row = i / g.nx, col = i - row * g.nx;
-        int js[4];
+    const unsigned mnx = 0xffffffffu / (unsigned)g.nx;
+    FOR_TEAM(i, N) {
+        int row, col, js[4];
+        divmod_nx(i, g.nx, mnx, row, col);
         neighbours4<MODE>(g, i, row, col, js);
         const float zi = z[i];
+        float d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) d[k] = js[k] != -1 ? __fsub_rn(zi, z[js[k]]) : 0.f;
         int r = i;
         float sr = 0.f, dbest = 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (js[k] == -1) continue;
-            const float d = __fsub_rn(zi, z[js[k]]);
-            if (d > dbest) {  // a smaller difference cannot give a larger quotient
-                const float q = __fdiv_rn(d, dx);
+        for (int k = 0; k < 4; ++k)
+            if (d[k] > dbest) {  // a smaller difference cannot give a larger quotient
+                const float q = __fdiv_rn(d[k], dx);
                 if (q > sr) {
                     sr = q;
                     r = js[k];
-                    dbest = d;
+                    dbest = d[k];
                 }
             }
-        }
         rec[i] = r;
-        rec_[i] = r;
         if (grad) grad[i] = sr;
     }
-    __syncthreads();
+    Tm.sync();
 }
 
-// reroute_flow(carve=True) (lakeflow.py:466-538) on receivers rec (with rec_ == rec).
+// reroute_flow(carve=True) (lakeflow.py:466-538), the reference's own steps by one block,
+// from outer iteration it (with rec_ == rec; outer as the first iteration set it).
 template <int MODE>
-__device__ void tile_reroute(const Grid &g, const BatchTile &T, const BatchArrays &A, const float *z, BatchShm &sh)
+__device__ __noinline__ void tile_reroute_steps(const Grid &g, const BatchTile &T, const BatchArrays &A, const float *z,
+                                                BatchShm &sh, int it, int outer)
 {
     const int N = g.nx * g.ny;
     const long long o = T.off, ob = T.boff;
@@ -657,11 +694,8 @@ __device__ void tile_reroute(const Grid &g, const BatchTile &T, const BatchArray
         __syncthreads();
         return n;
     };
-    const int ndep = list_pits();
-    if (ndep == 0) return;
-    const int outer = bceil_log2(ndep) + 1;
-    for (int it = 0; it < outer; ++it) {
-        const int nd = it > 0 ? list_pits() : ndep;
+    for (; it < outer; ++it) {
+        const int nd = list_pits();
         if (nd == 0) break;  // (the labels the reference computes first are overwritten)
         const bool acyclic = tile_labels_blocks<MODE>(g, N, rec_, rec__, bid, sh);
         if (!acyclic) tile_labels<MODE>(g, N, rec_, rec__, bid, A.mark + o, A.dnr + 4 * o, lrounds, sh, A.status);
@@ -672,18 +706,91 @@ __device__ void tile_reroute(const Grid &g, const BatchTile &T, const BatchArray
     }
 }
 
+// The same reroute by the single grid's device loop, the team's blocks together; a tile
+// where the carve closes a receiver cycle goes on with the reference's steps.
+//
+// The steps are functions of their own: inlined into one kernel they spilled 2-3 KB of
+// registers at 1024 threads.
 template <int MODE>
-__device__ void route_tile(const BatchTile &T, const BatchArrays &A, BatchShm &sh)
+__device__ __noinline__ void batch_front_steps(const LoopArgs &L, int32_t *R, ClusterTeam Tm, unsigned char *smem)
+{
+    reroute_tiles<MODE>(L, R, Tm, smem);
+    Tm.sync();
+    reroute_labels<MODE, true>(L, R, Tm);
+    Tm.sync();
+    reroute_first_border<MODE, false>(L, Tm, smem);
+    Tm.sync();
+}
+template <int MODE>
+__device__ __noinline__ int batch_loop(const LoopArgs &L, ClusterTeam Tm, unsigned char *smem, int *it_outer)
+{
+    int it = 0, outer = 0, n_outer = 0;
+    const int state = reroute_loop<MODE, true>(L, Tm, smem, it, outer, n_outer);
+    if (threadIdx.x == 0) {
+        it_outer[0] = it;
+        it_outer[1] = outer;
+    }
+    Tm.sync();
+    return state;
+}
+
+template <int MODE>
+__device__ __noinline__ void tile_reroute(const BatchTile &T, const BatchArrays &A, const float *z, BatchShm &sh,
+                                          ClusterTeam Tm, unsigned char *smem)
+{
+    const Grid g{T.nx, T.ny, MODE, MODE == 3 ? A.codes + T.off : nullptr};
+    const int N = g.nx * g.ny;
+    const long long o = T.off, ob = T.boff;
+    int32_t *R = reinterpret_cast<int32_t *>(A.p_) + o;  // later the segment list
+    if (Tm.r == 0)
+        for (int k = threadIdx.x; k < 64 + LOOP_ITS * LOOP_CTR; k += blockDim.x) sh.loop[k] = 0;
+    if (threadIdx.x == 0) {
+        LoopArgs &L = sh.la;
+        int *ctr = team_at(sh.loop, Tm);
+        int32_t *d = A.dnr + 4 * o, *e = A.dnr_ + 4 * o;  // 4 N entries each
+        const int ntiles = (g.nx + TILE_W - 1) / TILE_W * ((g.ny + TILE_H - 1) / TILE_H);  // at most N / 4
+        L.bid = A.bid + o; L.rec = A.rcv + o; L.rec_ = A.rec_ + o; L.J = A.rec__ + o;
+        L.z = z; L.zp = nullptr; L.isb = nullptr;
+        L.sad = A.saddle + ob; L.out = A.outlet + ob; L.snode = A.snode + ob;
+        L.tag = A.tag + o; L.tag_ = A.tag_ + o; L.inv = A.inv + ob;
+        L.fin = d; L.nf = d + N + 1;
+        L.alist[0] = d + 2 * N + 2;
+        L.dirty = d + 3 * N + 2; L.dtiles = L.dirty + ntiles;
+        L.akey = reinterpret_cast<long long *>(e); L.abid = e + 2 * N; L.pit0 = e + 3 * N;
+        L.pits[0] = A.ndnr + o; L.pits[1] = A.ndnr_ + o;
+        L.alist[1] = A.mark + o;
+        L.segs = R;
+        L.ctl = ctr; L.ctl_out = nullptr;
+        L.info = ctr + 16; L.bar = ctr + 24; L.it_ctr = ctr + 64;
+        L.g = g;
+    }
+    __syncthreads();
+    const int ntiles = (g.nx + TILE_W - 1) / TILE_W * ((g.ny + TILE_H - 1) / TILE_H);
+    FOR_TEAM(k, ntiles) sh.la.dirty[k] = 0;
+    Tm.sync();
+    batch_front_steps<MODE>(sh.la, R, Tm, smem);
+    const int state = batch_loop<MODE>(sh.la, Tm, smem, sh.it_outer);
+    if (state == RR_GENERAL || state == RR_RESUME) {
+        if (Tm.r == 0) tile_reroute_steps<MODE>(g, T, A, z, sh, state == RR_RESUME ? sh.it_outer[0] + 1 : 0, sh.it_outer[1]);
+        Tm.sync();
+    } else if (state == RR_WALKERR && Tm.r == 0 && threadIdx.x == 0) {
+        atomicOr(A.status, BST_CARVE);
+    }
+}
+
+template <int MODE>
+__device__ __forceinline__ void route_tile(const BatchTile &T, const BatchArrays &A, BatchShm &sh, ClusterTeam &Tm,
+                                           unsigned char *smem)
 {
     const Grid g{T.nx, T.ny, MODE, MODE == 3 ? A.codes + T.off : nullptr};
     const int N = T.nx * T.ny;
     const long long o = T.off;
     const float *z = A.z + o;
-    tile_receivers<MODE>(g, T.dx, z, A.rcv + o, A.rec_ + o, A.grad + o);
-    tile_reroute<MODE>(g, T, A, z, sh);
+    tile_receivers<MODE>(g, T.dx, z, A.rcv + o, A.grad + o, Tm);
+    tile_reroute<MODE>(T, A, z, sh, Tm, smem);
     // accumulate: Q holds the seed (flowfields.py:272-292).  Tiles the front takes (modes 0-2,
     // 3 x 3 and more) are accumulated after this launch, all together
-    if (T.item0 >= 0) return;
+    if (T.item0 >= 0 || Tm.r != 0) return;
     tile_accumulate(N, A.rcv + o, A.Q + o, A.counts + o, A.dnr + 4 * o, A.dnr_ + 4 * o, A.ndnr + o, A.ndnr_ + o,
                     A.src + o, A.p_ + o, A.c_ + o, A.mark + o, A.rec__ + o, sh);
 }
@@ -705,122 +812,132 @@ struct GfParams {
     float *trace;      // optional, per tile: niter x (max|dh|, mean|dh|)
 };
 
-// max and sum of v over the block (max as unsigned bits: |x| >= 0, NaN above all)
-__device__ __forceinline__ void bmaxsum(float m, float sum, BatchShm &sh, float *om, float *os)
+// max and sum of v over the team (max as unsigned bits: |x| >= 0, NaN above all)
+__device__ __forceinline__ void bmaxsum(float m, float sum, BatchShm &sh, ClusterTeam &Tm, float *om, float *os)
 {
     unsigned mu = __float_as_uint(m);
     for (int o = 16; o; o >>= 1) {
         mu = max(mu, __shfl_xor_sync(0xffffffffu, mu, o));
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) { sh.ws[0] = 0; sh.ws[1] = 0; }
-    __syncthreads();
+    int *ws = team_at(sh.ws, Tm);
+    Tm.sync();
+    if (Tm.r == 0 && threadIdx.x == 0) { sh.ws[0] = 0; sh.ws[1] = 0; }
+    Tm.sync();
     if ((threadIdx.x & 31) == 0) {
-        atomicMax((unsigned *)&sh.ws[0], mu);
-        atomicAdd((float *)&sh.ws[1], sum);
+        atomicMax((unsigned *)&ws[0], mu);
+        atomicAdd((float *)&ws[1], sum);
     }
-    __syncthreads();
-    *om = __uint_as_float((unsigned)sh.ws[0]);
-    *os = __int_as_float(sh.ws[1]);
-    __syncthreads();
+    Tm.sync();
+    *om = __uint_as_float((unsigned)vload(ws));
+    *os = __int_as_float(vload(ws + 1));
+    Tm.sync();
 }
 
 template <int MODE>
-__device__ void gf_tile(const BatchTile &T, const BatchArrays &A, const GfParams &P, BatchShm &sh)
+__device__ __forceinline__ void gf_tile(const BatchTile &T, const BatchArrays &A, const GfParams &P, BatchShm &sh,
+                                        ClusterTeam &Tm, unsigned char *smem)
 {
     const Grid g{T.nx, T.ny, MODE, MODE == 3 ? A.codes + T.off : nullptr};
-    const int N = T.nx * T.ny;
+    const int N = T.nx * T.ny, nx = T.nx;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
     const long long o = T.off;
     float *zh = const_cast<float *>(A.z) + o, *h = P.h + o, *Q = A.Q + o;
     int32_t *rec = A.rcv + o;
     // scratch of the routing arrays, free once the reroute is done
-    int32_t *ra = A.rec_ + o, *rb = A.rec__ + o;
-    float *zs = A.zp + o, *zn = A.p_ + o;
+    int2 *fa = reinterpret_cast<int2 *>(A.dnr + 4 * o), *fb = fa + N;  // fill records {pointer, surface}
     float *w = reinterpret_cast<float *>(A.dnr_) + 4 * o;
-    uint8_t *issrc = A.isb + o;
     float *temp = reinterpret_cast<float *>(A.ndnr) + o;
     float *href = reinterpret_cast<float *>(A.c_) + o;
-    float *dh = reinterpret_cast<float *>(A.ndnr_) + o;
     const float dx = T.dx, dx2 = P.cst[4 * T.id], prec_dx2 = P.cst[4 * T.id + 1], manning = P.cst[4 * T.id + 2];
     const float thr = P.cst[4 * T.id + 3];
     const int nr = bceil_log2(N);
     int it = 0;
     float rmax = 0.f, rmean = 0.f;
     for (; it < P.niter; ++it) {
-        FOR_CELLS(i, N) href[i] = h[i];
-        tile_receivers<MODE>(g, dx, zh, rec, A.rec_ + o, nullptr);
-        tile_reroute<MODE>(g, T, A, zh, sh);
-        // fill_z_add_delta (fill_topo.py:99-125): rounds on snapshots of z_ and rec_
-        FOR_CELLS(i, N) {
-            zs[i] = zh[i];
-            ra[i] = rec[i];
+        tile_receivers<MODE>(g, dx, zh, rec, nullptr, Tm);
+        tile_reroute<MODE>(T, A, zh, sh, Tm, smem);
+        // fill_z_add_delta (fill_topo.py:99-125): rounds on snapshots of the records.  The
+        // surface that a self-pointing cell's followers compare with is its initial one,
+        // which is also its record's where it points to itself from the start (bit 31).
+        FOR_TEAM(i, N) {
+            const int r = rec[i];
+            fa[i] = make_int2(r == i ? (i | (int)0x80000000) : r, __float_as_int(zh[i]));
         }
-        __syncthreads();
-        float *a = zs, *b = zn;
-        int32_t *pa = ra, *pb = rb;
+        Tm.sync();
+        int2 *a = fa, *b = fb;
         for (int r = 0; r < nr; ++r) {
             const float inc = (float)(ldexp(1.0, r - 1) * (double)P.eps);
-            int ch = 0;
-            FOR_CELLS(i, N) {
-                const int q = pa[i];
-                const int qq = pa[q];
-                pb[i] = qq;
-                const float zi = a[i];
-                float zo = zi;
-                if (!(i == q || (zi > zh[q] && qq == q))) zo = fmaxf(zi, __fadd_rn(a[q], inc));
-                b[i] = zo;
-                ch |= qq != q || __float_as_uint(zo) != __float_as_uint(zi);
+            bool ch = false;
+            FOR_TEAM(i, N) {
+                const int2 s = a[i];
+                const int q = s.x & 0x7FFFFFFF;
+                int2 n = s;
+                if (q != i) {
+                    const int2 t = a[q];
+                    const int qq = t.x & 0x7FFFFFFF;
+                    const float zi = __int_as_float(s.y), zq = __int_as_float(t.y);
+                    n.x = qq;
+                    if (!(qq == q && zi > (t.x < 0 ? zq : zh[q]))) n.y = __float_as_int(fmaxf(zi, __fadd_rn(zq, inc)));
+                    ch |= n.x != s.x || n.y != s.y;
+                }
+                b[i] = n;
             }
-            const bool any = __syncthreads_or(ch);
-            float *t = a; a = b; b = t;
-            int32_t *u = pa; pa = pb; pb = u;
-            // a round that changed nothing is a fixed point of every later round (see k_fill_round)
+            const bool any = team_any(ch, sh, Tm);
+            int2 *t = a; a = b; b = t;
+            // a round that changed nothing is a fixed point of every later round
             if (!any) break;
         }
-        FOR_CELLS(i, N) {
-            const float zf = a[i];
-            h[i] = __fadd_rn(h[i], __fsub_rn(zf, zh[i]));
+        FOR_TEAM(i, N) {
+            const float zf = __int_as_float(a[i].y), hi = h[i], zi = zh[i];
+            href[i] = hi;
+            h[i] = __fadd_rn(hi, __fsub_rn(zf, zi));
             zh[i] = zf;
         }
-        __syncthreads();
-        // diffusion: weights once, then 5 gather sweeps (Q <-> temp), ending in Q
-        FOR_CELLS(i, N) {
-            const int row = i / g.nx, col = i - row * g.nx;
-            if (leave<MODE>(g, i)) { issrc[i] = 0; continue; }
-            const float zi = zh[i];
-            float sk[4];
+        Tm.sync();
+        // diffusion: a cell's outgoing weights once (-1: not a source), then 5 gather sweeps
+        FOR_TEAM(i, N) {
+            int row, col, js[4];
+            divmod_nx(i, nx, mnx, row, col);
+            float sk[4] = {0.f, 0.f, 0.f, 0.f};
             float sums = 0.f;
-            int js[4];
-            neighbours4<MODE>(g, i, row, col, js);
+            if (!can_leave<MODE>(g, i, row, col)) {
+                const float zi = zh[i];
+                neighbours4<MODE>(g, i, row, col, js);
+                float zn[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                sk[k] = (js[k] != -1) ? fmaxf(0.f, __fdiv_rn(__fsub_rn(zi, zh[js[k]]), dx)) : 0.f;
-                sums = __fadd_rn(sums, sk[k]);
+                for (int k = 0; k < 4; ++k) zn[k] = js[k] != -1 ? zh[js[k]] : zi;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    sk[k] = (js[k] != -1) ? fmaxf(0.f, __fdiv_rn(__fsub_rn(zi, zn[k]), dx)) : 0.f;
+                    sums = __fadd_rn(sums, sk[k]);
+                }
             }
-            if (sums == 0.f) { issrc[i] = 0; continue; }
-            issrc[i] = 1;
+            const bool src = !(sums == 0.f);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) w[(size_t)k * N + i] = __fdiv_rn(sk[k], sums);
+            for (int k = 0; k < 4; ++k) w[(size_t)k * N + i] = src ? __fdiv_rn(sk[k], sums) : -1.f;
         }
-        __syncthreads();
+        Tm.sync();
         float *qa = Q, *qb = temp;
         for (int sw = 0; sw < 5; ++sw) {
-            FOR_CELLS(j, N) {
-                const int row = j / g.nx, col = j - row * g.nx;
+            FOR_TEAM(j, N) {
+                int row, col;
+                divmod_nx(j, nx, mnx, row, col);
                 float acc = prec_dx2;
-                if (MODE != 3 && row > 0 && row < g.ny - 1 && col > 0 && col < g.nx - 1) {
-                    const int nx = g.nx;
-                    if (issrc[j - nx]) acc = __fadd_rn(acc, __fmul_rn(w[3 * (size_t)N + j - nx], qa[j - nx]));
-                    if (issrc[j - 1]) acc = __fadd_rn(acc, __fmul_rn(w[2 * (size_t)N + j - 1], qa[j - 1]));
-                    if (issrc[j + 1]) acc = __fadd_rn(acc, __fmul_rn(w[(size_t)N + j + 1], qa[j + 1]));
-                    if (issrc[j + nx]) acc = __fadd_rn(acc, __fmul_rn(w[j + nx], qa[j + nx]));
+                if (MODE != 3 && row > 0 && row < g.ny - 1 && col > 0 && col < nx - 1) {
+                    const float wt = w[3 * (size_t)N + j - nx], wl = w[2 * (size_t)N + j - 1], wr = w[(size_t)N + j + 1],
+                                wb = w[j + nx];
+                    const float qt = qa[j - nx], ql = qa[j - 1], qr = qa[j + 1], qd = qa[j + nx];
+                    if (!(wt < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wt, qt));
+                    if (!(wl < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wl, ql));
+                    if (!(wr < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wr, qr));
+                    if (!(wb < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wb, qd));
                 } else {
                     int c[8];
                     const int n = donor_candidates(g, j, row, col, c);
                     for (int q = 0; q < n; ++q) {
                         const int i = c[q];
-                        if (!issrc[i]) continue;
+                        if (w[i] < 0.f) continue;
                         const float qi = qa[i];
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
@@ -829,106 +946,115 @@ __device__ void gf_tile(const BatchTile &T, const BatchArrays &A, const GfParams
                 }
                 qb[j] = acc;
             }
-            __syncthreads();
+            Tm.sync();
             float *t = qa; qa = qb; qb = t;
         }
-        if (qa != Q) {
-            FOR_CELLS(j, N) Q[j] = qa[j];
-            __syncthreads();
-        }
-        // Manning update, two loops as in the reference (h receives tdh twice)
-        FOR_CELLS(i, N) {
+        // Manning update; slopes from the fill's records, which hold the filled surface (h
+        // receives tdh twice, gf_hydrodynamics.py:127-129); the last sweep's result into Q
+        float m = 0.f, sum = 0.f;
+        FOR_TEAM(i, N) {
             const int r = rec[i];
+            const float zi = __int_as_float(a[i].y), qi = qa[i], hi = h[i];
             float tS = P.edgesw;
-            if (r != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zh[i], zh[r]), dx), 1e-4f);
-            float Qo = __fmul_rn(dx, (float)pow((double)h[i], (double)(5.0f / 3.0f)));
+            if (r != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zi, __int_as_float(a[r].y)), dx), 1e-4f);
+            Q[i] = qi;
+            float Qo = __fmul_rn(dx, pow53(hi));
             Qo = __fdiv_rn(Qo, manning);
             Qo = __fmul_rn(Qo, __fsqrt_rn(tS));
-            float tdh = __fdiv_rn(__fsub_rn(Q[i], Qo), dx2);
+            float tdh = __fdiv_rn(__fsub_rn(qi, Qo), dx2);
             tdh = __fmul_rn(tdh, P.dt);
-            const float h1 = __fadd_rn(h[i], tdh);
-            h[i] = h1;
+            const float h1 = __fadd_rn(hi, tdh);
             if (h1 < 0.f) tdh = __fadd_rn(tdh, h1);
-            dh[i] = tdh;
-        }
-        __syncthreads();
-        float m = 0.f, sum = 0.f;
-        FOR_CELLS(i, N) {
-            const float d = dh[i];
-            const float hn = __fadd_rn(h[i], d);
+            const float hn = __fadd_rn(h1, tdh);
             h[i] = hn;
-            zh[i] = __fadd_rn(zh[i], d);
+            zh[i] = __fadd_rn(zi, tdh);
             const float e = fabsf(__fsub_rn(hn, href[i]));
             m = __uint_as_float(max(__float_as_uint(m), __float_as_uint(e)));
             sum += e;
         }
-        bmaxsum(m, sum, sh, &rmax, &rmean);
+        bmaxsum(m, sum, sh, Tm, &rmax, &rmean);
         rmean /= (float)N;
-        if (P.trace && threadIdx.x == 0) {
+        if (P.trace && Tm.r == 0 && threadIdx.x == 0) {
             P.trace[((size_t)T.id * P.niter + it) * 2] = rmax;
             P.trace[((size_t)T.id * P.niter + it) * 2 + 1] = rmean;
         }
         if ((P.crit == 0 && rmax < thr) || (P.crit == 1 && rmean < thr)) { ++it; break; }
     }
-    if (threadIdx.x == 0) {
+    if (Tm.r == 0 && threadIdx.x == 0) {
         P.iters[T.id] = it;
         P.res[2 * T.id] = rmax;
         P.res[2 * T.id + 1] = rmean;
     }
-    __syncthreads();
 }
 
-// Persistent: each CTA takes the next tile (largest first) until the queue is empty.
+// The next tile of the queue for the whole team (largest first), or -1.
+__device__ __forceinline__ int next_tile(int ntiles, int *queue, BatchShm &sh, ClusterTeam &Tm)
+{
+    Tm.sync();  // the previous tile is done, and its number read
+    if (Tm.r == 0 && threadIdx.x == 0) sh.cur = atomicAdd(queue, 1);
+    Tm.sync();
+    const int k = *(volatile int *)team_at(&sh.cur, Tm);
+    Tm.sync();
+    return k < ntiles ? k : -1;
+}
+
+__device__ __forceinline__ ClusterTeam cluster_team()
+{
+    ClusterTeam Tm;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(Tm.r));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(Tm.n));
+    return Tm;
+}
+
+// Persistent: each team takes the next tile until the queue is empty.
 __global__ void __launch_bounds__(1024) k_batch_route(int ntiles, BatchArrays A)
 {
+    extern __shared__ __align__(16) unsigned char batch_smem[];
     __shared__ BatchShm sh;
+    ClusterTeam Tm = cluster_team();
+    if (threadIdx.x == 0) sh.any[0] = sh.any[1] = sh.any[2] = sh.any_r = 0;
     for (;;) {
-        if (threadIdx.x == 0) sh.cur = atomicAdd(A.queue, 1);
-        __syncthreads();
-        const int k = sh.cur;
-        __syncthreads();
-        if (k >= ntiles) return;
+        const int k = next_tile(ntiles, A.queue, sh, Tm);
+        if (k < 0) return;
         const BatchTile T = A.tiles[k];
         switch (T.mode) {
-        case 0: route_tile<0>(T, A, sh); break;
-        case 1: route_tile<1>(T, A, sh); break;
-        case 2: route_tile<2>(T, A, sh); break;
+        case 0: route_tile<0>(T, A, sh, Tm, batch_smem); break;
+        case 1: route_tile<1>(T, A, sh, Tm, batch_smem); break;
+        case 2: route_tile<2>(T, A, sh, Tm, batch_smem); break;
         case 3:
-            if (A.codes) route_tile<3>(T, A, sh);
+            if (A.codes) route_tile<3>(T, A, sh, Tm, batch_smem);
             else if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
             break;
         default:
             if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
             break;
         }
-        __syncthreads();
     }
 }
 
-// Persistent GraphFlood: each CTA runs whole tiles to their stop, largest first.
+// Persistent GraphFlood: each team runs whole tiles to their stop, largest first.
 __global__ void __launch_bounds__(1024) k_batch_graphflood(int ntiles, BatchArrays A, GfParams P)
 {
+    extern __shared__ __align__(16) unsigned char batch_smem[];
     __shared__ BatchShm sh;
+    ClusterTeam Tm = cluster_team();
+    if (threadIdx.x == 0) sh.any[0] = sh.any[1] = sh.any[2] = sh.any_r = 0;
     for (;;) {
-        if (threadIdx.x == 0) sh.cur = atomicAdd(A.queue, 1);
-        __syncthreads();
-        const int k = sh.cur;
-        __syncthreads();
-        if (k >= ntiles) return;
+        const int k = next_tile(ntiles, A.queue, sh, Tm);
+        if (k < 0) return;
         const BatchTile T = A.tiles[k];
         switch (T.mode) {
-        case 0: gf_tile<0>(T, A, P, sh); break;
-        case 1: gf_tile<1>(T, A, P, sh); break;
-        case 2: gf_tile<2>(T, A, P, sh); break;
+        case 0: gf_tile<0>(T, A, P, sh, Tm, batch_smem); break;
+        case 1: gf_tile<1>(T, A, P, sh, Tm, batch_smem); break;
+        case 2: gf_tile<2>(T, A, P, sh, Tm, batch_smem); break;
         case 3:
-            if (A.codes) gf_tile<3>(T, A, P, sh);
+            if (A.codes) gf_tile<3>(T, A, P, sh, Tm, batch_smem);
             else if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
             break;
         default:
             if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
             break;
         }
-        __syncthreads();
     }
 }
 
@@ -949,8 +1075,8 @@ struct BatchWs {
 };
 
 // Work items of the accumulation front: a tile nx x ny has ceil(nx/64) ceil(ny/24) <=
-// nx ny / 3 + 1 of them (tiles of at least 3 x 3).
-static size_t batch_item_cap(long long total, int ntiles) { return (size_t)(total / 3 + ntiles); }
+// nx ny / 37 + 1 of them (tiles of at least 3 x 3; 3 x (24 k + 1) comes closest).
+static size_t batch_item_cap(long long total, int ntiles) { return (size_t)(total / 37 + ntiles); }
 
 static BatchWs carve_batch(void *ws, size_t wsb, long long total, int ntiles, size_t *used = nullptr)
 {
@@ -1005,6 +1131,46 @@ extern "C" size_t pff_batch_workspace_bytes(long long total_cells, int ntiles)
 }
 
 namespace pff {
+// Blocks per tile (a cluster).  More blocks shorten the largest tile's chain, which bounds a
+// batch whose tiles differ much, and fill the GPU when tiles are few; each costs a share of
+// cluster barriers.
+static int batch_team(long long total, int ntiles, int slots)
+{
+    const long long avg = total / ntiles;
+    int t = 1;
+    while (t < 8 && (long long)ntiles * t * 2 <= slots && avg >= 2048LL * t) t *= 2;
+    if (avg >= 65536) t = std::max(t, 4);
+    return t;
+}
+
+template <class K, class... Args>
+static int launch_batch(K kernel, int threads, int ctas_per_sm, long long total, int ntiles, cudaStream_t st, Args... args)
+{
+    int dev = 0, nsm = 148, occ = 1;
+    PFF_CUDA(cudaGetDevice(&dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const size_t smem = (size_t)(threads / TILE_THREADS) * LOOP_GROUP_BYTES;
+    PFF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM));
+    PFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem));
+    if (ctas_per_sm < 1) ctas_per_sm = 1;
+    if (ctas_per_sm > occ) ctas_per_sm = occ > 0 ? occ : 1;
+    const int team = batch_team(total, ntiles, nsm * ctas_per_sm);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(std::min(std::max(nsm * ctas_per_sm / team, 1), ntiles) * team));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)team;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    PFF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    count_launch();
+    return PFF_OK;
+}
+
 static int batch_check(long long total, int ntiles, void *ws, size_t wsb, const char *who)
 {
     if (ntiles <= 0 || total <= 0) {
@@ -1099,12 +1265,6 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
         set_error("pff_batch_route: threads must be 256, 512 or 1024 (got %d)", threads);
         return PFF_ERR_ARG;
     }
-    int dev = 0, nsm = 148, occ = 1;
-    PFF_CUDA(cudaGetDevice(&dev));
-    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_route, threads, 0));
-    if (ctas_per_sm < 1) ctas_per_sm = 1;
-    if (ctas_per_sm > occ) ctas_per_sm = occ > 0 ? occ : 1;
     BatchWs w = carve_batch(workspace, workspace_bytes, total_cells, ntiles);
     BatchArrays A = w.A;
     A.z = z;
@@ -1114,9 +1274,8 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
     A.Q = Q;
     A.counts = counts;
     cudaStream_t st = S(stream);
-    const int grid = std::min(nsm * ctas_per_sm, ntiles);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
-    { k_batch_route<<<grid, threads, 0, st>>>(ntiles, A); count_launch(); }
+    PFF_TRY(launch_batch(k_batch_route, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A));
     if (total_cells < (1LL << 31)) {
         BatchAcc b{};
         b.rcv = receivers; b.Q = Q; b.counts = counts;
@@ -1163,12 +1322,6 @@ extern "C" int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, f
         set_error("pff_batch_graphflood: threads must be 256, 512 or 1024 (got %d)", threads);
         return PFF_ERR_ARG;
     }
-    int dev = 0, nsm = 148, occ = 1;
-    PFF_CUDA(cudaGetDevice(&dev));
-    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_graphflood, threads, 0));
-    if (ctas_per_sm < 1) ctas_per_sm = 1;
-    if (ctas_per_sm > occ) ctas_per_sm = occ > 0 ? occ : 1;
     BatchWs w = carve_batch(workspace, workspace_bytes, total_cells, ntiles);
     BatchArrays A = w.A;
     A.z = zh;
@@ -1179,8 +1332,7 @@ extern "C" int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, f
     A.counts = nullptr;
     GfParams P{tile_consts, edgesw, dt, 1e-3f, niter, crit, h, iters, residuals, trace};
     cudaStream_t st = S(stream);
-    const int grid = std::min(nsm * ctas_per_sm, ntiles);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
-    { k_batch_graphflood<<<grid, threads, 0, st>>>(ntiles, A, P); count_launch(); }
+    PFF_TRY(launch_batch(k_batch_graphflood, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A, P));
     return check_cuda("pff_batch_graphflood");
 }

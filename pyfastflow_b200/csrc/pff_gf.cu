@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include "pff_internal.h"
+#include "pff_pow.cuh"
 #include "pff_div.cuh"
 
 namespace pff {
@@ -430,7 +431,6 @@ static int l_diffuse_fused(const float *zh, float *Q, float *temp, int nsweeps, 
 // h^(5/3) with the exponent rounded to f32 (Taichi folds 5./3. to an f32
 // constant), evaluated in double and rounded once: the correctly rounded f32
 // power.  Both the oracle and this kernel use this definition.
-__device__ __forceinline__ float pow53(float h) { return (float)pow((double)h, (double)(5.0f / 3.0f)); }
 
 __global__ void __launch_bounds__(256) k_core1(float *h, const float *__restrict__ zh, float *dh,
                                                const int32_t *__restrict__ rec, const float *__restrict__ Q, int N,
@@ -803,4 +803,38 @@ extern "C" int pff_abs_diff_stats(const float *a, const float *b, int N, float *
     const int blocks = std::min(div_up(N, 256), 148 * 8);
     { k_abs_diff_stats<<<blocks, 256, 0, S(stream)>>>(a, b, N, out); count_launch(); }
     return check_cuda("pff_abs_diff_stats");
+}
+
+// pow53 against the full double-precision power on every float whose bits lie in [lo, hi]
+__global__ void k_pow53_selfcheck(unsigned lo, unsigned hi, unsigned long long *bad)
+{
+    unsigned long long nb = 0;
+    for (unsigned long long u = lo + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; u <= hi;
+         u += (unsigned long long)gridDim.x * blockDim.x) {
+        const float h = __uint_as_float((unsigned)u);
+        const float a = pow53(h), b = pow53_full(h);
+        nb += __float_as_uint(a) != __float_as_uint(b) && !(a != a && b != b);
+    }
+    if (nb) atomicAdd(bad, nb);
+}
+
+extern "C" int pff_pow53_selfcheck(uint32_t lo, uint32_t hi, long long *mismatches)
+{
+    clear_error();
+    if (!mismatches || lo > hi) {
+        set_error("pff_pow53_selfcheck: bad arguments");
+        return PFF_ERR_ARG;
+    }
+    unsigned long long *d = nullptr, bad = 0;
+    PFF_CUDA(cudaMalloc(&d, sizeof(unsigned long long)));
+    cudaMemset(d, 0, sizeof(unsigned long long));
+    k_pow53_selfcheck<<<148 * 8, 256>>>(lo, hi, d);
+    const cudaError_t e = cudaMemcpy(&bad, d, sizeof(bad), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) {
+        set_error("pff_pow53_selfcheck: %s", cudaGetErrorString(e));
+        return PFF_ERR_CUDA;
+    }
+    *mismatches = (long long)bad;
+    return PFF_OK;
 }

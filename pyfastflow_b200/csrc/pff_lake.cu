@@ -15,11 +15,10 @@
 #include <mutex>
 #include <cub/block/block_scan.cuh>
 #include "pff_internal.h"
+#include "pff_lake_loop.cuh"
 #include "pff_tiles.cuh"
 
 namespace pff {
-
-__device__ __forceinline__ long long invalid_key() { return pack_key(1e8f, 42); }  // lakeflow.py:127
 
 __device__ __forceinline__ int warp_agg_inc(int *ctr, bool pred)
 {
@@ -312,140 +311,6 @@ __device__ __forceinline__ void block_append(bool pred, int val, int *list, int 
     __syncthreads();
 }
 
-// Exact quotient and remainder of n / d for 0 <= n < 2^31 and d >= 2 without the
-// integer divide sequence: with m = floor(2^32 / d) or m = floor((2^32 - 1) / d) (one
-// less only when d divides 2^32), q = umulhi(n, m) is floor(n / d) or one less
-// (n m / 2^32 > n / d - 2 n / 2^32 > n / d - 1), and one correction of the remainder
-// fixes it.
-__device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int &r)
-{
-    q = (int)__umulhi((unsigned)n, m);
-    r = n - q * d;
-    if (r >= d) { ++q; r -= d; }
-}
-
-// Tile-local indices q of a thread's receivers r (its cells: rows ly0 + 4 k of column lx of
-// the w x h tile at (row0, col0), local index t + 256 k, grid index i0 + 4 k nx; r < 0: no
-// cell): the receiver's, or the cell's own where it is a root or its receiver lies outside.
-__device__ __forceinline__ void tile_locals(const int (&r)[TILE_PER_THREAD], int (&q)[TILE_PER_THREAD], int i0, int t,
-                                            int lx, int ly0, int row0, int col0, int w, int h, int nx, unsigned mnx)
-{
-    static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
-    int far = 0;  // receivers that are not the grid neighbour (wrapped edges, or no D4 link)
-#pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = t + k * TILE_THREADS, d = r[k] - (i0 + 4 * k * nx);
-        const int sx = (d == 1) - (d == -1), sy = (d == nx) - (d == -nx);
-        const bool in = r[k] >= 0 && (unsigned)(lx + sx) < (unsigned)w && (unsigned)(ly0 + 4 * k + sy) < (unsigned)h;
-        q[k] = in ? c + sx + TILE_W * sy : c;
-        if (r[k] >= 0 && d != 0 && (sx | sy) == 0) far |= 1 << k;
-    }
-    if (!far) return;
-#pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        if (!(far >> k & 1)) continue;
-        int rr, rc;
-        divmod_nx(r[k], nx, mnx, rr, rc);
-        rr -= row0;
-        rc -= col0;
-        if (rr >= 0 && rr < h && rc >= 0 && rc < w) q[k] = rr * TILE_W + rc;
-    }
-}
-
-// A thread's 8 pointers q to their tile terminals.  Four rounds of pointer doubling in p
-// (16-bit local pointers; a pointer then spans 16 cells or ends), then every pointer is
-// followed on its own over the settled array, without barriers: most paths in a tile
-// are shorter than 64 cells.  At most 2048 / 16 steps (a cycle ends there too).
-// Bound by the shared-memory gathers' latency and bank conflicts.
-template <class Sync>
-__device__ __forceinline__ void tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD], int t, Sync sync)
-{
-    int qq[TILE_PER_THREAD];
-#pragma unroll 1
-    for (int round = 0; round < 4; ++round) {
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k)
-            if (qq[k] != q[k]) {
-                p[t + k * TILE_THREADS] = (uint16_t)qq[k];
-                q[k] = qq[k];
-            }
-        sync();
-    }
-#pragma unroll 1
-    for (int step = 0; step < TILE_CELLS / 16 + 1; ++step) {
-        bool ch = false;
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) qq[k] = p[q[k]];
-#pragma unroll
-        for (int k = 0; k < TILE_PER_THREAD; ++k) {
-            ch |= qq[k] != q[k];
-            q[k] = qq[k];
-        }
-        if (!ch) break;
-    }
-}
-
-// Tile terminals of one tile by one block: J[i] = the receiver of the last in-tile cell of
-// i's path (the root itself, or the first cell past the tile).  info[0] pits (pits ==
-// nullptr: no pit list), info[2] set if some exit target is not a tile-border cell
-// (receivers that are not D4 neighbours).  copy: also rec_copy = rec.
-//
-template <int MODE>
-__device__ void tile_terminal_one(const int32_t *__restrict__ rec, int32_t *J, int32_t *R, int *pits, int *info,
-                                  const Grid &g, int tx, int ty, uint16_t *p, int *rv, int32_t *rec_copy)
-{
-    const int nx = g.nx, ny = g.ny;
-    const unsigned mnx = 0xffffffffu / (unsigned)nx;
-    const int col0 = tx * TILE_W, row0 = ty * TILE_H;
-    const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
-    const int lx = threadIdx.x & (TILE_W - 1), ly0 = threadIdx.x / TILE_W;
-    const int i0 = (row0 + ly0) * nx + col0 + lx;
-    int r[TILE_PER_THREAD], q[TILE_PER_THREAD];
-#pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k) r[k] = (lx < w && ly0 + 4 * k < h) ? rec[i0 + 4 * k * nx] : -1;
-    tile_locals(r, q, i0, threadIdx.x, lx, ly0, row0, col0, w, h, nx, mnx);
-    int term = 0;  // cells that are terminals
-#pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = threadIdx.x + k * TILE_THREADS;
-        p[c] = (uint16_t)q[k];
-        rv[c] = r[k];
-        if (q[k] == c) term |= 1 << k;
-        if (rec_copy && r[k] >= 0) rec_copy[i0 + 4 * k * nx] = r[k];
-    }
-    __syncthreads();
-    tile_jump(p, q, threadIdx.x, []() { __syncthreads(); });
-    bool nonlocal = false;
-#pragma unroll
-    for (int k = 0; k < TILE_PER_THREAD; ++k) {
-        const int c = threadIdx.x + k * TILE_THREADS, ly = ly0 + 4 * k, i = i0 + 4 * k * nx;
-        bool pit = false;
-        if (r[k] >= 0) {
-            const int j = rv[q[k]];
-            J[i] = j;
-            if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || r[k] == i) R[i] = j;
-            if ((term >> k & 1) && r[k] != i) {  // an exit
-                int rr, rc;
-                divmod_nx(r[k], nx, mnx, rr, rc);
-                if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
-            }
-            if (p[q[k]] != q[k] || (q[k] == c && !(term >> k & 1))) nonlocal = true;  // a cycle in the tile
-            pit = pits && r[k] == i && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, pit);
-        if (m) {
-            const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(info, __popc(m));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (pit) pits[base + __popc(m & ((1u << lane) - 1u))] = i;
-        }
-    }
-    if (nonlocal) info[2] = 1;
-}
-
 // Tile terminals of the tiles listed in tiles[0 .. *ntiles) (one block per tile,
 // the grid strides over the list; the count is read on the device), or of every
 // tile (tiles == NULL, a 2-D grid of tiles).
@@ -457,13 +322,15 @@ __global__ void __launch_bounds__(TILE_THREADS) k_tile_terminal(const int32_t *_
     __shared__ uint16_t p[TILE_CELLS];
     __shared__ int rv[TILE_CELLS];
     if (!tiles) {
-        tile_terminal_one<MODE>(rec, J, R, pits, info, g, blockIdx.x, blockIdx.y, p, rv, rec_copy);
+        tile_terminal_one<MODE>(rec, J, R, pits, info, g, blockIdx.x, blockIdx.y, p, rv, rec_copy, threadIdx.x,
+                                []() { __syncthreads(); });
         return;
     }
     const int ntx = (g.nx + TILE_W - 1) / TILE_W, n = *ntiles;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int t = tiles[k];
-        tile_terminal_one<MODE>(rec, J, R, pits, info, g, t % ntx, t / ntx, p, rv, nullptr);
+        tile_terminal_one<MODE>(rec, J, R, pits, info, g, t % ntx, t / ntx, p, rv, nullptr, threadIdx.x,
+                                []() { __syncthreads(); });
         __syncthreads();  // p and rv are reused by the next tile
     }
 }
@@ -566,54 +433,6 @@ __global__ void k_basin_reset_list(long long *saddle, long long *outlet, int32_t
 // in a per-warp shared buffer, flushed with one atomic per strip.
 constexpr int SAD_ROWS = 32;
 constexpr int SAD_AHEAD = 4;  // rows loaded per group (SAD_ROWS is a multiple)
-
-// The saddle candidate of a border cell goes to atomicMin(saddle + bi, key) (pass 2).
-// In the border-list pass, where most lanes hold a candidate and neighbouring list
-// entries share basins, saddle_min_warp makes that one atomic per basin per warp
-// (in the N-wide strip pass it cost more than it saved): the lanes holding a
-// candidate group by basin (match.any), take the group's minimum key as two 32-bit
-// reductions (the key's signed order is the unsigned order of key ^ 2^63: high
-// words first, then the low words of the lanes that hold the minimal high word),
-// and the group's first lane applies it.  The minimum over the same keys: the
-// saddle is the one the per-cell atomics produce.
-__device__ __forceinline__ void saddle_min_warp(long long *saddle, int bi, long long key, bool has)
-{
-    const unsigned act = __ballot_sync(0xffffffffu, has);
-    if (!has) return;
-    const unsigned peers = __match_any_sync(act, bi);
-    const unsigned long long u = (unsigned long long)key ^ 0x8000000000000000ull;
-    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
-    const unsigned mh = __reduce_min_sync(peers, hi);
-    const unsigned ml = __reduce_min_sync(peers, hi == mh ? lo : 0xffffffffu);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1)
-        atomicMin(saddle + bi, (long long)((((unsigned long long)mh << 32) | ml) ^ 0x8000000000000000ull));
-}
-
-// Passes 1-2 for one cell; key: the lowest (z', neighbour basin) of a border cell (a
-// saddle candidate if below the invalid key).  Returns 0 for a cell off every
-// border, 1 for a border cell of the outlet basin 0, 2 for a border cell of a pit basin.
-__device__ __forceinline__ int saddle_cell(int i, int bi, float zi, const int (&jn)[4], const int (&bn)[4],
-                                           const float (&zn)[4], uint8_t *is_border, float *zp, long long &key)
-{
-    bool border = false;
-    float zmin = 1e9f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (jn[k] != -1 && bn[k] != bi) { border = true; zmin = fminf(zmin, zn[k]); }
-    is_border[i] = border;
-    const float zpi = border ? fmaxf(zi, zmin) : 1e9f;
-    zp[i] = zpi;
-    if (!border) return 0;
-    long long res = 0x7fffffffffffffffll;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (jn[k] == -1 || bn[k] == bi) continue;
-        const long long c = pack_key(zpi, bn[k]);
-        res = c < res ? c : res;
-    }
-    key = res;
-    return bi != 0 ? 2 : 1;
-}
 
 template <int MODE>
 __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restrict__ bid, uint8_t *is_border,
@@ -1523,11 +1342,42 @@ __global__ void k_relabel_check(const int32_t *__restrict__ fin, const long long
     }
 }
 
-}  // namespace pff
+// ---- the device-driven loop's kernels ------------------------------------------
 
-#include "pff_lake_loop.cuh"
+// the loop's final state for the host (see RR_*)
+__device__ __forceinline__ void loop_report(const LoopArgs &A, int it, int outer, int n_outer, int state)
+{
+    const int c[4] = {it, outer, n_outer, state};
+    for (int k = 0; k < 4; ++k) {
+        A.ctl[k] = c[k];
+        ((volatile int *)A.ctl_out)[k] = c[k];
+    }
+    __threadfence_system();
+}
 
-namespace pff {
+template <int MODE>
+__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, int32_t *R)
+{
+    __shared__ int dead;
+    if (threadIdx.x == 0) dead = 0;
+    GridTeam T{GridBar{A.bar + 8, 0}, &dead};
+    __syncthreads();
+    reroute_labels<MODE, false>(A, R, T);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
+{
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    __shared__ int dead;
+    if (threadIdx.x == 0) dead = 0;
+    GridTeam T{GridBar{A.bar, 0}, &dead};
+    __syncthreads();
+    int it = 0, outer = 0, n_outer = 0;
+    const int state = reroute_loop<MODE, false>(A, T, loop_smem, it, outer, n_outer);
+    // block 0's first thread reports; a block whose barrier gave up says so whoever it is
+    if (threadIdx.x == 0 && (blockIdx.x == 0 || state == RR_BOUND)) loop_report(A, it, outer, n_outer, state);
+}
 
 // ---- launchers ---------------------------------------------------------------
 
@@ -1934,10 +1784,7 @@ template <int MODE>
 static void l_loop(const LoopArgs &A, int32_t *R, int blocks, int *rc, cudaStream_t st)
 {
     LoopArgs a = A;
-    const int ntx = div_up(a.g.nx, TILE_W);
-    long long nslots = (long long)ntx * div_up(a.g.ny, TILE_H) * BORDER_SLOTS;
-    int *flags = a.bar + 16;
-    void *largs[] = {&a, &R, &nslots, &flags};
+    void *largs[] = {&a, &R};
     cudaError_t e = cudaLaunchCooperativeKernel((void *)k_reroute_labels<MODE>, blocks, LOOP_THREADS, largs, 0, st);
     if (e == cudaSuccess) {
         count_launch();

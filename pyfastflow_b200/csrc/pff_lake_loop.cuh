@@ -1,5 +1,5 @@
 // The carve reroute's outer loop (lakeflow.py:498-538) as one persistent cooperative
-// kernel.  Included by pff_lake.cu, whose helpers it uses.
+// kernel, and the same loop for the tiles of a ragged batch (pff_batch.cu).
 //
 // What bounds it: latency.  One outer iteration is about ten dependent steps over
 // lists (border cells, pits, path segments, touched tiles) that shrink by 2-3x per
@@ -17,9 +17,204 @@
 // One block of 1024 threads per SM: the barrier's cost grows with the number of
 // blocks, and 32 warps hide the gathers of the list steps.
 #pragma once
+#include "pff_common.cuh"
 #include "pff_coop.cuh"
+#include "pff_tiles.cuh"
 
 namespace pff {
+
+__device__ __forceinline__ long long invalid_key() { return pack_key(1e8f, 42); }  // lakeflow.py:127
+
+
+// Exact quotient and remainder of n / d for 0 <= n < 2^31 and d >= 2 without the
+// integer divide sequence: with m = floor(2^32 / d) or m = floor((2^32 - 1) / d) (one
+// less only when d divides 2^32), q = umulhi(n, m) is floor(n / d) or one less
+// (n m / 2^32 > n / d - 2 n / 2^32 > n / d - 1), and one correction of the remainder
+// fixes it.
+__device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int &r)
+{
+    q = (int)__umulhi((unsigned)n, m);
+    r = n - q * d;
+    if (r >= d) { ++q; r -= d; }
+}
+
+// Tile-local indices q of a thread's receivers r (its cells: rows ly0 + 4 k of column lx of
+// the w x h tile at (row0, col0), local index t + 256 k, grid index i0 + 4 k nx; r < 0: no
+// cell): the receiver's, or the cell's own where it is a root or its receiver lies outside.
+__device__ __forceinline__ void tile_locals(const int (&r)[TILE_PER_THREAD], int (&q)[TILE_PER_THREAD], int i0, int t,
+                                            int lx, int ly0, int row0, int col0, int w, int h, int nx, unsigned mnx)
+{
+    static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
+    int far = 0;  // receivers that are not the grid neighbour (wrapped edges, or no D4 link)
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS, d = r[k] - (i0 + 4 * k * nx);
+        const int sx = (d == 1) - (d == -1), sy = (d == nx) - (d == -nx);
+        const bool in = r[k] >= 0 && (unsigned)(lx + sx) < (unsigned)w && (unsigned)(ly0 + 4 * k + sy) < (unsigned)h;
+        q[k] = in ? c + sx + TILE_W * sy : c;
+        if (r[k] >= 0 && d != 0 && (sx | sy) == 0) far |= 1 << k;
+    }
+    if (!far) return;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        if (!(far >> k & 1)) continue;
+        int rr, rc;
+        divmod_nx(r[k], nx, mnx, rr, rc);
+        rr -= row0;
+        rc -= col0;
+        if (rr >= 0 && rr < h && rc >= 0 && rc < w) q[k] = rr * TILE_W + rc;
+    }
+}
+
+// A thread's 8 pointers q to their tile terminals.  Four rounds of pointer doubling in p
+// (16-bit local pointers; a pointer then spans 16 cells or ends), then every pointer is
+// followed on its own over the settled array, without barriers: most paths in a tile
+// are shorter than 64 cells.  At most 2048 / 16 steps (a cycle ends there too).
+// Bound by the shared-memory gathers' latency and bank conflicts.
+template <class Sync>
+__device__ __forceinline__ void tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD], int t, Sync sync)
+{
+    int qq[TILE_PER_THREAD];
+    unsigned act = (1u << TILE_PER_THREAD) - 1;  // pointers not known to be terminals
+#pragma unroll 1
+    for (int round = 0; round < 4; ++round) {
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (act >> k & 1) qq[k] = p[q[k]];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (act >> k & 1) {
+                if (qq[k] != q[k]) {
+                    p[t + k * TILE_THREADS] = (uint16_t)qq[k];
+                    q[k] = qq[k];
+                } else {
+                    act &= ~(1u << k);
+                }
+            }
+        sync();
+    }
+#pragma unroll 1
+    for (int step = 0; act && step < TILE_CELLS / 16 + 1; ++step) {
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (act >> k & 1) qq[k] = p[q[k]];
+#pragma unroll
+        for (int k = 0; k < TILE_PER_THREAD; ++k)
+            if (act >> k & 1) {
+                if (qq[k] == q[k]) act &= ~(1u << k);
+                q[k] = qq[k];
+            }
+    }
+}
+
+// Tile terminals of one tile by a group of 256 threads (t: thread of the group): J[i] = the receiver of the last in-tile cell of
+// i's path (the root itself, or the first cell past the tile).  info[0] pits (pits ==
+// nullptr: no pit list), info[2] set if some exit target is not a tile-border cell
+// (receivers that are not D4 neighbours).  copy: also rec_copy = rec.
+//
+template <int MODE, class Sync>
+__device__ __forceinline__ void tile_terminal_one(const int32_t *rec, int32_t *J, int32_t *R, int *pits, int *info,
+                                                  const Grid &g, int tx, int ty, uint16_t *p, int *rv,
+                                                  int32_t *rec_copy, int t, Sync sync)
+{
+    const int nx = g.nx, ny = g.ny;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const int col0 = tx * TILE_W, row0 = ty * TILE_H;
+    const int w = min(TILE_W, nx - col0), h = min(TILE_H, ny - row0);
+    const int lx = t & (TILE_W - 1), ly0 = t / TILE_W;
+    const int i0 = (row0 + ly0) * nx + col0 + lx;
+    int r[TILE_PER_THREAD], q[TILE_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) r[k] = (lx < w && ly0 + 4 * k < h) ? rec[i0 + 4 * k * nx] : -1;
+    tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
+    int term = 0;  // cells that are terminals
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS;
+        p[c] = (uint16_t)q[k];
+        rv[c] = r[k];
+        if (q[k] == c) term |= 1 << k;
+        if (rec_copy && r[k] >= 0) rec_copy[i0 + 4 * k * nx] = r[k];
+    }
+    sync();
+    tile_jump(p, q, t, sync);
+    bool nonlocal = false;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; ++k) {
+        const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k, i = i0 + 4 * k * nx;
+        bool pit = false;
+        if (r[k] >= 0) {
+            const int j = rv[q[k]];
+            J[i] = j;
+            if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || r[k] == i) R[i] = j;
+            if ((term >> k & 1) && r[k] != i) {  // an exit
+                int rr, rc;
+                divmod_nx(r[k], nx, mnx, rr, rc);
+                if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
+            }
+            if (p[q[k]] != q[k] || (q[k] == c && !(term >> k & 1))) nonlocal = true;  // a cycle in the tile
+            pit = pits && r[k] == i && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, pit);
+        if (m) {
+            const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+            int base = 0;
+            if (lane == leader) base = atomicAdd(info, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (pit) pits[base + __popc(m & ((1u << lane) - 1u))] = i;
+        }
+    }
+    if (nonlocal) info[2] = 1;
+}
+
+// The saddle candidate of a border cell goes to atomicMin(saddle + bi, key) (pass 2).
+// In the border-list pass, where most lanes hold a candidate and neighbouring list
+// entries share basins, saddle_min_warp makes that one atomic per basin per warp
+// (in the N-wide strip pass it cost more than it saved): the lanes holding a
+// candidate group by basin (match.any), take the group's minimum key as two 32-bit
+// reductions (the key's signed order is the unsigned order of key ^ 2^63: high
+// words first, then the low words of the lanes that hold the minimal high word),
+// and the group's first lane applies it.  The minimum over the same keys: the
+// saddle is the one the per-cell atomics produce.
+__device__ __forceinline__ void saddle_min_warp(long long *saddle, int bi, long long key, bool has)
+{
+    const unsigned act = __ballot_sync(0xffffffffu, has);
+    if (!has) return;
+    const unsigned peers = __match_any_sync(act, bi);
+    const unsigned long long u = (unsigned long long)key ^ 0x8000000000000000ull;
+    const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
+    const unsigned mh = __reduce_min_sync(peers, hi);
+    const unsigned ml = __reduce_min_sync(peers, hi == mh ? lo : 0xffffffffu);
+    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1)
+        atomicMin(saddle + bi, (long long)((((unsigned long long)mh << 32) | ml) ^ 0x8000000000000000ull));
+}
+
+// Passes 1-2 for one cell; key: the lowest (z', neighbour basin) of a border cell (a
+// saddle candidate if below the invalid key).  Returns 0 for a cell off every
+// border, 1 for a border cell of the outlet basin 0, 2 for a border cell of a pit basin.
+template <bool WRITE = true>
+__device__ __forceinline__ int saddle_cell(int i, int bi, float zi, const int (&jn)[4], const int (&bn)[4],
+                                           const float (&zn)[4], uint8_t *is_border, float *zp, long long &key)
+{
+    bool border = false;
+    float zmin = 1e9f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (jn[k] != -1 && bn[k] != bi) { border = true; zmin = fminf(zmin, zn[k]); }
+    if (WRITE) is_border[i] = border;
+    const float zpi = border ? fmaxf(zi, zmin) : 1e9f;
+    if (WRITE) zp[i] = zpi;
+    if (!border) return 0;
+    long long res = 0x7fffffffffffffffll;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (jn[k] == -1 || bn[k] == bi) continue;
+        const long long c = pack_key(zpi, bn[k]);
+        res = c < res ? c : res;
+    }
+    key = res;
+    return bi != 0 ? 2 : 1;
+}
 
 // how the loop ended (final state words: [0] iteration, [1] outer, [2] n_outer, [3] state)
 enum { RR_RUN = 0, RR_NOPITS = 1, RR_DONE = 2, RR_GENERAL = 3, RR_RESUME = 4, RR_WALKERR = 5, RR_BOUND = 6 };
@@ -32,14 +227,39 @@ __device__ __forceinline__ int d_ceil_log2(long long n)
     return r;
 }
 
-constexpr int LOOP_THREADS = 1024, LOOP_GROUPS = LOOP_THREADS / TILE_THREADS;
+constexpr int LOOP_THREADS = 1024;              // threads of a block (the batch also runs it with 256 and 512)
 constexpr int LOOP_CAP = 128;                   // list entries buffered per warp
 constexpr int LOOP_ITS = 33, LOOP_CTR = 40;     // per-iteration counter slots (outer <= 32)
 constexpr int LOOP_JUMPS = 16;                  // label jump rounds (8 links each: chains up to 9^16)
 enum { LC_NP = 0, LC_NA = 1, LC_NSEG = 2, LC_NDIRTY = 3, LC_ODD = 4, LC_FLAG = 8 };  // in an iteration's slots
-constexpr int LOOP_GROUP_BYTES = TILE_CELLS * 6;  // per 256-thread group: 12 KB
-constexpr int LOOP_SMEM = LOOP_THREADS / 32 * LOOP_CAP * 16;  // border-list entries of 16 B
-static_assert(LOOP_SMEM >= LOOP_GROUPS * LOOP_GROUP_BYTES, "the group buffers share that memory");
+constexpr int LOOP_GROUP_BYTES = LOOP_CAP * 16 * 8;  // per 256 threads: 8 warps' border-list entries of 16 B
+constexpr int LOOP_SMEM = LOOP_THREADS / TILE_THREADS * LOOP_GROUP_BYTES;
+static_assert(LOOP_GROUP_BYTES >= TILE_CELLS * 6, "a tile pass uses its group's memory");
+
+// The blocks that work on one grid.  All blocks of a cooperative launch:
+struct GridTeam {
+    GridBar bar;
+    int *dead;
+    __device__ __forceinline__ int rank() const { return blockIdx.x; }
+    __device__ __forceinline__ int size() const { return gridDim.x; }
+    __device__ __forceinline__ bool sync() { return bar.sync(dead); }
+};
+// The blocks of a cluster (resident together by construction):
+struct ClusterTeam {
+    int r, n;
+    __device__ __forceinline__ int rank() const { return r; }
+    __device__ __forceinline__ int size() const { return n; }
+    __device__ __forceinline__ bool sync()
+    {
+        if (n == 1) {
+            __syncthreads();
+        } else {
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
+        return true;
+    }
+};
 
 struct LoopArgs {
     int32_t *bid, *rec, *rec_, *J;
@@ -196,38 +416,35 @@ __device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, un
     if (group_or(bar_id, local) && t == 0) loop_mark(A, nd, ty * ntx + tx);
 }
 
-// a barrier that gave up ends the kernel; the final state then says so
-#define LOOP_SYNC()                                                                  \
-    do {                                                                             \
-        if (!bar.sync(&dead)) {                                                      \
-            if (threadIdx.x == 0) A.ctl[3] = ((volatile int *)A.ctl_out)[3] = RR_BOUND; \
-            return;                                                                  \
-        }                                                                            \
+// a barrier that gave up ends the work
+#define LOOP_SYNC()                        \
+    do {                                   \
+        if (!T.sync()) return RR_BOUND;    \
     } while (0)
 
-template <int MODE>
-__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
+// The outer iterations of one grid.  BATCH: a batch tile, whose basin, border and z'
+// arrays are scratch: they are initialised for the pits only, the first border list
+// carries keys, and nothing is written that only a caller would read.  Returns the final
+// state (the same in every thread), the iteration it stopped in, its bound and count.
+template <int MODE, bool BATCH, class Team>
+__device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned char *loop_smem, int &it, int &outer,
+                                            int &n_outer)
 {
-    extern __shared__ __align__(16) unsigned char loop_smem[];
-    __shared__ int dead;
-    const Grid &g = A.g;
+    const Grid g = A.g;
     const int nx = g.nx, N = g.N();
     const unsigned mnx = 0xffffffffu / (unsigned)nx;
-    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-    const int nblk = gridDim.x, gtid = blockIdx.x * LOOP_THREADS + tid, gthreads = nblk * LOOP_THREADS;
-    const int grp = tid / TILE_THREADS, gt = tid & (TILE_THREADS - 1);
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wib = tid >> 5;
+    const int nblk = T.size(), gtid = T.rank() * nt + tid, gthreads = nblk * nt;
+    const int grp = tid / TILE_THREADS, gt = tid & (TILE_THREADS - 1), ngrp = nt / TILE_THREADS;
     unsigned char *gsm = loop_smem + grp * LOOP_GROUP_BYTES;
     const TileXY txy{(nx + TILE_W - 1) / TILE_W, mnx, nx};
     const long long iv = invalid_key();
-    if (tid == 0) dead = 0;
-    GridBar bar{A.bar, 0};
-    __syncthreads();
-
-    const int np0 = A.info[0];
-    int state = RR_RUN, it = 0, n_outer = 0;
-    const int outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;  // :500
+    const int np0 = vload(A.info);
+    int state = RR_RUN;
+    it = n_outer = 0;
+    outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;             // :500
     if (np0 == 0) state = RR_NOPITS;                        // :496-497
-    else if (A.info[2] || A.info[4]) state = RR_GENERAL;    // not D4, or a receiver cycle in the input
+    else if (vload(A.info + 2) || vload(A.info + 4)) state = RR_GENERAL;  // not D4, or a receiver cycle in the input
     if (state == RR_RUN) {
         // clear the carve tags of an earlier call
         if ((((uintptr_t)A.tag | (uintptr_t)A.tag_) & 15) == 0) {
@@ -279,7 +496,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                 __syncwarp();
                 nb = 0;
             };
-            int k0 = (blockIdx.x * (LOOP_THREADS / 32) + wib) * 32;
+            int k0 = (T.rank() * (nt / 32) + wib) * 32;
             int inext = k0 + lane < n ? aprev[k0 + lane] : -1;
             for (; k0 < n; k0 += gthreads) {
                 const bool has = k0 + lane < n;
@@ -304,7 +521,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                     bi = A.fin[bi];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) bn[q] = A.fin[bn[q]];
-                    code = saddle_cell(i, bi, zi, jn, bn, zn, A.isb, A.zp, key);
+                    code = saddle_cell<!BATCH>(i, bi, zi, jn, bn, zn, A.isb, A.zp, key);
                 }
                 saddle_min_warp(A.sad, bi, key, code != 0 && key < iv);
                 const unsigned m = __ballot_sync(0xffffffffu, code != 0);
@@ -333,7 +550,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                 if (jn[q] != -1 && label(jn[q]) == tb) here = true;
             if (here) atomicMax(A.snode + bi, i);
         };
-        if (first) {
+        if (first && !BATCH) {
             for (int k = gtid; 4 * k < na; k += gthreads) {  // the list's memory is padded to 16 bytes
                 const int4 v = reinterpret_cast<const int4 *>(alist)[k];
                 int i[4] = {v.x, v.y, v.z, v.w}, bi[4];
@@ -410,7 +627,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                 __syncwarp();
                 nb = 0;
             };
-            for (int kb = (blockIdx.x * (LOOP_THREADS / 32) + wib) * 32; kb < np; kb += gthreads) {
+            for (int kb = (T.rank() * (nt / 32) + wib) * 32; kb < np; kb += gthreads) {
                 const int k = kb + lane;
                 bool keep = false;
                 int x = -1, p = -1;
@@ -483,7 +700,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
         }
         // a group of 256 threads takes about 5 us per segment whatever its length, a thread
         // about 0.6 us per cell; segments are many while the paths are short
-        if (nseg > 2 * LOOP_GROUPS * nblk) {
+        if (nseg > 2 * ngrp * nblk) {
             for (int k = gtid; k < nseg; k += gthreads) {
                 const int start = A.segs[k], tl = txy.of(start);
                 int x = start;
@@ -502,7 +719,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
                 if (local) loop_mark(A, C + LC_NDIRTY, tl);
             }
         } else {
-            for (int k = grp * nblk + blockIdx.x; k < nseg; k += nblk * LOOP_GROUPS) {
+            for (int k = grp * nblk + T.rank(); k < nseg; k += nblk * ngrp) {
                 loop_walk(A, A.segs[k], txy.ntx, mnx, gt, grp + 1, gsm, C + LC_NDIRTY, txy);
             }
         }
@@ -535,7 +752,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
         else if (it + 2 >= LOOP_ITS) state = RR_BOUND;
         const bool go_on = state == RR_RUN;
         const int ndirty = vload(C + LC_NDIRTY);
-        for (int k = grp * nblk + blockIdx.x; k < ndirty; k += nblk * LOOP_GROUPS) {
+        for (int k = grp * nblk + T.rank(); k < ndirty; k += nblk * ngrp) {
             const int tile = A.dtiles[k];
             loop_tile(A, tile, txy.ntx, mnx, gt, grp + 1, gsm, go_on);
             if (gt == 0) A.dirty[tile] = 0;
@@ -555,7 +772,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
         LOOP_SYNC();
         ++it;
     }
-    if (state == RR_DONE || state == RR_WALKERR) {  // basin_id_init (:537)
+    if (!BATCH && (state == RR_DONE || state == RR_WALKERR)) {  // basin_id_init (:537)
         if (MODE != 3 && (nx & 3) == 0 && ((uintptr_t)A.bid & 15) == 0) {
             for (int q = gtid; 4 * q < N; q += gthreads) {
                 int row, col, lab[4];
@@ -572,32 +789,23 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
             }
         }
     }
-    if (gtid == 0) {
-        const int c[9] = {it, outer, n_outer, state, 0, 0, 0, 0, it + 1};
-        for (int k = 0; k < 9; ++k) {
-            A.ctl[k] = c[k];
-            ((volatile int *)A.ctl_out)[k] = c[k];
-        }
-        __threadfence_system();
-    }
+    return state;
 }
 
 // Labels of the first iteration: pointer jumping of R over the tile-border cells (8 links
 // per round and thread; chains of tiles up to 9^16 long), then one gather per cell and
 // the basins' initial entries (20 B per cell: the stores overlap the gathers).
-template <int MODE>
-__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, int32_t *R, long long nslots, int *flags)
+template <int MODE, bool BATCH, class Team>
+__device__ __forceinline__ int reroute_labels(const LoopArgs &A, int32_t *R, Team &T)
 {
-    __shared__ int dead;
-    if (A.info[0] == 0 || A.info[2]) return;  // the same for every block
-    const Grid &g = A.g;
+    if (vload(A.info) == 0 || vload(A.info + 2)) return RR_RUN;  // the same for every block
+    const Grid g = A.g;
     const int nx = g.nx, N = g.N();
     const unsigned mnx = 0xffffffffu / (unsigned)nx;
     const int ntx = (nx + TILE_W - 1) / TILE_W;
-    const int gtid = blockIdx.x * LOOP_THREADS + threadIdx.x, gthreads = gridDim.x * LOOP_THREADS;
-    if (threadIdx.x == 0) dead = 0;
-    GridBar bar{A.bar + 8, 0};
-    __syncthreads();
+    const long long nslots = (long long)ntx * ((g.ny + TILE_H - 1) / TILE_H) * BORDER_SLOTS;
+    const int gtid = T.rank() * blockDim.x + threadIdx.x, gthreads = T.size() * blockDim.x;
+    int *flags = A.bar + 16;
     for (int r = 0; r < LOOP_JUMPS; ++r) {
         bool ch = false;
         for (long long k = gtid; k < nslots; k += gthreads) {
@@ -618,7 +826,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, 
     }
     const long long iv = invalid_key();
     bool cyc = false;
-    if (MODE != 3 && (nx & 3) == 0 &&
+    if (!BATCH && MODE != 3 && (nx & 3) == 0 &&
         (((uintptr_t)A.J | (uintptr_t)A.bid | (uintptr_t)A.sad | (uintptr_t)A.out | (uintptr_t)A.snode) & 15) == 0 &&
         ((uintptr_t)A.inv & 3) == 0) {
         for (int q = gtid; 4 * q < N; q += gthreads) {
@@ -643,23 +851,114 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, 
     } else {
         for (int i = gtid; i < N; i += gthreads) {
             const int rt = R[A.J[i]];
-            A.sad[i] = iv;
-            A.out[i] = iv;
-            A.snode[i] = -1;
-            A.inv[i] = 0;
+            if (!BATCH) {
+                A.sad[i] = iv;
+                A.out[i] = iv;
+                A.snode[i] = -1;
+                A.inv[i] = 0;
+            }
             cyc |= A.rec_[rt] != rt;
             int row, col;
             divmod_nx(rt, nx, mnx, row, col);
             A.bid[i] = can_leave<MODE>(g, rt, row, col) ? 0 : rt + 1;
         }
     }
-    if (gtid == 0) {
+    if (BATCH) {
+        const int np = vload(A.info);
+        for (int k = gtid; k <= np; k += gthreads) {
+            const int b = k < np ? A.pit0[k] + 1 : 0;
+            A.sad[b] = iv;
+            A.out[b] = iv;
+            A.snode[b] = -1;
+            A.inv[b] = 0;
+        }
+    } else if (gtid == 0) {
         A.sad[N] = iv;
         A.out[N] = iv;
         A.snode[N] = -1;
         A.inv[N] = 0;
     }
     if (cyc) A.info[4] = 1;
+    return RR_RUN;
+}
+
+// The tile pass over the whole grid: rec_ = rec, tile terminals and the pit list.
+template <int MODE, class Team>
+__device__ __forceinline__ void reroute_tiles(const LoopArgs &A, int32_t *R, Team &T, unsigned char *smem)
+{
+    const int grp = threadIdx.x / TILE_THREADS, gt = threadIdx.x & (TILE_THREADS - 1), ngrp = blockDim.x / TILE_THREADS;
+    const Grid g = A.g;
+    const int ntx = (g.nx + TILE_W - 1) / TILE_W, ntiles = ntx * ((g.ny + TILE_H - 1) / TILE_H);
+    unsigned char *gsm = smem + grp * LOOP_GROUP_BYTES;
+    for (int k = grp * T.size() + T.rank(); k < ntiles; k += ngrp * T.size()) {
+        tile_terminal_one<MODE>(A.rec, A.J, R, A.pit0, A.info, g, k % ntx, k / ntx,
+                                reinterpret_cast<uint16_t *>(gsm), reinterpret_cast<int *>(gsm + 2 * TILE_CELLS), A.rec_,
+                                gt, [&]() { group_sync(grp + 1); });
+        group_sync(grp + 1);  // the buffers are reused by the group's next tile
+    }
+}
+
+// Passes 1-2 of the first iteration over every cell; the border cells with their labels
+// and keys.  A warp takes 32 consecutive cells: neighbours and their labels come from L1.
+template <int MODE, bool WRITE, class Team>
+__device__ __forceinline__ void reroute_first_border(const LoopArgs &A, Team &T, unsigned char *smem)
+{
+    if (vload(A.info) == 0 || vload(A.info + 2) || vload(A.info + 4)) return;
+    const Grid g = A.g;
+    const int nx = g.nx, N = g.N(), lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const int gthreads = T.size() * blockDim.x;
+    int *bufi = reinterpret_cast<int *>(smem) + wib * LOOP_CAP * 4, *bufb = bufi + LOOP_CAP;
+    long long *bufk = reinterpret_cast<long long *>(bufb + LOOP_CAP);
+    int *na = A.it_ctr + LC_NA;
+    int nb = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        int base = 0;
+        if (lane == 0 && nb) base = atomicAdd(na, nb);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int q = lane; q < nb; q += 32) {
+            A.alist[0][base + q] = bufi[q];
+            A.abid[base + q] = bufb[q];
+            A.akey[base + q] = bufk[q];
+        }
+        __syncwarp();
+        nb = 0;
+    };
+    for (int k0 = (T.rank() * (blockDim.x >> 5) + wib) * 32; k0 < N; k0 += gthreads) {
+        const int i = k0 + lane;
+        int code = 0, bi = 0;
+        long long key = 0;
+        if (i < N) {
+            int row, col;
+            divmod_nx(i, nx, mnx, row, col);
+            if (can_leave<MODE>(g, i, row, col)) {
+                if (WRITE) A.zp[i] = A.z[i];
+            } else {
+                int jn[4], bn[4];
+                float zn[4];
+                neighbours4<MODE>(g, i, row, col, jn);
+                bi = A.bid[i];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    bn[q] = jn[q] != -1 ? A.bid[jn[q]] : 0;
+                    zn[q] = jn[q] != -1 ? A.z[jn[q]] : 0.f;
+                }
+                code = saddle_cell<WRITE>(i, bi, A.z[i], jn, bn, zn, A.isb, A.zp, key);
+            }
+        }
+        if (code != 0 && key < invalid_key()) atomicMin(A.sad + bi, key);
+        const unsigned m = __ballot_sync(0xffffffffu, code != 0);
+        if (code != 0) {
+            const int at = nb + __popc(m & ((1u << lane) - 1u));
+            bufi[at] = i;
+            bufb[at] = bi;
+            bufk[at] = key;
+        }
+        nb += __popc(m);
+        if (nb > LOOP_CAP - 32) flush();
+    }
+    flush();
 }
 
 }  // namespace pff
