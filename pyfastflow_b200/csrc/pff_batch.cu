@@ -621,6 +621,11 @@ __device__ __forceinline__ T *team_at(T *p, const ClusterTeam &Tm)
     return q;
 }
 #define FOR_TEAM(i, N) for (int i = Tm.r * blockDim.x + threadIdx.x; i < (N); i += Tm.n * blockDim.x)
+// U cells per thread and trip (cells i0, i0 + stride, ...), so that their loads are in
+// flight together: the passes are bound by load latency at 32 warps per SM
+#define FOR_TEAM_U(i0, stride, U, N)                                                    \
+    for (int stride = Tm.n * blockDim.x, i0 = Tm.r * blockDim.x + threadIdx.x; i0 < (N); \
+         i0 += (U) * stride)
 
 // whether any thread of the team has p (a barrier)
 __device__ __forceinline__ bool team_any(bool p, BatchShm &sh, ClusterTeam &Tm)
@@ -640,32 +645,47 @@ __device__ __forceinline__ bool team_any(bool p, BatchShm &sh, ClusterTeam &Tm)
 // receivers (receivers.py:31-58): strict >, first k wins ties (and the gradient if
 // grad is not null).
 template <int MODE>
-__device__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, float *grad, ClusterTeam &Tm)
+__device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, float *grad,
+                                            ClusterTeam Tm)
 {
     const int N = g.nx * g.ny;
     const unsigned mnx = 0xffffffffu / (unsigned)g.nx;
-    FOR_TEAM(i, N) {
-        int row, col, js[4];
-        divmod_nx(i, g.nx, mnx, row, col);
-        neighbours4<MODE>(g, i, row, col, js);
-        const float zi = z[i];
-        float d[4];
+    constexpr int U = 4;
+    FOR_TEAM_U(i0, stride, U, N) {
+        int js[U][4];
+        float zi[U], zn[U][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) d[k] = js[k] != -1 ? __fsub_rn(zi, z[js[k]]) : 0.f;
-        int r = i;
-        float sr = 0.f, dbest = 0.f;
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * stride;
+            if (i >= N) break;
+            int row, col;
+            divmod_nx(i, g.nx, mnx, row, col);
+            neighbours4<MODE>(g, i, row, col, js[u]);
+            zi[u] = z[i];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (d[k] > dbest) {  // a smaller difference cannot give a larger quotient
-                const float q = __fdiv_rn(d[k], dx);
-                if (q > sr) {
-                    sr = q;
-                    r = js[k];
-                    dbest = d[k];
+            for (int k = 0; k < 4; ++k) zn[u][k] = js[u][k] != -1 ? z[js[u][k]] : zi[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * stride;
+            if (i >= N) break;
+            int r = i;
+            float sr = 0.f, dbest = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float d = __fsub_rn(zi[u], zn[u][k]);
+                if (js[u][k] != -1 && d > dbest) {  // a smaller difference cannot give a larger quotient
+                    const float q = __fdiv_rn(d, dx);
+                    if (q > sr) {
+                        sr = q;
+                        r = js[u][k];
+                        dbest = d;
+                    }
                 }
             }
-        rec[i] = r;
-        if (grad) grad[i] = sr;
+            rec[i] = r;
+            if (grad) grad[i] = sr;
+        }
     }
     Tm.sync();
 }
@@ -725,7 +745,7 @@ template <int MODE>
 __device__ __noinline__ int batch_loop(const LoopArgs &L, ClusterTeam Tm, unsigned char *smem, int *it_outer)
 {
     int it = 0, outer = 0, n_outer = 0;
-    const int state = reroute_loop<MODE, true>(L, Tm, smem, it, outer, n_outer);
+    const int state = reroute_loop<MODE, true, true>(L, Tm, smem, it, outer, n_outer);
     if (threadIdx.x == 0) {
         it_outer[0] = it;
         it_outer[1] = outer;
@@ -834,13 +854,210 @@ __device__ __forceinline__ void bmaxsum(float m, float sum, BatchShm &sh, Cluste
     Tm.sync();
 }
 
+// The steps of an iteration are functions of their own: inlined into one kernel they
+// spilled registers at 1024 threads.
+
+// fill_z_add_delta (fill_topo.py:99-125): rounds on snapshots of the records {pointer,
+// surface}; the buffer that holds the final ones is returned.
+__device__ __noinline__ const int2 *gf_fill(int N, int2 *fa, int2 *fb, const int32_t *rec, float *zh, float *h, float *href,
+                                    int nr, float eps, BatchShm &sh, ClusterTeam Tm)
+{
+    FOR_TEAM(i, N) {
+        const int r = rec[i];
+        fa[i] = make_int2(r == i ? (i | (int)0x80000000) : r, __float_as_int(zh[i]));
+    }
+    Tm.sync();
+    int2 *a = fa, *b = fb;
+    for (int r = 0; r < nr; ++r) {
+        const float inc = (float)(ldexp(1.0, r - 1) * (double)eps);
+        bool ch = false;
+        FOR_TEAM_U(i0, stride, 4, N) {
+            int2 sv[4], tv[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * stride;
+                sv[u] = i < N ? a[i] : make_int2(0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) tv[u] = a[sv[u].x & 0x7FFFFFFF];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * stride, q = sv[u].x & 0x7FFFFFFF;
+                if (i >= N) break;
+                int2 n = sv[u];
+                if (q != i) {
+                    const int qq = tv[u].x & 0x7FFFFFFF;
+                    const float zi = __int_as_float(n.y), zq = __int_as_float(tv[u].y);
+                    n.x = qq;
+                    if (!(qq == q && zi > (tv[u].x < 0 ? zq : zh[q]))) n.y = __float_as_int(fmaxf(zi, __fadd_rn(zq, inc)));
+                    ch |= n.x != sv[u].x || n.y != sv[u].y;
+                }
+                b[i] = n;
+            }
+        }
+        const bool any = team_any(ch, sh, Tm);
+        int2 *t = a; a = b; b = t;
+        // a round that changed nothing is a fixed point of every later round
+        if (!any) break;
+    }
+    FOR_TEAM(i, N) {
+        const float zf = __int_as_float(a[i].y), hi = h[i], zi = zh[i];
+        href[i] = hi;
+        h[i] = __fadd_rn(hi, __fsub_rn(zf, zi));
+        zh[i] = zf;
+    }
+    Tm.sync();
+    return a;
+}
+
+// diffuse_Q_constant_prec (gf_hydrodynamics.py:24-75): a cell's outgoing weights once (-1:
+// not a source), then 5 gather sweeps; the last one's result is in the returned array.
+template <int MODE>
+__device__ __noinline__ void gf_weights(const Grid &g, float dx, const float *zh, float *w, ClusterTeam Tm)
+{
+    const int N = g.nx * g.ny, nx = g.nx;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    FOR_TEAM_U(i0, stride, 2, N) {
+        int js[2][4];
+        float zi[2], zn[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + u * stride;
+            int row, col;
+            divmod_nx(i, nx, mnx, row, col);
+            if (i < N && !can_leave<MODE>(g, i, row, col)) neighbours4<MODE>(g, i, row, col, js[u]);
+            else js[u][0] = js[u][1] = js[u][2] = js[u][3] = -1;  // leaving cells have no slopes
+            zi[u] = i < N ? zh[i] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) zn[u][k] = js[u][k] != -1 ? zh[js[u][k]] : zi[u];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + u * stride;
+            if (i >= N) break;
+            float sk[4];
+            float sums = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                sk[k] = (js[u][k] != -1) ? fmaxf(0.f, __fdiv_rn(__fsub_rn(zi[u], zn[u][k]), dx)) : 0.f;
+                sums = __fadd_rn(sums, sk[k]);
+            }
+            const bool src = !(sums == 0.f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[(size_t)k * N + i] = src ? __fdiv_rn(sk[k], sums) : -1.f;
+        }
+    }
+    Tm.sync();
+}
+template <int MODE>
+__device__ __noinline__ const float *gf_sweeps(const Grid &g, const float *w, float *Q, float *temp, float prec_dx2,
+                                       ClusterTeam Tm)
+{
+    const int N = g.nx * g.ny, nx = g.nx;
+    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const bool sym = MODE != 3 && nx >= 3 && g.ny >= 3;
+    float *qa = Q, *qb = temp;
+    for (int sw = 0; sw < 5; ++sw) {
+        FOR_TEAM_U(j0, stride, 2, N) {
+            float wv[2][4], qv[2][4];
+            int js[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = j0 + u * stride;
+                int row, col;
+                divmod_nx(j, nx, mnx, row, col);
+                // modes 0-2 on grids of at least 3 x 3: j's sources are its own neighbours,
+                // and neighbour k sends to j through its opposite link 3 - k
+                if (sym && j < N) neighbours4<MODE>(g, j, row, col, js[u]);
+                else js[u][0] = js[u][1] = js[u][2] = js[u][3] = -1;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = js[u][k];
+                    wv[u][k] = i != -1 ? w[(size_t)(3 - k) * N + i] : -1.f;
+                    qv[u][k] = i != -1 ? qa[i] : 0.f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = j0 + u * stride;
+                if (j >= N) break;
+                float acc = prec_dx2;
+                if (sym) {
+                    // ascending source: top, left, right, bottom, except beside a wrap
+                    int (&x)[4] = js[u];
+                    if (MODE != 0 && !(x[0] < x[1] && x[1] < x[2] && x[2] < x[3])) {
+                        auto cs = [&](int p, int q) {
+                            if (x[p] > x[q]) {
+                                const int ti = x[p]; x[p] = x[q]; x[q] = ti;
+                                float tf = wv[u][p]; wv[u][p] = wv[u][q]; wv[u][q] = tf;
+                                tf = qv[u][p]; qv[u][p] = qv[u][q]; qv[u][q] = tf;
+                            }
+                        };
+                        cs(0, 1); cs(2, 3); cs(0, 2); cs(1, 3); cs(1, 2);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (!(wv[u][k] < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wv[u][k], qv[u][k]));
+                } else {
+                    int row, col, c[8];
+                    divmod_nx(j, nx, mnx, row, col);
+                    const int n = donor_candidates(g, j, row, col, c);
+                    for (int q = 0; q < n; ++q) {
+                        const int i = c[q];
+                        if (w[i] < 0.f) continue;
+                        const float qi = qa[i];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (neighbour_i<MODE>(g, i, k) == j)
+                                acc = __fadd_rn(acc, __fmul_rn(w[(size_t)k * N + i], qi));
+                    }
+                }
+                qb[j] = acc;
+            }
+        }
+        Tm.sync();
+        float *t = qa; qa = qb; qb = t;
+    }
+    return qa;
+}
+
+// Manning update (gf_hydrodynamics.py:79-129; h receives tdh twice, :127-129); slopes from
+// the fill's records a, which hold the filled surface; the diffused qa goes into Q.
+// Returns this thread's largest |dh| and the sum.
+__device__ __noinline__ float2 gf_update(int N, const int2 *a, const int32_t *rec, const float *qa, float *Q, float *h,
+                                 float *zh, const float *href, float dx, float dx2, float manning,
+                                 float edgesw, float dt, ClusterTeam Tm)
+{
+    float m = 0.f, sum = 0.f;
+    FOR_TEAM(i, N) {
+        const int r = rec[i];
+        const float zi = __int_as_float(a[i].y), qi = qa[i], hi = h[i];
+        float tS = edgesw;
+        if (r != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zi, __int_as_float(a[r].y)), dx), 1e-4f);
+        Q[i] = qi;
+        float Qo = __fmul_rn(dx, pow53(hi));
+        Qo = __fdiv_rn(Qo, manning);
+        Qo = __fmul_rn(Qo, __fsqrt_rn(tS));
+        float tdh = __fdiv_rn(__fsub_rn(qi, Qo), dx2);
+        tdh = __fmul_rn(tdh, dt);
+        const float h1 = __fadd_rn(hi, tdh);
+        if (h1 < 0.f) tdh = __fadd_rn(tdh, h1);
+        const float hn = __fadd_rn(h1, tdh);
+        h[i] = hn;
+        zh[i] = __fadd_rn(zi, tdh);
+        const float e = fabsf(__fsub_rn(hn, href[i]));
+        m = __uint_as_float(max(__float_as_uint(m), __float_as_uint(e)));
+        sum += e;
+    }
+    return make_float2(m, sum);
+}
+
 template <int MODE>
 __device__ __forceinline__ void gf_tile(const BatchTile &T, const BatchArrays &A, const GfParams &P, BatchShm &sh,
                                         ClusterTeam &Tm, unsigned char *smem)
 {
     const Grid g{T.nx, T.ny, MODE, MODE == 3 ? A.codes + T.off : nullptr};
-    const int N = T.nx * T.ny, nx = T.nx;
-    const unsigned mnx = 0xffffffffu / (unsigned)nx;
+    const int N = T.nx * T.ny;
     const long long o = T.off;
     float *zh = const_cast<float *>(A.z) + o, *h = P.h + o, *Q = A.Q + o;
     int32_t *rec = A.rcv + o;
@@ -857,122 +1074,11 @@ __device__ __forceinline__ void gf_tile(const BatchTile &T, const BatchArrays &A
     for (; it < P.niter; ++it) {
         tile_receivers<MODE>(g, dx, zh, rec, nullptr, Tm);
         tile_reroute<MODE>(T, A, zh, sh, Tm, smem);
-        // fill_z_add_delta (fill_topo.py:99-125): rounds on snapshots of the records.  The
-        // surface that a self-pointing cell's followers compare with is its initial one,
-        // which is also its record's where it points to itself from the start (bit 31).
-        FOR_TEAM(i, N) {
-            const int r = rec[i];
-            fa[i] = make_int2(r == i ? (i | (int)0x80000000) : r, __float_as_int(zh[i]));
-        }
-        Tm.sync();
-        int2 *a = fa, *b = fb;
-        for (int r = 0; r < nr; ++r) {
-            const float inc = (float)(ldexp(1.0, r - 1) * (double)P.eps);
-            bool ch = false;
-            FOR_TEAM(i, N) {
-                const int2 s = a[i];
-                const int q = s.x & 0x7FFFFFFF;
-                int2 n = s;
-                if (q != i) {
-                    const int2 t = a[q];
-                    const int qq = t.x & 0x7FFFFFFF;
-                    const float zi = __int_as_float(s.y), zq = __int_as_float(t.y);
-                    n.x = qq;
-                    if (!(qq == q && zi > (t.x < 0 ? zq : zh[q]))) n.y = __float_as_int(fmaxf(zi, __fadd_rn(zq, inc)));
-                    ch |= n.x != s.x || n.y != s.y;
-                }
-                b[i] = n;
-            }
-            const bool any = team_any(ch, sh, Tm);
-            int2 *t = a; a = b; b = t;
-            // a round that changed nothing is a fixed point of every later round
-            if (!any) break;
-        }
-        FOR_TEAM(i, N) {
-            const float zf = __int_as_float(a[i].y), hi = h[i], zi = zh[i];
-            href[i] = hi;
-            h[i] = __fadd_rn(hi, __fsub_rn(zf, zi));
-            zh[i] = zf;
-        }
-        Tm.sync();
-        // diffusion: a cell's outgoing weights once (-1: not a source), then 5 gather sweeps
-        FOR_TEAM(i, N) {
-            int row, col, js[4];
-            divmod_nx(i, nx, mnx, row, col);
-            float sk[4] = {0.f, 0.f, 0.f, 0.f};
-            float sums = 0.f;
-            if (!can_leave<MODE>(g, i, row, col)) {
-                const float zi = zh[i];
-                neighbours4<MODE>(g, i, row, col, js);
-                float zn[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) zn[k] = js[k] != -1 ? zh[js[k]] : zi;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    sk[k] = (js[k] != -1) ? fmaxf(0.f, __fdiv_rn(__fsub_rn(zi, zn[k]), dx)) : 0.f;
-                    sums = __fadd_rn(sums, sk[k]);
-                }
-            }
-            const bool src = !(sums == 0.f);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[(size_t)k * N + i] = src ? __fdiv_rn(sk[k], sums) : -1.f;
-        }
-        Tm.sync();
-        float *qa = Q, *qb = temp;
-        for (int sw = 0; sw < 5; ++sw) {
-            FOR_TEAM(j, N) {
-                int row, col;
-                divmod_nx(j, nx, mnx, row, col);
-                float acc = prec_dx2;
-                if (MODE != 3 && row > 0 && row < g.ny - 1 && col > 0 && col < nx - 1) {
-                    const float wt = w[3 * (size_t)N + j - nx], wl = w[2 * (size_t)N + j - 1], wr = w[(size_t)N + j + 1],
-                                wb = w[j + nx];
-                    const float qt = qa[j - nx], ql = qa[j - 1], qr = qa[j + 1], qd = qa[j + nx];
-                    if (!(wt < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wt, qt));
-                    if (!(wl < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wl, ql));
-                    if (!(wr < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wr, qr));
-                    if (!(wb < 0.f)) acc = __fadd_rn(acc, __fmul_rn(wb, qd));
-                } else {
-                    int c[8];
-                    const int n = donor_candidates(g, j, row, col, c);
-                    for (int q = 0; q < n; ++q) {
-                        const int i = c[q];
-                        if (w[i] < 0.f) continue;
-                        const float qi = qa[i];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (neighbour_i<MODE>(g, i, k) == j) acc = __fadd_rn(acc, __fmul_rn(w[(size_t)k * N + i], qi));
-                    }
-                }
-                qb[j] = acc;
-            }
-            Tm.sync();
-            float *t = qa; qa = qb; qb = t;
-        }
-        // Manning update; slopes from the fill's records, which hold the filled surface (h
-        // receives tdh twice, gf_hydrodynamics.py:127-129); the last sweep's result into Q
-        float m = 0.f, sum = 0.f;
-        FOR_TEAM(i, N) {
-            const int r = rec[i];
-            const float zi = __int_as_float(a[i].y), qi = qa[i], hi = h[i];
-            float tS = P.edgesw;
-            if (r != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zi, __int_as_float(a[r].y)), dx), 1e-4f);
-            Q[i] = qi;
-            float Qo = __fmul_rn(dx, pow53(hi));
-            Qo = __fdiv_rn(Qo, manning);
-            Qo = __fmul_rn(Qo, __fsqrt_rn(tS));
-            float tdh = __fdiv_rn(__fsub_rn(qi, Qo), dx2);
-            tdh = __fmul_rn(tdh, P.dt);
-            const float h1 = __fadd_rn(hi, tdh);
-            if (h1 < 0.f) tdh = __fadd_rn(tdh, h1);
-            const float hn = __fadd_rn(h1, tdh);
-            h[i] = hn;
-            zh[i] = __fadd_rn(zi, tdh);
-            const float e = fabsf(__fsub_rn(hn, href[i]));
-            m = __uint_as_float(max(__float_as_uint(m), __float_as_uint(e)));
-            sum += e;
-        }
-        bmaxsum(m, sum, sh, Tm, &rmax, &rmean);
+        const int2 *a = gf_fill(N, fa, fb, rec, zh, h, href, nr, P.eps, sh, Tm);
+        gf_weights<MODE>(g, dx, zh, w, Tm);
+        const float *qa = gf_sweeps<MODE>(g, w, Q, temp, prec_dx2, Tm);
+        const float2 e = gf_update(N, a, rec, qa, Q, h, zh, href, dx, dx2, manning, P.edgesw, P.dt, Tm);
+        bmaxsum(e.x, e.y, sh, Tm, &rmax, &rmean);
         rmean /= (float)N;
         if (P.trace && Tm.r == 0 && threadIdx.x == 0) {
             P.trace[((size_t)T.id * P.niter + it) * 2] = rmax;
@@ -1333,6 +1439,18 @@ extern "C" int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, f
     GfParams P{tile_consts, edgesw, dt, 1e-3f, niter, crit, h, iters, residuals, trace};
     cudaStream_t st = S(stream);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
+    // more tiles than SMs: two half-size blocks per SM hold twice the tiles at once, and the
+    // steps are bound by latency, not by threads (256 tiles of 128 x 128 on 148 SMs took two
+    // rounds of one block each)
+    if (threads == 1024 && ctas_per_sm <= 1) {
+        int dev = 0, nsm = 148;
+        PFF_CUDA(cudaGetDevice(&dev));
+        PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        if (ntiles > nsm) {
+            threads = 512;
+            ctas_per_sm = 2;
+        }
+    }
     PFF_TRY(launch_batch(k_batch_graphflood, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A, P));
     return check_cuda("pff_batch_graphflood");
 }

@@ -1374,8 +1374,30 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
     GridTeam T{GridBar{A.bar, 0}, &dead};
     __syncthreads();
     int it = 0, outer = 0, n_outer = 0;
-    const int state = reroute_loop<MODE, false>(A, T, loop_smem, it, outer, n_outer);
+    const int state = reroute_loop<MODE, false, false>(A, T, loop_smem, it, outer, n_outer);
     // block 0's first thread reports; a block whose barrier gave up says so whoever it is
+    if (threadIdx.x == 0 && (blockIdx.x == 0 || state == RR_BOUND)) loop_report(A, it, outer, n_outer, state);
+}
+
+// The whole reroute of a grid whose steps do not fill the GPU, in one launch: with one
+// block per 2048 cells below one per SM, the four launches' latency (8-10 us of about
+// 60 at 48 x 33) is more than their wider grids save.
+template <int MODE>
+__global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_whole(LoopArgs A, int32_t *R, int nzero)
+{
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    __shared__ int dead;
+    if (threadIdx.x == 0) dead = 0;
+    if (gridDim.x == 1)  // one block clears its counters itself
+        for (int k = threadIdx.x; k < nzero; k += LOOP_THREADS) A.ctl[k] = 0;
+    GridTeam T{GridBar{A.bar, 0}, &dead};
+    __syncthreads();
+    reroute_tiles<MODE>(A, R, T, loop_smem);
+    int it = 0, outer = 0, n_outer = 0, state = RR_BOUND;
+    if (T.sync() && reroute_labels<MODE, false>(A, R, T) == RR_RUN && T.sync()) {
+        reroute_first_border<MODE, true>(A, T, loop_smem);
+        if (T.sync()) state = reroute_loop<MODE, false, true>(A, T, loop_smem, it, outer, n_outer);
+    }
     if (threadIdx.x == 0 && (blockIdx.x == 0 || state == RR_BOUND)) loop_report(A, it, outer, n_outer, state);
 }
 
@@ -1711,7 +1733,7 @@ namespace pff {
 // ---- the outer loop of reroute_flow driven on the device (carve rerouting) -------------
 // Four launches per call: the tile pass (with rec_ = rec and the pit list), the labels
 // and the strip saddle pass of iteration 0, then the loop kernel, which goes on to
-// the end (pff_lake_loop.cuh).  The rare cases that need the reference's N-wide steps
+// the end (pff_lake_loop.cuh); small grids take one (k_reroute_whole).  The rare cases that need the reference's N-wide steps
 // (non-D4 receivers, receiver cycles) stop it in a recorded state; the host then runs
 // those steps from there.
 
@@ -1741,9 +1763,10 @@ static void l_loop_ready(int dev, int *ready)
     if (!v) {
         int per = 0, per2 = 0, coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        if (cudaFuncSetAttribute(k_reroute_loop<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) == cudaSuccess) {
+        if (cudaFuncSetAttribute(k_reroute_loop<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) == cudaSuccess &&
+            cudaFuncSetAttribute(k_reroute_whole<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) == cudaSuccess) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_reroute_loop<MODE>, LOOP_THREADS, LOOP_SMEM);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_reroute_labels<MODE>, LOOP_THREADS, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_reroute_whole<MODE>, LOOP_THREADS, LOOP_SMEM);
         }
         cudaGetLastError();
         v = coop && per > 0 && per2 > 0 ? 1 : -1;
@@ -1751,13 +1774,14 @@ static void l_loop_ready(int dev, int *ready)
     }
     *ready = v;
 }
-static int loop_blocks(const Grid &g)
+static int loop_blocks(const Grid &g, int *fill)
 {
     int dev = 0, nsm = 0, ready = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     PFF_MODE_DISPATCH(g.mode, l_loop_ready, dev, &ready);
     if (ready < 0) return 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    *fill = nsm;
     return g.N() <= LOOP_ONE ? 1 : std::min(nsm, div_up(g.N(), LOOP_CELLS));
 }
 
@@ -1781,9 +1805,22 @@ static void l_strip(const LoopArgs &A, cudaStream_t st)
 }
 
 template <int MODE>
-static void l_loop(const LoopArgs &A, int32_t *R, int blocks, int *rc, cudaStream_t st)
+static void l_loop(const LoopArgs &A, int32_t *R, int blocks, bool whole, int nzero, int *rc, cudaStream_t st)
 {
     LoopArgs a = A;
+    if (whole) {
+        void *args[] = {&a, &R, &nzero};
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel((void *)k_reroute_whole<MODE>, blocks, LOOP_THREADS, args, LOOP_SMEM, st);
+        count_launch();
+        if (e != cudaSuccess) {
+            set_error("pff_reroute_flow: cooperative launch: %s", cudaGetErrorString(e));
+            cudaGetLastError();
+            *rc = PFF_ERR_CUDA;
+        }
+        return;
+    }
+    l_tile_terminal<MODE>(a.rec, a.J, R, a.pit0, a.info, a.g, a.rec_, st);  // :491, :493
     void *largs[] = {&a, &R};
     cudaError_t e = cudaLaunchCooperativeKernel((void *)k_reroute_labels<MODE>, blocks, LOOP_THREADS, largs, 0, st);
     if (e == cudaSuccess) {
@@ -1808,7 +1845,8 @@ static int reroute_device(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *re
                           uint8_t *tag_, const Grid &g, RerouteWs &w, int *ctl_out, cudaStream_t st)
 {
     if (!rr_device_on()) return PFF_ERR_UNSUPPORTED;
-    const int blocks = loop_blocks(g);
+    int nsm = 0;
+    const int blocks = loop_blocks(g, &nsm);
     if (blocks < 1) return PFF_ERR_UNSUPPORTED;
     const int ntiles = div_up(g.nx, TILE_W) * div_up(g.ny, TILE_H);
     LoopArgs A{};
@@ -1828,10 +1866,10 @@ static int reroute_device(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *re
     A.dirty = A.it_ctr + LOOP_ITS * LOOP_CTR;
     A.ctl_out = ctl_out;
     A.g = g;
-    PFF_CUDA(cudaMemsetAsync(w.loop, 0, sizeof(int) * ((size_t)RR_SYNC + LOOP_ITS * LOOP_CTR + ntiles), st));
-    PFF_MODE_DISPATCH(g.mode, l_tile_terminal, rec, rec__, w.R, w.pit0, A.info, g, rec_, st);  // :491, :493
+    const int nzero = RR_SYNC + LOOP_ITS * LOOP_CTR + ntiles;
+    if (blocks > 1) PFF_CUDA(cudaMemsetAsync(w.loop, 0, sizeof(int) * (size_t)nzero, st));
     int rc = PFF_OK;
-    PFF_MODE_DISPATCH(g.mode, l_loop, A, w.R, blocks, &rc, st);
+    PFF_MODE_DISPATCH(g.mode, l_loop, A, w.R, blocks, blocks < nsm, nzero, &rc, st);
     PFF_TRY(rc);
     return check_cuda("pff_reroute_flow");
 }

@@ -423,10 +423,11 @@ __device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, un
     } while (0)
 
 // The outer iterations of one grid.  BATCH: a batch tile, whose basin, border and z'
-// arrays are scratch: they are initialised for the pits only, the first border list
-// carries keys, and nothing is written that only a caller would read.  Returns the final
+// arrays are scratch: they are initialised for the pits only, and nothing is written that
+// only a caller would read.  KEYED: the first border list carries labels and keys (from
+// reroute_first_border, not from the strip pass).  Returns the final
 // state (the same in every thread), the iteration it stopped in, its bound and count.
-template <int MODE, bool BATCH, class Team>
+template <int MODE, bool BATCH, bool KEYED, class Team>
 __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned char *loop_smem, int &it, int &outer,
                                             int &n_outer)
 {
@@ -550,7 +551,7 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
                 if (jn[q] != -1 && label(jn[q]) == tb) here = true;
             if (here) atomicMax(A.snode + bi, i);
         };
-        if (first && !BATCH) {
+        if (first && !KEYED) {
             for (int k = gtid; 4 * k < na; k += gthreads) {  // the list's memory is padded to 16 bytes
                 const int4 v = reinterpret_cast<const int4 *>(alist)[k];
                 int i[4] = {v.x, v.y, v.z, v.w}, bi[4];
@@ -849,18 +850,30 @@ __device__ __forceinline__ int reroute_labels(const LoopArgs &A, int32_t *R, Tea
             reinterpret_cast<int4 *>(A.bid)[q] = make_int4(lab[0], lab[1], lab[2], lab[3]);
         }
     } else {
-        for (int i = gtid; i < N; i += gthreads) {
-            const int rt = R[A.J[i]];
-            if (!BATCH) {
-                A.sad[i] = iv;
-                A.out[i] = iv;
-                A.snode[i] = -1;
-                A.inv[i] = 0;
+        constexpr int U = 4;  // cells per trip, their gathers in flight together
+        for (int i0 = gtid; i0 < N; i0 += U * gthreads) {
+            int rt[U], rr[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) rt[u] = i0 + u * gthreads < N ? A.J[i0 + u * gthreads] : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) rt[u] = i0 + u * gthreads < N ? R[rt[u]] : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) rr[u] = A.rec_[rt[u]];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * gthreads;
+                if (i >= N) break;
+                if (!BATCH) {
+                    A.sad[i] = iv;
+                    A.out[i] = iv;
+                    A.snode[i] = -1;
+                    A.inv[i] = 0;
+                }
+                cyc |= rr[u] != rt[u];
+                int row, col;
+                divmod_nx(rt[u], nx, mnx, row, col);
+                A.bid[i] = can_leave<MODE>(g, rt[u], row, col) ? 0 : rt[u] + 1;
             }
-            cyc |= A.rec_[rt] != rt;
-            int row, col;
-            divmod_nx(rt, nx, mnx, row, col);
-            A.bid[i] = can_leave<MODE>(g, rt, row, col) ? 0 : rt + 1;
         }
     }
     if (BATCH) {
