@@ -424,6 +424,9 @@ int pff_conv3x3_wgrad(const uint16_t *x, int csx, int offx, const uint16_t *dy, 
 int pff_bias_grad(const uint16_t *dy, int cs, int off, float *db, long long P, int C, void *stream);
 int pff_relu_bwd(uint16_t *g, int csg, int offg, const uint16_t *y, int csy, int offy, long long P, int C,
                  void *stream);
+/* pff_relu_bwd (y may be NULL: no ReLU), then pff_bias_grad of the result, in one pass. */
+int pff_relu_bias_bwd(uint16_t *g, int csg, int offg, const uint16_t *y, int csy, int offy, float *db, long long P,
+                      int C, void *stream);
 int pff_avgpool2(const uint16_t *x, int csx, int offx, uint16_t *y, int csy, int offy, int B, int H, int W,
                  int C, void *stream);
 int pff_avgpool2_bwd(const uint16_t *dy, int csd, int offd, uint16_t *dx, int csx, int offx, int B, int H,

@@ -77,6 +77,7 @@ SIGNATURES = {
     "pff_conv3x3_wflip": (_i32, [_vp, _vp, _i32, _i32, _vp]),
     "pff_conv3x3_wgrad": (_i32, [_vp, _i32, _i32, _vp, _i32, _i32, _vp] + [_i32] * 5 + [_vp]),
     "pff_bias_grad": (_i32, [_vp, _i32, _i32, _vp, _i64, _i32, _vp]),
+    "pff_relu_bias_bwd": (_i32, [_vp, _i32, _i32, _vp, _i32, _i32, _vp, _i64, _i32, _vp]),
     "pff_relu_bwd": (_i32, [_vp, _i32, _i32, _vp, _i32, _i32, _i64, _i32, _vp]),
     "pff_avgpool2": (_i32, [_vp, _i32, _i32, _vp, _i32, _i32] + [_i32] * 4 + [_vp]),
     "pff_avgpool2_bwd": (_i32, [_vp, _i32, _i32, _vp, _i32, _i32] + [_i32] * 5 + [_vp]),

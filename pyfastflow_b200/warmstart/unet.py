@@ -192,11 +192,10 @@ class UNet:
             b, h, w = self._dims(lev)
             P = b * h * w
             cd = BUFFERS[dst][0]
-            if relu:
-                _call("pff_relu_bwd", gr[dst].data_ptr(), cd, do, bf[dst].data_ptr(), cd, do, P, cout, st)
+            _call("pff_relu_bias_bwd", gr[dst].data_ptr(), cd, do, bf[dst].data_ptr() if relu else None, cd, do,
+                  self.g.data_ptr() + 4 * bo, P, cout, st)
             _call("pff_conv3x3_wgrad", bf[src].data_ptr(), BUFFERS[src][0], so, gr[dst].data_ptr(), cd, do,
                   self.g.data_ptr() + 4 * wo, b, h, w, cin, cout, st)
-            _call("pff_bias_grad", gr[dst].data_ptr(), cd, do, self.g.data_ptr() + 4 * bo, P, cout, st)
             if need_dx:
                 _call("pff_conv3x3_fwd", gr[dst].data_ptr(), cd, do, self.wt[name].data_ptr(), None,
                       gr[dsrc].data_ptr(), BUFFERS[dsrc][0], dso, b, h, w, cout, cin, 0, 0, st)
