@@ -163,6 +163,11 @@ int pff_accumulate_tree(const int32_t *receivers, const float *weights, float va
 int pff_accumulate_tree_status(int nx, int ny, int local, void *workspace, size_t workspace_bytes,
                                int *status, void *stream);
 
+/* pff_accumulate_tree and pff_accumulate_tree_status with one synchronisation. */
+int pff_accumulate_tree_run(const int32_t *receivers, const float *weights, float value, float *Q, uint32_t *counts,
+                            int nx, int ny, int local, void *workspace, size_t workspace_bytes, int *status,
+                            void *stream);
+
 /* ---- lake / depression rerouting -----------------------------------------------
  * Replaces pyfastflow/flow/lakeflow.py:466-538 reroute_flow(bid, rec, rec_, rec__,
  * z, z_prime, is_border, outlet, basin_saddle, basin_saddlenode, tag, tag_,

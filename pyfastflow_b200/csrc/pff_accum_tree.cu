@@ -24,13 +24,16 @@
 //             a block's nodes in shared memory.  Nodes whose parent lies in another block are
 //             the next level's nodes.  The top level is one block over the grid.
 //   down      from the top: each level's nodes receive the totals of the nodes of
-//             the level above that drain into them (integer atomics), and the walks
+//             the level above that drain into them (integer atomics), and the rounds
 //             run again with those inflows added to the seeds, giving every node
-//             its full total; level 0 then gives every cell its full total.
+//             its full total; at level 0 the inflows of a tile's entries are added
+//             along their in-tile paths to the totals kept from the way up.
+// A constant seed needs only the counts: its totals are count x seed.
 // A receiver cycle shows as a successor pointer that outlives the rounds; it is
 // reported in the status word (the result is then unspecified).
 #include <algorithm>
 #include <cmath>
+#include "pff_coop.cuh"
 #include "pff_internal.h"
 
 namespace pff {
@@ -43,6 +46,7 @@ constexpr int TR_S1 = 8;                 // level-1 block side in tiles
 constexpr int TR_MAXLEV = 20;
 constexpr int TR_SMEM_NODES = 8192;      // nodes of a block kept in shared memory
 constexpr int TR_NODE_BYTES = 24;        // lo, hi, cnt, lpar, jmp, tn
+constexpr int TR_ALL_TILES = 4;          // one launch for the whole accumulation up to so many tiles per SM
 
 // status bits
 constexpr int TR_ERR_RCV = 1;       // a receiver index out of range
@@ -75,7 +79,11 @@ struct TreeArgs {
     long long *In0;
     unsigned *Inc0;
     int *up0;            // per cell: level-1 position of its tile terminal, or -1
-    int *status;         // [0] error bits, [1] max |seed| bits
+    long long *T0;       // per cell: in-tile total (weighted seeds)
+    unsigned *C0;        // per cell: in-tile count
+    int *status;         // [0] error bits, [1] max |seed| bits, [2] finished tiles, [8..9] grid barrier
+    int *out;            // the caller's copy of status[0] (mapped host memory), or null
+    int nzero;           // ints from status on that start at zero (status, then the levels' counts)
     long long *scr_acc;  // fallback storage for blocks larger than TR_SMEM_NODES
     unsigned *scr_cnt;
     int *scr_lpar, *scr_pend, *scr_tn;
@@ -145,7 +153,7 @@ __device__ __forceinline__ float from_fixed(long long v, int s)
 }
 
 // max |seed| over the grid (as f32 bits: non-negative floats order as integers)
-__global__ void k_tree_seedmax(const float *__restrict__ w, int N, int *status)
+__device__ __forceinline__ void tree_seedmax(const float *__restrict__ w, int N, int *status)
 {
     unsigned m = 0;
     bool bad = false;
@@ -170,6 +178,8 @@ __global__ void k_tree_seedmax(const float *__restrict__ w, int N, int *status)
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&status[0], TR_ERR_SEED);
 }
 
+__global__ void k_tree_seedmax(const float *__restrict__ w, int N, int *status) { tree_seedmax(w, N, status); }
+
 // ---- accumulation by pointer doubling -------------------------------------------------------
 // Within a block, with A the donor -> receiver adjacency restricted to the block,
 // the upstream sums are Q = sum_j A^j w = prod_i (I + A^(2^i)) w (A is nilpotent
@@ -182,7 +192,7 @@ __global__ void k_tree_seedmax(const float *__restrict__ w, int N, int *status)
 //
 // jmp[k]: successor 2^i steps down, or -1.  Register copies of each thread's
 // nodes (RPT per thread) hold the start-of-round values.
-template <int RPT, int NT>
+template <int RPT, int NT, bool VAL>
 __device__ __forceinline__ bool doubling_rounds(int n, int *jmp, unsigned *lo, unsigned *hi, unsigned *cnt,
                                                 int max_rounds)
 {
@@ -199,8 +209,10 @@ __device__ __forceinline__ bool doubling_rounds(int n, int *jmp, unsigned *lo, u
             if (k < n) {
                 sj[j] = jmp[k];
                 if (sj[j] >= 0) {
-                    sl[j] = lo[k];
-                    sh[j] = hi[k];
+                    if (VAL) {
+                        sl[j] = lo[k];
+                        sh[j] = hi[k];
+                    }
                     sc[j] = cnt[k];
                     nj[j] = jmp[sj[j]];
                     live = true;
@@ -212,8 +224,10 @@ __device__ __forceinline__ bool doubling_rounds(int n, int *jmp, unsigned *lo, u
         for (int j = 0; j < RPT; ++j) {
             if (sj[j] >= 0) {
                 const int k = threadIdx.x + j * NT;
-                const unsigned old = atomicAdd(&lo[sj[j]], sl[j]);
-                atomicAdd(&hi[sj[j]], sh[j] + (old + sl[j] < old ? 1u : 0u));
+                if (VAL) {
+                    const unsigned old = atomicAdd(&lo[sj[j]], sl[j]);
+                    atomicAdd(&hi[sj[j]], sh[j] + (old + sl[j] < old ? 1u : 0u));
+                }
                 atomicAdd(&cnt[sj[j]], sc[j]);
                 jmp[k] = nj[j];
             }
@@ -226,43 +240,76 @@ __device__ __forceinline__ bool doubling_rounds(int n, int *jmp, unsigned *lo, u
     return !__syncthreads_or(live);
 }
 
-// ---- level 0: one CTA per tile ---------------------------------------------------------------
-// The same doubling rounds as doubling_rounds(), with each 64-bit total held as
-// two 32-bit halves in shared memory: 32-bit shared atomics are single
-// operations, 64-bit ones are not.  The low half's atomic returns the old value,
-// so the adder whose addition wraps it adds the carry to the high half; every
-// wrap is counted exactly once, and the 64-bit sum is exact.
+// ---- level 0: a group of 256 threads per tile ---------------------------------------------
+// The cells of a tw x th tile that another tile's exit can enter: its perimeter when the
+// receivers are local, else every cell.  Entry e as a local index (row * 32 + column).
+__device__ __forceinline__ int tree_entries(const TreeArgs &a, int tw, int th)
+{
+    if (!a.local) return tw * th;
+    return tw + (th > 1 ? tw : 0) + max(th - 2, 0) * (tw > 1 ? 2 : 1);
+}
+__device__ __forceinline__ int tree_entry(const TreeArgs &a, int e, int tw, int th)
+{
+    int lx, ly;
+    if (!a.local) { ly = e / tw; lx = e - ly * tw; }
+    else if (e < tw) { lx = e; ly = 0; }
+    else if (e < 2 * tw && th > 1) { lx = e - tw; ly = th - 1; }
+    else if (tw > 1) { const int f = e - 2 * tw; lx = (f & 1) ? tw - 1 : 0; ly = 1 + (f >> 1); }
+    else { lx = 0; ly = 1 + e - 2; }
+    return ly * TR_T + lx;
+}
+
+// Pass 0, level 0, one tile by a group of 256 threads (t: thread of the group; sync: the
+// group's barrier).  The same doubling rounds as doubling_rounds(), with each 64-bit total
+// held as two 32-bit halves in shared memory: 32-bit shared atomics are single
+// operations, 64-bit ones are not.  The low half's atomic returns the old value, so the
+// adder whose addition wraps it adds the carry to the high half; every wrap is counted
+// exactly once, and the 64-bit sum is exact.
 //
-// DOWN = false: in-tile totals, level-1 nodes for the exits, up0 for the cells
-// other tiles can drain into.  DOWN = true: totals with the inflows, written as
-// Q (f32) and counts.
-template <bool DOWN>
-__global__ void __launch_bounds__(TR_T0_THREADS) k_tree_tile(const int32_t *__restrict__ rcv,
-                                                             const float *__restrict__ w, float value,
-                                                             float *Q, unsigned *counts, TreeArgs a)
+// VAL = false (a constant seed): only the counts are formed; a total is count x seed, the
+// same integer.
+//
+// Writes the in-tile totals of every cell (T0, C0), the level-1 nodes of the exits, and
+// up0 for the cells other tiles can drain into.
+//
+// Bound by the rounds' shared-memory atomics (about 7 rounds; 72 % issue active).
+template <bool VAL, class Sync>
+__device__ __forceinline__ void tree_tile_up(const TreeArgs &a, const int32_t *__restrict__ rcv,
+                                             const float *__restrict__ w, int s, int tile, unsigned char *smem, int t,
+                                             Sync sync)
 {
     constexpr int RPT = TR_TC / TR_T0_THREADS;
-    __shared__ unsigned lo[TR_TC], hi[TR_TC];
-    __shared__ unsigned cnt[TR_TC];
-    __shared__ int jmp[TR_TC];
-    __shared__ int lpar[TR_TC];  // -2 no cell, -1 root, -3 exit, else in-tile receiver
-    __shared__ int s_n, s_base, s_err;
-    const int tile = blockIdx.x;
+    unsigned *cnt = reinterpret_cast<unsigned *>(smem), *lo = cnt + TR_TC, *hi = lo + (VAL ? TR_TC : 0);
+    uint16_t *jmp = reinterpret_cast<uint16_t *>(hi + (VAL ? TR_TC : 0));
+    int16_t *lpar = reinterpret_cast<int16_t *>(jmp + TR_TC);  // -2 no cell, -1 root, -3 exit, else in-tile receiver
+    int *sv = reinterpret_cast<int *>(lpar + TR_TC);           // [0] exits, [1] base, [2] error, [3] live rounds flag
+    constexpr uint16_t DEAD = 0xffff;
     const int tx = tile % a.ntx, ty = tile / a.ntx;
     const int x0 = tx * TR_T, y0 = ty * TR_T;
     const int tw = min(TR_T, a.nx - x0), th = min(TR_T, a.ny - y0);
-    const int s = fixed_shift(w ? (unsigned)a.status[1] : __float_as_uint(fabsf(value)), a.N);
-    const long long cval = w ? 0 : to_fixed(value, s);
-    if (threadIdx.x == 0) { s_n = 0; s_err = 0; }
-    for (int k = threadIdx.x; k < TR_TC; k += TR_T0_THREADS) {
-        const int lx = k & (TR_T - 1), ly = k >> 5;
+    const int lx = t & (TR_T - 1), ly0 = t >> 5;  // a thread's cells: rows ly0 + 8 j
+    if (t < 4) sv[t] = 0;
+    sync();
+    int rr[RPT];
+    float wv[RPT];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const bool in = lx < tw && ly0 + 8 * j < th;
+        const int gi = (y0 + ly0 + 8 * j) * a.nx + x0 + lx;
+        rr[j] = in ? rcv[gi] : -1;
+        wv[j] = VAL && in ? w[gi] : 0.f;
+    }
+    unsigned alive = 0;  // this thread's cells whose pointer is still alive
+    bool exit_[RPT];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const int k = t + j * TR_T0_THREADS, ly = ly0 + 8 * j;
         int lp = -2;
-        unsigned long long sv = 0;
-        unsigned sc = 0;
+        unsigned long long v = 0;
         if (lx < tw && ly < th) {
             const int gi = (y0 + ly) * a.nx + x0 + lx;
-            int r = rcv[gi];
-            if (r < 0 || r >= a.N) { atomicOr(&s_err, TR_ERR_RCV); r = gi; }
+            int r = rr[j];
+            if (r < 0 || r >= a.N) { atomicOr(&sv[2], TR_ERR_RCV); r = gi; }
             const int d = r - gi;
             if (d == 0) lp = -1;
             else if (d == 1 && lx + 1 < tw) lp = k + 1;  // D4 neighbours without a division
@@ -273,141 +320,254 @@ __global__ void __launch_bounds__(TR_T0_THREADS) k_tree_tile(const int32_t *__re
                 const int ry = r / a.nx, rx = r - ry * a.nx;
                 lp = (rx >= x0 && rx < x0 + tw && ry >= y0 && ry < y0 + th) ? (ry - y0) * TR_T + rx - x0 : -3;
             }
-            sv = (unsigned long long)(w ? to_fixed(w[gi], s) : cval);
-            sc = 1;
-            if (DOWN && a.marker[gi]) {
-                sv += (unsigned long long)a.In0[gi];
-                sc += a.Inc0[gi];
-            }
+            if (VAL) v = (unsigned long long)to_fixed(wv[j], s);
         }
-        lpar[k] = lp;
-        jmp[k] = lp >= 0 ? lp : -1;
-        lo[k] = (unsigned)sv;
-        hi[k] = (unsigned)(sv >> 32);
-        cnt[k] = sc;
+        lpar[k] = (int16_t)lp;
+        exit_[j] = lp == -3;
+        jmp[k] = lp >= 0 ? (uint16_t)lp : DEAD;
+        alive |= (lp >= 0 ? 1u : 0u) << j;
+        cnt[k] = lp != -2 ? 1u : 0u;
+        if (VAL) {
+            lo[k] = (unsigned)v;
+            hi[k] = (unsigned)(v >> 32);
+        }
     }
-    __syncthreads();
+    sync();
     // doubling rounds: the longest in-tile path is < 1024 = 2^10 cells
     bool cyc = false;
-    unsigned alive = 0;  // this thread's cells whose pointer is still alive
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) alive |= (jmp[threadIdx.x + j * TR_T0_THREADS] >= 0 ? 1u : 0u) << j;
     for (int r = 0;; ++r) {
         int sj[RPT], nj[RPT];
         unsigned sl[RPT], sh[RPT], sc[RPT];
+        if (alive) sv[3] = r + 1;
 #pragma unroll
         for (int j = 0; j < RPT; ++j) {
-            const int k = threadIdx.x + j * TR_T0_THREADS;
+            const int k = t + j * TR_T0_THREADS;
             sj[j] = -1;
             if (alive >> j & 1u) {
                 sj[j] = jmp[k];
-                sl[j] = lo[k];
-                sh[j] = hi[k];
+                if (VAL) {
+                    sl[j] = lo[k];
+                    sh[j] = hi[k];
+                }
                 sc[j] = cnt[k];
                 nj[j] = jmp[sj[j]];
-                if (nj[j] < 0) alive &= ~(1u << j);
+                if (nj[j] == DEAD) alive &= ~(1u << j);
             }
         }
-        if (!__syncthreads_or(sj[0] >= 0 || sj[1] >= 0 || sj[2] >= 0 || sj[3] >= 0)) break;
+        sync();
+        if (sv[3] != r + 1) break;
         if (r == 10) { cyc = true; break; }  // a path longer than the tile: a cycle
 #pragma unroll
         for (int j = 0; j < RPT; ++j) {
             if (sj[j] >= 0) {
-                const int k = threadIdx.x + j * TR_T0_THREADS;
-                const unsigned old = atomicAdd(&lo[sj[j]], sl[j]);
-                atomicAdd(&hi[sj[j]], sh[j] + (old + sl[j] < old ? 1u : 0u));
+                const int k = t + j * TR_T0_THREADS;
+                if (VAL) {
+                    const unsigned old = atomicAdd(&lo[sj[j]], sl[j]);
+                    atomicAdd(&hi[sj[j]], sh[j] + (old + sl[j] < old ? 1u : 0u));
+                }
                 atomicAdd(&cnt[sj[j]], sc[j]);
-                jmp[k] = nj[j];
+                jmp[k] = (uint16_t)nj[j];
             }
         }
-        __syncthreads();
+        sync();
     }
-    if (cyc && threadIdx.x == 0) s_err |= TR_ERR_CYCLE;
+    if (cyc && t == 0) atomicOr(&sv[2], TR_ERR_CYCLE);
 
-    if (DOWN) {
-        for (int k = threadIdx.x; k < TR_TC; k += TR_T0_THREADS) {
-            const int lx = k & (TR_T - 1), ly = k >> 5;
-            if (lx < tw && ly < th) {
-                const int gi = (y0 + ly) * a.nx + x0 + lx;
-                if (Q) Q[gi] = from_fixed((long long)(((unsigned long long)hi[k] << 32) | lo[k]), s);
-                if (counts) counts[gi] = cnt[k];
-                a.marker[gi] = 0;  // leave the markers clear for the next call
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0 && s_err) atomicOr(&a.status[0], s_err);
-        return;
-    }
-
-    // exits -> level-1 nodes of this tile's level-1 block
+    // totals, and exits -> level-1 nodes of this tile's level-1 block
     const TreeLevel &L1 = a.lv[1];
     const int bx = tx / L1.side, by = ty / L1.side;
     const int b1 = by * L1.nbx + bx;
     const BlockGeo g1 = block_geo(bx, by, L1.side, a.ntx, a.nty);
-    int mine = 0;
-    for (int k = threadIdx.x; k < TR_TC; k += TR_T0_THREADS) mine += lpar[k] == -3;
-    for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&s_n, mine);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_base = s_n ? atomicAdd(&L1.cnt[b1], s_n) : 0;
-        if (s_base + s_n > g1.tiles * a.cap0) { s_err |= TR_ERR_CAP; s_n = -1; }
-        s_n = s_n < 0 ? -1 : 0;  // reused as the rank counter below (-1: no room)
+    int rank[RPT];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const unsigned m = __ballot_sync(0xffffffffu, exit_[j]);
+        int base = 0;
+        if (m && (t & 31) == 0) base = atomicAdd(&sv[0], __popc(m));
+        rank[j] = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << (t & 31)) - 1u));
     }
-    __syncthreads();
-    const int slot0 = g1.tile_off * a.cap0 + s_base;
-    int *q = jmp;  // free after the rounds: level-1 position of each exit
-    for (int k = threadIdx.x; k < TR_TC; k += TR_T0_THREADS) {
+    sync();
+    if (t == 0) {
+        const int n = sv[0];
+        int base = n ? atomicAdd(&L1.cnt[b1], n) : 0;
+        if (base + n > g1.tiles * a.cap0) {
+            atomicOr(&sv[2], TR_ERR_CAP);
+            base = -1;
+        }
+        sv[1] = base;
+    }
+    sync();
+    const int base = sv[1], slot0 = g1.tile_off * a.cap0 + base;
+    int *q = reinterpret_cast<int *>(cnt);  // level-1 position of each exit, once its count is written
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const int k = t + j * TR_T0_THREADS, ly = ly0 + 8 * j;
         int qk = -1;
-        if (lpar[k] == -3 && s_n >= 0) {
-            const int lx = k & (TR_T - 1), ly = k >> 5;
+        if (lx < tw && ly < th) {
             const int gi = (y0 + ly) * a.nx + x0 + lx;
-            const int r = rcv[gi];
-            qk = slot0 + atomicAdd(&s_n, 1);
-            L1.W[qk] = (long long)(((unsigned long long)hi[k] << 32) | lo[k]);
-            L1.C[qk] = cnt[k];
-            L1.rawpar[qk] = r;
-            L1.src[qk] = gi;
-            a.In0[r] = 0;
-            a.Inc0[r] = 0;
-            a.marker[r] = 1;
-            if (a.local) {  // the entry must be on the perimeter of its own tile
-                const int ry = r / a.nx, rx = r - ry * a.nx;
-                const int ex = rx % TR_T, ey = ry % TR_T;
-                if (!(ex == 0 || ey == 0 || ex == TR_T - 1 || ey == TR_T - 1 || rx == a.nx - 1 || ry == a.ny - 1))
-                    atomicOr(&s_err, TR_ERR_NONLOCAL);
+            const long long tot = VAL ? (long long)(((unsigned long long)hi[k] << 32) | lo[k]) : 0;
+            const unsigned c = cnt[k];
+            a.C0[gi] = c;
+            if (VAL) a.T0[gi] = tot;
+            if (exit_[j] && base >= 0) {
+                const int r = rr[j];
+                qk = slot0 + rank[j];
+                if (VAL) L1.W[qk] = tot;
+                L1.C[qk] = c;
+                L1.rawpar[qk] = r;
+                L1.src[qk] = gi;
+                if (VAL) a.In0[r] = 0;
+                a.Inc0[r] = 0;
+                a.marker[r] = 1;
+                if (a.local) {  // the entry must be on the perimeter of its own tile
+                    const int ry = r / a.nx, rx = r - ry * a.nx;
+                    const int ex = rx % TR_T, ey = ry % TR_T;
+                    if (!(ex == 0 || ey == 0 || ex == TR_T - 1 || ey == TR_T - 1 || rx == a.nx - 1 || ry == a.ny - 1))
+                        atomicOr(&sv[2], TR_ERR_NONLOCAL);
+                }
             }
         }
         q[k] = qk;
     }
-    __syncthreads();
+    sync();
     // up0 = level-1 position of the cell's tile terminal (if that is an exit), for
     // the cells another tile's exit can enter: the perimeter when local, every cell
     // otherwise; each walks down to its terminal
-    const int per = a.local ? (tw + tw + max(th - 2, 0) * 2 - (th == 1 ? tw : 0)) : tw * th;
-    for (int e = threadIdx.x; e < per; e += TR_T0_THREADS) {
-        int lx, ly;
-        if (!a.local) { ly = e / tw; lx = e - ly * tw; }
-        else if (e < tw) { lx = e; ly = 0; }
-        else if (e < 2 * tw && th > 1) { lx = e - tw; ly = th - 1; }
-        else { const int f = e - 2 * tw; lx = (f & 1) ? tw - 1 : 0; ly = 1 + (f >> 1); }
-        int t = ly * TR_T + lx;
-        for (int st = 0; st < TR_TC && lpar[t] >= 0; ++st) t = lpar[t];
-        a.up0[(y0 + ly) * a.nx + x0 + lx] = lpar[t] == -3 ? q[t] : -1;
+    const int per = tree_entries(a, tw, th);
+    for (int e = t; e < per; e += TR_T0_THREADS) {
+        int u = tree_entry(a, e, tw, th);
+        const int gi = (y0 + (u >> 5)) * a.nx + x0 + (u & (TR_T - 1));
+        for (int st = 0; st < TR_TC && lpar[u] >= 0; ++st) u = lpar[u];
+        a.up0[gi] = lpar[u] == -3 ? q[u] : -1;
     }
-    if (threadIdx.x == 0 && s_err) atomicOr(&a.status[0], s_err);
+    if (t == 0 && sv[2]) atomicOr(&a.status[0], sv[2]);
+}
+
+// The last pass, level 0: each cell's full total = its in-tile total plus the inflows of the
+// tile's entries upstream of it.  The entries (at most 124 when local, most tiles have
+// 30-60) each walk their in-tile path and add; every other cell only reads its total back.
+// The pass was a second run of the doubling rounds with the inflows in the seeds (318 us
+// at 4096^2 against 382 for the first); reading the totals back costs 12 B per cell.
+template <bool VAL, class Sync>
+__device__ __forceinline__ void tree_tile_finish(const TreeArgs &a, const int32_t *__restrict__ rcv, int s, long long cval,
+                                                 float *Q, unsigned *counts, int tile, unsigned char *smem, int t,
+                                                 Sync sync)
+{
+    constexpr int RPT = TR_TC / TR_T0_THREADS;
+    unsigned *cnt = reinterpret_cast<unsigned *>(smem), *lo = cnt + TR_TC, *hi = lo + (VAL ? TR_TC : 0);
+    int16_t *lpar = reinterpret_cast<int16_t *>(hi + (VAL ? TR_TC : 0));  // in-tile receiver or -1
+    const int tx = tile % a.ntx, ty = tile / a.ntx;
+    const int x0 = tx * TR_T, y0 = ty * TR_T;
+    const int tw = min(TR_T, a.nx - x0), th = min(TR_T, a.ny - y0);
+    const int lx = t & (TR_T - 1), ly0 = t >> 5;
+    int rr[RPT];
+    unsigned cv[RPT];
+    long long tv[RPT];
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const bool in = lx < tw && ly0 + 8 * j < th;
+        const int gi = (y0 + ly0 + 8 * j) * a.nx + x0 + lx;
+        rr[j] = in ? rcv[gi] : -1;
+        cv[j] = in ? a.C0[gi] : 0u;
+        tv[j] = VAL && in ? a.T0[gi] : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const int k = t + j * TR_T0_THREADS, ly = ly0 + 8 * j;
+        int lp = -1;
+        if (lx < tw && ly < th) {
+            const int gi = (y0 + ly) * a.nx + x0 + lx, r = rr[j], d = r - gi;
+            if (d == 1 && lx + 1 < tw) lp = k + 1;
+            else if (d == -1 && lx > 0) lp = k - 1;
+            else if (d == a.nx && ly + 1 < th) lp = k + TR_T;
+            else if (d == -a.nx && ly > 0) lp = k - TR_T;
+            else if (d != 0 && r >= 0 && r < a.N) {
+                const int ry = r / a.nx, rx = r - ry * a.nx;
+                if (rx >= x0 && rx < x0 + tw && ry >= y0 && ry < y0 + th) lp = (ry - y0) * TR_T + rx - x0;
+            }
+        }
+        lpar[k] = (int16_t)lp;
+        cnt[k] = cv[j];
+        if (VAL) {
+            lo[k] = (unsigned)(unsigned long long)tv[j];
+            hi[k] = (unsigned)((unsigned long long)tv[j] >> 32);
+        }
+    }
+    sync();
+    const int per = tree_entries(a, tw, th);
+    for (int e = t; e < per; e += TR_T0_THREADS) {
+        int u = tree_entry(a, e, tw, th);
+        const int gi = (y0 + (u >> 5)) * a.nx + x0 + (u & (TR_T - 1));
+        if (!a.marker[gi]) continue;
+        const unsigned ic = a.Inc0[gi];
+        const unsigned long long iv = VAL ? (unsigned long long)a.In0[gi] : 0;
+        for (int st = 0; st < TR_TC && u >= 0; ++st) {
+            atomicAdd(&cnt[u], ic);
+            if (VAL) {
+                const unsigned old = atomicAdd(&lo[u], (unsigned)iv);
+                atomicAdd(&hi[u], (unsigned)(iv >> 32) + (old + (unsigned)iv < old ? 1u : 0u));
+            }
+            u = lpar[u];
+        }
+    }
+    sync();
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const int k = t + j * TR_T0_THREADS, ly = ly0 + 8 * j;
+        if (lx < tw && ly < th) {
+            const int gi = (y0 + ly) * a.nx + x0 + lx;
+            const unsigned c = cnt[k];
+            if (Q) {
+                const long long v = VAL ? (long long)(((unsigned long long)hi[k] << 32) | lo[k]) : cval * (long long)c;
+                Q[gi] = from_fixed(v, s);
+            }
+            if (counts) counts[gi] = c;
+        }
+    }
+}
+
+template <bool VAL>
+struct TreeTile {
+    static constexpr int BYTES = TR_TC * 4 * (VAL ? 3 : 1) + TR_TC * 4 + 16;  // shared memory of a tile pass
+};
+
+// the shift of the fixed-point seeds
+__device__ __forceinline__ int tree_shift(const TreeArgs &a, const float *w, float value)
+{
+    return fixed_shift(w ? (unsigned)vload(a.status + 1) : __float_as_uint(fabsf(value)), a.N);
+}
+
+template <bool VAL>
+__global__ void __launch_bounds__(TR_T0_THREADS) k_tree_up(const int32_t *__restrict__ rcv, const float *__restrict__ w,
+                                                           float value, TreeArgs a)
+{
+    __shared__ __align__(16) unsigned char sm[TreeTile<VAL>::BYTES];
+    tree_tile_up<VAL>(a, rcv, w, tree_shift(a, w, value), blockIdx.x, sm, threadIdx.x, []() { __syncthreads(); });
+}
+
+template <bool VAL>
+__global__ void __launch_bounds__(TR_T0_THREADS) k_tree_finish(const int32_t *__restrict__ rcv, const float *__restrict__ w,
+                                                               float value, float *Q, unsigned *counts, TreeArgs a)
+{
+    __shared__ __align__(16) unsigned char sm[TreeTile<VAL>::BYTES];
+    const int s = tree_shift(a, w, value);
+    tree_tile_finish<VAL>(a, rcv, s, w ? 0 : to_fixed(value, s), Q, counts, blockIdx.x, sm, threadIdx.x,
+                          []() { __syncthreads(); });
+    // the status is final since the passes before: the first block reports it
+    if (a.out && blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile int *)a.out = a.status[0];
+        __threadfence_system();
+    }
 }
 
 // ---- levels >= 1: one CTA per block -----------------------------------------------------------
 // MODE 0 up (local totals, next-level nodes, up pointers), 1 down (totals with the
 // inflows, scattered one level down), 2 top (up with no exits, then scattered).
-template <int MODE>
-__global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
+template <int MODE, bool VAL>
+__device__ __forceinline__ void tree_level(int L, const TreeArgs &a, int b, unsigned char *tsm)
 {
-    extern __shared__ __align__(16) unsigned char tsm[];
     __shared__ int s_n, s_base, s_err;
     const TreeLevel &V = a.lv[L];
-    const int b = blockIdx.x;
     const int bx = b % V.nbx, by = b / V.nbx;
     const BlockGeo g = block_geo(bx, by, V.side, a.ntx, a.nty);
     const int base = g.tile_off * a.cap0;
@@ -455,17 +615,19 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
         const int lp = p < 0 ? -1 : (p >= base && p < base + n ? p - base : -3);
         lpar[k] = lp;
         jmp[k] = lp >= 0 ? lp : -1;
-        unsigned long long sv = (unsigned long long)V.W[pos];
+        unsigned long long sv = VAL ? (unsigned long long)V.W[pos] : 0;
         unsigned sc = V.C[pos];
         if (MODE == 1) {
-            sv += (unsigned long long)V.In[pos];
+            if (VAL) sv += (unsigned long long)V.In[pos];
             sc += V.Inc[pos];
         } else {
-            V.In[pos] = 0;
+            if (VAL) V.In[pos] = 0;
             V.Inc[pos] = 0;
         }
-        lo[k] = (unsigned)sv;
-        hi[k] = (unsigned)(sv >> 32);
+        if (VAL) {
+            lo[k] = (unsigned)sv;
+            hi[k] = (unsigned)(sv >> 32);
+        }
         cnt[k] = sc;
     }
     __syncthreads();
@@ -473,7 +635,7 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
     while ((1 << rounds) < n) ++rounds;
     bool ok;
     if (in_smem) {
-        ok = doubling_rounds<TR_SMEM_NODES / TR_LB_THREADS, TR_LB_THREADS>(n, jmp, lo, hi, cnt, rounds + 1);
+        ok = doubling_rounds<TR_SMEM_NODES / TR_LB_THREADS, TR_LB_THREADS, VAL>(n, jmp, lo, hi, cnt, rounds + 1);
     } else {
         // the same rounds with the start-of-round values in a second scratch (tn holds the next pointers)
         ok = true;
@@ -489,7 +651,7 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
             for (int k = threadIdx.x; k < n; k += TR_LB_THREADS) {  // start-of-round snapshot
                 const int j = jmp[k];
                 if (j >= 0) {
-                    a.scr_acc2[base + k] = (long long)(((unsigned long long)hi[k] << 32) | lo[k]);
+                    if (VAL) a.scr_acc2[base + k] = (long long)(((unsigned long long)hi[k] << 32) | lo[k]);
                     a.scr_cnt2[base + k] = cnt[k];
                 }
             }
@@ -497,9 +659,11 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
             for (int k = threadIdx.x; k < n; k += TR_LB_THREADS) {
                 const int j = jmp[k];
                 if (j >= 0) {
-                    const unsigned long long x = (unsigned long long)a.scr_acc2[base + k];
-                    const unsigned old = atomicAdd(&lo[j], (unsigned)x);
-                    atomicAdd(&hi[j], (unsigned)(x >> 32) + (old + (unsigned)x < old ? 1u : 0u));
+                    if (VAL) {
+                        const unsigned long long x = (unsigned long long)a.scr_acc2[base + k];
+                        const unsigned old = atomicAdd(&lo[j], (unsigned)x);
+                        atomicAdd(&hi[j], (unsigned)(x >> 32) + (old + (unsigned)x < old ? 1u : 0u));
+                    }
                     atomicAdd(&cnt[j], a.scr_cnt2[base + k]);
                 }
             }
@@ -519,14 +683,14 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
             if (L == 1) {
                 const int cell = V.rawpar[pos];
                 if (cell < 0 || cell >= a.N) continue;  // flagged in the up pass
-                atomicAdd((unsigned long long *)&a.In0[cell], ((unsigned long long)hi[k] << 32) | lo[k]);
+                if (VAL) atomicAdd((unsigned long long *)&a.In0[cell], ((unsigned long long)hi[k] << 32) | lo[k]);
                 atomicAdd(&a.Inc0[cell], cnt[k]);
             } else {
                 const TreeLevel &D = a.lv[L - 1];
                 const int sp = V.src[pos];
                 const int t = (sp >= 0 && sp < a.slots) ? D.par[sp] : -1;
                 if (t < 0 || t >= a.slots) continue;
-                atomicAdd((unsigned long long *)&D.In[t], ((unsigned long long)hi[k] << 32) | lo[k]);
+                if (VAL) atomicAdd((unsigned long long *)&D.In[t], ((unsigned long long)hi[k] << 32) | lo[k]);
                 atomicAdd(&D.Inc[t], cnt[k]);
             }
         }
@@ -567,7 +731,7 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
         if (lpar[k] == -3 && s_n >= 0) {
             const int pos = base + k;
             q = slot0 + atomicAdd(&s_n, 1);
-            U.W[q] = (long long)(((unsigned long long)hi[k] << 32) | lo[k]);
+            if (VAL) U.W[q] = (long long)(((unsigned long long)hi[k] << 32) | lo[k]);
             U.C[q] = cnt[k];
             U.rawpar[q] = V.par[pos];
             U.src[q] = pos;
@@ -580,6 +744,74 @@ __global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
         V.up[base + k] = lpar[t] == -3 ? jmp[t] : -1;
     }
     if (threadIdx.x == 0 && s_err) atomicOr(&a.status[0], s_err);
+}
+
+template <int MODE, bool VAL>
+__global__ void __launch_bounds__(TR_LB_THREADS) k_tree_level(int L, TreeArgs a)
+{
+    extern __shared__ __align__(16) unsigned char tsm[];
+    tree_level<MODE, VAL>(L, a, blockIdx.x, tsm);
+}
+
+// The whole accumulation in one cooperative launch, a grid barrier between the passes, for
+// grids whose passes are shorter than their launches: at 512 x 512 the seven launches,
+// four memsets and the status read took 64 us of device time and 111 us in all.  Larger
+// grids take the separate launches, whose tile passes hold twice the threads per SM.
+template <bool VAL>
+__global__ void __launch_bounds__(TR_LB_THREADS, 1) k_tree_all(const int32_t *__restrict__ rcv, const float *__restrict__ w,
+                                                               float value, float *Q, unsigned *counts, TreeArgs a)
+{
+    extern __shared__ __align__(16) unsigned char tsm[];
+    __shared__ int dead;
+    const int gtid = blockIdx.x * TR_LB_THREADS + threadIdx.x, gthreads = gridDim.x * TR_LB_THREADS;
+    const int grp = threadIdx.x / TR_T0_THREADS, gt = threadIdx.x & (TR_T0_THREADS - 1);
+    constexpr int ngrp = TR_LB_THREADS / TR_T0_THREADS;
+    if (threadIdx.x == 0) dead = 0;
+    if (gridDim.x == 1)  // one block clears its counters itself
+        for (int k = threadIdx.x; k < a.nzero; k += TR_LB_THREADS) a.status[k] = 0;
+    GridBar bar{a.status + 8, 0};
+    __syncthreads();
+    if (((uintptr_t)a.marker & 15) == 0) {
+        for (int k = gtid; k < (a.N + 15) / 16; k += gthreads)  // the array is padded to 256 bytes
+            reinterpret_cast<uint4 *>(a.marker)[k] = make_uint4(0, 0, 0, 0);
+    } else {
+        for (int k = gtid; k < a.N; k += gthreads) a.marker[k] = 0;
+    }
+    if (VAL) tree_seedmax(w, a.N, a.status);
+    if (!bar.sync(&dead)) return;
+    const int s = tree_shift(a, w, value), ntiles = a.ntx * a.nty;
+    auto gsync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "n"(TR_T0_THREADS) : "memory"); };
+    unsigned char *gsm = tsm + grp * ((TreeTile<VAL>::BYTES + 15) / 16 * 16);
+    for (int k = grp * gridDim.x + blockIdx.x; k < ntiles; k += ngrp * gridDim.x) {
+        tree_tile_up<VAL>(a, rcv, w, s, k, gsm, gt, gsync);
+        gsync();
+    }
+    if (!bar.sync(&dead)) return;
+    for (int L = 1; L < a.nlev; ++L) {
+        for (int b = blockIdx.x; b < a.lv[L].nbx * a.lv[L].nby; b += gridDim.x) {
+            tree_level<0, VAL>(L, a, b, tsm);
+            __syncthreads();
+        }
+        if (!bar.sync(&dead)) return;
+    }
+    if (blockIdx.x == 0) tree_level<2, VAL>(a.nlev, a, 0, tsm);
+    if (!bar.sync(&dead)) return;
+    for (int L = a.nlev - 1; L >= 1; --L) {
+        for (int b = blockIdx.x; b < a.lv[L].nbx * a.lv[L].nby; b += gridDim.x) {
+            tree_level<1, VAL>(L, a, b, tsm);
+            __syncthreads();
+        }
+        if (!bar.sync(&dead)) return;
+    }
+    const long long cval = w ? 0 : to_fixed(value, s);
+    for (int k = grp * gridDim.x + blockIdx.x; k < ntiles; k += ngrp * gridDim.x) {
+        tree_tile_finish<VAL>(a, rcv, s, cval, Q, counts, k, gsm, gt, gsync);
+        gsync();
+    }
+    if (a.out && gtid == 0) {
+        *(volatile int *)a.out = vload(a.status);
+        __threadfence_system();
+    }
 }
 
 // ---- host --------------------------------------------------------------------------------------
@@ -611,58 +843,24 @@ static TreePlan tree_plan(int nx, int ny, int local)
     return p;
 }
 
-static size_t tree_bytes(const TreePlan &p, int N)
+// The workspace's layout; a.status and the levels' counts are contiguous.
+static TreeArgs tree_carve(const TreePlan &p, int nx, int ny, int local, void *workspace, size_t bytes, size_t *used)
 {
-    const size_t S = (size_t)p.slots;
-    size_t b = 0;
-    b += Carver::round((size_t)N) + Carver::round(8 * (size_t)N) + 2 * Carver::round(4 * (size_t)N);  // level 0
-    b += Carver::round(sizeof(int) * 64);                                                             // status
-    b += 2 * Carver::round(8 * S) + 5 * Carver::round(4 * S);                                         // scratch
-    for (int L = 1; L <= p.nlev; ++L)
-        b += 2 * Carver::round(8 * S) + 6 * Carver::round(4 * S) + Carver::round(sizeof(int) * (size_t)p.nb[L]);
-    return b + 4096;
-}
-
-}  // namespace pff
-
-using namespace pff;
-
-extern "C" size_t pff_accumulate_tree_workspace_bytes(int nx, int ny, int local)
-{
-    if (nx < 1 || ny < 1 || (long long)nx * ny > (1LL << 30)) return 0;
-    return tree_bytes(tree_plan(nx, ny, local), nx * ny);
-}
-
-extern "C" int pff_accumulate_tree(const int32_t *receivers, const float *weights, float value, float *Q,
-                                   uint32_t *counts, int nx, int ny, int local, void *workspace,
-                                   size_t workspace_bytes, void *stream)
-{
-    clear_error();
-    if (nx < 1 || ny < 1 || (long long)nx * ny > (1LL << 30) || !receivers || (!Q && !counts)) {
-        set_error("pff_accumulate_tree: bad arguments");
-        return PFF_ERR_ARG;
-    }
+    Carver cv(workspace, bytes);
     const int N = nx * ny;
-    const TreePlan p = tree_plan(nx, ny, local);
-    if (!workspace || workspace_bytes < tree_bytes(p, N)) {
-        set_error("pff_accumulate_tree: workspace too small");
-        return PFF_ERR_WORKSPACE;
-    }
-    if (!weights && !(fabsf(value) <= 3.4028235e38f)) {
-        set_error("pff_accumulate_tree: non-finite seed value");
-        return PFF_ERR_ARG;
-    }
-    cudaStream_t st = S(stream);
-    Carver cv(workspace, workspace_bytes);
     TreeArgs a{};
     a.nx = nx; a.ny = ny; a.ntx = p.ntx; a.nty = p.nty; a.N = N;
     a.cap0 = p.cap0; a.nlev = p.nlev; a.local = local ? 1 : 0;
     a.slots = (int)p.slots;
     a.marker = cv.take<unsigned char>(N);
     a.In0 = cv.take<long long>(N);
+    a.T0 = cv.take<long long>(N);
     a.Inc0 = cv.take<unsigned>(N);
+    a.C0 = cv.take<unsigned>(N);
     a.up0 = cv.take<int>(N);
-    a.status = cv.take<int>(64);
+    a.nzero = 64;
+    for (int L = 1; L <= p.nlev; ++L) a.nzero += p.nb[L];
+    a.status = cv.take<int>(a.nzero);
     const size_t S = (size_t)p.slots;
     a.scr_acc = cv.take<long long>(S);
     a.scr_cnt = cv.take<unsigned>(S);
@@ -671,6 +869,7 @@ extern "C" int pff_accumulate_tree(const int32_t *receivers, const float *weight
     a.scr_tn = cv.take<int>(S);
     a.scr_acc2 = cv.take<long long>(S);
     a.scr_cnt2 = cv.take<unsigned>(S);
+    int *cnt = a.status ? a.status + 64 : nullptr;
     for (int L = 1; L <= p.nlev; ++L) {
         TreeLevel &V = a.lv[L];
         V.W = cv.take<long long>(S);
@@ -681,44 +880,133 @@ extern "C" int pff_accumulate_tree(const int32_t *receivers, const float *weight
         V.par = cv.take<int>(S);
         V.up = cv.take<int>(S);
         V.src = cv.take<int>(S);
-        V.cnt = cv.take<int>(p.nb[L]);
+        V.cnt = cnt;
+        if (cnt) cnt += p.nb[L];
         V.side = p.side[L];
         V.nbx = p.nbx[L];
         V.nby = p.nby[L];
     }
     // the top level's exits would go to level nlev+1: there are none (one block)
     a.lv[p.nlev + 1] = a.lv[p.nlev];
+    if (used) *used = cv.off;
+    return a;
+}
 
-    PFF_CUDA(cudaMemsetAsync(a.marker, 0, (size_t)N, st));
-    PFF_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int) * 64, st));
-    for (int L = 1; L <= p.nlev; ++L) PFF_CUDA(cudaMemsetAsync(a.lv[L].cnt, 0, sizeof(int) * p.nb[L], st));
-    if (weights) {
-        int dev = 0, nsm = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const int grid = std::min(div_up(N, 256), nsm * 8);
-        { k_tree_seedmax<<<grid, 256, 0, st>>>(weights, N, a.status); count_launch(); }
-    }
+static size_t tree_bytes(const TreePlan &p, int nx, int ny)
+{
+    size_t used = 0;
+    tree_carve(p, nx, ny, 1, nullptr, 0, &used);
+    return used + 4096;
+}
+
+template <bool VAL>
+static int launch_tree(const TreePlan &p, const TreeArgs &a_, const int32_t *receivers, const float *weights, float value,
+                       float *Q, uint32_t *counts, cudaStream_t st)
+{
+    TreeArgs a = a_;
+    int dev = 0, nsm = 148, coop = 0;
+    PFF_CUDA(cudaGetDevice(&dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     const size_t smem = (size_t)TR_SMEM_NODES * TR_NODE_BYTES;  // per-device attribute: set on every call
-    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PFF_PROBED("k_tree_tile<up>", st,
-               k_tree_tile<false><<<p.ntiles, TR_T0_THREADS, 0, st>>>(receivers, weights, value, Q, counts, a));
+    if (coop && p.ntiles <= TR_ALL_TILES * nsm) {
+        const int blocks = std::min(nsm, div_up(p.ntiles, TR_LB_THREADS / TR_T0_THREADS));
+        if (blocks > 1) PFF_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int) * (size_t)a.nzero, st));
+        PFF_CUDA(cudaFuncSetAttribute(k_tree_all<VAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        void *args[] = {(void *)&receivers, (void *)&weights, &value, &Q, &counts, &a};
+        PFF_CUDA(cudaLaunchCooperativeKernel((void *)k_tree_all<VAL>, blocks, TR_LB_THREADS, args, smem, st));
+        count_launch();
+        return check_cuda("pff_accumulate_tree");
+    }
+    PFF_CUDA(cudaMemsetAsync(a.marker, 0, (size_t)a.N, st));
+    PFF_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int) * (size_t)a.nzero, st));
+    if (VAL) {
+        const int grid = std::min(div_up(a.N, 256), nsm * 8);
+        { k_tree_seedmax<<<grid, 256, 0, st>>>(weights, a.N, a.status); count_launch(); }
+    }
+    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<0, VAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<1, VAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PFF_CUDA(cudaFuncSetAttribute(k_tree_level<2, VAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PFF_PROBED("k_tree_tile<up>", st, k_tree_up<VAL><<<p.ntiles, TR_T0_THREADS, 0, st>>>(receivers, weights, value, a));
     count_launch();
     for (int L = 1; L < p.nlev; ++L) {
-        k_tree_level<0><<<p.nb[L], TR_LB_THREADS, smem, st>>>(L, a);
+        k_tree_level<0, VAL><<<p.nb[L], TR_LB_THREADS, smem, st>>>(L, a);
         count_launch();
     }
-    { k_tree_level<2><<<1, TR_LB_THREADS, smem, st>>>(p.nlev, a); count_launch(); }
+    { k_tree_level<2, VAL><<<1, TR_LB_THREADS, smem, st>>>(p.nlev, a); count_launch(); }
     for (int L = p.nlev - 1; L >= 1; --L) {
-        k_tree_level<1><<<p.nb[L], TR_LB_THREADS, smem, st>>>(L, a);
+        k_tree_level<1, VAL><<<p.nb[L], TR_LB_THREADS, smem, st>>>(L, a);
         count_launch();
     }
     PFF_PROBED("k_tree_tile<down>", st,
-               k_tree_tile<true><<<p.ntiles, TR_T0_THREADS, 0, st>>>(receivers, weights, value, Q, counts, a));
+               k_tree_finish<VAL><<<p.ntiles, TR_T0_THREADS, 0, st>>>(receivers, weights, value, Q, counts, a));
     count_launch();
     return check_cuda("pff_accumulate_tree");
+}
+
+static int accumulate_tree(const int32_t *receivers, const float *weights, float value, float *Q, uint32_t *counts, int nx,
+                           int ny, int local, void *workspace, size_t workspace_bytes, int *out, cudaStream_t st)
+{
+    if (nx < 1 || ny < 1 || (long long)nx * ny > (1LL << 30) || !receivers || (!Q && !counts)) {
+        set_error("pff_accumulate_tree: bad arguments");
+        return PFF_ERR_ARG;
+    }
+    const TreePlan p = tree_plan(nx, ny, local);
+    if (!workspace || workspace_bytes < tree_bytes(p, nx, ny)) {
+        set_error("pff_accumulate_tree: workspace too small");
+        return PFF_ERR_WORKSPACE;
+    }
+    if (!weights && !(fabsf(value) <= 3.4028235e38f)) {
+        set_error("pff_accumulate_tree: non-finite seed value");
+        return PFF_ERR_ARG;
+    }
+    TreeArgs a = tree_carve(p, nx, ny, local, workspace, workspace_bytes, nullptr);
+    a.out = out;
+    return weights ? launch_tree<true>(p, a, receivers, weights, value, Q, counts, st)
+                   : launch_tree<false>(p, a, receivers, weights, value, Q, counts, st);
+}
+
+}  // namespace pff
+
+using namespace pff;
+
+extern "C" size_t pff_accumulate_tree_workspace_bytes(int nx, int ny, int local)
+{
+    if (nx < 1 || ny < 1 || (long long)nx * ny > (1LL << 30)) return 0;
+    return tree_bytes(tree_plan(nx, ny, local), nx, ny);
+}
+
+extern "C" int pff_accumulate_tree(const int32_t *receivers, const float *weights, float value, float *Q,
+                                   uint32_t *counts, int nx, int ny, int local, void *workspace,
+                                   size_t workspace_bytes, void *stream)
+{
+    clear_error();
+    return accumulate_tree(receivers, weights, value, Q, counts, nx, ny, local, workspace, workspace_bytes, nullptr,
+                           S(stream));
+}
+
+extern "C" int pff_accumulate_tree_run(const int32_t *receivers, const float *weights, float value, float *Q,
+                                       uint32_t *counts, int nx, int ny, int local, void *workspace,
+                                       size_t workspace_bytes, int *status, void *stream)
+{
+    clear_error();
+    if (!status) {
+        set_error("pff_accumulate_tree_run: null pointer");
+        return PFF_ERR_ARG;
+    }
+    int *host = nullptr, *dptr = nullptr;
+    PFF_TRY(pinned_ints(&host, &dptr));
+    host[0] = -1;
+    PFF_TRY(accumulate_tree(receivers, weights, value, Q, counts, nx, ny, local, workspace, workspace_bytes, dptr,
+                            S(stream)));
+    PFF_CUDA(cudaStreamSynchronize(S(stream)));
+    PFF_TRY(check_cuda("pff_accumulate_tree_run"));
+    *status = *(volatile int *)host;
+    if (*status < 0) {
+        set_error("pff_accumulate_tree_run: the passes did not end");
+        return PFF_ERR_NOCONV;
+    }
+    return PFF_OK;
 }
 
 extern "C" int pff_accumulate_tree_status(int nx, int ny, int local, void *workspace, size_t workspace_bytes,
@@ -729,18 +1017,12 @@ extern "C" int pff_accumulate_tree_status(int nx, int ny, int local, void *works
         set_error("pff_accumulate_tree_status: bad arguments");
         return PFF_ERR_ARG;
     }
-    const int N = nx * ny;
     const TreePlan p = tree_plan(nx, ny, local);
-    if (!workspace || workspace_bytes < tree_bytes(p, N)) {
+    if (!workspace || workspace_bytes < tree_bytes(p, nx, ny)) {
         set_error("pff_accumulate_tree_status: workspace too small");
         return PFF_ERR_WORKSPACE;
     }
-    Carver cv(workspace, workspace_bytes);
-    cv.take<unsigned char>(N);
-    cv.take<long long>(N);
-    cv.take<unsigned>(N);
-    cv.take<int>(N);
-    int *stw = cv.take<int>(64);
-    PFF_TRY(read_ints(IntReads().add(stw, 1), status, S(stream)));
+    const TreeArgs a = tree_carve(p, nx, ny, local, workspace, workspace_bytes, nullptr);
+    PFF_TRY(read_ints(IntReads().add(a.status, 1), status, S(stream)));
     return PFF_OK;
 }

@@ -199,12 +199,11 @@ class FlowRouter:
                 wp, wn = self._ws_tree.get(lib.pff_accumulate_tree_workspace_bytes(self.nx, self.ny, local),
                                            self.device)
                 seeds = None if value is not None else self.Q.data_ptr()
-                _lib.call("pff_accumulate_tree", self.receivers.data_ptr(), seeds,
-                          float(value) if value is not None else 0.0, self.Q.data_ptr(),
-                          self.counts.data_ptr() if counts else None, self.nx, self.ny, local, wp, wn,
-                          _dev.stream())
                 st = C.c_int()
-                _lib.call("pff_accumulate_tree_status", self.nx, self.ny, local, wp, wn, C.byref(st), _dev.stream())
+                _lib.call("pff_accumulate_tree_run", self.receivers.data_ptr(), seeds,
+                          float(value) if value is not None else 0.0, self.Q.data_ptr(),
+                          self.counts.data_ptr() if counts else None, self.nx, self.ny, local, wp, wn, C.byref(st),
+                          _dev.stream())
                 if st.value == 0:
                     return
                 if st.value & 1:
