@@ -315,37 +315,53 @@ __device__ __forceinline__ Pub pick4(int q, const Pub &a, const Pub &b, const Pu
     return q == 0 ? a : (q == 1 ? b : (q == 2 ? c : d));
 }
 
-// One active node's round: the reference's swap-remove scan (downstream_propag.py:131-162)
-// on start-of-round donor states.  Returns 0: keeps donors, 1: finished (Q and count
-// written).  last: the start-of-round value is the result (fuse(.., logn), :59-74).
-__device__ __forceinline__ int acc_node(int t, const Pub *cur, Pub *nxt, int4 *priv, float *Q, uint32_t *counts,
-                                        bool last)
+// The scan for a node with two donors of n0 and n1 donors (their first ones f0 and f1): which
+// are absorbed, and the slots left.  A removed first donor leaves its slot to the second.
+struct Two {
+    int todo, w0, w1;
+    bool a0, a1;
+};
+__device__ __forceinline__ Two two_donors(int n0, int n1, int own0, int own1, int f0, int f1)
+{
+    const int x0 = n0 == 1 ? f0 : own0, x1 = n1 == 1 ? f1 : own1;
+    return Two{(n0 != 0) + (n1 != 0), n0 != 0 ? x0 : x1, x1, n0 <= 1, n1 <= 1};
+}
+
+// The result of an active node's round into the next buffers: 0 keeps donors, 1 finished
+// (Q and count written).
+__device__ __forceinline__ int acc_store(int t, const Pub &s, bool worked, int todo, float p, uint32_t c, int w0, int w1,
+                                         int w2, int w3, Pub *nxt, int4 *priv, float *Q, uint32_t *counts)
+{
+    if (!worked) {
+        nxt[t] = s;
+        return 0;
+    }
+    nxt[t] = Pub{todo, p, c, todo > 0 ? w0 : s.d0};
+    if (todo > 1) priv[t] = make_int4(w1, w2, w3, -1);
+    if (todo > 0) return 0;
+    Q[t] = p;
+    if (counts) counts[t] = c;
+    return 1;
+}
+
+// A node with three or more donors (2-3 % of them): the reference's swap-remove scan
+// (downstream_propag.py:131-162) on start-of-round donor states, loaded up front (every
+// one it can need is a start-of-round slot); then slot k holds donor w_k whose preloaded
+// state is q_k.
+__device__ __noinline__ int acc_node_many(int t, const Pub *cur, Pub *nxt, int4 *priv, float *Q, uint32_t *counts)
 {
     const Pub s = cur[t];
-    if (last) {
-        Q[t] = s.p;
-        if (counts) counts[t] = s.c;
-        return 2;
-    }
+    const int4 pq = priv[t];
     int todo = s.ndnr;
-    int own[4] = {s.d0, -1, -1, -1};
-    if (todo > 1) {
-        const int4 pq = priv[t];
-        own[1] = pq.x; own[2] = pq.y; own[3] = pq.z;
-    }
-    // Every donor state this round can need is one of the start-of-round slots: load
-    // them all up front (independent loads).  The scan then runs on registers: slot k
-    // holds donor w_k whose preloaded state is q_k.
-    Pub P0 = s, P1 = s, P2 = s, P3 = s;
-    if (todo > 0) P0 = cur[own[0]];
-    if (todo > 1) P1 = cur[own[1]];
-    if (todo > 2) P2 = cur[own[2]];
+    const int own[4] = {s.d0, pq.x, pq.y, pq.z};
+    Pub P3 = s;
+    const Pub P0 = cur[own[0]], P1 = cur[own[1]], P2 = cur[own[2]];
     if (todo > 3) P3 = cur[own[3]];
     int w0 = own[0], w1 = own[1], w2 = own[2], w3 = own[3];
     int q0 = 0, q1 = 1, q2 = 2, q3 = 3;
     bool worked = false;
-    float padd = 0.f;
-    uint32_t cadd = 0;
+    float padd = s.p;
+    uint32_t cadd = s.c;
     int i = 0;
 #pragma unroll
     for (int step = 0; step < 8; ++step) {  // each step advances i or removes a donor
@@ -353,7 +369,6 @@ __device__ __forceinline__ int acc_node(int t, const Pub *cur, Pub *nxt, int4 *p
         const int q = sel4(i, q0, q1, q2, q3);
         const Pub ds = pick4(q, P0, P1, P2, P3);
         if (ds.ndnr <= 1) {
-            if (!worked) { padd = s.p; cadd = s.c; }
             worked = true;
             padd = __fadd_rn(padd, ds.p);
             cadd += ds.c;
@@ -371,16 +386,7 @@ __device__ __forceinline__ int acc_node(int t, const Pub *cur, Pub *nxt, int4 *p
             ++i;
         }
     }
-    if (!worked) {
-        nxt[t] = s;
-        return 0;
-    }
-    nxt[t] = Pub{todo, padd, cadd, todo > 0 ? w0 : own[0]};
-    if (todo > 1) priv[t] = make_int4(w1, w2, w3, -1);
-    if (todo > 0) return 0;
-    Q[t] = padd;
-    if (counts) counts[t] = cadd;
-    return 1;
+    return acc_store(t, s, worked, todo, padd, cadd, w0, w1, w2, w3, nxt, priv, Q, counts);
 }
 
 // Every remaining round in one cooperative launch, a grid barrier between rounds.  Round
@@ -391,10 +397,12 @@ __device__ __forceinline__ int acc_node(int t, const Pub *cur, Pub *nxt, int4 *p
 //
 // What bounds it: the late rounds, whose lists are nearly empty.  One launch per round
 // cost 2-4 us each for about 20 of them (285 us for the 24 rounds at 2048 x 2048); a
-// barrier costs 1.3 us, and the empty ones at the end are skipped.  Each warp takes 32
-// entries and collects what it keeps in shared memory, so the lists stay in runs of
-// ascending cells whose donors share cache lines.
-constexpr int ACC_THREADS = 1024, ACC_CAP = 96;
+// barrier costs 1.3 us, and the empty ones at the end are skipped.  The early rounds wait on
+// dependent loads (entry, record, slots, donors; DRAM 23 % busy at 32 warps per SM), so a
+// warp takes 64 entries, two per thread, and issues each level's loads for both.  It
+// collects what it keeps in shared memory, so the lists stay in runs of ascending cells
+// whose donors share cache lines.
+constexpr int ACC_THREADS = 1024, ACC_CAP = 128;
 struct AccRounds {
     const int32_t *rcv;
     Pub *buf[2];
@@ -455,38 +463,74 @@ __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
             __syncwarp();
             n = 0;
         };
-        for (int k0 = (blockIdx.x * (ACC_THREADS / 32) + wib) * 32; k0 < total; k0 += gthreads) {
-            const int idx = k0 + lane;
-            int t = -1, r = 2;
-            if (idx < nA) {
-                t = la[idx];
-                bool last = it == logn;
-                if (a.tiles && it >= logmin) {  // the tile's own last round
-                    int lo = 0, hi = a.ntiles - 1;  // tiles sorted by offset: see k_batch_front
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (a.tiles[mid].off <= t) lo = mid;
-                        else hi = mid - 1;
+        for (int k0 = (blockIdx.x * (ACC_THREADS / 32) + wib) * 64; k0 < total; k0 += 2 * gthreads) {
+            int t[2], d1[2], res[2];
+            Pub sc[2], P0[2], P1[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int idx = k0 + 32 * u + lane;
+                t[u] = idx < nA ? la[idx] : (idx < total ? lf[idx - nA] : -1);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) sc[u] = t[u] >= 0 ? cur[t[u]] : Pub{0, 0.f, 0u, -1};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool act = k0 + 32 * u + lane < nA;
+                d1[u] = act && sc[u].ndnr == 2 ? a.priv[t[u]].x : -1;
+                P0[u] = act ? cur[sc[u].d0] : sc[u];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) P1[u] = d1[u] >= 0 ? cur[d1[u]] : P0[u];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int idx = k0 + 32 * u + lane;
+                res[u] = 2;
+                if (idx < nA) {
+                    bool last = it == logn;
+                    if (a.tiles && it >= logmin) {  // the tile's own last round
+                        int lo = 0, hi = a.ntiles - 1;  // tiles sorted by offset: see k_batch_front
+                        while (lo < hi) {
+                            const int mid = (lo + hi + 1) >> 1;
+                            if (a.tiles[mid].off <= t[u]) lo = mid;
+                            else hi = mid - 1;
+                        }
+                        last = it == a.tiles[lo].logn;
                     }
-                    last = it == a.tiles[lo].logn;
-                }
-                r = acc_node(t, cur, nxt, a.priv, a.Q, a.counts, last);
-            } else if (idx < total) {
-                const int f = lf[idx - nA];
-                const Pub s = cur[f];
-                nxt[f] = s;
-                if (fin_q) {
-                    a.Q[f] = s.p;
-                    if (a.counts) a.counts[f] = s.c;
+                    const Pub &s = sc[u];
+                    if (last) {  // the start-of-round value is the result (fuse(.., logn), :59-74)
+                        a.Q[t[u]] = s.p;
+                        if (a.counts) a.counts[t[u]] = s.c;
+                    } else if (s.ndnr > 2) {
+                        res[u] = acc_node_many(t[u], cur, nxt, a.priv, a.Q, a.counts);
+                    } else {
+                        const Two r = s.ndnr == 2 ? two_donors(P0[u].ndnr, P1[u].ndnr, s.d0, d1[u], P0[u].d0, P1[u].d0)
+                                                  : Two{P0[u].ndnr != 0, P0[u].ndnr == 1 ? P0[u].d0 : s.d0, -1,
+                                                        P0[u].ndnr <= 1, false};
+                        float p = s.p;
+                        uint32_t c = s.c;
+                        if (r.a0) { p = __fadd_rn(p, P0[u].p); c += P0[u].c; }
+                        if (r.a1) { p = __fadd_rn(p, P1[u].p); c += P1[u].c; }
+                        res[u] = acc_store(t[u], s, r.a0 || r.a1, r.todo, p, c, r.w0, r.w1, -1, -1, nxt, a.priv, a.Q,
+                                           a.counts);
+                    }
+                } else if (idx < total) {
+                    nxt[t[u]] = sc[u];
+                    if (fin_q) {
+                        a.Q[t[u]] = sc[u].p;
+                        if (a.counts) a.counts[t[u]] = sc[u].c;
+                    }
                 }
             }
-            const unsigned ma = __ballot_sync(0xffffffffu, r == 0), mf = __ballot_sync(0xffffffffu, r == 1);
-            if (r == 0) sa[wib][na + __popc(ma & ((1u << lane) - 1u))] = t;
-            if (r == 1) sf[wib][nf + __popc(mf & ((1u << lane) - 1u))] = t;
-            na += __popc(ma);
-            nf += __popc(mf);
-            if (na > ACC_CAP - 32) flush(sa[wib], na, la2, c2);
-            if (nf > ACC_CAP - 32) flush(sf[wib], nf, lf2, c2 + 1);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const unsigned ma = __ballot_sync(0xffffffffu, res[u] == 0), mf = __ballot_sync(0xffffffffu, res[u] == 1);
+                if (res[u] == 0) sa[wib][na + __popc(ma & ((1u << lane) - 1u))] = t[u];
+                if (res[u] == 1) sf[wib][nf + __popc(mf & ((1u << lane) - 1u))] = t[u];
+                na += __popc(ma);
+                nf += __popc(mf);
+            }
+            if (na > ACC_CAP - 64) flush(sa[wib], na, la2, c2);
+            if (nf > ACC_CAP - 64) flush(sf[wib], nf, lf2, c2 + 1);
         }
         if (na) flush(sa[wib], na, la2, c2);
         if (nf) flush(sf[wib], nf, lf2, c2 + 1);
@@ -552,10 +596,17 @@ __device__ __forceinline__ FrontNode front_round(const float *pc, const uint32_t
         const uint32_t c = sc + cc[own0];
         return FrontNode{dnd == 0 ? 0 : 1, p, c, dnd == 0 ? own0 : (int)(dn & NONE), own1, own2, own3, true};
     }
-    uint32_t N0 = nc[own0], N1 = snd, N2 = snd, N3 = snd;
-    float P0 = pc[own0], P1 = sp, P2 = sp, P3 = sp;
-    uint32_t C0 = cc[own0], C1 = sc, C2 = sc, C3 = sc;
-    if (todo > 1) { N1 = nc[own1]; P1 = pc[own1]; C1 = cc[own1]; }
+    uint32_t N0 = nc[own0], N1 = nc[own1], N2 = snd, N3 = snd;
+    float P0 = pc[own0], P1 = pc[own1], P2 = sp, P3 = sp;
+    uint32_t C0 = cc[own0], C1 = cc[own1], C2 = sc, C3 = sc;
+    if (todo == 2) {  // two donors: both are absorbed (or not) in slot order; the scan unrolled
+        const Two r = two_donors((int)(N0 >> 16), (int)(N1 >> 16), own0, own1, (int)(N0 & NONE), (int)(N1 & NONE));
+        float p = sp;
+        uint32_t c = sc;
+        if (r.a0) { p = __fadd_rn(p, P0); c += C0; }
+        if (r.a1) { p = __fadd_rn(p, P1); c += C1; }
+        return FrontNode{r.todo, p, c, r.w0, r.w1, own2, own3, r.a0 || r.a1};
+    }
     if (todo > 2) { N2 = nc[own2]; P2 = pc[own2]; C2 = cc[own2]; }
     if (todo > 3) { N3 = nc[own3]; P3 = pc[own3]; C3 = cc[own3]; }
     int w0 = own0, w1 = own1, w2 = own2, w3 = own3;

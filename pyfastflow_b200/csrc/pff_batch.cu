@@ -744,8 +744,9 @@ __device__ __noinline__ void batch_front_steps(const LoopArgs &L, int32_t *R, Cl
 template <int MODE>
 __device__ __noinline__ int batch_loop(const LoopArgs &L, ClusterTeam Tm, unsigned char *smem, int *it_outer)
 {
-    int it = 0, outer = 0, n_outer = 0;
+    int it = it_outer[0], outer = it_outer[1], n_outer = 0;
     const int state = reroute_loop<MODE, true, true>(L, Tm, smem, it, outer, n_outer);
+    __syncthreads();
     if (threadIdx.x == 0) {
         it_outer[0] = it;
         it_outer[1] = outer;
@@ -786,16 +787,30 @@ __device__ __noinline__ void tile_reroute(const BatchTile &T, const BatchArrays 
     }
     __syncthreads();
     const int ntiles = (g.nx + TILE_W - 1) / TILE_W * ((g.ny + TILE_H - 1) / TILE_H);
-    FOR_TEAM(k, ntiles) sh.la.dirty[k] = 0;
-    Tm.sync();
-    batch_front_steps<MODE>(sh.la, R, Tm, smem);
-    const int state = batch_loop<MODE>(sh.la, Tm, smem, sh.it_outer);
-    if (state == RR_GENERAL || state == RR_RESUME) {
-        if (Tm.r == 0) tile_reroute_steps<MODE>(g, T, A, z, sh, state == RR_RESUME ? sh.it_outer[0] + 1 : 0, sh.it_outer[1]);
+    if (threadIdx.x == 0) sh.it_outer[0] = sh.it_outer[1] = 0;
+    for (;;) {
+        FOR_TEAM(k, ntiles) sh.la.dirty[k] = 0;
         Tm.sync();
-    } else if (state == RR_WALKERR && Tm.r == 0 && threadIdx.x == 0) {
-        atomicOr(A.status, BST_CARVE);
+        batch_front_steps<MODE>(sh.la, R, Tm, smem);
+        const int state = batch_loop<MODE>(sh.la, Tm, smem, sh.it_outer);
+        if (state == RR_WALKERR && Tm.r == 0 && threadIdx.x == 0) atomicOr(A.status, BST_CARVE);
+        if (state != RR_GENERAL && state != RR_RESUME) break;
+        // the carve closed a receiver cycle, or left one: one iteration of the reference's
+        // steps by the first block (their N-wide passes take 5-30 ms on a tile of 10^6
+        // cells), then the fast loop again from the receivers it leaves
+        const int gi = state == RR_RESUME ? sh.it_outer[0] + 1 : sh.it_outer[0], outer = sh.it_outer[1];
+        if (gi >= outer) break;
+        if (Tm.r == 0) {
+            tile_reroute_steps<MODE>(g, T, A, z, sh, gi, gi + 1);
+            __syncthreads();
+            for (int k = threadIdx.x; k < 64 + LOOP_ITS * LOOP_CTR; k += blockDim.x) sh.loop[k] = 0;
+        }
+        Tm.sync();
+        if (threadIdx.x == 0) sh.it_outer[0] = gi + 1;
+        __syncthreads();
+        if (gi + 1 >= outer) break;
     }
+    Tm.sync();
 }
 
 template <int MODE>
@@ -1327,7 +1342,7 @@ extern "C" long long pff_batch_plan(const int32_t *tile_nx, const int32_t *tile_
     for (int t = 0; t < ntiles; ++t) {
         const int nx = tile_nx[t], ny = tile_ny[t], logn = bceil_log2(cells(t)) + 1;
         // packed cell ids of the accumulation are 32-bit
-        const bool front = batch_front_takes(nx, ny, tile_mode[t]) && total < (1LL << 31);
+        const bool front = batch_front_takes(nx, ny, tile_mode[t]) && total < 2000000000LL;
         hp[t] = BatchTile{tile_offset[t], tile_offset[t] + t, nx, ny, tile_mode[t], t, tile_dx[t],
                           front ? (int)items.size() : -1, logn, 0};
         if (!front) continue;
@@ -1382,7 +1397,7 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
     cudaStream_t st = S(stream);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
     PFF_TRY(launch_batch(k_batch_route, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A));
-    if (total_cells < (1LL << 31)) {
+    if (total_cells < 2000000000LL) {
         BatchAcc b{};
         b.rcv = receivers; b.Q = Q; b.counts = counts;
         b.bufA = A.dnr; b.bufB = A.dnr_; b.priv = w.priv;

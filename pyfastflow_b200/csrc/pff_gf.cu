@@ -229,6 +229,12 @@ __global__ void __launch_bounds__(256) k_diffuse_sweep(const float *__restrict__
 // band, double-buffered in shared memory.  Traffic: zh and Q over the region once,
 // temp once.
 //
+// Bound by instruction issue.  The weights are stored at the cell that receives them (plane
+// k: the weight of the link through which the cell's top, left, right, bottom neighbour
+// reaches it), so a sweep's loads are all at the cell's own place, and away from the grid's
+// edges a thread takes four cells of a row with 16-byte loads: 9 loads for 4 cells, not 32
+// (the row's rim columns then hold values that no tile cell depends on).
+//
 // Periodic modes load the halo with wrap-around, so in modes 0-2 (nx, ny >= 3) the
 // k-th neighbour of a cell is always the adjacent shared-memory cell, and it exists
 // exactly when that cell lies in the grid along the non-periodic axes.  A cell that
@@ -239,10 +245,12 @@ __global__ void __launch_bounds__(256) k_diffuse_sweep(const float *__restrict__
 // ny-1: bottom, top, left, right.  Flag byte per region cell: bit 0 in the grid,
 // bit 1 a source, bits 2-3 that order.
 constexpr int DF_TX = 64, DF_TY = 32, DF_HMAX = 8, DF_THREADS = 512;
-__host__ __device__ constexpr int df_region(int H) { return (DF_TX + 2 * H) * (DF_TY + 2 * H); }
+__host__ __device__ constexpr int df_px(int H) { return (DF_TX + 2 * H + 3) / 4 * 4; }  // a region row in shared memory
+__host__ __device__ constexpr int df_region(int H) { return df_px(H) * (DF_TY + 2 * H) + 8; }
 __host__ __device__ constexpr int df_ring(int H) { return (DF_TX + 2 * H + 2) * (DF_TY + 2 * H + 2); }
-// zh over the region and its ring, four weight planes, two Q buffers, the flags
+// four weight planes, two Q buffers (16-byte aligned), zh over the region and its ring, the flags
 constexpr size_t df_smem(int H) { return sizeof(float) * (size_t)(df_ring(H) + 6 * df_region(H)) + df_region(H); }
+static_assert(df_region(1) % 4 == 0 && df_region(5) % 4 == 0 && df_region(8) % 4 == 0, "16-byte planes");
 
 template <int MODE>
 __device__ __forceinline__ bool df_inside(const Grid &g, int r, int c)
@@ -265,12 +273,13 @@ template <int MODE, int H>
 __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__restrict__ zh, const float *__restrict__ Qin,
                                                        float *__restrict__ out, Grid g, DivC dc, float prec_dx2)
 {
-    constexpr int RX = DF_TX + 2 * H, RY = DF_TY + 2 * H, ZX = RX + 2, ZY = RY + 2, P = RX * RY;
+    constexpr int RX = DF_TX + 2 * H, RY = DF_TY + 2 * H, ZX = RX + 2, ZY = RY + 2, PX = df_px(H), P = df_region(H);
     extern __shared__ __align__(16) float df_sm[];
-    float *zs = df_sm;
-    float *w0 = zs + ZX * ZY, *w1 = w0 + P, *w2 = w1 + P, *w3 = w2 + P;
+    // planes with 4 floats in front (a row's left neighbour column at index -1)
+    float *w0 = df_sm + 4, *w1 = w0 + P, *w2 = w1 + P, *w3 = w2 + P;
     float *qa = w3 + P, *qb = qa + P;
-    unsigned char *fl = reinterpret_cast<unsigned char *>(qb + P);
+    float *zs = df_sm + 6 * P;
+    unsigned char *fl = reinterpret_cast<unsigned char *>(zs + ZX * ZY);
     const int x0 = blockIdx.x * DF_TX - H, y0 = blockIdx.y * DF_TY - H;  // region origin (unwrapped)
     const int nx = g.nx, ny = g.ny;
     // the region and its ring strictly inside the grid: every region cell is an interior
@@ -286,8 +295,8 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
         }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < P; t += blockDim.x) {
-        const int ry = t / RX, rx = t % RX, r = y0 + ry, c = x0 + rx;
+    for (int t = threadIdx.x; t < RX * RY; t += blockDim.x) {
+        const int ry = t / RX, rx = t % RX, r = y0 + ry, c = x0 + rx, i = ry * PX + rx;
         unsigned char f = 0;
         float q = 0.f, wk[4] = {DF_SKIP, DF_SKIP, DF_SKIP, DF_SKIP};
         if (inner || df_inside<MODE>(g, r, c)) {
@@ -305,27 +314,46 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
                 const int z = (ry + 1) * ZX + rx + 1;
                 const float zi = zs[z];
                 const float zn[4] = {zs[z - ZX], zs[z - 1], zs[z + 1], zs[z + ZX]};
-                float sk[4], sums = 0.f;
-                // max(0, (zi - zj) / dx) is +0 unless zi > zj (NaN compares false and
-                // max(0, NaN) is 0), and 0 / sums is +0 for the sums > 0 of a source:
-                // only the descending links divide
+                // max(0, (zi - zj) / dx), with Markstein's exact quotient for all four links
+                // at once where every descending one lies in its range (a level or rising
+                // link, or a NaN, gives +0); likewise the weights, with y = RN(1 / sums)
+                float m[4], sk[4], sums = 0.f, mx = 0.f;
+                bool ok = true;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    sk[k] = zi > zn[k] ? fmaxf(0.f, div_dx(__fsub_rn(zi, zn[k]), dc)) : 0.f;
-                    sums = __fadd_rn(sums, sk[k]);
+                    m[k] = fmaxf(__fsub_rn(zi, zn[k]), 0.f);
+                    ok = ok && (m[k] == 0.f || m[k] >= dc.mlo);
+                    mx = fmaxf(mx, m[k]);
+                    sk[k] = div_markstein(m[k], dc);
                 }
-                if (sums != 0.f) {
+                if (!(ok && mx <= dc.mhi)) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) wk[k] = sk[k] != 0.f ? __fdiv_rn(sk[k], sums) : 0.f;
+                    for (int k = 0; k < 4; ++k) sk[k] = m[k] > 0.f ? fmaxf(0.f, div_dx(m[k], dc)) : 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sums = __fadd_rn(sums, sk[k]);
+                if (sums != 0.f) {
+                    // quotients in [2^-100, 1]: nothing under- or overflows on the way
+                    bool fast = sums >= 0x1p-40f && sums <= 0x1p40f;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) fast = fast && (sk[k] == 0.f || sk[k] >= 0x1p-60f);
+                    const DivC ds{sums, __frcp_rn(sums), 0.f, 0.f};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) wk[k] = div_markstein(sk[k], ds);
+                    if (!fast) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) wk[k] = sk[k] != 0.f ? __fdiv_rn(sk[k], sums) : 0.f;
+                    }
                 }
             }
         }
-        w0[t] = wk[0];
-        w1[t] = wk[1];
-        w2[t] = wk[2];
-        w3[t] = wk[3];
-        qa[t] = q;
-        fl[t] = f;
+        // to the cells the links lead to, within the region
+        if (ry > 0) w3[i - PX] = wk[0];
+        if (rx > 0) w2[i - 1] = wk[1];
+        if (rx < RX - 1) w1[i + 1] = wk[2];
+        if (ry < RY - 1) w0[i + PX] = wk[3];
+        qa[i] = q;
+        fl[i] = f;
     }
     __syncthreads();
     float *qc = qa, *qn = qb;
@@ -333,15 +361,22 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
     for (int sw = 1; sw <= H; ++sw) {
         const int bw = RX - 2 * sw, bh = RY - 2 * sw;
         if (inner) {  // every cell inside the grid, off its edges: summation order top, left, right, bottom
-            for (int t = threadIdx.x; t < bw * bh; t += blockDim.x) {
-                const int i = (sw + t / bw) * RX + sw + t % bw;
-                const int u = i - RX, l = i - 1, rt = i + 1, d = i + RX;
-                float acc = prec_dx2;
-                acc = df_add(acc, w3[u], qc[u]);
-                acc = df_add(acc, w2[l], qc[l]);
-                acc = df_add(acc, w1[rt], qc[rt]);
-                acc = df_add(acc, w0[d], qc[d]);
-                qn[i] = acc;
+            for (int t = threadIdx.x; t < PX / 4 * bh; t += blockDim.x) {
+                const int i = (sw + t / (PX / 4)) * PX + t % (PX / 4) * 4;
+                auto ld = [](const float *p) { return *reinterpret_cast<const float4 *>(p); };
+                const float4 a0 = ld(w0 + i), a1 = ld(w1 + i), a2 = ld(w2 + i), a3 = ld(w3 + i);
+                const float4 u = ld(qc + i - PX), m = ld(qc + i), d = ld(qc + i + PX);
+                const float l = qc[i - 1], rt = qc[i + 4];
+                auto cell = [&](float x0, float x1, float x2, float x3, float qu, float ql, float qr, float qd) {
+                    float acc = prec_dx2;
+                    acc = df_add(acc, x0, qu);
+                    acc = df_add(acc, x1, ql);
+                    acc = df_add(acc, x2, qr);
+                    return df_add(acc, x3, qd);
+                };
+                *reinterpret_cast<float4 *>(qn + i) =
+                    make_float4(cell(a0.x, a1.x, a2.x, a3.x, u.x, l, m.y, d.x), cell(a0.y, a1.y, a2.y, a3.y, u.y, m.x, m.z, d.y),
+                                cell(a0.z, a1.z, a2.z, a3.z, u.z, m.y, m.w, d.z), cell(a0.w, a1.w, a2.w, a3.w, u.w, m.z, rt, d.w));
             }
             __syncthreads();
             float *tq = qc;
@@ -350,38 +385,36 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
             continue;
         }
         for (int t = threadIdx.x; t < bw * bh; t += blockDim.x) {
-            const int i = (sw + t / bw) * RX + sw + t % bw;
+            const int i = (sw + t / bw) * PX + sw + t % bw;
             const unsigned char f = fl[i];
             if (!(f & 1)) continue;
-            // the source above reaches i through its bottom link (w3), the left one
-            // through its right link (w2), the right one its left (w1), below its top (w0);
             // a neighbour that is not a source has the weight DF_SKIP on every link
-            const int u = i - RX, l = i - 1, rt = i + 1, d = i + RX;
+            const int u = i - PX, l = i - 1, rt = i + 1, d = i + PX;
             float acc = prec_dx2;
             switch (f >> 2) {
             case 0:
-                acc = df_add(acc, w3[u], qc[u]);
-                acc = df_add(acc, w2[l], qc[l]);
-                acc = df_add(acc, w1[rt], qc[rt]);
-                acc = df_add(acc, w0[d], qc[d]);
+                acc = df_add(acc, w0[i], qc[u]);
+                acc = df_add(acc, w1[i], qc[l]);
+                acc = df_add(acc, w2[i], qc[rt]);
+                acc = df_add(acc, w3[i], qc[d]);
                 break;
             case 1:
-                acc = df_add(acc, w3[u], qc[u]);
-                acc = df_add(acc, w1[rt], qc[rt]);
-                acc = df_add(acc, w2[l], qc[l]);
-                acc = df_add(acc, w0[d], qc[d]);
+                acc = df_add(acc, w0[i], qc[u]);
+                acc = df_add(acc, w2[i], qc[rt]);
+                acc = df_add(acc, w1[i], qc[l]);
+                acc = df_add(acc, w3[i], qc[d]);
                 break;
             case 2:
-                acc = df_add(acc, w2[l], qc[l]);
-                acc = df_add(acc, w1[rt], qc[rt]);
-                acc = df_add(acc, w0[d], qc[d]);
-                acc = df_add(acc, w3[u], qc[u]);
+                acc = df_add(acc, w1[i], qc[l]);
+                acc = df_add(acc, w2[i], qc[rt]);
+                acc = df_add(acc, w3[i], qc[d]);
+                acc = df_add(acc, w0[i], qc[u]);
                 break;
             default:
-                acc = df_add(acc, w0[d], qc[d]);
-                acc = df_add(acc, w3[u], qc[u]);
-                acc = df_add(acc, w2[l], qc[l]);
-                acc = df_add(acc, w1[rt], qc[rt]);
+                acc = df_add(acc, w3[i], qc[d]);
+                acc = df_add(acc, w0[i], qc[u]);
+                acc = df_add(acc, w1[i], qc[l]);
+                acc = df_add(acc, w2[i], qc[rt]);
                 break;
             }
             qn[i] = acc;
@@ -394,7 +427,7 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
     for (int t = threadIdx.x; t < DF_TX * DF_TY; t += blockDim.x) {
         const int ly = t / DF_TX, lx = t % DF_TX;
         const int row = y0 + H + ly, col = x0 + H + lx;
-        if (row < ny && col < nx) out[row * nx + col] = qc[(H + ly) * RX + H + lx];
+        if (row < ny && col < nx) out[row * nx + col] = qc[(H + ly) * PX + H + lx];
     }
 }
 

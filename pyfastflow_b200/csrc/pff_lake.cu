@@ -315,7 +315,7 @@ __device__ __forceinline__ void block_append(bool pred, int val, int *list, int 
 // the grid strides over the list; the count is read on the device), or of every
 // tile (tiles == NULL, a 2-D grid of tiles).
 template <int MODE>
-__global__ void __launch_bounds__(TILE_THREADS) k_tile_terminal(const int32_t *__restrict__ rec, int32_t *J, int32_t *R,
+__global__ void __launch_bounds__(TILE_THREADS, 5) k_tile_terminal(const int32_t *__restrict__ rec, int32_t *J, int32_t *R,
                                                                 int *pits, int *info, Grid g, const int *tiles,
                                                                 const int *ntiles, int32_t *rec_copy)
 {

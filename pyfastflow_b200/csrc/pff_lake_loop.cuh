@@ -41,8 +41,11 @@ __device__ __forceinline__ void divmod_nx(int n, int d, unsigned m, int &q, int 
 // Tile-local indices q of a thread's receivers r (its cells: rows ly0 + 4 k of column lx of
 // the w x h tile at (row0, col0), local index t + 256 k, grid index i0 + 4 k nx; r < 0: no
 // cell): the receiver's, or the cell's own where it is a root or its receiver lies outside.
-__device__ __forceinline__ void tile_locals(const int (&r)[TILE_PER_THREAD], int (&q)[TILE_PER_THREAD], int i0, int t,
-                                            int lx, int ly0, int row0, int col0, int w, int h, int nx, unsigned mnx)
+// True if some receiver outside is not a tile-border cell (a receiver one column or row away
+// always is one).
+__device__ __forceinline__ bool tile_locals(const int (&r)[TILE_PER_THREAD], int (&q)[TILE_PER_THREAD], int i0, int t,
+                                            int lx, int ly0, int row0, int col0, int w, int h, int nx, int ny,
+                                            unsigned mnx)
 {
     static_assert(TILE_THREADS == 4 * TILE_W, "a thread's cells are 4 rows apart");
     int far = 0;  // receivers that are not the grid neighbour (wrapped edges, or no D4 link)
@@ -54,25 +57,27 @@ __device__ __forceinline__ void tile_locals(const int (&r)[TILE_PER_THREAD], int
         q[k] = in ? c + sx + TILE_W * sy : c;
         if (r[k] >= 0 && d != 0 && (sx | sy) == 0) far |= 1 << k;
     }
-    if (!far) return;
+    bool nonlocal = false;
+    if (!far) return nonlocal;
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
         if (!(far >> k & 1)) continue;
         int rr, rc;
         divmod_nx(r[k], nx, mnx, rr, rc);
-        rr -= row0;
-        rc -= col0;
-        if (rr >= 0 && rr < h && rc >= 0 && rc < w) q[k] = rr * TILE_W + rc;
+        if (rr >= row0 && rr < row0 + h && rc >= col0 && rc < col0 + w) q[k] = (rr - row0) * TILE_W + rc - col0;
+        else if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
     }
+    return nonlocal;
 }
 
 // A thread's 8 pointers q to their tile terminals.  Four rounds of pointer doubling in p
 // (16-bit local pointers; a pointer then spans 16 cells or ends), then every pointer is
 // followed on its own over the settled array, without barriers: most paths in a tile
-// are shorter than 64 cells.  At most 2048 / 16 steps (a cycle ends there too).
+// are shorter than 64 cells.  At most 2048 / 16 steps; true if a pointer is then still
+// moving (a cycle).
 // Bound by the shared-memory gathers' latency and bank conflicts.
 template <class Sync>
-__device__ __forceinline__ void tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD], int t, Sync sync)
+__device__ __forceinline__ bool tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD], int t, Sync sync)
 {
     int qq[TILE_PER_THREAD];
     unsigned act = (1u << TILE_PER_THREAD) - 1;  // pointers not known to be terminals
@@ -105,6 +110,7 @@ __device__ __forceinline__ void tile_jump(uint16_t *p, int (&q)[TILE_PER_THREAD]
                 q[k] = qq[k];
             }
     }
+    return act != 0;
 }
 
 // Tile terminals of one tile by a group of 256 threads (t: thread of the group): J[i] = the receiver of the last in-tile cell of
@@ -126,7 +132,7 @@ __device__ __forceinline__ void tile_terminal_one(const int32_t *rec, int32_t *J
     int r[TILE_PER_THREAD], q[TILE_PER_THREAD];
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) r[k] = (lx < w && ly0 + 4 * k < h) ? rec[i0 + 4 * k * nx] : -1;
-    tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
+    bool nonlocal = tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, ny, mnx);
     int term = 0;  // cells that are terminals
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
@@ -137,8 +143,9 @@ __device__ __forceinline__ void tile_terminal_one(const int32_t *rec, int32_t *J
         if (rec_copy && r[k] >= 0) rec_copy[i0 + 4 * k * nx] = r[k];
     }
     sync();
-    tile_jump(p, q, t, sync);
-    bool nonlocal = false;
+    nonlocal |= tile_jump(p, q, t, sync);
+    // a tile off the grid's rim has no cell that can leave (modes 0-2)
+    const bool rim = MODE == 3 || row0 == 0 || col0 == 0 || row0 + h == ny || col0 + w == nx;
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
         const int c = t + k * TILE_THREADS, ly = ly0 + 4 * k, i = i0 + 4 * k * nx;
@@ -147,13 +154,9 @@ __device__ __forceinline__ void tile_terminal_one(const int32_t *rec, int32_t *J
             const int j = rv[q[k]];
             J[i] = j;
             if (lx == 0 || ly == 0 || lx == w - 1 || ly == h - 1 || r[k] == i) R[i] = j;
-            if ((term >> k & 1) && r[k] != i) {  // an exit
-                int rr, rc;
-                divmod_nx(r[k], nx, mnx, rr, rc);
-                if (!is_tile_border(nx, ny, rr, rc)) nonlocal = true;
-            }
-            if (p[q[k]] != q[k] || (q[k] == c && !(term >> k & 1))) nonlocal = true;  // a cycle in the tile
-            pit = pits && r[k] == i && !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
+            if (q[k] == c && !(term >> k & 1)) nonlocal = true;  // a cycle in the tile
+            pit = pits && r[k] == i;
+            if (rim && pit) pit = !can_leave<MODE>(g, i, row0 + ly, col0 + lx);
         }
         const unsigned m = __ballot_sync(0xffffffffu, pit);
         if (m) {
@@ -340,7 +343,7 @@ __device__ __forceinline__ void loop_tile(const LoopArgs &A, int tile, int ntx, 
         }
     if (!go_on) return;
     int q[TILE_PER_THREAD];
-    tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
+    tile_locals(r, q, i0, t, lx, ly0, row0, col0, w, h, nx, ny, mnx);
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
         p[t + k * TILE_THREADS] = (uint16_t)q[k];
@@ -376,7 +379,7 @@ __device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, un
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k)
         r[k] = (lx < w && ly0 + 4 * k < h) ? A.rec_[i0 + 4 * k * nx] : -1;
-    tile_locals(r, j, i0, t, lx, ly0, row0, col0, w, h, nx, mnx);
+    tile_locals(r, j, i0, t, lx, ly0, row0, col0, w, h, nx, ny, mnx);
 #pragma unroll
     for (int k = 0; k < TILE_PER_THREAD; ++k) {
         const int c = t + k * TILE_THREADS;
@@ -425,7 +428,8 @@ __device__ __forceinline__ void loop_walk(const LoopArgs &A, int s0, int ntx, un
 // The outer iterations of one grid.  BATCH: a batch tile, whose basin, border and z'
 // arrays are scratch: they are initialised for the pits only, and nothing is written that
 // only a caller would read.  KEYED: the first border list carries labels and keys (from
-// reroute_first_border, not from the strip pass).  Returns the final
+// reroute_first_border, not from the strip pass).  it and outer on entry: the iteration to
+// begin with, and (if that is not the first) the loop's bound.  Returns the final
 // state (the same in every thread), the iteration it stopped in, its bound and count.
 template <int MODE, bool BATCH, bool KEYED, class Team>
 __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned char *loop_smem, int &it, int &outer,
@@ -441,10 +445,11 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
     const TileXY txy{(nx + TILE_W - 1) / TILE_W, mnx, nx};
     const long long iv = invalid_key();
     const int np0 = vload(A.info);
+    const int it0 = it;
     int state = RR_RUN;
-    it = n_outer = 0;
-    outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;             // :500
-    if (np0 == 0) state = RR_NOPITS;                        // :496-497
+    n_outer = 0;
+    if (it0 == 0) outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;  // :500
+    if (np0 == 0) state = it0 == 0 ? RR_NOPITS : RR_DONE;      // :496-497, :512-514
     else if (vload(A.info + 2) || vload(A.info + 4)) state = RR_GENERAL;  // not D4, or a receiver cycle in the input
     if (state == RR_RUN) {
         // clear the carve tags of an earlier call
@@ -464,8 +469,8 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
         }
     }
     while (state == RR_RUN) {
-        const bool first = it == 0;
-        int *C = A.it_ctr + it * LOOP_CTR, *Cn = C + LOOP_CTR;
+        const bool first = it == it0;
+        int *C = A.it_ctr + (it - it0) * LOOP_CTR, *Cn = C + LOOP_CTR;
         const int np = first ? np0 : vload(C + LC_NP);
         const int *pits = first ? A.pit0 : A.pits[it & 1];
         int *pnext = A.pits[(it + 1) & 1];
