@@ -650,7 +650,7 @@ __device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float
 {
     const int N = g.nx * g.ny;
     const unsigned mnx = 0xffffffffu / (unsigned)g.nx;
-    constexpr int U = 4;
+    constexpr int U = 2;
     FOR_TEAM_U(i0, stride, U, N) {
         int js[U][4];
         float zi[U], zn[U][4];
@@ -669,17 +669,38 @@ __device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float
         for (int u = 0; u < U; ++u) {
             const int i = i0 + u * stride;
             if (i >= N) break;
-            int r = i;
-            float sr = 0.f, dbest = 0.f;
+            // one quotient per cell, as in k_receivers_lean: division by dx is monotone, and the
+            // first direction whose rounded quotient is the largest has a drop within 2^-21 of
+            // the largest drop; when that direction's drop is the largest itself, it is the
+            // answer.  Anything else (a near tie, a quotient that under- or overflows) takes
+            // the ordered scan.
+            float d[4], dmax = 0.f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const float d = __fsub_rn(zi[u], zn[u][k]);
-                if (js[u][k] != -1 && d > dbest) {  // a smaller difference cannot give a larger quotient
-                    const float q = __fdiv_rn(d, dx);
-                    if (q > sr) {
-                        sr = q;
-                        r = js[u][k];
-                        dbest = d;
+                d[k] = js[u][k] != -1 ? __fsub_rn(zi[u], zn[u][k]) : 0.f;
+                dmax = fmaxf(dmax, d[k]);
+            }
+            int r = i;
+            float sr = 0.f;
+            if (dmax > 0.f) {
+                const float near = __fmul_rn(dmax, 1.0f - 0x1p-21f);
+                int kf = 3;
+                float df = d[3];
+#pragma unroll
+                for (int k = 2; k >= 0; --k)
+                    if (d[k] >= near) { kf = k; df = d[k]; }
+                sr = __fdiv_rn(dmax, dx);
+                r = kf == 0 ? js[u][0] : (kf == 1 ? js[u][1] : (kf == 2 ? js[u][2] : js[u][3]));
+                if (df != dmax || !(sr >= 0x1p-100f && sr <= 0x1p100f)) {
+                    r = i;
+                    sr = 0.f;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float q = d[k] > 0.f ? __fdiv_rn(d[k], dx) : 0.f;
+                        if (q > sr) {
+                            sr = q;
+                            r = js[u][k];
+                        }
                     }
                 }
             }

@@ -469,20 +469,21 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
         }
     }
     while (state == RR_RUN) {
-        const bool first = it == it0;
-        int *C = A.it_ctr + (it - it0) * LOOP_CTR, *Cn = C + LOOP_CTR;
+        const int rel = it - it0;  // the lists and counters begin with this call
+        const bool first = rel == 0;
+        int *C = A.it_ctr + rel * LOOP_CTR, *Cn = C + LOOP_CTR;
         const int np = first ? np0 : vload(C + LC_NP);
-        const int *pits = first ? A.pit0 : A.pits[it & 1];
-        int *pnext = A.pits[(it + 1) & 1];
-        const int *alist = A.alist[it & 1];
+        const int *pits = first ? A.pit0 : A.pits[rel & 1];
+        int *pnext = A.pits[(rel + 1) & 1];
+        const int *alist = A.alist[rel & 1];
         auto label = [&](int i) -> int {
             const int b = A.bid[i];
             return first ? b : A.fin[b];
         };
         // ---- passes 1-2 over the previous border cells (the first list comes from the strip pass)
         if (!first) {
-            const int *aprev = A.alist[(it & 1) ^ 1];
-            int *anext = A.alist[it & 1];
+            const int *aprev = A.alist[(rel & 1) ^ 1];
+            int *anext = A.alist[rel & 1];
             const int n = vload(C - LOOP_CTR + LC_NA);
             // each warp on its own: the entries that stay on a border collect in its buffer,
             // and the next trip's cells are loaded ahead
@@ -755,7 +756,7 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
         else if (last) state = RR_DONE;
         else if (!settled) state = RR_RESUME;       // the carve closed a receiver cycle
         else if (vload(Cn + LC_NP) == 0) { ++n_outer; state = RR_DONE; }
-        else if (it + 2 >= LOOP_ITS) state = RR_BOUND;
+        else if (rel + 2 >= LOOP_ITS) state = RR_BOUND;
         const bool go_on = state == RR_RUN;
         const int ndirty = vload(C + LC_NDIRTY);
         for (int k = grp * nblk + T.rank(); k < ndirty; k += nblk * ngrp) {
@@ -943,38 +944,49 @@ __device__ __forceinline__ void reroute_first_border(const LoopArgs &A, Team &T,
         __syncwarp();
         nb = 0;
     };
-    for (int k0 = (T.rank() * (blockDim.x >> 5) + wib) * 32; k0 < N; k0 += gthreads) {
-        const int i = k0 + lane;
-        int code = 0, bi = 0;
-        long long key = 0;
-        if (i < N) {
-            int row, col;
-            divmod_nx(i, nx, mnx, row, col);
-            if (can_leave<MODE>(g, i, row, col)) {
-                if (WRITE) A.zp[i] = A.z[i];
-            } else {
-                int jn[4], bn[4];
-                float zn[4];
-                neighbours4<MODE>(g, i, row, col, jn);
-                bi = A.bid[i];
+    for (int k0 = (T.rank() * (blockDim.x >> 5) + wib) * 64; k0 < N; k0 += 2 * gthreads) {
+        int jn[2][4], bn[2][4], bi[2];
+        float zn[2][4], zi[2];
+        bool on[2];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    bn[q] = jn[q] != -1 ? A.bid[jn[q]] : 0;
-                    zn[q] = jn[q] != -1 ? A.z[jn[q]] : 0.f;
+        for (int u = 0; u < 2; ++u) {  // two cells per thread, their loads in flight together
+            const int i = k0 + 32 * u + lane;
+            on[u] = false;
+            if (i < N) {
+                int row, col;
+                divmod_nx(i, nx, mnx, row, col);
+                if (can_leave<MODE>(g, i, row, col)) {
+                    if (WRITE) A.zp[i] = A.z[i];
+                } else {
+                    on[u] = true;
+                    neighbours4<MODE>(g, i, row, col, jn[u]);
+                    bi[u] = A.bid[i];
+                    zi[u] = A.z[i];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        bn[u][q] = jn[u][q] != -1 ? A.bid[jn[u][q]] : 0;
+                        zn[u][q] = jn[u][q] != -1 ? A.z[jn[u][q]] : 0.f;
+                    }
                 }
-                code = saddle_cell<WRITE>(i, bi, A.z[i], jn, bn, zn, A.isb, A.zp, key);
             }
         }
-        if (code != 0 && key < invalid_key()) atomicMin(A.sad + bi, key);
-        const unsigned m = __ballot_sync(0xffffffffu, code != 0);
-        if (code != 0) {
-            const int at = nb + __popc(m & ((1u << lane) - 1u));
-            bufi[at] = i;
-            bufb[at] = bi;
-            bufk[at] = key;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = k0 + 32 * u + lane;
+            int code = 0;
+            long long key = 0;
+            if (on[u]) code = saddle_cell<WRITE>(i, bi[u], zi[u], jn[u], bn[u], zn[u], A.isb, A.zp, key);
+            if (code != 0 && key < invalid_key()) atomicMin(A.sad + bi[u], key);
+            const unsigned m = __ballot_sync(0xffffffffu, code != 0);
+            if (code != 0) {
+                const int at = nb + __popc(m & ((1u << lane) - 1u));
+                bufi[at] = i;
+                bufb[at] = bi[u];
+                bufk[at] = key;
+            }
+            nb += __popc(m);
+            if (nb > LOOP_CAP - 32) flush();
         }
-        nb += __popc(m);
-        if (nb > LOOP_CAP - 32) flush();
     }
     flush();
 }
