@@ -551,9 +551,11 @@ __global__ void __launch_bounds__(TR_T0_THREADS) k_tree_finish(const int32_t *__
 {
     __shared__ __align__(16) unsigned char sm[TreeTile<VAL>::BYTES];
     const int s = tree_shift(a, w, value);
-    tree_tile_finish<VAL>(a, rcv, s, w ? 0 : to_fixed(value, s), Q, counts, blockIdx.x, sm, threadIdx.x,
-                          []() { __syncthreads(); });
-    // the status is final since the passes before: the first block reports it
+    // the status is final since the passes before; after a problem Q keeps its seeds for the
+    // caller's other path
+    if (vload(a.status) == 0)
+        tree_tile_finish<VAL>(a, rcv, s, w ? 0 : to_fixed(value, s), Q, counts, blockIdx.x, sm, threadIdx.x,
+                              []() { __syncthreads(); });
     if (a.out && blockIdx.x == 0 && threadIdx.x == 0) {
         *(volatile int *)a.out = a.status[0];
         __threadfence_system();
@@ -804,7 +806,8 @@ __global__ void __launch_bounds__(TR_LB_THREADS, 1) k_tree_all(const int32_t *__
         if (!bar.sync(&dead)) return;
     }
     const long long cval = w ? 0 : to_fixed(value, s);
-    for (int k = grp * gridDim.x + blockIdx.x; k < ntiles; k += ngrp * gridDim.x) {
+    const int n = vload(a.status) == 0 ? ntiles : 0;  // after a problem Q keeps its seeds
+    for (int k = grp * gridDim.x + blockIdx.x; k < n; k += ngrp * gridDim.x) {
         tree_tile_finish<VAL>(a, rcv, s, cval, Q, counts, k, gsm, gt, gsync);
         gsync();
     }
@@ -910,7 +913,8 @@ static int launch_tree(const TreePlan &p, const TreeArgs &a_, const int32_t *rec
     PFF_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     const size_t smem = (size_t)TR_SMEM_NODES * TR_NODE_BYTES;  // per-device attribute: set on every call
     if (coop && p.ntiles <= TR_ALL_TILES * nsm) {
-        const int blocks = std::min(nsm, div_up(p.ntiles, TR_LB_THREADS / TR_T0_THREADS));
+        // a block has room for 4 tiles at a time, but tiles on SMs of their own are faster
+        const int blocks = p.ntiles <= TR_LB_THREADS / TR_T0_THREADS ? 1 : std::min(nsm, p.ntiles);
         if (blocks > 1) PFF_CUDA(cudaMemsetAsync(a.status, 0, sizeof(int) * (size_t)a.nzero, st));
         PFF_CUDA(cudaFuncSetAttribute(k_tree_all<VAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         void *args[] = {(void *)&receivers, (void *)&weights, &value, &Q, &counts, &a};

@@ -86,16 +86,16 @@ constexpr int RCV4_AHEAD = 2;  // rows loaded per group there (RCV4_ROWS is a mu
 
 template <int MODE>
 __global__ void __launch_bounds__(128) k_receivers(const float *__restrict__ z, int32_t *__restrict__ rcv,
-                                                   float *__restrict__ grad, Grid g, float dx)
+                                                   float *__restrict__ grad, Grid g, float dx, int rows)
 {
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nstrips = (g.nx + 31) >> 5;
     const int strip = warp % nstrips, band = warp / nstrips;
     const int col = (strip << 5) + lane;
-    const int row0 = band * RCV_ROWS;
+    const int row0 = band * rows;
     if (row0 >= g.ny) return;
-    const int row1 = min(row0 + RCV_ROWS, g.ny);
+    const int row1 = min(row0 + rows, g.ny);
     const bool incol = col < g.nx;
     const int nx = g.nx;
     // register window: above, centre, below (column `col`); rows are loaded in groups
@@ -578,8 +578,12 @@ static void launch_receivers(const float *z, int32_t *rcv, float *grad, const Gr
         count_launch();
         return;
     }
-    const long long warps = (long long)((g.nx + 31) / 32) * ((g.ny + RCV_ROWS - 1) / RCV_ROWS);
-    PFF_PROBED("k_receivers", st, k_receivers<MODE><<<div_up(warps, 4), 128, 0, st>>>(z, rcv, grad, g, dx));
+    // bands of RCV_ROWS rows, shorter while they would leave the GPU with less than 32 warps
+    // per SM (1001 x 777 has 800 bands of 32 rows, 30 us; of 4 rows it takes 10 us)
+    int rows = RCV_ROWS;
+    while (rows > RCV_AHEAD && (long long)((g.nx + 31) / 32) * ((g.ny + rows - 1) / rows) < 148 * 32) rows /= 2;
+    const long long warps = (long long)((g.nx + 31) / 32) * ((g.ny + rows - 1) / rows);
+    PFF_PROBED("k_receivers", st, k_receivers<MODE><<<div_up(warps, 4), 128, 0, st>>>(z, rcv, grad, g, dx, rows));
     count_launch();
 }
 

@@ -522,27 +522,43 @@ __global__ void __launch_bounds__(256) k_core_fused(float *h, float *zh, const f
                                                     int N, float dx, float dx2, float manning, float edgesw, float dt,
                                                     const float *__restrict__ href, float *dhmax)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float m = 0.f;
-    if (i < N) {
-        int r = rec[i];
-        if ((unsigned)r >= (unsigned)N) r = i;  // as in k_core1
-        const float zi = zf[i];
+    // two cells per thread: the receivers' gathers of both are in flight together (one
+    // cell per thread waited on them: 49 us at 2048^2 against 34)
+    constexpr int U = 2;
+    float m = 0.f, zi[U], zr[U], hi[U], qi[U];
+    int r[U];
+    const int i0 = blockIdx.x * (256 * U) + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int i = i0 + 256 * u;
+        r[u] = i < N ? rec[i] : 0;
+        zi[u] = i < N ? zf[i] : 0.f;
+        hi[u] = i < N ? h[i] : 0.f;
+        qi[u] = i < N ? Q[i] : 0.f;
+        if ((unsigned)r[u] >= (unsigned)N) r[u] = i;  // as in k_core1
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) zr[u] = i0 + 256 * u < N ? zf[r[u]] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int i = i0 + 256 * u;
+        if (i >= N) break;
         float tS = edgesw;
-        if (r != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zi, zf[r]), dx), 1e-4f);
-        const float hi = h[i];
-        float Qo = __fmul_rn(dx, pow53(hi));
+        if (r[u] != i) tS = fmaxf(__fdiv_rn(__fsub_rn(zi[u], zr[u]), dx), 1e-4f);
+        float Qo = __fmul_rn(dx, pow53(hi[u]));
         Qo = __fdiv_rn(Qo, manning);
         Qo = __fmul_rn(Qo, __fsqrt_rn(tS));
-        float tdh = __fdiv_rn(__fsub_rn(Q[i], Qo), dx2);
+        float tdh = __fdiv_rn(__fsub_rn(qi[u], Qo), dx2);
         tdh = __fmul_rn(tdh, dt);
-        const float h1 = __fadd_rn(hi, tdh);
+        const float h1 = __fadd_rn(hi[u], tdh);
         if (h1 < 0.f) tdh = __fadd_rn(tdh, h1);
         dh[i] = tdh;
         const float hn = __fadd_rn(h1, tdh);  // k_core2
         h[i] = hn;
-        zh[i] = __fadd_rn(zi, tdh);
-        if (dhmax && href) m = fabsf(__fsub_rn(hn, href[i]));
+        zh[i] = __fadd_rn(zi[u], tdh);
+        // as unsigned bits: NaN sorts above every finite value
+        if (dhmax && href)
+            m = __uint_as_float(max(__float_as_uint(m), __float_as_uint(fabsf(__fsub_rn(hn, href[i])))));
     }
     if (!dhmax || !href) return;
     unsigned mu = __float_as_uint(m);
@@ -823,7 +839,7 @@ extern "C" int pff_graphflood_core_filled(float *h, float *zh, const float *zf, 
     }
     cudaStream_t st = S(stream);
     PFF_PROBED("k_core_fused", st,
-               k_core_fused<<<div_up(N, 256), 256, 0, st>>>(h, zh, zf, dh, rec, Q, N, dx, dx2, manning, edgesw, dt,
+               k_core_fused<<<div_up(N, 512), 256, 0, st>>>(h, zh, zf, dh, rec, Q, N, dx, dx2, manning, edgesw, dt,
                                                              h_ref, dhmax));
     count_launch();
     return check_cuda("pff_graphflood_core_filled");

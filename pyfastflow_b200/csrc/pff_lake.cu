@@ -1380,7 +1380,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
 }
 
 // The whole reroute of a grid whose steps do not fill the GPU, in one launch: with one
-// block per 2048 cells below one per SM, the four launches' latency (8-10 us of about
+// block per 1024 cells below one per SM, the four launches' latency (8-10 us of about
 // 60 at 48 x 33) is more than their wider grids save.
 template <int MODE>
 __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_whole(LoopArgs A, int32_t *R, int nzero)
@@ -1754,7 +1754,10 @@ static bool rr_device_on()
 
 // Blocks of the cooperative kernels: one per LOOP_CELLS cells up to one per SM (the device's
 // occupancy for them, asked once), 0 where they cannot be launched.
-constexpr int LOOP_CELLS = 2048, LOOP_ONE = 8192;
+// 1024 cells: one per thread; the whole reroute of 256 x 256 cells takes 156 us, 159 with 2048 cells per
+// block and 170 with 4096 (barriers over more blocks against fewer cells in flight).  Up to
+// LOOP_ONE cells one block and __syncthreads: at 48 x 33 a grid barrier costs more than the steps.
+constexpr int LOOP_CELLS = 1024, LOOP_ONE = 8192;
 template <int MODE>
 static void l_loop_ready(int dev, int *ready)
 {

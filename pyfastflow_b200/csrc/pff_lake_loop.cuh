@@ -274,7 +274,7 @@ struct LoopArgs {
     uint8_t *tag, *tag_;
     uint8_t *inv;
     int32_t *fin, *nf;
-    int *pit0, *pits[2];   // the first pit list; those of odd and even later iterations: [it & 1]
+    int *pit0, *pits[2];   // the first pit list; those of later iterations: [(it - it0) & 1]
     int *alist[2];         // border cells (the first list marks pit-basin cells by the sign bit)
     int *abid;             // later lists: a border cell's label,
     long long *akey;       // and its lowest (z', neighbour basin) key

@@ -34,7 +34,7 @@ def codes_like(mode, nx, ny, seed):
     return c
 
 
-# <= 8192 cells: one block; < 2048 per SM: several; 360,000: four launches (148 SMs)
+# <= 8192 cells: one block; < 1024 per SM: several; 360,000: four launches (148 SMs)
 @pytest.mark.parametrize("nx,ny", [(2, 2), (48, 33), (64, 32), (65, 127), (92, 90), (513, 130), (600, 601)])
 @pytest.mark.parametrize("kind", ["zeros", "int", "spectral", "high"])
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
