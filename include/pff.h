@@ -187,12 +187,12 @@ int pff_reroute_flow(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *rec__, 
  * queue more work behind the reroute before it looks at the result (no reference
  * counterpart; the Flooder's pipelined loop uses it).
  *   - pff_reroute_flow_async launches the device-driven outer loop and returns; the
- *     graph's last node copies its final state (9 ints) into ctl_out (device memory, or
+ *     loop's kernel writes its final state (9 ints) into ctl_out (device memory, or
  *     pinned host memory, which it writes through its unified address).
- *     Returns PFF_ERR_UNAVAILABLE where that loop cannot run (graphs switched off by
+ *     Returns PFF_ERR_UNAVAILABLE where that loop cannot run (switched off by
  *     pff_reroute_use_graphs / PFF_REROUTE_NO_GRAPH, or not supported).
  *   - pff_reroute_flow_finish takes a host copy of those 9 ints, once the launch has
- *     completed, and does what pff_reroute_flow does after its graph: nothing if the
+ *     completed, and does what pff_reroute_flow does after its loop: nothing if the
  *     loop finished on the device (ctl[3] = 1 no pits, or 2 done), the reference's
  *     steps on the host if it stopped for them (3, 4; synchronises), an error
  *     otherwise.  Same buffers and workspace as the async call; *n_outer_out as in

@@ -155,7 +155,7 @@ class FlowRouter:
     def reroute_flow_async(self, ctl: torch.Tensor) -> bool:
         """Launch the carve reroute's device-driven loop without waiting for it; its
         final state (9 int32) lands in `ctl` (a device tensor).  False where that
-        loop is not available (graphs switched off): call reroute_flow instead.
+        loop is not available (switched off): call reroute_flow instead.
         Complete with reroute_flow_finish once a host copy of `ctl` is readable."""
         if not self.lakeflow:
             raise RuntimeError("Flow field not compiled for lakeflow")
@@ -281,22 +281,15 @@ class FlowRouter:
                     wb[b].copy_(weights[k].reshape(-1), non_blocking=True)
             ev_in[b].record(h2d)
 
-        load(0)
-        for k in range(n):
+        def put(k):  # DEM k and its seeds into the router's fields
             b = k & 1
-            if k + 1 < n:
-                load(k + 1)
             main.wait_event(ev_in[b])
             self.z.copy_(zb[b])
-            if wb is not None:
-                self.Q.copy_(wb[b])
-            else:
-                self.Q.fill_(1.0)
+            self._seed_many(wb, b)
             ev_used[b].record(main)
-            self.compute_receivers()
-            if self.lakeflow:
-                self.reroute_flow(carve)
-            self._accumulate(True)
+
+        def take(k):  # the results of DEM k to the host
+            b = k & 1
             if k >= 2:
                 main.wait_event(ev_drained[b])  # results of DEM k-2 have left this buffer
             qb[b].copy_(self.Q)
@@ -309,8 +302,56 @@ class FlowRouter:
                 if out_counts is not None:
                     out_counts[k].reshape(-1).copy_(cb[b], non_blocking=True)
             ev_drained[b].record(d2h)
+
+        # While DEM k is accumulated the host enqueues its results' copies and DEM k+1's
+        # fields, then reads the accumulation's status: the GPU waited 70-80 us per DEM for
+        # those calls when they followed the read.  DEM k's own seeds stay in wb[b] until
+        # load(k+2), for the rare receivers that need another accumulation.
+        load(0)
+        put(0)
+        for k in range(n):
+            if k + 1 < n:
+                load(k + 1)
+            self.compute_receivers()
+            if self.lakeflow:
+                self.reroute_flow(carve)
+            read = self._accumulate_begin()
+            take(k)
+            if k + 1 < n:
+                put(k + 1)
+            if read() != 0:
+                self._seed_many(wb, k & 1)
+                ev_used[k & 1].record(main)
+                self._accumulate(True)
+                main.wait_event(ev_drained[k & 1])  # the seeds' copies of the first take
+                take(k)
+                if k + 1 < n:
+                    self._seed_many(wb, (k + 1) & 1)
+                    ev_used[(k + 1) & 1].record(main)
         main.wait_stream(d2h)
         main.wait_stream(h2d)
+
+    def _seed_many(self, wb, b):
+        if wb is not None:
+            self.Q.copy_(wb[b])
+        else:
+            self.Q.fill_(1.0)
+
+    def _accumulate_begin(self):
+        """Launch the tree accumulation of Q (with counts) without waiting; the returned
+        function reads its status (0: done; else _accumulate has to run on the seeds)."""
+        import ctypes as C
+
+        wp, wn = self._ws_tree.get(_lib.load().pff_accumulate_tree_workspace_bytes(self.nx, self.ny, 1), self.device)
+        _lib.call("pff_accumulate_tree", self.receivers.data_ptr(), self.Q.data_ptr(), 0.0, self.Q.data_ptr(),
+                  self.counts.data_ptr(), self.nx, self.ny, 1, wp, wn, _dev.stream())
+
+        def read():
+            st = C.c_int()
+            _lib.call("pff_accumulate_tree_status", self.nx, self.ny, 1, wp, wn, C.byref(st), _dev.stream())
+            return st.value
+
+        return read
 
     def accumulate_weighted_Q(self, weights, counts=True, exact_order=False):
         """Upstream sum of per-cell weights (e.g. precipitation-weighted

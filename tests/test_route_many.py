@@ -31,3 +31,40 @@ def test_route_many_matches_single_calls(cuda):
         torch.cuda.synchronize()
         assert np.array_equal(qh[k].numpy().view(np.uint32), r1.Q.cpu().numpy().view(np.uint32)), k
         assert np.array_equal(ch[k].numpy(), r1.counts.cpu().numpy()), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("failing", [(0,), (1, 2), (0, 1, 2, 3, 4)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_route_many_repeats_a_refused_accumulation(cuda, failing, weighted):
+    """A nonzero status after the next DEM's fields are queued: the results are still those
+    of every DEM's own seeds, bit for bit.  The status is made up on the host."""
+    torch = cuda
+    import pyfastflow_b200 as pf
+
+    n = 96
+    dems = [synthetic.routing_lakes(n, seed=s)["z"] for s in (3, 4, 5, 6, 7)]
+    zh = [torch.from_numpy(d.ravel().copy()).pin_memory() for d in dems]
+    wh = [torch.from_numpy(synthetic.lognormal_weights(n * n, 10 + k)).pin_memory() for k in range(5)]
+
+    def run(fail):
+        qh = [torch.empty(n * n, dtype=torch.float32).pin_memory() for _ in dems]
+        ch = [torch.empty(n * n, dtype=torch.int32).pin_memory() for _ in dems]
+        r = pf.flow.FlowRouter(n, n, 30.0)
+        begin, calls = r._accumulate_begin, []
+
+        def refused():
+            calls.append(0)
+            if len(calls) - 1 not in fail:
+                return begin()
+            r.counts.fill_(-1)
+            return lambda: 4
+
+        r._accumulate_begin = refused
+        r.route_many(zh, wh if weighted else None, qh, ch)
+        torch.cuda.synchronize()
+        return qh, ch
+
+    for a, b in zip(run(()), run(failing)):
+        for k in range(5):
+            assert torch.equal(a[k].view(torch.int32), b[k].view(torch.int32)), k
