@@ -269,11 +269,8 @@ __device__ __forceinline__ int swr(int r, int c)
     return CH % 8 ? r * CH + (c ^ ((r >> 1) & 3)) : r * CH + (c ^ (r & 7));
 }
 
-// BM x BN = 64 x 64, or 32 x 96 where Cout <= 32: the full-resolution layers have Cout = 32
-// (8 in the head) and K = 9 Cin = 288 or 864, so 64 x 64 tiles were half padding.  A
-// thread's pixels advance by WG_BK per stage: their positions are kept, not divided out
-// (two 64-bit divisions per 16 bytes loaded had cost more than the products: 1120 us for
-// the 15 launches of a training step at 16 x 128 x 128).
+// The form for rows whose tiles k_conv3x3_wgrad9 cannot address in 32 bits.  A thread's
+// pixels advance by WG_BK per stage: their positions are kept, not divided out.
 template <int BM, int BN>
 __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(WgradArgs a)
 {
@@ -390,6 +387,209 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(WgradArgs a)
                 if (k + 1 < K) atomicAdd(a.dw + (long long)co * K + k + 1, acc[i][j][2 * hf + 1]);
             }
         }
+}
+
+// The weight gradient: all nine taps of a CO x CI
+// channel block in one CTA.  With one tile of the GEMM per CTA every pixel's activations
+// crossed from L2 once per tap and column tile (24 to 32 products per byte); here a stage
+// is a tile of 8 rows of 16 pixels and its halo, which the taps read shifted, at 144
+// products per byte (32 x 32) or 230 (64 x 64).  12 warps = 3 tap rows x 4: quadrants of
+// 32 x 32 channels, or where the block has fewer, groups that take every 2nd or 4th row
+// and meet in shared memory at the end.  A warp keeps three taps' 32 x 32 sums (96
+// registers) and loads dy's fragments once for the three.  For one pixel tile per pass the
+// tensor pipe is the bound; what is left are the few passes per CTA (4 to 20) and the
+// adds into dw.  At 16 x 128 x 128 (full resolution), old and new: 96 -> 32 channels 117 and
+// 50 us, 32 -> 32 39 and 23; at 16 x 32 x 32, 384 -> 128 channels 83 and 45 us.
+// Halo rows are 24 pixels apart in shared memory, a multiple of the swizzle's period, so
+// that a fragment's address moves by a constant from row to row.
+constexpr int W9_TW = 16, W9_HW = W9_TW + 2, W9_PITCH = 24, W9_ST = 3, W9_THREADS = 384;
+__host__ __device__ constexpr int w9_rows(int CO, int CI) { return CO * CI == 4096 ? 8 : 16; }
+__host__ __device__ constexpr int w9_smem(int CO, int CI)
+{
+    return W9_ST * 2 * (W9_TW * w9_rows(CO, CI) * CO + W9_PITCH * (w9_rows(CO, CI) + 2) * CI);
+}
+
+struct Wgrad9Args {
+    const bf16_t *x;
+    int csx, offx;
+    const bf16_t *dy;
+    int csd, offd;
+    float *dw;
+    int B, H, W, Cin, Cout;
+    int ntx, nty, ntiles;  // pixel tiles across, down, in all
+    int pair;              // dw takes 8-byte adds
+};
+
+template <int CO, int CI>
+__global__ void __launch_bounds__(W9_THREADS, 1) k_conv3x3_wgrad9(Wgrad9Args a)
+{
+    constexpr int CA = CO / 8, CB = CI / 8, QM = CO / 32, Q = QM * (CI / 32), KG = 4 / Q;
+    constexpr int TH = w9_rows(CO, CI);
+    constexpr int SA = W9_TW * TH * CA, SB = W9_PITCH * (TH + 2) * CB;  // 16-byte chunks of a stage
+    extern __shared__ __align__(128) uint4 w9[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int trow = warp % 3, grp = warp / 3, quad = grp % Q, kg = grp / Q;
+    const int qm = quad % QM * 32, qn = quad / QM * 32;
+    const int m0 = blockIdx.y * CO, n0 = blockIdx.x * CI;
+    const int t0 = (int)((long long)a.ntiles * blockIdx.z / gridDim.z);
+    const int nt = (int)((long long)a.ntiles * (blockIdx.z + 1) / gridDim.z) - t0;
+
+    // the next tile to load and the next to multiply
+    int lx = t0 % a.ntx, ly = t0 / a.ntx % a.nty, lb = t0 / a.ntx / a.nty, cx = lx, cy = ly;
+    auto load_stage = [&](int st) {
+        const int y0 = ly * TH, x0 = lx * W9_TW;
+        const long long at = ((long long)lb * a.H + y0) * a.W + x0;  // the tile's first pixel
+        const bf16_t *da = a.dy + at * a.csd + a.offd + m0, *xb = a.x + (at - a.W - 1) * a.csx + a.offx + n0;
+        uint4 *A = w9 + st * (SA + SB), *B = A + SA;
+#pragma unroll
+        for (int j = 0; j < (SA + W9_THREADS - 1) / W9_THREADS; ++j) {
+            const int e = tid + W9_THREADS * j, r = e / CA, c = e % CA, y = r / W9_TW, x = r % W9_TW;
+            if (SA % W9_THREADS && e >= SA) break;
+            const bool v = y0 + y < a.H && x0 + x < a.W && m0 + c * 8 < a.Cout;
+            cp_async16(smem_u32(A + swr<CA>(r, c)), v ? da + ((y * a.W + x) * a.csd + c * 8) : a.dy, v);
+        }
+#pragma unroll
+        for (int j = 0; j < (W9_HW * (TH + 2) * CB + W9_THREADS - 1) / W9_THREADS; ++j) {
+            const int e = tid + W9_THREADS * j, r = e / CB, c = e % CB, y = r / W9_HW, x = r % W9_HW;
+            if (e >= W9_HW * (TH + 2) * CB) break;
+            const bool v = (unsigned)(y0 + y - 1) < (unsigned)a.H && (unsigned)(x0 + x - 1) < (unsigned)a.W &&
+                           n0 + c * 8 < a.Cin;
+            cp_async16(smem_u32(B + swr<CB>(y * W9_PITCH + x, c)), v ? xb + ((y * a.W + x) * a.csx + c * 8) : a.x, v);
+        }
+        if (++lx == a.ntx) {
+            lx = 0;
+            if (++ly == a.nty) ly = 0, ++lb;
+        }
+    };
+    float acc[3][2][4][4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[d][i][j][q] = 0.f;
+#pragma unroll
+    for (int s = 0; s < W9_ST - 1; ++s) {
+        if (s < nt) load_stage(s);
+        cp_commit();
+    }
+    // fragment addresses in the first stage, at the group's first row
+    const int ar = kg * W9_TW + (lane & 7) + ((lane >> 4) << 3), ac = qm / 8 + ((lane >> 3) & 1);
+    const int br = (kg + trow) * W9_PITCH + (lane & 7) + (((lane >> 3) & 1) << 3), bc = qn / 8 + (lane >> 4);
+    const unsigned s0 = smem_u32(w9);
+    unsigned fa[2], fb[3][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) fa[i] = 16 * swr<CA>(ar, ac + 2 * i);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) fb[d][j] = 16 * (SA + swr<CB>(br + d, bc + 2 * j));
+    for (int k = 0; k < nt; ++k) {
+        cp_wait<W9_ST - 2>();
+        __syncthreads();
+        if (k + W9_ST - 1 < nt) load_stage((k + W9_ST - 1) % W9_ST);
+        cp_commit();
+        const unsigned sk = s0 + k % W9_ST * (16 * (SA + SB));
+        const int rows = a.H - cy * TH;  // rows below the image are left out
+        // the column right of the image has dy = 0 but the image's last x at its left tap:
+        // that x is taken out of the fragments, as 0 times an infinity is no 0
+        const int xe = a.W - cx * W9_TW;
+        unsigned mask[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            mask[h] = xe < W9_TW && (xe >> 1) == (lane & 3) + 4 * h ? (xe & 1 ? 0x0000ffffu : 0xffff0000u) : 0xffffffffu;
+        if (++cx == a.ntx) {
+            cx = 0;
+            if (++cy == a.nty) cy = 0;
+        }
+        auto row_products = [&](int m) {  // the group's m-th row
+            unsigned af[2][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                ldsm_x4_t(sk + fa[i] + m * (KG * W9_TW * CA * 16), af[i][0], af[i][1], af[i][2], af[i][3]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                unsigned bf[4][2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    ldsm_x4_t(sk + fb[d][j] + m * (KG * W9_PITCH * CB * 16), bf[2 * j][0], bf[2 * j][1],
+                              bf[2 * j + 1][0], bf[2 * j + 1][1]);
+                if (d == 0) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) bf[j][0] &= mask[0], bf[j][1] &= mask[1];
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        mma16816(acc[d][i][j], af[i][0], af[i][1], af[i][2], af[i][3], bf[j][0], bf[j][1]);
+            }
+        };
+        if (rows >= TH) {
+#pragma unroll 4
+            for (int m = 0; m < TH / KG; ++m) row_products(m);
+        } else {
+#pragma unroll 1
+            for (int m = 0; kg + m * KG < rows; ++m) row_products(m);
+        }
+    }
+    cp_wait<0>();
+    if (KG > 1) {  // the row groups' sums, one group at a time (3 Q warps of 96 x 32 floats)
+        float *red = reinterpret_cast<float *>(w9) + (trow * Q + quad) * 96 * 32 + lane;
+        for (int g = 1; g < KG; ++g) {
+            __syncthreads();
+            if (kg == g) {
+#pragma unroll
+                for (int e = 0; e < 96; ++e) red[e * 32] = acc[e / 32][e / 16 % 2][e / 4 % 4][e % 4];
+            }
+            __syncthreads();
+            if (kg == 0) {
+#pragma unroll
+                for (int e = 0; e < 96; ++e) acc[e / 32][e / 16 % 2][e / 4 % 4][e % 4] += red[e * 32];
+            }
+        }
+        if (kg) return;
+    }
+    const long long K = 9LL * a.Cin;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int co = m0 + qm + i * 16 + (lane >> 2) + hf * 8;
+                if (co >= a.Cout) continue;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int ci = n0 + qn + j * 8 + 2 * (lane & 3);
+                    if (ci >= a.Cin) continue;
+                    float *o = a.dw + co * K + (3 * trow + d) * a.Cin + ci;
+                    const float v0 = acc[d][i][j][2 * hf], v1 = acc[d][i][j][2 * hf + 1];
+                    if (a.pair)
+                        atomicAdd(reinterpret_cast<float2 *>(o), make_float2(v0, v1));
+                    else
+                        atomicAdd(o, v0), atomicAdd(o + 1, v1);
+                }
+            }
+}
+
+template <int CO, int CI>
+static int launch_wgrad9(Wgrad9Args a, cudaStream_t st)
+{
+    static_assert(CO * CI == 4096 || w9_smem(CO, CI) >= 3 * 96 * 32 * 4 * (CO * CI / 1024), "room for the groups' sums");
+    auto kern = k_conv3x3_wgrad9<CO, CI>;
+    PFF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, w9_smem(CO, CI)));
+    const int nb = (a.Cin + CI - 1) / CI, mb = (a.Cout + CO - 1) / CO;
+    a.ntx = (a.W + W9_TW - 1) / W9_TW;
+    a.nty = (a.H + w9_rows(CO, CI) - 1) / w9_rows(CO, CI);
+    a.ntiles = a.B * a.ntx * a.nty;
+    // one CTA per SM: as many ranges of pixel tiles as that takes
+    const int split = std::max(1, std::min(a.ntiles, 148 / (nb * mb)));
+    kern<<<dim3(nb, mb, split), W9_THREADS, w9_smem(CO, CI), st>>>(a);
+    count_launch();
+    return PFF_OK;
 }
 
 // ---- small ops --------------------------------------------------------------------------
@@ -739,8 +939,21 @@ extern "C" int pff_conv3x3_wgrad(const bf16_t *x, int csx, int offx, const bf16_
     PFF_TRY(check_slice("pff_conv3x3_wgrad input", csx, offx, Cin));
     PFF_TRY(check_slice("pff_conv3x3_wgrad dy", csd, offd, Cout));
     const long long P = (long long)B * H * W;
+    // always, where a tile's offsets and the number of tiles fit 32 bits (also with 8 channels on
+    // one side, three quarters of a block padding: 8 -> 32 at 16 x 128 x 128 23 us against 31,
+    // 32 -> 8 22 against 39)
+    if (Cin <= 32768 && Cout <= 32768 && P < (1LL << 30) &&
+        (20LL * W + 32) * std::max(csx, csd) < (1LL << 31)) {
+        Wgrad9Args a{x, csx, offx, dy, csd, offd, dw, B, H, W, Cin, Cout, 0, 0, 0, ((uintptr_t)dw & 7) == 0};
+        // channel blocks of 64 where at most 31 of the last one's are padding
+        const bool co64 = (Cout + 31) / 32 % 2 == 0, ci64 = (Cin + 31) / 32 % 2 == 0;
+        const int rc = co64 ? ci64 ? launch_wgrad9<64, 64>(a, S(stream)) : launch_wgrad9<64, 32>(a, S(stream))
+                            : ci64 ? launch_wgrad9<32, 64>(a, S(stream)) : launch_wgrad9<32, 32>(a, S(stream));
+        if (rc != PFF_OK) return rc;
+        return check_cuda("pff_conv3x3_wgrad");
+    }
     const int K = 9 * Cin;
-    const int bm = Cout <= 32 ? 32 : 64, bn = Cout <= 32 ? 96 : 64;
+    constexpr int bm = 64, bn = 64;
     const int tiles = ((K + bn - 1) / bn) * ((Cout + bm - 1) / bm);
     // enough pixel chunks for ~4 CTAs per SM, each at least 512 pixels
     long long chunks = std::max<long long>(1, (148LL * 4 + tiles - 1) / tiles);
@@ -753,8 +966,7 @@ extern "C" int pff_conv3x3_wgrad(const bf16_t *x, int csx, int offx, const bf16_
     }
     WgradArgs a{x, csx, offx, dy, csd, offd, dw, B, H, W, Cin, Cout, pchunk};
     dim3 grid((unsigned)((K + bn - 1) / bn), (unsigned)((Cout + bm - 1) / bm), (unsigned)chunks);
-    if (bm == 32) k_conv3x3_wgrad<32, 96><<<grid, WG_THREADS, 0, S(stream)>>>(a);
-    else k_conv3x3_wgrad<64, 64><<<grid, WG_THREADS, 0, S(stream)>>>(a);
+    k_conv3x3_wgrad<bm, bn><<<grid, WG_THREADS, 0, S(stream)>>>(a);
     count_launch();
     return check_cuda("pff_conv3x3_wgrad");
 }

@@ -236,6 +236,63 @@ def test_conv_tiles_by_channel_count(cuda, cin, cout, B, H, W):
     assert ((dw.double() - rw).abs() <= B * H * W * 2.0 ** -24 * mw + 1e-30).all()
 
 
+# channel blocks of 32 and 64 with and without padding; pixel tiles of 8 or 16 rows of 16 with remainders
+@pytest.mark.parametrize("cin,cout", [(24, 24), (64, 32), (32, 64), (64, 64), (104, 72)])
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (2, 8, 16), (3, 9, 17), (1, 15, 31), (2, 33, 40), (70, 8, 8)])
+def test_weight_gradient_tiles(cuda, cin, cout, B, H, W):
+    """The nine-tap weight gradient on channel slices, added onto dw, 4- and 8-byte aligned,
+    against torch in f64 (tolerance as above).  An infinity in the last column reaches the
+    same sums and no others."""
+    torch = cuda
+    import torch.nn.functional as F
+
+    from pyfastflow_b200 import _dev, _lib
+
+    x, dy = _bf(torch, B, H, W, cin + 16, seed=1).cuda(), _bf(torch, B, H, W, cout + 8, seed=2).cuda()
+    n = cout * 9 * cin
+    for inf, off in ((False, 0), (False, 1), (True, 0)):
+        if inf:
+            x[0, 0, W - 1, 8] = float("inf")
+        xs, ds = x[..., 8:8 + cin].double(), dy[..., 8:].double()
+        buf = torch.full((n + 1,), 0.5, device="cuda")
+        dw = buf[off:off + n]
+        _lib.call("pff_conv3x3_wgrad", x.data_ptr(), cin + 16, 8, dy.data_ptr(), cout + 8, 8, dw.data_ptr(), B, H, W, cin,
+                  cout, _dev.stream())
+        got = dw.double().reshape(cout, 9, cin)
+
+        def ref(u, v):
+            up = F.pad(u, (0, 0, 1, 1, 1, 1))
+            taps = [torch.einsum("bhwo,bhwi->oi", v, up[:, t // 3:t // 3 + H, t % 3:t % 3 + W]) for t in range(9)]
+            return torch.stack(taps, 1)
+
+        fin = torch.where(torch.isfinite(xs), xs, torch.zeros((), dtype=torch.float64, device="cuda"))
+        rw, mw = ref(fin, ds) + 0.5, ref(fin.abs(), ds.abs()) + 0.5
+        hit = ref((~torch.isfinite(xs)).double(), ds.abs()) != 0
+        assert torch.equal(~torch.isfinite(got), hit)
+        assert ((got - rw).abs()[~hit] <= ((B * H * W + 150) * 2.0 ** -24 * mw + 1e-30)[~hit]).all()
+        assert buf[n * (1 - off)].item() == 0.5
+
+
+def test_weight_gradient_long_rows(cuda):
+    """A channel stride beyond the tiles' 32-bit offsets takes the general kernel: the same
+    gradient as for dense rows (tolerance as above, twice)."""
+    torch = cuda
+    from pyfastflow_b200 import _dev, _lib
+
+    cs, cin, cout, W = 41_297_768, 24, 40, 3  # (20 W + 32) cs >= 2^31
+    x, dy = _bf(torch, 1, 1, W, cin, seed=1).cuda(), _bf(torch, 1, 1, W, cout, seed=2).cuda()
+    wide = torch.zeros(W * cs, dtype=torch.bfloat16, device="cuda")
+    wide.view(W, cs)[:, 16:16 + cin] = x[0, 0]
+    out = []
+    for t, c, off in ((x, cin, 0), (wide, cs, 16)):
+        dw = torch.zeros(cout, 9, cin, device="cuda")
+        _lib.call("pff_conv3x3_wgrad", t.data_ptr(), c, off, dy.data_ptr(), cout, 0, dw.data_ptr(), 1, 1, W, cin, cout,
+                  _dev.stream())
+        out.append(dw)
+    mag = dy.abs().float().amax() * x.abs().float().amax() * W
+    assert out[0].abs().sum() > 0 and ((out[0] - out[1]).abs() <= 2 * W * 2.0 ** -24 * mag).all()
+
+
 @pytest.mark.parametrize("C_,B,H,W", [(8, 1, 2, 2), (24, 3, 6, 10), (96, 2, 16, 8), (256, 1, 4, 6)])
 def test_small_ops_16_byte_forms(cuda, C_, B, H, W):
     """Resampling and the ReLU / bias gradient on 8 channels per thread against the
