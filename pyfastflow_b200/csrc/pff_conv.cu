@@ -78,6 +78,39 @@ struct ConvArgs {
 // 64-byte rows (4 chunks of 16 B), chunk c of row r stored at c ^ ((r >> 1) & 3)
 __device__ __forceinline__ int sw64(int r, int c) { return r * 4 + (c ^ ((r >> 1) & 3)); }
 
+// Rows of CH 16-byte chunks, chunk c of row r stored at c ^ (r & 7) within its group of 8, or at
+// c ^ ((r >> 1) & 3) within 4 (CH = 4, 12): ldmatrix reads 8 rows of a chunk without conflicts.
+template <int CH>
+__device__ __forceinline__ int swr(int r, int c)
+{
+    return CH % 8 ? r * CH + (c ^ ((r >> 1) & 3)) : r * CH + (c ^ (r & 7));
+}
+
+// bias, ReLU and the store of channels co, co + 1 of pixel p (bf16 pairs, or f32)
+__device__ __forceinline__ void conv_store(const ConvArgs &a, long long p, int co, float v0, float v1)
+{
+    const bool two = co + 1 < a.Cout;
+    if (a.bias) {
+        v0 += a.bias[co];
+        if (two) v1 += a.bias[co + 1];
+    }
+    if (a.relu) {
+        v0 = fmaxf(v0, 0.f);
+        v1 = fmaxf(v1, 0.f);
+    }
+    if (a.out_f32) {
+        float *yo = (float *)a.y + p * a.csy + a.offy + co;
+        yo[0] = v0;
+        if (two) yo[1] = v1;
+    } else {
+        bf16_t *yo = (bf16_t *)a.y + p * a.csy + a.offy + co;
+        if (two)
+            *reinterpret_cast<unsigned *>(yo) = (unsigned)f2bf(v0) | ((unsigned)f2bf(v1) << 16);
+        else
+            yo[0] = f2bf(v0);
+    }
+}
+
 // BN output channels per CTA: 64 (2 x 2 warps of 64 x 32), or 32 and 16 (4 warps of
 // 32 x BN) where Cout is that small.  The U-Net's full-resolution layers have 32 (and the
 // head 8) output channels and only 9 to 27 K steps, so half to seven eighths of a 64-wide
@@ -205,30 +238,133 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv3x3(ConvArgs a)
             for (int j = 0; j < NJ; ++j) {
                 const int co = n0 + wn * (8 * NJ) + j * 8 + 2 * (lane & 3);
                 if (co >= a.Cout) continue;
-                float v0 = acc[i][j][2 * hf], v1 = acc[i][j][2 * hf + 1];
-                if (a.bias) {
-                    v0 += a.bias[co];
-                    if (co + 1 < a.Cout) v1 += a.bias[co + 1];
+                conv_store(a, p, co, acc[i][j][2 * hf], acc[i][j][2 * hf + 1]);
+            }
+        }
+}
+
+// The convolution with 32, 64 or 96 input channels: the im2col form above fetches every
+// pixel nine times from L2 and a thread's addresses cost more than its products.  Here a
+// CTA keeps the weights of NB output channels in shared memory and walks over tiles of 16
+// rows of 16 pixels, double-buffered with their halo; the taps read the tile shifted.  A
+// warp takes MI rows of pixels; K steps go through taps and channels in the order of the
+// form above, so every sum is the same.  Bound by
+// fragment loads (6 per 16 products) and the tensor pipe; 16 x 128 x 128, before and now:
+// 96 -> 32 channels 74 and 54 us, 32 -> 96 90 and 56, 32 -> 32 31 and 27, 32 -> 8 27 and 20;
+// 64 -> 32 at 16 x 64 x 64 19 and 15.
+constexpr int CT_TW = 16, CT_TH = 16, CT_HW = CT_TW + 2, CT_PITCH = 24;
+__host__ __device__ constexpr int ct_smem(int CC, int NB) { return 16 * (NB * (9 * CC + 1) + 2 * CT_PITCH * (CT_TH + 2) * CC); }
+
+template <int CC, int NB, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_conv3x3_tile(ConvArgs a, int ntx, int nty, int ntiles)
+{
+    constexpr int MI = CT_TH / WARPS, NJ = NB / 8, THREADS = 32 * WARPS;
+    constexpr int WR = 9 * CC + 1;  // chunks per weight row, odd: 8 rows on 8 bank groups
+    constexpr int ST = CT_PITCH * (CT_TH + 2) * CC;
+    extern __shared__ __align__(128) uint4 ct[];
+    uint4 *sW = ct, *sX = ct + NB * WR;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n0 = blockIdx.y * NB;
+    for (int e = tid; e < NB * 9 * CC; e += THREADS) {
+        const int n = e / (9 * CC), q = e % (9 * CC);
+        const bool v = n0 + n < a.Cout;
+        cp_async16(smem_u32(sW + n * WR + q), v ? a.w + ((long long)(n0 + n) * 9 * CC + q) * 8 : a.w, v);
+    }
+    auto load_tile = [&](int st, int t) {
+        const int tx = t % ntx, u = t / ntx, ty = u % nty, b = u / nty;
+        const int y0 = ty * CT_TH - 1, x0 = tx * CT_TW - 1;
+        const bf16_t *xb = a.x + (((long long)b * a.H + y0) * a.W + x0) * a.csx + a.offx;
+        uint4 *X = sX + st * ST;
+        for (int e = tid; e < CT_HW * (CT_TH + 2) * CC; e += THREADS) {
+            const int r = e / CC, c = e % CC, y = r / CT_HW, x = r % CT_HW;
+            const bool v = (unsigned)(y0 + y) < (unsigned)a.H && (unsigned)(x0 + x) < (unsigned)a.W;
+            cp_async16(smem_u32(X + swr<CC>(y * CT_PITCH + x, c)), v ? xb + ((y * a.W + x) * a.csx + c * 8) : a.x, v);
+        }
+        cp_commit();
+    };
+    const unsigned wb = smem_u32(sW) + 16 * (((lane & 7) + ((lane >> 4) << 3)) * WR + ((lane >> 3) & 1));
+    const unsigned xs = smem_u32(sX);
+    int t = blockIdx.x;
+    load_tile(0, t);  // the weights' copies are in the same group
+    for (int k = 0; t < ntiles; ++k, t += gridDim.x) {
+        if (t + (int)gridDim.x < ntiles)
+            load_tile((k + 1) & 1, t + gridDim.x);
+        else
+            cp_commit();
+        cp_wait<1>();
+        __syncthreads();
+        float acc[MI][NJ][4];
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+        const unsigned xb = xs + 16 * ((k & 1) * ST + warp * MI * CT_PITCH * CC);
+#pragma unroll 1
+        for (int kh = 0; kh < 3; ++kh) {
+#pragma unroll
+            for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+                for (int s = 0; s < CC / 2; ++s) {
+                    unsigned af[MI][4], bf[NJ][2];
+                    const unsigned xa = xb + 16 * (kh * CT_PITCH * CC + swr<CC>(kw + (lane & 15), 2 * s + (lane >> 4)));
+#pragma unroll
+                    for (int i = 0; i < MI; ++i)
+                        ldsm_x4(xa + i * (16 * CT_PITCH * CC), af[i][0], af[i][1], af[i][2], af[i][3]);
+#pragma unroll
+                    for (int j = 0; j < NJ / 2; ++j)
+                        ldsm_x4(wb + 16 * (j * 16 * WR + (3 * kh + kw) * CC + 2 * s), bf[2 * j][0], bf[2 * j][1],
+                                bf[2 * j + 1][0], bf[2 * j + 1][1]);
+#pragma unroll
+                    for (int i = 0; i < MI; ++i)
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j)
+                            mma16816(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bf[j][0], bf[j][1]);
                 }
-                if (a.relu) {
-                    v0 = fmaxf(v0, 0.f);
-                    v1 = fmaxf(v1, 0.f);
-                }
-                if (a.out_f32) {
-                    float *yo = (float *)a.y + p * a.csy + a.offy + co;
-                    yo[0] = v0;
-                    if (co + 1 < a.Cout) yo[1] = v1;
-                } else {
-                    bf16_t *yo = (bf16_t *)a.y + p * a.csy + a.offy + co;
-                    if (co + 1 < a.Cout) {
-                        const unsigned pk = (unsigned)f2bf(v0) | ((unsigned)f2bf(v1) << 16);
-                        *reinterpret_cast<unsigned *>(yo) = pk;
-                    } else {
-                        yo[0] = f2bf(v0);
-                    }
+        }
+        __syncthreads();  // the tile's buffer is free for the load after next
+        const int tx = t % ntx, u = t / ntx, ty = u % nty, b = u / nty;
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            const int y = ty * CT_TH + warp * MI + i;
+            if (y >= a.H) break;
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int x = tx * CT_TW + (lane >> 2) + hf * 8;
+                if (x >= a.W) continue;
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    const int co = n0 + j * 8 + 2 * (lane & 3);
+                    if (co < a.Cout)
+                        conv_store(a, ((long long)b * a.H + y) * a.W + x, co, acc[i][j][2 * hf], acc[i][j][2 * hf + 1]);
                 }
             }
         }
+    }
+    cp_wait<0>();
+}
+
+template <int CC, int NB, int WARPS>
+static int launch_conv_tile(const ConvArgs &a, cudaStream_t st)
+{
+    auto kern = k_conv3x3_tile<CC, NB, WARPS>;
+    constexpr int smem = ct_smem(CC, NB), per = 227 * 1024 / (smem + 1024);
+    static_assert(per >= 1, "shared memory of an SM");
+    PFF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const int ntx = (a.W + CT_TW - 1) / CT_TW, nty = (a.H + CT_TH - 1) / CT_TH, nt = a.B * ntx * nty;
+    const int ny = (a.Cout + NB - 1) / NB;
+    // resident CTAs, each with the same number of tiles but for one
+    const int most = std::max(1, 148 * std::min(per, 3) / ny), each = (nt + most - 1) / most;
+    kern<<<dim3((nt + each - 1) / each, ny), 32 * WARPS, smem, st>>>(a, ntx, nty, nt);
+    count_launch();
+    return PFF_OK;
+}
+
+template <int CC, int WARPS>
+static int launch_conv_tile(const ConvArgs &a, cudaStream_t st)
+{
+    return a.Cout > 16 ? launch_conv_tile<CC, 32, WARPS>(a, st) : launch_conv_tile<CC, 16, WARPS>(a, st);
 }
 
 // wt[ci][tap'][co] = w[co][8 - tap'][ci]: the data gradient of a 3x3 convolution is
@@ -260,14 +396,6 @@ struct WgradArgs {
     int B, H, W, Cin, Cout;
     long long pchunk;  // pixels per CTA (multiple of WG_BK)
 };
-
-// Rows of CH 16-byte chunks, chunk c of row r stored at c ^ (r & 7) within its group of 8, or at
-// c ^ ((r >> 1) & 3) within 4 (CH = 4, 12): ldmatrix reads 8 rows of a chunk without conflicts.
-template <int CH>
-__device__ __forceinline__ int swr(int r, int c)
-{
-    return CH % 8 ? r * CH + (c ^ ((r >> 1) & 3)) : r * CH + (c ^ (r & 7));
-}
 
 // The form for rows whose tiles k_conv3x3_wgrad9 cannot address in 32 bits.  A thread's
 // pixels advance by WG_BK per stage: their positions are kept, not divided out.
@@ -906,6 +1034,14 @@ extern "C" int pff_conv3x3_fwd(const bf16_t *x, int csx, int offx, const bf16_t 
         return conv3x3_tc(x, csx, offx, w, bias, y, csy, offy, B, H, W, Cin, Cout, relu, out_f32, S(stream));
     ConvArgs a{x, csx, offx, w, bias, y, csy, offy, B, H, W, Cin, Cout, relu, out_f32};
     const long long P = (long long)B * H * W;
+    // whole tiles of 32, 64 or 96 channels fit shared memory twice beside the weights; other counts,
+    // and rows beyond 32-bit offsets within a tile, take the im2col form
+    if (Cin % 32 == 0 && Cin <= 96 && P < (1LL << 30) && (20LL * W + 32) * csx < (1LL << 31)) {
+        const int rc = Cin == 32 ? launch_conv_tile<4, 4>(a, S(stream))
+                     : Cin == 64 ? launch_conv_tile<8, 8>(a, S(stream)) : launch_conv_tile<12, 8>(a, S(stream));
+        if (rc != PFF_OK) return rc;
+        return check_cuda("pff_conv3x3_fwd");
+    }
     const int bn = Cout > 32 ? 64 : (Cout > 16 ? 32 : 16);
     dim3 grid((unsigned)((P + CV_BM - 1) / CV_BM), (unsigned)((Cout + bn - 1) / bn));
     if (bn == 64) k_conv3x3<64><<<grid, CV_THREADS, 0, S(stream)>>>(a);

@@ -273,6 +273,51 @@ def test_weight_gradient_tiles(cuda, cin, cout, B, H, W):
         assert buf[n * (1 - off)].item() == 0.5
 
 
+@pytest.mark.parametrize("cin", [32, 64, 96])
+@pytest.mark.parametrize("cout,f32", [(8, 0), (17, 1), (40, 0)])
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (2, 16, 16), (1, 17, 18)])
+def test_conv_tile_is_the_im2col_form(cuda, cin, cout, f32, B, H, W):
+    """Tiles with a halo in shared memory against the im2col kernel, which a channel stride
+    beyond 32-bit tile offsets takes: bit for bit."""
+    torch = cuda
+    from pyfastflow_b200 import _dev, _lib
+
+    cs = (2 ** 31 // (20 * W + 32) + 8) // 8 * 8
+    x = _bf(torch, B * H * W, cin, seed=1).cuda()
+    w, bias = _bf(torch, cout, 9, cin, seed=3).cuda(), torch.linspace(-1, 1, cout, device="cuda")
+    wide = torch.empty(B * H * W * cs, dtype=torch.bfloat16, device="cuda")
+    wide.view(B * H * W, cs)[:, 16:16 + cin] = x
+    out = []
+    _lib.call("pff_conv_set_path", 1)
+    try:
+        for t, c, off in ((x, cin, 0), (wide, cs, 16)):
+            y = torch.full((B * H * W, cout + 8), 7.0, device="cuda").to(torch.float32 if f32 else torch.bfloat16)
+            _lib.call("pff_conv3x3_fwd", t.data_ptr(), c, off, w.data_ptr(), bias.data_ptr(), y.data_ptr(), cout + 8, 4,
+                      B, H, W, cin, cout, 1, f32, _dev.stream())
+            out.append(y)
+    finally:
+        _lib.call("pff_conv_set_path", 0)
+    assert (out[0][:, :4] == 7).all() and (out[0][:, 4 + cout:] == 7).all() and (out[0][:, 4:4 + cout] == 0).any()
+    dt = torch.int32 if f32 else torch.int16
+    assert torch.equal(out[0].view(dt), out[1].view(dt))
+
+
+def test_conv_tile_many_tiles(cuda):
+    """More tiles than CTAs: two images' rows against each image by itself, bit for bit."""
+    torch = cuda
+    from pyfastflow_b200 import _dev, _lib
+
+    B, H, W, cin, cout = 9, 120, 136, 32, 96
+    x, w = _bf(torch, B, H, W, cin, seed=1).cuda(), _bf(torch, cout, 9, cin, seed=3).cuda()
+    y, z = (torch.zeros(B, H, W, cout, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    _lib.call("pff_conv3x3_fwd", x.data_ptr(), cin, 0, w.data_ptr(), None, y.data_ptr(), cout, 0, B, H, W, cin, cout, 0, 0,
+              _dev.stream())
+    for b in range(B):
+        _lib.call("pff_conv3x3_fwd", x[b].data_ptr(), cin, 0, w.data_ptr(), None, z[b].data_ptr(), cout, 0, 1, H, W, cin,
+                  cout, 0, 0, _dev.stream())
+    assert y.abs().sum() > 0 and torch.equal(y.view(torch.int16), z.view(torch.int16))
+
+
 def test_weight_gradient_long_rows(cuda):
     """A channel stride beyond the tiles' 32-bit offsets takes the general kernel: the same
     gradient as for dense rows (tolerance as above, twice)."""
