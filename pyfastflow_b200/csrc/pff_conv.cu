@@ -524,9 +524,9 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(WgradArgs a)
 // products per byte (32 x 32) or 230 (64 x 64).  12 warps = 3 tap rows x 4: quadrants of
 // 32 x 32 channels, or where the block has fewer, groups that take every 2nd or 4th row
 // and meet in shared memory at the end.  A warp keeps three taps' 32 x 32 sums (96
-// registers) and loads dy's fragments once for the three.  For one pixel tile per pass the
-// tensor pipe is the bound; what is left are the few passes per CTA (4 to 20) and the
-// adds into dw.  At 16 x 128 x 128 (full resolution), old and new: 96 -> 32 channels 117 and
+// registers) and loads dy's fragments once for the three.  Bound by the
+// mma.sync pipe (active 57 to 65 % of the kernel; L2 11 %); the rest are the first loads, the
+// few passes per CTA (4 to 20) and the adds into dw.  At 16 x 128 x 128 (full resolution), old and new: 96 -> 32 channels 117 and
 // 50 us, 32 -> 32 39 and 23; at 16 x 32 x 32, 384 -> 128 channels 83 and 45 us.
 // Halo rows are 24 pixels apart in shared memory, a multiple of the swizzle's period, so
 // that a fragment's address moves by a constant from row to row.
@@ -1036,7 +1036,7 @@ extern "C" int pff_conv3x3_fwd(const bf16_t *x, int csx, int offx, const bf16_t 
     const long long P = (long long)B * H * W;
     // whole tiles of 32, 64 or 96 channels fit shared memory twice beside the weights; other counts,
     // and rows beyond 32-bit offsets within a tile, take the im2col form
-    if (Cin % 32 == 0 && Cin <= 96 && P < (1LL << 30) && (20LL * W + 32) * csx < (1LL << 31)) {
+    if (Cin % 32 == 0 && Cin <= 96 && Cout <= 1 << 20 && P < (1LL << 30) && (20LL * W + 32) * csx < (1LL << 31)) {
         const int rc = Cin == 32 ? launch_conv_tile<4, 4>(a, S(stream))
                      : Cin == 64 ? launch_conv_tile<8, 8>(a, S(stream)) : launch_conv_tile<12, 8>(a, S(stream));
         if (rc != PFF_OK) return rc;

@@ -1,4 +1,4 @@
-"""Ragged batches: many independent DEM tiles routed in one persistent launch.
+"""Ragged batches: many independent DEM tiles routed together by persistent kernels.
 
 The reference routes one grid per process (its grid size is a module global,
 pyfastflow/constants.py).  ``RaggedRouter`` holds many tiles of their own shape,
@@ -10,9 +10,10 @@ user runs tile by tile:
     reroute_flow(carve=True)            (flow/lakeflow.py:466-538)
     accumulate_constant_Q / weighted    (flow/flowfields.py:254-292)
 
-Results are bit-identical to those per-tile calls.  One launch covers the whole
-batch; ``route(graph=True)`` replays it from a captured CUDA graph, and ``tune()``
-picks the CTA size and residency by timing the candidates on the batch itself.
+Results are bit-identical to those per-tile calls.  The routing of the whole batch is
+one launch and its accumulation two; ``route(graph=True)`` replays them from a captured
+CUDA graph, and ``tune()`` picks the CTA size and residency by timing the candidates on
+the batch itself.
 """
 from __future__ import annotations
 
@@ -173,9 +174,9 @@ class RaggedRouter:
                   self.ws.data_ptr(), self.ws_bytes, _dev.stream())
 
     def route(self, graph: bool = False, check: bool = True):
-        """receivers -> reroute(carve) -> accumulate for every tile, one launch.
+        """receivers -> reroute(carve) -> accumulate for every tile.
 
-        graph=True captures the launch (with the seed copy) in a CUDA graph on the
+        graph=True captures the launches (with the seed copy) in a CUDA graph on the
         first call and replays it afterwards.  check=True reads the status word
         (one host synchronisation) and raises on an error bit."""
         if graph:
