@@ -83,7 +83,7 @@ __device__ __forceinline__ int sw64(int r, int c) { return r * 4 + (c ^ ((r >> 1
 template <int CH>
 __device__ __forceinline__ int swr(int r, int c)
 {
-    return CH % 8 ? r * CH + (c ^ ((r >> 1) & 3)) : r * CH + (c ^ (r & 7));
+    return CH == 1 ? r : CH % 8 ? r * CH + (c ^ ((r >> 1) & 3)) : r * CH + (c ^ (r & 7));
 }
 
 // bias, ReLU and the store of channels co, co + 1 of pixel p (bf16 pairs, or f32)
@@ -243,31 +243,33 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv3x3(ConvArgs a)
         }
 }
 
-// The convolution with 32, 64 or 96 input channels: the im2col form above fetches every
+// The convolution with 8, 32, 64 or 96 input channels: the im2col form above fetches every
 // pixel nine times from L2 and a thread's addresses cost more than its products.  Here a
 // CTA keeps the weights of NB output channels in shared memory and walks over tiles of 16
 // rows of 16 pixels, double-buffered with their halo; the taps read the tile shifted.  A
 // warp takes MI rows of pixels; K steps go through taps and channels in the order of the
 // form above, so every sum is the same.  Bound by
 // fragment loads (6 per 16 products) and the tensor pipe; 16 x 128 x 128, before and now:
-// 96 -> 32 channels 74 and 54 us, 32 -> 96 90 and 56, 32 -> 32 31 and 27, 32 -> 8 27 and 20;
-// 64 -> 32 at 16 x 64 x 64 19 and 15.
+// 96 -> 32 channels 74 and 54 us, 32 -> 96 90 and 56, 32 -> 32 31 and 27, 32 -> 8 27 and 20,
+// 8 -> 32 25 and 17 (two taps per K step); 64 -> 32 at 16 x 64 x 64 19 and 15.
 constexpr int CT_TW = 16, CT_TH = 16, CT_HW = CT_TW + 2, CT_PITCH = 24;
-__host__ __device__ constexpr int ct_smem(int CC, int NB) { return 16 * (NB * (9 * CC + 1) + 2 * CT_PITCH * (CT_TH + 2) * CC); }
+// 16-byte chunks of a weight row: odd, so that 8 rows lie on 8 bank groups
+__host__ __device__ constexpr int ct_wrow(int CC) { return CC == 1 ? 11 : 9 * CC + 1; }
+__host__ __device__ constexpr int ct_smem(int CC, int NB) { return 16 * (NB * ct_wrow(CC) + 2 * CT_PITCH * (CT_TH + 2) * CC); }
 
 template <int CC, int NB, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) k_conv3x3_tile(ConvArgs a, int ntx, int nty, int ntiles)
 {
     constexpr int MI = CT_TH / WARPS, NJ = NB / 8, THREADS = 32 * WARPS;
-    constexpr int WR = 9 * CC + 1;  // chunks per weight row, odd: 8 rows on 8 bank groups
+    constexpr int WR = ct_wrow(CC), WC = CC == 1 ? 10 : 9 * CC;  // 8 channels: a tenth tap of zeros
     constexpr int ST = CT_PITCH * (CT_TH + 2) * CC;
     extern __shared__ __align__(128) uint4 ct[];
     uint4 *sW = ct, *sX = ct + NB * WR;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n0 = blockIdx.y * NB;
-    for (int e = tid; e < NB * 9 * CC; e += THREADS) {
-        const int n = e / (9 * CC), q = e % (9 * CC);
-        const bool v = n0 + n < a.Cout;
+    for (int e = tid; e < NB * WC; e += THREADS) {
+        const int n = e / WC, q = e % WC;
+        const bool v = n0 + n < a.Cout && q < 9 * CC;
         cp_async16(smem_u32(sW + n * WR + q), v ? a.w + ((long long)(n0 + n) * 9 * CC + q) * 8 : a.w, v);
     }
     auto load_tile = [&](int st, int t) {
@@ -301,27 +303,38 @@ __global__ void __launch_bounds__(32 * WARPS) k_conv3x3_tile(ConvArgs a, int ntx
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
         const unsigned xb = xs + 16 * ((k & 1) * ST + warp * MI * CT_PITCH * CC);
+        // one K step of 16: A rows at xa, weight chunks from q
+        auto step = [&](unsigned xa, int q, bool last) {
+            unsigned af[MI][4], bf[NJ][2];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                ldsm_x4(xa + i * (16 * CT_PITCH * CC), af[i][0], af[i][1], af[i][2], af[i][3]);
+                if (last) af[i][2] = af[i][3] = 0;  // past the last tap: 0 times an infinity is no 0
+            }
+#pragma unroll
+            for (int j = 0; j < NJ / 2; ++j)
+                ldsm_x4(wb + 16 * (j * 16 * WR + q), bf[2 * j][0], bf[2 * j][1], bf[2 * j + 1][0], bf[2 * j + 1][1]);
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+                    mma16816(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bf[j][0], bf[j][1]);
+        };
+        if constexpr (CC == 1) {  // two taps per step
+#pragma unroll
+            for (int q = 0; q < 10; q += 2) {
+                const int tap = min(q + (lane >> 4), 8);
+                step(xb + 16 * (tap / 3 * CT_PITCH + tap % 3 + (lane & 15)), q, q == 8);
+            }
+        } else {
 #pragma unroll 1
-        for (int kh = 0; kh < 3; ++kh) {
+            for (int kh = 0; kh < 3; ++kh)
 #pragma unroll
-            for (int kw = 0; kw < 3; ++kw)
+                for (int kw = 0; kw < 3; ++kw)
 #pragma unroll
-                for (int s = 0; s < CC / 2; ++s) {
-                    unsigned af[MI][4], bf[NJ][2];
-                    const unsigned xa = xb + 16 * (kh * CT_PITCH * CC + swr<CC>(kw + (lane & 15), 2 * s + (lane >> 4)));
-#pragma unroll
-                    for (int i = 0; i < MI; ++i)
-                        ldsm_x4(xa + i * (16 * CT_PITCH * CC), af[i][0], af[i][1], af[i][2], af[i][3]);
-#pragma unroll
-                    for (int j = 0; j < NJ / 2; ++j)
-                        ldsm_x4(wb + 16 * (j * 16 * WR + (3 * kh + kw) * CC + 2 * s), bf[2 * j][0], bf[2 * j][1],
-                                bf[2 * j + 1][0], bf[2 * j + 1][1]);
-#pragma unroll
-                    for (int i = 0; i < MI; ++i)
-#pragma unroll
-                        for (int j = 0; j < NJ; ++j)
-                            mma16816(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bf[j][0], bf[j][1]);
-                }
+                    for (int s = 0; s < CC / 2; ++s)
+                        step(xb + 16 * (kh * CT_PITCH * CC + swr<CC>(kw + (lane & 15), 2 * s + (lane >> 4))),
+                             (3 * kh + kw) * CC + 2 * s, false);
         }
         __syncthreads();  // the tile's buffer is free for the load after next
         const int tx = t % ntx, u = t / ntx, ty = u % nty, b = u / nty;
@@ -355,7 +368,7 @@ static int launch_conv_tile(const ConvArgs &a, cudaStream_t st)
     const int ntx = (a.W + CT_TW - 1) / CT_TW, nty = (a.H + CT_TH - 1) / CT_TH, nt = a.B * ntx * nty;
     const int ny = (a.Cout + NB - 1) / NB;
     // resident CTAs, each with the same number of tiles but for one
-    const int most = std::max(1, 148 * std::min(per, 3) / ny), each = (nt + most - 1) / most;
+    const int most = std::max(1, 148 * std::min(per, 4) / ny), each = (nt + most - 1) / most;
     kern<<<dim3((nt + each - 1) / each, ny), 32 * WARPS, smem, st>>>(a, ntx, nty, nt);
     count_launch();
     return PFF_OK;
@@ -1034,10 +1047,11 @@ extern "C" int pff_conv3x3_fwd(const bf16_t *x, int csx, int offx, const bf16_t 
         return conv3x3_tc(x, csx, offx, w, bias, y, csy, offy, B, H, W, Cin, Cout, relu, out_f32, S(stream));
     ConvArgs a{x, csx, offx, w, bias, y, csy, offy, B, H, W, Cin, Cout, relu, out_f32};
     const long long P = (long long)B * H * W;
-    // whole tiles of 32, 64 or 96 channels fit shared memory twice beside the weights; other counts,
+    // whole tiles of 8, 32, 64 or 96 channels fit shared memory twice beside the weights; other counts,
     // and rows beyond 32-bit offsets within a tile, take the im2col form
-    if (Cin % 32 == 0 && Cin <= 96 && Cout <= 1 << 20 && P < (1LL << 30) && (20LL * W + 32) * csx < (1LL << 31)) {
-        const int rc = Cin == 32 ? launch_conv_tile<4, 4>(a, S(stream))
+    if ((Cin == 8 || (Cin % 32 == 0 && Cin <= 96)) && Cout <= 1 << 20 && P < (1LL << 30) && (20LL * W + 32) * csx < (1LL << 31)) {
+        const int rc = Cin == 8 ? launch_conv_tile<1, 4>(a, S(stream))
+                     : Cin == 32 ? launch_conv_tile<4, 4>(a, S(stream))
                      : Cin == 64 ? launch_conv_tile<8, 8>(a, S(stream)) : launch_conv_tile<12, 8>(a, S(stream));
         if (rc != PFF_OK) return rc;
         return check_cuda("pff_conv3x3_fwd");

@@ -273,17 +273,18 @@ def test_weight_gradient_tiles(cuda, cin, cout, B, H, W):
         assert buf[n * (1 - off)].item() == 0.5
 
 
-@pytest.mark.parametrize("cin", [32, 64, 96])
+@pytest.mark.parametrize("cin", [8, 32, 64, 96])
 @pytest.mark.parametrize("cout,f32", [(8, 0), (17, 1), (40, 0)])
 @pytest.mark.parametrize("B,H,W", [(1, 1, 1), (2, 16, 16), (1, 17, 18)])
 def test_conv_tile_is_the_im2col_form(cuda, cin, cout, f32, B, H, W):
     """Tiles with a halo in shared memory against the im2col kernel, which a channel stride
-    beyond 32-bit tile offsets takes: bit for bit."""
+    beyond 32-bit tile offsets takes: bit for bit, with an infinity in the last pixel."""
     torch = cuda
     from pyfastflow_b200 import _dev, _lib
 
     cs = (2 ** 31 // (20 * W + 32) + 8) // 8 * 8
     x = _bf(torch, B * H * W, cin, seed=1).cuda()
+    x[-1, 3] = float("inf")
     w, bias = _bf(torch, cout, 9, cin, seed=3).cuda(), torch.linspace(-1, 1, cout, device="cuda")
     wide = torch.empty(B * H * W * cs, dtype=torch.bfloat16, device="cuda")
     wide.view(B * H * W, cs)[:, 16:16 + cin] = x
