@@ -46,6 +46,13 @@ const char *pff_last_error_string(void);
 /* Total number of CUDA kernels this library has launched in this process (no
  * counterpart in the reference: used to report GPU launches per step). */
 long long pff_launch_count(void);
+/* Failure test of the barriers between the blocks of cooperative launches.  The calling
+ * thread's later launches of the named kernels (1 reroute loop, 2 reroute labels, 4 tree
+ * accumulation, 8 reference-order rounds; summed) wait at every barrier for `absent` (0 or 1)
+ * blocks more than there are, at most limit_us (1 to 2000000) microseconds; the call that made
+ * the launch then fails with PFF_ERR_NOCONV.  kernels = 0: as usual again, no block more and
+ * two seconds. */
+int pff_barrier_test(int kernels, int absent, int limit_us);
 /* Kernel timing probes (no reference counterpart; used by benchmarks to time the
  * dominant kernels inside a call).  pff_probe_enable(1) clears and arms them: each
  * probed launch made outside stream capture is then bracketed by two CUDA events on

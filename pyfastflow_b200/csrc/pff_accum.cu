@@ -414,6 +414,7 @@ struct AccRounds {
     int *nonlocal, *overflow;
     int N, first, logn;
     int *bar, *over_out;
+    BarWait wait;
     // ragged batch: rounds end tile by tile (N is then the packed total, nonlocal unused)
     const BatchTile *tiles;
     int ntiles;
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int gthreads = gridDim.x * ACC_THREADS;
     if (threadIdx.x == 0) dead = 0;
-    GridBar bar{a.bar, 0};
+    GridBar bar{a.bar, a.wait};
     __syncthreads();
     int it = a.first, logn = a.logn, logmin = a.logn;
     if (a.tiles) {
@@ -976,7 +977,7 @@ int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st)
     a.Q = b.Q; a.counts = b.counts;
     for (int k = 0; k < 2; ++k) { a.la[k] = b.la[k]; a.lf[k] = b.lf[k]; }
     a.cnt = cnt; a.nonlocal = nonlocal; a.overflow = nonlocal + 1;
-    a.N = (int)b.total; a.first = BATCH_FR; a.bar = bar;
+    a.N = (int)b.total; a.first = BATCH_FR; a.bar = bar; a.wait = bar_wait(BAR_ROUNDS);
     a.tiles = b.by_offset; a.ntiles = b.ntiles; a.limits = b.limits;
     return launch_rounds(a, (int)b.total, st);
 }
@@ -1109,7 +1110,7 @@ extern "C" int pff_accumulate_grid(const int32_t *receivers, float *Q, uint32_t 
     for (int k = 0; k < 2; ++k) { a.la[k] = la[k]; a.lf[k] = lf[k]; }
     a.cnt = ctr; a.nonlocal = nonlocal; a.overflow = overflow;
     a.N = N; a.first = front ? FR : 0; a.logn = logn;
-    a.bar = bar; a.over_out = dptr;
+    a.bar = bar; a.wait = bar_wait(BAR_ROUNDS); a.over_out = dptr;
     PFF_TRY(launch_rounds(a, N, st));
     PFF_CUDA(cudaStreamSynchronize(st));
     PFF_TRY(check_cuda("pff_accumulate"));

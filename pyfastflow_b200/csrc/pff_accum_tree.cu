@@ -81,7 +81,8 @@ struct TreeArgs {
     int *up0;            // per cell: level-1 position of its tile terminal, or -1
     long long *T0;       // per cell: in-tile total (weighted seeds)
     unsigned *C0;        // per cell: in-tile count
-    int *status;         // [0] error bits, [1] max |seed| bits, [2] finished tiles, [8..9] grid barrier
+    int *status;         // [0] error bits, [1] max |seed| bits, [8] grid barrier
+    BarWait wait;
     int *out;            // the caller's copy of status[0] (mapped host memory), or null
     int nzero;           // ints from status on that start at zero (status, then the levels' counts)
     long long *scr_acc;  // fallback storage for blocks larger than TR_SMEM_NODES
@@ -771,7 +772,7 @@ __global__ void __launch_bounds__(TR_LB_THREADS, 1) k_tree_all(const int32_t *__
     if (threadIdx.x == 0) dead = 0;
     if (gridDim.x == 1)  // one block clears its counters itself
         for (int k = threadIdx.x; k < a.nzero; k += TR_LB_THREADS) a.status[k] = 0;
-    GridBar bar{a.status + 8, 0};
+    GridBar bar{a.status + 8, a.wait};
     __syncthreads();
     if (((uintptr_t)a.marker & 15) == 0) {
         for (int k = gtid; k < (a.N + 15) / 16; k += gthreads)  // the array is padded to 256 bytes
@@ -907,6 +908,7 @@ static int launch_tree(const TreePlan &p, const TreeArgs &a_, const int32_t *rec
                        float *Q, uint32_t *counts, cudaStream_t st)
 {
     TreeArgs a = a_;
+    a.wait = bar_wait(BAR_TREE);
     int dev = 0, nsm = 148, coop = 0;
     PFF_CUDA(cudaGetDevice(&dev));
     PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));

@@ -692,6 +692,10 @@ int pinned_ints(int **host, int **dptr)
     return PFF_OK;
 }
 
+static thread_local int g_bar_kernels = 0;
+static thread_local BarWait g_bar_wait = {0, 2000000};
+BarWait bar_wait(int kernel) { return g_bar_kernels & kernel ? g_bar_wait : BarWait{0, 2000000}; }
+
 int read_ints(const IntReads &r, int *out, cudaStream_t st)
 {
     if (r.k > 8) {
@@ -782,6 +786,18 @@ void probe_end(ProbeMark m, cudaStream_t st)
 }
 
 }  // namespace pff
+
+extern "C" int pff_barrier_test(int kernels, int absent, int limit_us)
+{
+    clear_error();
+    if (kernels < 0 || kernels > 15 || absent < 0 || absent > 1 || (kernels && (limit_us < 1 || limit_us > 2000000))) {
+        set_error("pff_barrier_test: bad arguments");
+        return PFF_ERR_ARG;
+    }
+    g_bar_kernels = kernels;
+    g_bar_wait = BarWait{absent, (unsigned)limit_us};
+    return PFF_OK;
+}
 
 extern "C" long long pff_launch_count(void) { return g_launches.load(); }
 

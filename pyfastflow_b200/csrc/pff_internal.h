@@ -91,6 +91,15 @@ struct Carver {
     static size_t round(size_t n) { return (n + 255) & ~size_t(255); }
 };
 
+// How long the blocks of a cooperative launch wait at a barrier, and for how many more blocks
+// than there are (pff_barrier_test; otherwise two seconds and none).
+enum { BAR_REROUTE = 1, BAR_LABELS = 2, BAR_TREE = 4, BAR_ROUNDS = 8 };
+struct BarWait {
+    int absent;
+    unsigned limit_us;
+};
+BarWait bar_wait(int kernel);
+
 // A tile of a ragged batch.
 struct BatchTile {
     long long off;   // first cell of the tile in the packed arrays

@@ -1360,7 +1360,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, 
 {
     __shared__ int dead;
     if (threadIdx.x == 0) dead = 0;
-    GridTeam T{GridBar{A.bar + 8, 0}, &dead};
+    GridTeam T{GridBar{A.bar + 8, A.labels_wait}, &dead};
     __syncthreads();
     reroute_labels<MODE, false>(A, R, T);
 }
@@ -1371,12 +1371,12 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_loop(LoopArgs A)
     extern __shared__ __align__(16) unsigned char loop_smem[];
     __shared__ int dead;
     if (threadIdx.x == 0) dead = 0;
-    GridTeam T{GridBar{A.bar, 0}, &dead};
+    GridTeam T{GridBar{A.bar, A.wait}, &dead};
     __syncthreads();
     int it = 0, outer = 0, n_outer = 0;
     const int state = reroute_loop<MODE, false, false>(A, T, loop_smem, it, outer, n_outer);
-    // block 0's first thread reports; a block whose barrier gave up says so whoever it is
-    if (threadIdx.x == 0 && (blockIdx.x == 0 || state == RR_BOUND)) loop_report(A, it, outer, n_outer, state);
+    // all blocks end in the same state (see GridBar)
+    if (threadIdx.x == 0 && blockIdx.x == 0) loop_report(A, it, outer, n_outer, state);
 }
 
 // The whole reroute of a grid whose steps do not fill the GPU, in one launch: with one
@@ -1390,7 +1390,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_whole(LoopArgs A, i
     if (threadIdx.x == 0) dead = 0;
     if (gridDim.x == 1)  // one block clears its counters itself
         for (int k = threadIdx.x; k < nzero; k += LOOP_THREADS) A.ctl[k] = 0;
-    GridTeam T{GridBar{A.bar, 0}, &dead};
+    GridTeam T{GridBar{A.bar, A.wait}, &dead};
     __syncthreads();
     reroute_tiles<MODE>(A, R, T, loop_smem);
     int it = 0, outer = 0, n_outer = 0, state = RR_BOUND;
@@ -1398,7 +1398,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_whole(LoopArgs A, i
         reroute_first_border<MODE, true>(A, T, loop_smem);
         if (T.sync()) state = reroute_loop<MODE, false, true>(A, T, loop_smem, it, outer, n_outer);
     }
-    if (threadIdx.x == 0 && (blockIdx.x == 0 || state == RR_BOUND)) loop_report(A, it, outer, n_outer, state);
+    if (threadIdx.x == 0 && blockIdx.x == 0) loop_report(A, it, outer, n_outer, state);
 }
 
 // ---- launchers ---------------------------------------------------------------
@@ -1864,10 +1864,12 @@ static int reroute_device(int32_t *bid, int32_t *rec, int32_t *rec_, int32_t *re
     A.segs = w.segs; A.dtiles = w.dtiles;
     A.ctl = w.loop;
     A.info = w.loop + 16;
-    A.bar = w.loop + 24;  // [0..1] the loop's, [8..9] the labels', [16..31] the labels' round flags
+    A.bar = w.loop + 24;  // [0] the loop's, [8] the labels', [16..31] the labels' round flags
     A.it_ctr = w.loop + RR_SYNC;
     A.dirty = A.it_ctr + LOOP_ITS * LOOP_CTR;
     A.ctl_out = ctl_out;
+    A.wait = bar_wait(BAR_REROUTE);
+    A.labels_wait = bar_wait(BAR_LABELS);
     A.g = g;
     const int nzero = RR_SYNC + LOOP_ITS * LOOP_CTR + ntiles;
     if (blocks > 1) PFF_CUDA(cudaMemsetAsync(w.loop, 0, sizeof(int) * (size_t)nzero, st));

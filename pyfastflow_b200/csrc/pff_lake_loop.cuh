@@ -282,7 +282,8 @@ struct LoopArgs {
     int *it_ctr;           // LOOP_ITS x LOOP_CTR counters, zeroed before the prologue
     int *info;             // prologue: [0] pits, [2] non-D4 receivers, [4] unresolved labels
     int *ctl, *ctl_out;    // final state words (RR_*), and the caller's copy
-    int *bar;              // [0] barrier arrivals, [1] error
+    int *bar;              // barrier arrivals
+    BarWait wait, labels_wait;
     Grid g;
 };
 
