@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(128) k_saddle_p12_strip(const int32_t *__restr
                                                           Grid g, int *blist, int *nblist, int *alist, int *nalist,
                                                           const int *info)
 {
-    if (info && (info[0] == 0 || info[2] || info[4])) return;  // nothing to do, or the host's steps
+    if (info && (info[0] == 0 || info[2] || info[4] || info[5])) return;  // nothing to do, or the host's steps
     __shared__ int buf[4][32 * SAD_ROWS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int warp = blockIdx.x * 4 + wib;
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(128, 4) k_saddle_p12_strip4(const int32_t *__r
                                                               const int *info)
 {
     static_assert(MODE >= 0 && MODE <= 2, "custom codes take k_saddle_p12_strip");
-    if (info && (info[0] == 0 || info[2] || info[4])) return;  // nothing to do, or the host's steps
+    if (info && (info[0] == 0 || info[2] || info[4] || info[5])) return;  // nothing to do, or the host's steps
     __shared__ int buf[4][128 * SAD4_ROWS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int warp = blockIdx.x * 4 + wib;
@@ -1362,7 +1362,8 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1) k_reroute_labels(LoopArgs A, 
     if (threadIdx.x == 0) dead = 0;
     GridTeam T{GridBar{A.bar + 8, A.labels_wait}, &dead};
     __syncthreads();
-    reroute_labels<MODE, false>(A, R, T);
+    // no labels: the passes behind this launch leave the grid alone
+    if (reroute_labels<MODE, false>(A, R, T) != RR_RUN && blockIdx.x == 0 && threadIdx.x == 0) A.info[5] = 1;
 }
 
 template <int MODE>

@@ -280,7 +280,7 @@ struct LoopArgs {
     long long *akey;       // and its lowest (z', neighbour basin) key
     int *segs, *dirty, *dtiles;
     int *it_ctr;           // LOOP_ITS x LOOP_CTR counters, zeroed before the prologue
-    int *info;             // prologue: [0] pits, [2] non-D4 receivers, [4] unresolved labels
+    int *info;             // prologue: [0] pits, [2] non-D4 receivers, [4] unresolved labels, [5] no labels
     int *ctl, *ctl_out;    // final state words (RR_*), and the caller's copy
     int *bar;              // barrier arrivals
     BarWait wait, labels_wait;
@@ -450,7 +450,8 @@ __device__ __forceinline__ int reroute_loop(const LoopArgs &A, Team &T, unsigned
     int state = RR_RUN;
     n_outer = 0;
     if (it0 == 0) outer = np0 > 0 ? d_ceil_log2(np0) + 1 : 0;  // :500
-    if (np0 == 0) state = it0 == 0 ? RR_NOPITS : RR_DONE;      // :496-497, :512-514
+    if (vload(A.info + 5)) state = RR_BOUND;                   // the labels' launch gave up
+    else if (np0 == 0) state = it0 == 0 ? RR_NOPITS : RR_DONE;      // :496-497, :512-514
     else if (vload(A.info + 2) || vload(A.info + 4)) state = RR_GENERAL;  // not D4, or a receiver cycle in the input
     if (state == RR_RUN) {
         // clear the carve tags of an earlier call

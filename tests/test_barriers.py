@@ -65,14 +65,36 @@ def test_a_barrier_that_gives_up_is_an_error(cuda, barrier_test, nx, ny, kernels
         assert np.array_equal(a, b)
 
 
+@pytest.mark.gpu
+def test_labels_that_give_up_end_the_reroute(cuda, barrier_test):
+    """The labels are a launch of their own on larger grids: the saddle pass and the loop behind
+    it must not run on what an earlier call left.  The receivers stay as they were."""
+    from pyfastflow_b200._lib import PFFError
+
+    r = router(600, 601)
+    chain(r, False)
+    want = results(r)
+    r.compute_receivers()
+    before = r.receivers.cpu().numpy().copy()
+    barrier_test(LABELS, 1, 1000)
+    with pytest.raises(PFFError, match="status 3"):
+        r.reroute_flow()
+    assert np.array_equal(before, r.receivers.cpu().numpy())
+    barrier_test(0, 0, 0)
+    chain(r, False)
+    for a, b in zip(want, results(r)):
+        assert np.array_equal(a, b)
+
+
 # limits around the blocks' distance: some waits end in time and others do not
 @pytest.mark.gpu
-@pytest.mark.parametrize("kernels,exact", [(REROUTE, False), (TREE, False), (ROUNDS, True)])
-def test_blocks_agree_on_a_barrier_given_up(cuda, barrier_test, kernels, exact):
+@pytest.mark.parametrize("n,kernels,exact", [(380, REROUTE, False), (600, LABELS, False), (380, TREE, False),
+                                             (380, ROUNDS, True)])
+def test_blocks_agree_on_a_barrier_given_up(cuda, barrier_test, n, kernels, exact):
     """Every call is an error or gives the usual results."""
     from pyfastflow_b200._lib import PFFError
 
-    r = router(380, 390)
+    r = router(n, n + 10)
     chain(r, exact)
     want = results(r)
     ended = []
