@@ -161,7 +161,8 @@ int pff_accumulate_set_front(int rounds);
  * Asynchronous (no host synchronisation).  Problems are recorded in a status word
  * read by pff_accumulate_tree_status (synchronizes `stream`): 1 receiver out of
  * range, 2 receiver cycle, 4 a tile with too many exits, 8 local = 1 violated,
- * 16 non-finite seed; Q and counts are unspecified when it is nonzero.
+ * 16 non-finite seed; Q and counts are unspecified when it is nonzero.  The status call
+ * itself returns PFF_ERR_NOCONV if the passes did not end.
  * workspace: pff_accumulate_tree_workspace_bytes(nx, ny, local) bytes. */
 size_t pff_accumulate_tree_workspace_bytes(int nx, int ny, int local);
 int pff_accumulate_tree(const int32_t *receivers, const float *weights, float value, float *Q,

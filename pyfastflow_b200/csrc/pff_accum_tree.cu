@@ -1029,6 +1029,12 @@ extern "C" int pff_accumulate_tree_status(int nx, int ny, int local, void *works
         return PFF_ERR_WORKSPACE;
     }
     const TreeArgs a = tree_carve(p, nx, ny, local, workspace, workspace_bytes, nullptr);
-    PFF_TRY(read_ints(IntReads().add(a.status, 1), status, S(stream)));
+    int words[2] = {0, 0};
+    PFF_TRY(read_ints(IntReads().add(a.status, 1).add(a.status + 8, 1), words, S(stream)));
+    if (words[1] & BAR_HALT) {
+        set_error("pff_accumulate_tree_status: the passes did not end");
+        return PFF_ERR_NOCONV;
+    }
+    *status = words[0];
     return PFF_OK;
 }

@@ -86,6 +86,27 @@ def test_labels_that_give_up_end_the_reroute(cuda, barrier_test):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.gpu
+def test_tree_status_reports_a_barrier_given_up(cuda, barrier_test):
+    """pff_accumulate_tree and its status call apart, as FlowRouter.route_many makes them."""
+    torch = cuda
+    from pyfastflow_b200._lib import PFFError
+
+    r = router(300, 200)
+    z = [r.z.cpu().pin_memory() for _ in range(3)]
+    q = [torch.full((r.N,), -1.0).pin_memory() for _ in z]
+    r.route_many(z, None, q)
+    torch.cuda.synchronize()
+    want = q[0].clone()
+    barrier_test(TREE, 1, 1000)
+    with pytest.raises(PFFError, match="status 3"):
+        r.route_many(z, None, q)
+    barrier_test(0, 0, 0)
+    r.route_many(z, None, q)
+    torch.cuda.synchronize()
+    assert all(torch.equal(want, t) for t in q)
+
+
 # limits around the blocks' distance: some waits end in time and others do not
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,kernels,exact", [(380, REROUTE, False), (600, LABELS, False), (380, TREE, False),
