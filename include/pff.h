@@ -365,7 +365,8 @@ int pff_erode_deposit(float *z, const uint8_t *bound, int32_t *rcv, const float 
  * threads: 256, 512 or 1024 per CTA; ctas_per_sm is clamped to the occupancy.
  * pff_batch_status: error bits of the last launch (synchronizes `stream`):
  * 1 = a bad tile mode (or a custom-mode tile without codes), 8 = cells of one receiver cycle ended with
- * different serial labels, 16 = a carve did not converge. */
+ * different serial labels, 16 = a carve did not converge, 32 = the accumulation's rounds
+ * did not end (Q and counts are unspecified). */
 size_t pff_batch_workspace_bytes(long long total_cells, int ntiles);
 long long pff_batch_plan(const int32_t *tile_nx, const int32_t *tile_ny, const int32_t *tile_mode,
                          const float *tile_dx, int ntiles, long long *tile_offset, int32_t *order,

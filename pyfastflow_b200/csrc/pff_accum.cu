@@ -419,6 +419,7 @@ struct AccRounds {
     const BatchTile *tiles;
     int ntiles;
     const int *limits;  // [0] smallest, [1] largest logn of the tiles
+    int *status;        // BST_* bits
 };
 
 __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
@@ -535,7 +536,10 @@ __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
         }
         if (na) flush(sa[wib], na, la2, c2);
         if (nf) flush(sf[wib], nf, lf2, c2 + 1);
-        if (!bar.sync(&dead)) return;
+        if (!bar.sync(&dead)) {  // a single grid's caller misses over_out
+            if (a.status && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.status, BST_ROUNDS);
+            return;
+        }
     }
     if (a.over_out && blockIdx.x == 0 && threadIdx.x == 0) {
         ((volatile int *)a.over_out)[0] = *a.overflow;
@@ -978,7 +982,7 @@ int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st)
     for (int k = 0; k < 2; ++k) { a.la[k] = b.la[k]; a.lf[k] = b.lf[k]; }
     a.cnt = cnt; a.nonlocal = nonlocal; a.overflow = nonlocal + 1;
     a.N = (int)b.total; a.first = BATCH_FR; a.bar = bar; a.wait = bar_wait(BAR_ROUNDS);
-    a.tiles = b.by_offset; a.ntiles = b.ntiles; a.limits = b.limits;
+    a.tiles = b.by_offset; a.ntiles = b.ntiles; a.limits = b.limits; a.status = b.status;
     return launch_rounds(a, (int)b.total, st);
 }
 

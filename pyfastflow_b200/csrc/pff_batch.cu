@@ -42,7 +42,6 @@ struct BatchArrays {
     int *status;             // [0] error bits (see pff_batch_status)
 };
 
-enum : int { BST_MODE = 1, BST_CYCLE_LABELS = 8, BST_CARVE = 16 };
 
 constexpr int LB_SIDE = 32, LB_CELLS = LB_SIDE * LB_SIDE;  // label sub-blocks
 
@@ -1424,7 +1423,7 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
         b.bufA = A.dnr; b.bufB = A.dnr_; b.priv = w.priv;
         b.la[0] = A.ndnr; b.la[1] = A.ndnr_;
         b.lf[0] = A.src; b.lf[1] = reinterpret_cast<int *>(A.p_);
-        b.ctr = w.acc_ctr;
+        b.ctr = w.acc_ctr; b.status = A.status;
         b.by_offset = w.by_offset; b.items = w.items; b.limits = w.limits;
         b.total = total_cells; b.ntiles = ntiles;
         PFF_TRY(launch_batch_accumulate(b, st));

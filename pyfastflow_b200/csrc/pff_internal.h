@@ -112,6 +112,9 @@ struct BatchTile {
     int pad;
 };
 
+// error bits of a batch's status word
+enum : int { BST_MODE = 1, BST_CYCLE_LABELS = 8, BST_CARVE = 16, BST_ROUNDS = 32 };
+
 // The accumulation of a ragged batch (pff_accum.cu), over packed arrays.
 constexpr int BATCH_ACC_CTR = 256;
 struct BatchAcc {
@@ -121,6 +124,7 @@ struct BatchAcc {
     void *bufA, *bufB, *priv;  // 16 B per cell each
     int *la[2], *lf[2];   // 4 B per cell each
     int *ctr;             // BATCH_ACC_CTR ints
+    int *status;          // BST_* bits
     const BatchTile *by_offset;  // the tiles in packed order
     const int *items;     // work item -> tile (packed order)
     const int *limits;    // [0] smallest and [1] largest logn of the front's tiles, [2] work items

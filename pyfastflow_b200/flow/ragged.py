@@ -200,7 +200,7 @@ class RaggedRouter:
                   _dev.stream())
         if st.value:
             raise _lib.PFFError(f"ragged routing status {st.value} (1: bad tile mode, 8: receiver cycle with "
-                                "mixed serial labels, 16: carve did not converge)")
+                                "mixed serial labels, 16: carve did not converge, 32: the accumulation did not end)")
 
     def tune(self, candidates=TUNE_CANDIDATES, reps: int = 2) -> tuple[int, int]:
         """Time each (threads, CTAs per SM) candidate on this batch, keep the fastest."""

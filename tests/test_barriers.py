@@ -107,6 +107,29 @@ def test_tree_status_reports_a_barrier_given_up(cuda, barrier_test):
     assert all(torch.equal(want, t) for t in q)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [False, True])
+def test_batch_status_reports_a_barrier_given_up(cuda, barrier_test, graph):
+    from pyfastflow_b200._lib import PFFError
+    from pyfastflow_b200.flow import RaggedRouter
+
+    shapes = [(60 + 9 * k, 150 - 11 * k) for k in range(8)]
+    rr = RaggedRouter(shapes, 30.0, "normal")
+    rr.set_z([synthetic.spectral_dem(nx, ny, k, relief=300.0, npits=20, pit_scale=0.1)
+              for k, (ny, nx) in enumerate(shapes)])
+    rr.seed_constant()
+    rr.route()
+    want = [t.cpu().numpy().copy() for t in (rr.receivers, rr.Q, rr.counts)]
+    barrier_test(ROUNDS, 1, 1000)
+    with pytest.raises(PFFError, match="status 32"):
+        rr.route(graph=graph)
+    rr._graph = None  # it holds the launch made for the test
+    barrier_test(0, 0, 0)
+    rr.route(graph=graph)
+    for a, b in zip(want, (rr.receivers, rr.Q, rr.counts)):
+        assert np.array_equal(a, b.cpu().numpy())
+
+
 # limits around the blocks' distance: some waits end in time and others do not
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,kernels,exact", [(380, REROUTE, False), (600, LABELS, False), (380, TREE, False),
