@@ -73,6 +73,7 @@ class FlowRouter:
         self._ws_fill = _dev.Scratch()
         self._ws_diff = _dev.Scratch()
         self.last_n_outer = 0
+        self._refused = None  # status with which the last _accumulate_begin was refused
         # global configuration, as the reference writes it (flowfields.py:163-182)
         cte.NX, cte.NY, cte.DX = self.nx, self.ny, self.dx
         cte.RAND_RCV = self.stochastic_receivers  # flowfields.py:166
@@ -182,34 +183,39 @@ class FlowRouter:
         self.last_n_outer = nout.value
         return int(ctl_host[3])
 
-    def _accumulate(self, counts: bool = True, exact_order: bool = False, value=None):
+    def _accumulate(self, counts: bool = True, exact_order: bool = False, value=None, refused=None):
         """Upstream sums of the seeds (Q, or `value` per cell) into Q and counts.
 
         Default: the tile-hierarchy accumulation (pff_accumulate_tree) -- exact
         integer sums, Q rounded once to f32, exact counts.  exact_order=True, and
         receivers the tree path reports it cannot take (a receiver cycle), use the
         rake-and-compress rounds with the reference's f32 summation order
-        (pff_accumulate_grid), bit-identical to the reference's Q."""
+        (pff_accumulate_grid), bit-identical to the reference's Q.
+
+        refused: the status with which the tree path has just refused these receivers
+        and seeds, where it has."""
         lib = _lib.load()
         if not exact_order:
             import ctypes as C
 
-            local = 1
+            local, status = 1, refused
             for _ in range(2):
-                wp, wn = self._ws_tree.get(lib.pff_accumulate_tree_workspace_bytes(self.nx, self.ny, local),
-                                           self.device)
-                seeds = None if value is not None else self.Q.data_ptr()
-                st = C.c_int()
-                _lib.call("pff_accumulate_tree_run", self.receivers.data_ptr(), seeds,
-                          float(value) if value is not None else 0.0, self.Q.data_ptr(),
-                          self.counts.data_ptr() if counts else None, self.nx, self.ny, local, wp, wn, C.byref(st),
-                          _dev.stream())
-                if st.value == 0:
+                if status is None:
+                    wp, wn = self._ws_tree.get(lib.pff_accumulate_tree_workspace_bytes(self.nx, self.ny, local),
+                                               self.device)
+                    seeds = None if value is not None else self.Q.data_ptr()
+                    st = C.c_int()
+                    _lib.call("pff_accumulate_tree_run", self.receivers.data_ptr(), seeds,
+                              float(value) if value is not None else 0.0, self.Q.data_ptr(),
+                              self.counts.data_ptr() if counts else None, self.nx, self.ny, local, wp, wn, C.byref(st),
+                              _dev.stream())
+                    status = st.value
+                if status == 0:
                     return
-                if st.value & 1:
+                if status & 1:
                     raise _lib.PFFError("accumulate: a receiver index is out of range")
-                if st.value == 8 and local == 1:
-                    local = 0  # receivers that are not D4 neighbours (jump rerouting): general form
+                if status == 8 and local == 1:
+                    local, status = 0, None  # receivers that are not D4 neighbours (jump rerouting): general form
                     continue
                 break
             # a receiver cycle (or a tile with more than 256 outside receivers): the
@@ -274,7 +280,9 @@ class FlowRouter:
             b = k & 1
             h2d.wait_event(start)
             if k >= 2:
-                h2d.wait_event(ev_used[b])  # DEM k-2 has left this buffer
+                # DEM k-1 is in the router's fields, so DEM k-2 has left this buffer; earlier, the
+                # transfer would slow DEM k-2's accumulation (15 us per DEM at 1536 x 1280)
+                h2d.wait_event(ev_used[b ^ 1])
             with torch.cuda.stream(h2d):
                 zb[b].copy_(dems[k].reshape(-1), non_blocking=True)
                 if wb is not None:
@@ -288,13 +296,16 @@ class FlowRouter:
             self._seed_many(wb, b)
             ev_used[b].record(main)
 
-        def take(k):  # the results of DEM k to the host
+        def keep(k):  # the results of DEM k out of the router's fields
             b = k & 1
             if k >= 2:
                 main.wait_event(ev_drained[b])  # results of DEM k-2 have left this buffer
             qb[b].copy_(self.Q)
             cb[b].copy_(self.counts)
             ev_out[b].record(main)
+
+        def send(k):  # and to the host
+            b = k & 1
             d2h.wait_event(ev_out[b])
             with torch.cuda.stream(d2h):
                 if out_Q is not None:
@@ -303,31 +314,38 @@ class FlowRouter:
                     out_counts[k].reshape(-1).copy_(cb[b], non_blocking=True)
             ev_drained[b].record(d2h)
 
-        # While DEM k is accumulated the host enqueues its results' copies and DEM k+1's
-        # fields, then reads the accumulation's status: the GPU waited 70-80 us per DEM for
-        # those calls when they followed the read.  DEM k's own seeds stay in wb[b] until
-        # load(k+2), for the rare receivers that need another accumulation.
+        # While DEM k is accumulated the host enqueues its results' copies on the device, DEM
+        # k+1's fields and DEM k+2's transfer, then reads the accumulation's status: the GPU
+        # waited 70-80 us per DEM for those calls when they followed the read.  Nothing goes
+        # to the host before the status is known.  Receivers that need another accumulation
+        # (rare) fetch DEM k's seeds from the host again.
         load(0)
         put(0)
+        if n > 1:
+            load(1)
+        self.compute_receivers()
         for k in range(n):
-            if k + 1 < n:
-                load(k + 1)
-            self.compute_receivers()
             if self.lakeflow:
                 self.reroute_flow(carve)
             read = self._accumulate_begin()
-            take(k)
+            keep(k)
             if k + 1 < n:
                 put(k + 1)
+            if k + 2 < n:
+                load(k + 2)
             if read() != 0:
-                self._seed_many(wb, k & 1)
-                ev_used[k & 1].record(main)
-                self._accumulate(True)
-                main.wait_event(ev_drained[k & 1])  # the seeds' copies of the first take
-                take(k)
+                if wb is not None:
+                    self.Q.copy_(weights[k].reshape(-1))
+                else:
+                    self.Q.fill_(1.0)
+                self._accumulate(True, refused=self._refused)
+                keep(k)
                 if k + 1 < n:
                     self._seed_many(wb, (k + 1) & 1)
                     ev_used[(k + 1) & 1].record(main)
+            if k + 1 < n:
+                self.compute_receivers()  # runs while the host enqueues the copies
+            send(k)
         main.wait_stream(d2h)
         main.wait_stream(h2d)
 
@@ -339,9 +357,11 @@ class FlowRouter:
 
     def _accumulate_begin(self):
         """Launch the tree accumulation of Q (with counts) without waiting; the returned
-        function reads its status (0: done; else _accumulate has to run on the seeds)."""
+        function reads its status (0: done; else _accumulate has to run on the seeds, and
+        _refused is that status)."""
         import ctypes as C
 
+        self._refused = None
         wp, wn = self._ws_tree.get(_lib.load().pff_accumulate_tree_workspace_bytes(self.nx, self.ny, 1), self.device)
         _lib.call("pff_accumulate_tree", self.receivers.data_ptr(), self.Q.data_ptr(), 0.0, self.Q.data_ptr(),
                   self.counts.data_ptr(), self.nx, self.ny, 1, wp, wn, _dev.stream())
@@ -349,6 +369,7 @@ class FlowRouter:
         def read():
             st = C.c_int()
             _lib.call("pff_accumulate_tree_status", self.nx, self.ny, 1, wp, wn, C.byref(st), _dev.stream())
+            self._refused = st.value or None
             return st.value
 
         return read
