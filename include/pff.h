@@ -362,7 +362,8 @@ int pff_erode_deposit(float *z, const uint8_t *bound, int32_t *rcv, const float 
  * can be captured in a CUDA graph.  Q: per-cell seed in, upstream sum out.  codes:
  * packed uint8 boundary codes (N per tile, read for custom-mode tiles only; NULL if
  * the batch has none).
- * threads: 256, 512 or 1024 per CTA; ctas_per_sm is clamped to the occupancy.
+ * threads: 256, 512 or 1024 per CTA; ctas_per_sm is clamped to 1 ... the occupancy.  One to
+ * eight CTAs (a cluster) work on a tile together.
  * pff_batch_status: error bits of the last launch (synchronizes `stream`):
  * 1 = a bad tile mode (or a custom-mode tile without codes), 8 = cells of one receiver cycle ended with
  * different serial labels, 16 = a carve did not converge, 32 = the accumulation's rounds
@@ -387,12 +388,20 @@ int pff_batch_status(long long total_cells, int ntiles, void *workspace, size_t 
  * max|dh|/dt < tol*prec with threshold = tol*prec*dt), 1 when mean|dh| < threshold,
  * -1 never.  Per tile (caller order): iters = iterations run, residuals = the last
  * (max|dh|, mean|dh|); trace (optional): niter x (max, mean) per tile.  The mean is
- * summed in an unspecified order.  Asynchronous; status bits as pff_batch_status. */
+ * summed in an unspecified order.  Asynchronous; status bits as pff_batch_status.
+ * ctas_per_sm < 1 leaves the shape to the library: one CTA of `threads` per SM, but two of
+ * 512 in place of one of 1024 where tiles outnumber the SMs. */
 int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, float *Q, const float *tile_consts,
                          float edgesw, float dt,
                          int niter, int crit, int32_t *iters, float *residuals, float *trace,
                          long long total_cells, int ntiles, int threads, int ctas_per_sm, void *workspace,
                          size_t workspace_bytes, void *stream);
+
+/* The launch that pff_batch_route (graphflood = 0) or pff_batch_graphflood makes on the current
+ * device for these values: threads and ctas_per_sm as asked for on entry, as used on
+ * return; team = CTAs per tile. */
+int pff_batch_shape(int graphflood, long long total_cells, int ntiles, int *threads, int *ctas_per_sm, int *team);
+
 
 /* ---- Warm-start network (BF16 tensor-core convolutions) ---------------------------
  * No reference counterpart: the reference has no learned component.  These serve

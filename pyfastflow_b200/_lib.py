@@ -68,6 +68,7 @@ SIGNATURES = {
     "pff_batch_plan": (_i64, [_vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp, _sz, _vp]),
     "pff_batch_route": (_i32, [_vp] * 6 + [_i64, _i32, _i32, _i32, _vp, _sz, _vp]),
     "pff_batch_status": (_i32, [_i64, _i32, _vp, _sz, C.POINTER(C.c_int), _vp]),
+    "pff_batch_shape": (_i32, [_i32, _i64, _i32] + [C.POINTER(C.c_int)] * 3),
     "pff_batch_graphflood": (_i32, [_vp, _vp, _vp, _vp, _vp, _f32, _f32, _i32, _i32, _vp, _vp, _vp, _i64, _i32,
                                     _i32, _i32, _vp, _sz, _vp]),
     "pff_conv3x3_fwd": (_i32, [_vp, _i32, _i32, _vp, _vp, _vp, _i32, _i32] + [_i32] * 7 + [_vp]),

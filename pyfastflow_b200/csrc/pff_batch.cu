@@ -1284,8 +1284,13 @@ static int batch_team(long long total, int ntiles, int slots)
     return t;
 }
 
-template <class K, class... Args>
-static int launch_batch(K kernel, int threads, int ctas_per_sm, long long total, int ntiles, cudaStream_t st, Args... args)
+struct BatchShape {
+    int threads, ctas_per_sm, team, blocks;
+};
+
+// The launch of `kernel` for the shape asked for: ctas_per_sm clamped to [1, occupancy].
+template <class K>
+static int batch_shape(K kernel, int threads, int ctas_per_sm, long long total, int ntiles, BatchShape *s)
 {
     int dev = 0, nsm = 148, occ = 1;
     PFF_CUDA(cudaGetDevice(&dev));
@@ -1296,14 +1301,40 @@ static int launch_batch(K kernel, int threads, int ctas_per_sm, long long total,
     if (ctas_per_sm < 1) ctas_per_sm = 1;
     if (ctas_per_sm > occ) ctas_per_sm = occ > 0 ? occ : 1;
     const int team = batch_team(total, ntiles, nsm * ctas_per_sm);
+    *s = BatchShape{threads, ctas_per_sm, team, std::min(std::max(nsm * ctas_per_sm / team, 1), ntiles) * team};
+    return PFF_OK;
+}
+
+// GraphFlood with the shape left to the library (ctas_per_sm < 1).  More tiles than SMs: two
+// half-size blocks per SM hold twice the tiles at once, and the steps are bound by latency,
+// not by threads (256 tiles of 128 x 128 on 148 SMs took two rounds of one block each).
+static int gf_choose(int ntiles, int *threads, int *ctas_per_sm)
+{
+    if (*ctas_per_sm >= 1) return PFF_OK;
+    int dev = 0, nsm = 148;
+    PFF_CUDA(cudaGetDevice(&dev));
+    PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    *ctas_per_sm = 1;
+    if (*threads == 1024 && ntiles > nsm) {
+        *threads = 512;
+        *ctas_per_sm = 2;
+    }
+    return PFF_OK;
+}
+
+template <class K, class... Args>
+static int launch_batch(K kernel, int threads, int ctas_per_sm, long long total, int ntiles, cudaStream_t st, Args... args)
+{
+    BatchShape s{};
+    PFF_TRY(batch_shape(kernel, threads, ctas_per_sm, total, ntiles, &s));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(std::min(std::max(nsm * ctas_per_sm / team, 1), ntiles) * team));
+    cfg.gridDim = dim3((unsigned)s.blocks);
     cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = (size_t)(threads / TILE_THREADS) * LOOP_GROUP_BYTES;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)team;
+    at[0].val.clusterDim.x = (unsigned)s.team;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
@@ -1474,18 +1505,29 @@ extern "C" int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, f
     GfParams P{tile_consts, edgesw, dt, 1e-3f, niter, crit, h, iters, residuals, trace};
     cudaStream_t st = S(stream);
     { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
-    // more tiles than SMs: two half-size blocks per SM hold twice the tiles at once, and the
-    // steps are bound by latency, not by threads (256 tiles of 128 x 128 on 148 SMs took two
-    // rounds of one block each)
-    if (threads == 1024 && ctas_per_sm <= 1) {
-        int dev = 0, nsm = 148;
-        PFF_CUDA(cudaGetDevice(&dev));
-        PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        if (ntiles > nsm) {
-            threads = 512;
-            ctas_per_sm = 2;
-        }
-    }
+    PFF_TRY(gf_choose(ntiles, &threads, &ctas_per_sm));
     PFF_TRY(launch_batch(k_batch_graphflood, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A, P));
     return check_cuda("pff_batch_graphflood");
+}
+
+extern "C" int pff_batch_shape(int graphflood, long long total_cells, int ntiles, int *threads, int *ctas_per_sm,
+                               int *team)
+{
+    clear_error();
+    if (!threads || !ctas_per_sm || !team || total_cells <= 0 || ntiles <= 0 ||
+        (*threads != 256 && *threads != 512 && *threads != 1024)) {
+        set_error("pff_batch_shape: bad arguments");
+        return PFF_ERR_ARG;
+    }
+    BatchShape s{};
+    if (graphflood) {
+        PFF_TRY(gf_choose(ntiles, threads, ctas_per_sm));
+        PFF_TRY(batch_shape(k_batch_graphflood, *threads, *ctas_per_sm, total_cells, ntiles, &s));
+    } else {
+        PFF_TRY(batch_shape(k_batch_route, *threads, *ctas_per_sm, total_cells, ntiles, &s));
+    }
+    *threads = s.threads;
+    *ctas_per_sm = s.ctas_per_sm;
+    *team = s.team;
+    return PFF_OK;
 }

@@ -43,8 +43,13 @@ class RaggedFlooder:
         """Up to `niter` iterations per tile; stop "max" ends a tile when
         max|dh|/dt < tol_ratio * P (the reference's residual), "mean" when
         mean|dh|/dt < tol_ratio * P, None never.  Returns (iterations per tile,
-        last (max|dh|, mean|dh|) per tile[, trace niter x 2 per tile])."""
+        last (max|dh|, mean|dh|) per tile[, trace niter x 2 per tile]).
+
+        The default launch shape, 1024 threads and one CTA per SM, leaves the choice to the
+        library: two CTAs of 512 threads where tiles outnumber the SMs."""
         r = self.router
+        if (threads, ctas_per_sm) == (1024, 1):
+            ctas_per_sm = 0
         cst = self._consts(tol_ratio)
         tr = torch.zeros(r.ntiles * max(niter, 1) * 2, dtype=torch.float32, device=r.device) if trace else None
         _lib.call("pff_batch_graphflood", r.z.data_ptr(), r.codes.data_ptr() if r.codes is not None else None,

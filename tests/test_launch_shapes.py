@@ -149,6 +149,25 @@ def test_batch_graphflood_teams_match_flooder(cuda, ntiles, mode):
         assert np.array_equal(rr.get_Q(t).view(np.uint32), r.get_Q().view(np.uint32)), t
 
 
+def batch_shape(graphflood, total, ntiles, threads, ctas):
+    from pyfastflow_b200 import _lib
+
+    v = [C.c_int(threads), C.c_int(ctas), C.c_int()]
+    _lib.call("pff_batch_shape", graphflood, total, ntiles, *map(C.byref, v))
+    return tuple(x.value for x in v)
+
+
+def test_batch_graphflood_takes_the_shape_asked_for(cuda):
+    """More tiles than SMs change only a shape that is left to the library."""
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    for n in (sms, sms + 1):
+        for threads, ctas in ((1024, 1), (512, 1), (512, 2), (256, 2)):
+            assert batch_shape(1, 1000 * n, n, threads, ctas)[:2] == (threads, ctas)
+    assert batch_shape(1, 1000 * sms, sms, 1024, 0)[:2] == (1024, 1)
+    assert batch_shape(1, 1000 * (sms + 1), sms + 1, 1024, 0)[:2] == (512, 2)
+    assert batch_shape(1, 1000 * (sms + 1), sms + 1, 512, 0)[:2] == (512, 1)
+
+
 @pytest.mark.parametrize("scale", [1e-37, 1e-20, 1e-9, 1.0, 1e9, 1e25, 1e36])
 def test_diffusion_quotients_in_and_out_of_range(cuda, scale):
     """Mode 0's fused pass (Markstein quotients) against mode 3 with the same boundary
