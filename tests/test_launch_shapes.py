@@ -126,6 +126,17 @@ def test_batch_teams_match_single_grids(cuda, ntiles, side, mode):
         assert np.array_equal(rr.get_Q(t).view(np.uint32), f.get_Q().view(np.uint32)), t
 
 
+# a team of 4 by the number of tiles, and by their average of more than 65536 cells
+@pytest.mark.parametrize("ntiles,side", [(16, 75), (40, 262)])
+def test_batch_teams_of_four(cuda, ntiles, side):
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    total = sum((side + k % 3) * (side - k % 5) for k in range(ntiles))
+    team = batch_shape(0, total, ntiles, 1024, 1)[2]
+    if sms == 148:
+        assert team == 4
+    test_batch_teams_match_single_grids(cuda, ntiles, side, "normal")
+
+
 @pytest.mark.parametrize("ntiles", [1, 20, 160])  # 8 blocks, 1 block, two half-size blocks per SM
 @pytest.mark.parametrize("mode", ["normal", "periodic_EW", "periodic_NS"])
 def test_batch_graphflood_teams_match_flooder(cuda, ntiles, mode):
