@@ -17,12 +17,33 @@ __device__ __forceinline__ int vload(const int *p) { return *(const volatile int
 // About 1.3 us over 148 blocks (one atomic and one polled load through L2); one block only
 // synchronises its threads.
 constexpr int BAR_HALT = 1 << 30;
+constexpr int BAR_POLLS = 32;  // about 20 us
+
+__device__ __forceinline__ int bar_poll(const int *ctr)
+{
+    int seen;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
+    return seen;
+}
+
+// The rest of a long wait for *ctr to reach target, at most limit_us; the counter's value.
+static __device__ __noinline__ int bar_long_wait(int *ctr, int target, unsigned limit_us)
+{
+    const long long t0 = clock64();
+    for (;;) {
+        const int seen = bar_poll(ctr);
+        if (seen >= target) return seen;
+        // cycles at 1.965 GHz: a little longer at lower clocks.  The swap fails if a block has
+        // arrived meanwhile: then look again
+        if (clock64() - t0 > 1965LL * limit_us && atomicCAS(ctr, seen, seen | BAR_HALT) == seen) return seen | BAR_HALT;
+    }
+}
 
 struct GridBar {
     int *ctr;
-    unsigned limit_ns;
+    const BarWait &wait;
     int target;
-    __device__ __forceinline__ GridBar(int *counter, const BarWait &w) : ctr(counter), limit_ns(w.limit_us * 1000u), target(w.absent) {}
+    __device__ __forceinline__ GridBar(int *counter, const BarWait &w) : ctr(counter), wait(w), target(w.absent) {}
     __device__ __forceinline__ bool sync(int *dead)
     {
         __syncthreads();
@@ -31,26 +52,11 @@ struct GridBar {
             if (threadIdx.x == 0) {
                 __threadfence();
                 atomicAdd(ctr, 1);
-                unsigned long long t0;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-                int spin = 0, seen;
-                for (;;) {
-                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
-                    if (seen >= target) break;  // all arrived, or BAR_HALT
-                    if ((++spin & 15) == 0) {
-                        unsigned long long t;
-                        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-                        if (t - t0 > limit_ns) {
-                            const int was = atomicCAS(ctr, seen, seen | BAR_HALT);
-                            if (was == seen) seen |= BAR_HALT;
-                            else if (was < target) continue;  // an arrival in between: look again
-                            else seen = was;
-                            break;
-                        }
-                    }
-                }
-                __threadfence();
+                int seen = bar_poll(ctr);
+                for (int spin = 0; seen < target && spin < BAR_POLLS; ++spin) seen = bar_poll(ctr);
+                if (seen < target) seen = bar_long_wait(ctr, target, wait.limit_us);
                 if (seen & BAR_HALT) *dead = 1;
+                __threadfence();
             }
             __syncthreads();
         }
