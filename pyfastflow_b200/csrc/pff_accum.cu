@@ -231,6 +231,19 @@ __device__ __forceinline__ void acc_list0(Pub *A, Pub *B, int4 *priv, int *list,
     }
 }
 
+__global__ void __launch_bounds__(256) k_acc_init(Pub *A, Pub *B, int4 *priv, const float *Q, uint32_t *counts, int N)
+{
+    acc_init(A, B, priv, Q, counts, N);
+}
+__global__ void __launch_bounds__(256) k_acc_scatter(const int32_t *rcv, Pub *A, int4 *priv, int N, int *overflow)
+{
+    acc_scatter(rcv, A, priv, N, overflow);
+}
+__global__ void __launch_bounds__(256) k_acc_list0(Pub *A, Pub *B, int4 *priv, int *list, int *nlist, int N)
+{
+    acc_list0<256>(A, B, priv, list, nlist, N);
+}
+
 // Gather-form initialisation for D4 receivers: the donors of t are the cells
 // among its grid neighbours and wrap partners whose receiver is t; visiting
 // them in ascending index gives the reference's serial slot order without
@@ -344,19 +357,13 @@ __device__ __forceinline__ int acc_store(int t, const Pub &s, bool worked, int t
     return 1;
 }
 
-// A node with three or more donors (2-3 % of them): the reference's swap-remove scan
-// (downstream_propag.py:131-162) on start-of-round donor states, loaded up front (every
-// one it can need is a start-of-round slot); then slot k holds donor w_k whose preloaded
-// state is q_k.
-__device__ __noinline__ int acc_node_many(int t, const Pub *cur, Pub *nxt, int4 *priv, float *Q, uint32_t *counts)
+// The reference's swap-remove scan (downstream_propag.py:131-162) of a node t with record s over
+// the start-of-round states P0 .. P3 of its donors `own`, loaded up front (every one it
+// can need is a start-of-round slot); slot k holds donor w_k whose preloaded state is q_k.
+__device__ __forceinline__ int acc_scan(int t, const Pub &s, const int (&own)[4], const Pub &P0, const Pub &P1,
+                                        const Pub &P2, const Pub &P3, Pub *nxt, int4 *priv, float *Q, uint32_t *counts)
 {
-    const Pub s = cur[t];
-    const int4 pq = priv[t];
     int todo = s.ndnr;
-    const int own[4] = {s.d0, pq.x, pq.y, pq.z};
-    Pub P3 = s;
-    const Pub P0 = cur[own[0]], P1 = cur[own[1]], P2 = cur[own[2]];
-    if (todo > 3) P3 = cur[own[3]];
     int w0 = own[0], w1 = own[1], w2 = own[2], w3 = own[3];
     int q0 = 0, q1 = 1, q2 = 2, q3 = 3;
     bool worked = false;
@@ -387,6 +394,32 @@ __device__ __noinline__ int acc_node_many(int t, const Pub *cur, Pub *nxt, int4 
         }
     }
     return acc_store(t, s, worked, todo, padd, cadd, w0, w1, w2, w3, nxt, priv, Q, counts);
+}
+
+// A node with three or more donors (2-3 % of them).
+__device__ __noinline__ int acc_node_many(int t, const Pub *cur, Pub *nxt, int4 *priv, float *Q, uint32_t *counts)
+{
+    const Pub s = cur[t];
+    const int4 pq = priv[t];
+    const int own[4] = {s.d0, pq.x, pq.y, pq.z};
+    const Pub P0 = cur[own[0]], P1 = cur[own[1]], P2 = cur[own[2]];
+    const Pub P3 = s.ndnr > 3 ? cur[own[3]] : s;
+    return acc_scan(t, s, own, P0, P1, P2, P3, nxt, priv, Q, counts);
+}
+
+// An active node's round: its record s, its first donor's P0, its second donor d1 and that one's P1
+// (where it has two).
+__device__ __forceinline__ int acc_node(int t, const Pub &s, int d1, const Pub &P0, const Pub &P1, const Pub *cur, Pub *nxt,
+                                        int4 *priv, float *Q, uint32_t *counts)
+{
+    if (s.ndnr > 2) return acc_node_many(t, cur, nxt, priv, Q, counts);
+    const Two r = s.ndnr == 2 ? two_donors(P0.ndnr, P1.ndnr, s.d0, d1, P0.d0, P1.d0)
+                              : Two{P0.ndnr != 0, P0.ndnr == 1 ? P0.d0 : s.d0, -1, P0.ndnr <= 1, false};
+    float p = s.p;
+    uint32_t c = s.c;
+    if (r.a0) { p = __fadd_rn(p, P0.p); c += P0.c; }
+    if (r.a1) { p = __fadd_rn(p, P1.p); c += P1.c; }
+    return acc_store(t, s, r.a0 || r.a1, r.todo, p, c, r.w0, r.w1, -1, -1, nxt, priv, Q, counts);
 }
 
 // Every remaining round in one cooperative launch, a grid barrier between rounds.  Round
@@ -421,6 +454,51 @@ struct AccRounds {
     const int *limits;  // [0] smallest, [1] largest logn of the tiles
     int *status;        // BST_* bits
 };
+
+// One round over a long list as a launch of its own, where no tile front takes the first rounds
+// (custom boundaries, or no grid): 40 warps per SM, and one atomic per list and 256 entries
+// where the cooperative rounds have 32 and one per 64 to 128; the lists keep their order.
+// Nodes with three or four donors, for which that kernel calls a function, stay with their
+// warp.  Every round by
+// k_acc_rounds and with these: custom boundaries 2522 and 2339 us at 4096 x 4096, 698 and 682
+// at 2048 x 2048, no grid 336 and 296 at 1200 x 1200.  Not the last round, nor after the
+// gather has found other receivers.
+constexpr int ACC_WIDE = 1 << 20;     // nodes from which they are used
+constexpr int ACC_WIDE_ROUNDS = 7;    // 4 rounds: 2452 us at 4096 x 4096
+template <int BS>
+__global__ void __launch_bounds__(BS, 5) k_acc_round_wide(AccRounds a, int it)
+{
+    if (*a.nonlocal) return;
+    const Pub *cur = a.buf[it & 1];
+    Pub *nxt = a.buf[(it & 1) ^ 1];
+    const int *la = a.la[it & 1], *lf = a.lf[it & 1];
+    int *c2 = a.cnt + 2 * (it + 1);
+    const int nA = a.cnt[2 * it], total = nA + a.cnt[2 * it + 1];
+    const int stride = gridDim.x * BS, trips = (total + stride - 1) / stride;
+    for (int k = 0; k < trips; ++k) {
+        const int idx = k * stride + blockIdx.x * BS + threadIdx.x;
+        int t = -1, res = 2;
+        if (idx < nA) {
+            t = la[idx];
+            const Pub s = cur[t];
+            int own[4] = {s.d0, -1, -1, -1};
+            if (s.ndnr > 1) {
+                const int4 pq = a.priv[t];
+                own[1] = pq.x; own[2] = pq.y; own[3] = pq.z;
+            }
+            Pub P0 = s, P1 = s, P2 = s, P3 = s;
+            P0 = cur[own[0]];
+            if (s.ndnr > 1) P1 = cur[own[1]];
+            if (s.ndnr > 2) P2 = cur[own[2]];
+            if (s.ndnr > 3) P3 = cur[own[3]];
+            res = acc_scan(t, s, own, P0, P1, P2, P3, nxt, a.priv, a.Q, a.counts);
+        } else if (idx < total) {
+            t = lf[idx - nA];
+            nxt[t] = cur[t];
+        }
+        block_append2<BS>(res == 0, res == 1, t, a.la[(it & 1) ^ 1], c2, a.lf[(it & 1) ^ 1], c2 + 1);
+    }
+}
 
 __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
 {
@@ -502,18 +580,8 @@ __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
                     if (last) {  // the start-of-round value is the result (fuse(.., logn), :59-74)
                         a.Q[t[u]] = s.p;
                         if (a.counts) a.counts[t[u]] = s.c;
-                    } else if (s.ndnr > 2) {
-                        res[u] = acc_node_many(t[u], cur, nxt, a.priv, a.Q, a.counts);
                     } else {
-                        const Two r = s.ndnr == 2 ? two_donors(P0[u].ndnr, P1[u].ndnr, s.d0, d1[u], P0[u].d0, P1[u].d0)
-                                                  : Two{P0[u].ndnr != 0, P0[u].ndnr == 1 ? P0[u].d0 : s.d0, -1,
-                                                        P0[u].ndnr <= 1, false};
-                        float p = s.p;
-                        uint32_t c = s.c;
-                        if (r.a0) { p = __fadd_rn(p, P0[u].p); c += P0[u].c; }
-                        if (r.a1) { p = __fadd_rn(p, P1[u].p); c += P1[u].c; }
-                        res[u] = acc_store(t[u], s, r.a0 || r.a1, r.todo, p, c, r.w0, r.w1, -1, -1, nxt, a.priv, a.Q,
-                                           a.counts);
+                        res[u] = acc_node(t[u], s, d1[u], P0[u], P1[u], cur, nxt, a.priv, a.Q, a.counts);
                     }
                 } else if (idx < total) {
                     nxt[t[u]] = sc[u];
@@ -940,14 +1008,16 @@ static void l_acc_gather(const int32_t *rcv, Pub *A, Pub *B, int4 *priv, const f
 
 // Blocks of the cooperative rounds over n nodes: one per 8192 up to one per SM.  More blocks
 // make each barrier dearer than the shorter lists save: one per 2048 takes the whole call at
-// 700 x 500 from 437 to 453 us, 48 tiles of 32 to 160 from 422 to 432.
-static int launch_rounds(AccRounds &a, int n, cudaStream_t st)
+// 700 x 500 from 437 to 453 us, 48 tiles of 32 to 160 from 422 to 432.  Where no grid is given
+// the scatter's passes over every node are in the same launch, and one per 2048 is the better:
+// 155 against 205 us at 200 x 200, 229 against 246 at 700 x 500.
+static int launch_rounds(AccRounds &a, int n, int per_block, cudaStream_t st)
 {
     int dev = 0, nsm = 0;
     PFF_CUDA(cudaGetDevice(&dev));
     PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     void *args[] = {&a};
-    PFF_CUDA(cudaLaunchCooperativeKernel((void *)k_acc_rounds, std::max(1, std::min(nsm, div_up(n, 8192))), ACC_THREADS,
+    PFF_CUDA(cudaLaunchCooperativeKernel((void *)k_acc_rounds, std::max(1, std::min(nsm, div_up(n, per_block))), ACC_THREADS,
                                          args, 0, st));
     count_launch();
     return PFF_OK;
@@ -983,7 +1053,7 @@ int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st)
     a.cnt = cnt; a.nonlocal = nonlocal; a.overflow = nonlocal + 1;
     a.N = (int)b.total; a.first = BATCH_FR; a.bar = bar; a.wait = bar_wait(BAR_ROUNDS);
     a.tiles = b.by_offset; a.ntiles = b.ntiles; a.limits = b.limits; a.status = b.status;
-    return launch_rounds(a, (int)b.total, st);
+    return launch_rounds(a, (int)b.total, 8192, st);
 }
 
 }  // namespace pff
@@ -1098,6 +1168,13 @@ extern "C" int pff_accumulate_grid(const int32_t *receivers, float *Q, uint32_t 
         Grid g{nx, ny, mode, codes};
         PFF_MODE_DISPATCH(mode, l_acc_gather, receivers, A, B, priv, Q, counts, lA0, ctr + 0, nonlocal, overflow, g,
                           st);
+    } else if (N >= ACC_WIDE) {
+        int dev = 0, nsm = 148;
+        PFF_CUDA(cudaGetDevice(&dev));
+        PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        { k_acc_init<<<8 * nsm, 256, 0, st>>>(A, B, priv, Q, counts, N); count_launch(); }
+        { k_acc_scatter<<<8 * nsm, 256, 0, st>>>(receivers, A, priv, N, overflow); count_launch(); }
+        { k_acc_list0<<<8 * nsm, 256, 0, st>>>(A, B, priv, lA0, ctr, N); count_launch(); }
     } else {
         PFF_CUDA(cudaMemsetAsync(nonlocal, 1, sizeof(int), st));
     }
@@ -1114,8 +1191,17 @@ extern "C" int pff_accumulate_grid(const int32_t *receivers, float *Q, uint32_t 
     for (int k = 0; k < 2; ++k) { a.la[k] = la[k]; a.lf[k] = lf[k]; }
     a.cnt = ctr; a.nonlocal = nonlocal; a.overflow = overflow;
     a.N = N; a.first = front ? FR : 0; a.logn = logn;
+    if (!front && N >= ACC_WIDE) {
+        int dev = 0, nsm = 148;
+        PFF_CUDA(cudaGetDevice(&dev));
+        PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        for (; a.first < ACC_WIDE_ROUNDS; ++a.first) {
+            k_acc_round_wide<256><<<5 * nsm, 256, 0, st>>>(a, a.first);
+            count_launch();
+        }
+    }
     a.bar = bar; a.wait = bar_wait(BAR_ROUNDS); a.over_out = dptr;
-    PFF_TRY(launch_rounds(a, N, st));
+    PFF_TRY(launch_rounds(a, N, nx > 0 ? 8192 : 2048, st));
     PFF_CUDA(cudaStreamSynchronize(st));
     PFF_TRY(check_cuda("pff_accumulate"));
     const int over = *(volatile int *)host;

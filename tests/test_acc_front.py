@@ -106,3 +106,41 @@ def test_front_hands_over_nonlocal_receivers(orc, cuda, front):
     Q, c = _run(torch, rcv, w, nx, ny, 1, front)
     assert np.array_equal(c, co)
     assert np.array_equal(Q.view(np.uint32), Qo.view(np.uint32))
+
+
+# the scatter inside the rounds' launch, and with launches of its own and rounds over long lists
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(90, 70), (1100, 1000)])
+def test_rounds_without_a_front(cuda, nx, ny):
+    """No grid given, and custom boundaries that are the normal ones: the sums of the front's
+    path bit for bit (the same additions in the same order)."""
+    torch = cuda
+    from pyfastflow_b200 import _dev, _lib, synthetic
+    from pyfastflow_b200.flow import FlowRouter
+
+    lib = _lib.load()
+    n = nx * ny
+    codes = np.ones((ny, nx), np.uint8)
+    codes[0, :] = codes[-1, :] = codes[:, 0] = codes[:, -1] = 3
+    z = synthetic.spectral_dem(nx, ny, 4, relief=300.0, npits=n // 800, pit_scale=0.1)
+    w = torch.from_numpy(synthetic.lognormal_weights(n, 5)).cuda()
+    out = []
+    for mode in ("normal", "custom"):
+        r = FlowRouter(nx, ny, 30.0, mode, boundaries=codes if mode == "custom" else None)
+        r.set_z(z)
+        r.compute_receivers()
+        r.reroute_flow()
+        r.accumulate_weighted_Q(w, exact_order=True)
+        out.append((r.receivers, r.Q, r.counts))
+    wb = lib.pff_accumulate_workspace_bytes(n)
+    ws = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    Q, counts = w.clone(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    _lib.call("pff_accumulate", r.receivers.data_ptr(), Q.data_ptr(), counts.data_ptr(), n, ws.data_ptr(), wb,
+              _dev.stream())
+    out.append((r.receivers, Q, counts))
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    star = torch.zeros(n, dtype=torch.int32, device="cuda")  # a node with more than four donors
+    rc = lib.pff_accumulate(star.data_ptr(), Q.data_ptr(), counts.data_ptr(), n, ws.data_ptr(), wb, _dev.stream())
+    assert rc == 1 and b"more than 4 donors" in lib.pff_last_error_string()
