@@ -942,7 +942,7 @@ __global__ void __launch_bounds__(Front<BATCH_FR>::BS) k_batch_front(BatchAcc b,
                                                                      int *la, int *nla, int *lf, int *nlf, int *nonlocal)
 {
     using F = Front<BATCH_FR>;
-    const int n = b.limits[2];
+    const int n = b.small && *b.small ? 0 : b.limits[2];
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const BatchTile T = b.by_offset[b.items[k]];
         const Grid g{T.nx, T.ny, T.mode, nullptr};
@@ -1038,7 +1038,6 @@ int launch_batch_accumulate(const BatchAcc &b, cudaStream_t st)
     PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     using F = Front<BATCH_FR>;
     PFF_CUDA(cudaFuncSetAttribute(k_batch_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::SMEM));
-    PFF_CUDA(cudaMemsetAsync(b.ctr, 0, sizeof(int) * BATCH_ACC_CTR, st));
     int *cnt = b.ctr, *nonlocal = b.ctr + 128, *bar = b.ctr + 136;
     constexpr int pa = BATCH_FR & 1;
     Pub *buf[2] = {(Pub *)b.bufA, (Pub *)b.bufB};

@@ -39,11 +39,16 @@ struct BatchArrays {
     uint32_t *c_;
     const BatchTile *tiles;  // in largest-first order
     int *queue;              // [0] next tile
+    const int *small;        // whether the batch is k_batch_small's; null: it is not
     int *status;             // [0] error bits (see pff_batch_status)
 };
 
 
 constexpr int LB_SIDE = 32, LB_CELLS = LB_SIDE * LB_SIDE;  // label sub-blocks
+
+// Cells up to which GraphFlood's reroutes are the reference's steps by one block: 5 iterations on 40 tiles of
+// 24 x 24 take 483 us, 563 by the list loop; of 32 x 32 753 and 644.
+constexpr int GF_SMALL = 900;
 
 struct BatchShm {
     LoopArgs la;  // the current tile's reroute
@@ -641,15 +646,14 @@ __device__ __forceinline__ bool team_any(bool p, BatchShm &sh, ClusterTeam &Tm)
     return res;
 }
 
-// receivers (receivers.py:31-58): strict >, first k wins ties (and the gradient if
-// grad is not null).
-template <int MODE>
-__device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, float *grad,
-                                            ClusterTeam Tm)
+// receivers (receivers.py:31-58): strict >, first k wins ties (and the gradient and a copy of the
+// receivers if grad and rec_ are not null).
+template <int MODE, int U>
+__device__ __forceinline__ void receivers_cells(const Grid &g, float dx, const float *z, int32_t *rec, int32_t *rec_,
+                                                float *grad, ClusterTeam Tm)
 {
     const int N = g.nx * g.ny;
     const unsigned mnx = 0xffffffffu / (unsigned)g.nx;
-    constexpr int U = 2;
     FOR_TEAM_U(i0, stride, U, N) {
         int js[U][4];
         float zi[U], zn[U][4];
@@ -704,17 +708,26 @@ __device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float
                 }
             }
             rec[i] = r;
+            if (rec_) rec_[i] = r;
             if (grad) grad[i] = sr;
         }
     }
     Tm.sync();
 }
 
-// reroute_flow(carve=True) (lakeflow.py:466-538), the reference's own steps by one block,
-// from outer iteration it (with rec_ == rec; outer as the first iteration set it).
 template <int MODE>
-__device__ __noinline__ void tile_reroute_steps(const Grid &g, const BatchTile &T, const BatchArrays &A, const float *z,
-                                                BatchShm &sh, int it, int outer)
+__device__ __noinline__ void tile_receivers(const Grid &g, float dx, const float *z, int32_t *rec, float *grad,
+                                            ClusterTeam Tm)
+{
+    receivers_cells<MODE, 2>(g, dx, z, rec, nullptr, grad, Tm);
+}
+
+// reroute_flow(carve=True) (lakeflow.py:466-538), the reference's own steps by one block,
+// from outer iteration it (with rec_ == rec; outer as the first iteration set it, or -1 to set
+// it here).
+template <int MODE>
+__device__ __forceinline__ void reroute_steps(const Grid &g, const BatchTile &T, const BatchArrays &A, const float *z,
+                                              BatchShm &sh, int it, int outer)
 {
     const int N = g.nx * g.ny;
     const long long o = T.off, ob = T.boff;
@@ -734,9 +747,10 @@ __device__ __noinline__ void tile_reroute_steps(const Grid &g, const BatchTile &
         __syncthreads();
         return n;
     };
-    for (; it < outer; ++it) {
+    for (; outer < 0 || it < outer; ++it) {
         const int nd = list_pits();
         if (nd == 0) break;  // (the labels the reference computes first are overwritten)
+        if (outer < 0) outer = bceil_log2(nd) + 1;  // :500
         const bool acyclic = tile_labels_blocks<MODE>(g, N, rec_, rec__, bid, sh);
         if (!acyclic) tile_labels<MODE>(g, N, rec_, rec__, bid, A.mark + o, A.dnr + 4 * o, lrounds, sh, A.status);
         const int32_t *bl = acyclic ? pl : nullptr;  // basin ids: the pits', or any (labels of a cycle)
@@ -744,6 +758,28 @@ __device__ __noinline__ void tile_reroute_steps(const Grid &g, const BatchTile &
                               A.inv + ob, z, bl, nd);
         tile_carve(N, rec, rec_, A.mark + o, A.tag + o, A.snode + ob, A.outlet + ob, bl, nd, A.status);
     }
+}
+
+template <int MODE>
+__device__ __noinline__ void tile_reroute_steps(const Grid &g, const BatchTile &T, const BatchArrays &A, const float *z,
+                                                BatchShm &sh, int it, int outer)
+{
+    reroute_steps<MODE>(g, T, A, z, sh, it, outer);
+}
+
+// A small tile, start to end, by one block: the reference's steps need fewer barriers than the list
+// loop and its front.
+template <int MODE>
+__device__ __forceinline__ void small_tile(const BatchTile *tile, const BatchArrays &A, BatchShm &sh)
+{
+    const BatchTile T = *tile;
+    const Grid g{T.nx, T.ny, MODE, MODE == 3 ? A.codes + T.off : nullptr};
+    const long long o = T.off;
+    const float *z = A.z + o;
+    receivers_cells<MODE, 1>(g, T.dx, z, A.rcv + o, A.rec_ + o, A.grad + o, ClusterTeam{0, 1});
+    reroute_steps<MODE>(g, T, A, z, sh, 0, -1);
+    tile_accumulate(T.nx * T.ny, A.rcv + o, A.Q + o, A.counts + o, A.dnr + 4 * o, A.dnr_ + 4 * o, A.ndnr + o,
+                    A.ndnr_ + o, A.src + o, A.p_ + o, A.c_ + o, A.mark + o, A.rec__ + o, sh);
 }
 
 // The same reroute by the single grid's device loop, the team's blocks together; a tile
@@ -783,6 +819,15 @@ __device__ __noinline__ void tile_reroute(const BatchTile &T, const BatchArrays 
     const int N = g.nx * g.ny;
     const long long o = T.off, ob = T.boff;
     int32_t *R = reinterpret_cast<int32_t *>(A.p_) + o;  // later the segment list
+    if (N <= GF_SMALL) {
+        if (Tm.r == 0) {
+            FOR_CELLS(i, N) A.rec_[o + i] = A.rcv[o + i];
+            __syncthreads();
+            tile_reroute_steps<MODE>(g, T, A, z, sh, 0, -1);
+        }
+        Tm.sync();
+        return;
+    }
     if (Tm.r == 0)
         for (int k = threadIdx.x; k < 64 + LOOP_ITS * LOOP_CTR; k += blockDim.x) sh.loop[k] = 0;
     if (threadIdx.x == 0) {
@@ -1152,6 +1197,7 @@ __global__ void __launch_bounds__(1024) k_batch_route(int ntiles, BatchArrays A)
 {
     extern __shared__ __align__(16) unsigned char batch_smem[];
     __shared__ BatchShm sh;
+    if (A.small && *A.small) return;  // k_batch_small's batch
     ClusterTeam Tm = cluster_team();
     if (threadIdx.x == 0) sh.any[0] = sh.any[1] = sh.any[2] = sh.any_r = 0;
     for (;;) {
@@ -1170,6 +1216,35 @@ __global__ void __launch_bounds__(1024) k_batch_route(int ntiles, BatchArrays A)
             if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
             break;
         }
+    }
+}
+
+// A batch of small tiles, one block per tile.  A kernel of its own: without the list loop's shared
+// memory the steps' scratch stays in L1 (2000 tiles of 32 x 32 cells 1476 us, 1791 inside
+// k_batch_route), and with nothing else inlined they spill nothing.
+__global__ void __launch_bounds__(1024) k_batch_small(int ntiles, BatchArrays A)
+{
+    __shared__ BatchShm sh;
+    if (!*A.small) return;
+    for (;;) {
+        if (threadIdx.x == 0) sh.cur = atomicAdd(A.queue, 1);
+        __syncthreads();
+        const int k = sh.cur;
+        __syncthreads();
+        if (k >= ntiles) return;
+        switch (A.tiles[k].mode) {
+        case 0: small_tile<0>(A.tiles + k, A, sh); break;
+        case 1: small_tile<1>(A.tiles + k, A, sh); break;
+        case 2: small_tile<2>(A.tiles + k, A, sh); break;
+        case 3:
+            if (A.codes) small_tile<3>(A.tiles + k, A, sh);
+            else if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
+            break;
+        default:
+            if (threadIdx.x == 0) atomicOr(A.status, BST_MODE);
+            break;
+        }
+        __syncthreads();
     }
 }
 
@@ -1199,10 +1274,10 @@ __global__ void __launch_bounds__(1024) k_batch_graphflood(int ntiles, BatchArra
     }
 }
 
-__global__ void k_batch_reset(int *ctr)
+__global__ void k_batch_reset(int *ctr, int *acc_ctr)
 {
-    ctr[0] = 0;
-    ctr[1] = 0;
+    if (threadIdx.x < 2) ctr[threadIdx.x] = 0;
+    if (acc_ctr) acc_ctr[threadIdx.x] = 0;
 }
 
 // Workspace layout, identical for the plan and the launches.
@@ -1282,6 +1357,24 @@ static int batch_team(long long total, int ntiles, int slots)
     while (t < 8 && (long long)ntiles * t * 2 <= slots && avg >= 2048LL * t) t *= 2;
     if (avg >= 65536) t = std::max(t, 4);
     return t;
+}
+
+// A batch whose largest tile has at most so many cells is k_batch_small's, by the threads of a block
+// (1024, 512, 256).  The steps beat the list loop while barriers cost more than passes over
+// every cell.  Tiles of 24 x 24 cells: 40 of them take 118 us with 1024 threads and 183 by the loop, 2000
+// take 900 and 1150; 48 x 48: 205 and 250, but 2000 of them 2198 and 2126, and 40 of 56 x 56
+// with 512 threads 264 and 259; with 256 threads 40 of 40 x 40 237 and 239.  Mixed batches go by their
+// largest tile, the last to end: 40 of 24 to 60 cells a side 219 and 234, of 24 to 75 289 and
+// 275.  Where blocks of 1024 threads have two tiles each, the smaller ones make up for
+// it: 200 of 24 to 75 384 and 476 (but of 64 x 64 567 and 503).
+constexpr int SMALL_CLASSES = 3;
+static int small_class(int threads) { return threads == 1024 ? 0 : (threads == 512 ? 1 : 2); }
+static int small_cells(int cls, int ntiles, long long total)
+{
+    if (cls == 2) return 1900;
+    if (ntiles > 300) return 2600;
+    if (cls == 1) return 3100;
+    return ntiles > 148 && total <= 2600LL * ntiles ? 5600 : 3600;
 }
 
 struct BatchShape {
@@ -1389,11 +1482,16 @@ extern "C" long long pff_batch_plan(const int32_t *tile_nx, const int32_t *tile_
     std::stable_sort(ord, ord + ntiles, [&](int a, int b) { return cells(a) > cells(b); });
     std::vector<BatchTile> hp(ntiles), ht(ntiles);  // packed order, largest first
     std::vector<int> items;
-    int limits[3] = {64, 0, 0};
+    int limits[3 + SMALL_CLASSES] = {64, 0, 0};  // from [3] on, per class, whether the batch is k_batch_small's
+    bool small = true;  // with every launch shape
+    for (int c = 0; c < SMALL_CLASSES; ++c) {
+        limits[3 + c] = cells(ord[0]) <= small_cells(c, ntiles, total);
+        small = small && limits[3 + c];
+    }
     for (int t = 0; t < ntiles; ++t) {
         const int nx = tile_nx[t], ny = tile_ny[t], logn = bceil_log2(cells(t)) + 1;
         // packed cell ids of the accumulation are 32-bit
-        const bool front = batch_front_takes(nx, ny, tile_mode[t]) && total < 2000000000LL;
+        const bool front = !small && batch_front_takes(nx, ny, tile_mode[t]) && total < 2000000000LL;
         hp[t] = BatchTile{tile_offset[t], tile_offset[t] + t, nx, ny, tile_mode[t], t, tile_dx[t],
                           front ? (int)items.size() : -1, logn, 0};
         if (!front) continue;
@@ -1446,7 +1544,17 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
     A.Q = Q;
     A.counts = counts;
     cudaStream_t st = S(stream);
-    { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
+    { k_batch_reset<<<1, BATCH_ACC_CTR, 0, st>>>(w.ctr, w.acc_ctr); count_launch(); }
+    const int cls = small_class(threads);
+    if (total_cells <= (long long)small_cells(cls, ntiles, total_cells) * ntiles) {  // else the largest tile is larger
+        A.small = w.limits + 3 + cls;
+        int dev = 0, nsm = 148, occ = 1;
+        PFF_CUDA(cudaGetDevice(&dev));
+        PFF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        PFF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch_small, threads, 0));
+        const int grid = std::min(nsm * std::max(std::min(ctas_per_sm, occ), 1), ntiles);
+        { k_batch_small<<<grid, threads, 0, st>>>(ntiles, A); count_launch(); }
+    }
     PFF_TRY(launch_batch(k_batch_route, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A));
     if (total_cells < 2000000000LL) {
         BatchAcc b{};
@@ -1454,7 +1562,7 @@ extern "C" int pff_batch_route(const float *z, const uint8_t *codes, int32_t *re
         b.bufA = A.dnr; b.bufB = A.dnr_; b.priv = w.priv;
         b.la[0] = A.ndnr; b.la[1] = A.ndnr_;
         b.lf[0] = A.src; b.lf[1] = reinterpret_cast<int *>(A.p_);
-        b.ctr = w.acc_ctr; b.status = A.status;
+        b.ctr = w.acc_ctr; b.status = A.status; b.small = A.small;
         b.by_offset = w.by_offset; b.items = w.items; b.limits = w.limits;
         b.total = total_cells; b.ntiles = ntiles;
         PFF_TRY(launch_batch_accumulate(b, st));
@@ -1504,7 +1612,7 @@ extern "C" int pff_batch_graphflood(float *zh, const uint8_t *codes, float *h, f
     A.counts = nullptr;
     GfParams P{tile_consts, edgesw, dt, 1e-3f, niter, crit, h, iters, residuals, trace};
     cudaStream_t st = S(stream);
-    { k_batch_reset<<<1, 1, 0, st>>>(w.ctr); count_launch(); }
+    { k_batch_reset<<<1, BATCH_ACC_CTR, 0, st>>>(w.ctr, nullptr); count_launch(); }
     PFF_TRY(gf_choose(ntiles, &threads, &ctas_per_sm));
     PFF_TRY(launch_batch(k_batch_graphflood, threads, ctas_per_sm, total_cells, ntiles, st, ntiles, A, P));
     return check_cuda("pff_batch_graphflood");

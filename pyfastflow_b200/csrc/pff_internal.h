@@ -123,7 +123,8 @@ struct BatchAcc {
     uint32_t *counts;
     void *bufA, *bufB, *priv;  // 16 B per cell each
     int *la[2], *lf[2];   // 4 B per cell each
-    int *ctr;             // BATCH_ACC_CTR ints
+    int *ctr;             // BATCH_ACC_CTR ints, zero
+    const int *small;     // null, or whether the sums are there already
     int *status;          // BST_* bits
     const BatchTile *by_offset;  // the tiles in packed order
     const int *items;     // work item -> tile (packed order)

@@ -160,6 +160,47 @@ def test_batch_graphflood_teams_match_flooder(cuda, ntiles, mode):
         assert np.array_equal(rr.get_Q(t).view(np.uint32), r.get_Q().view(np.uint32)), t
 
 
+# batches of small tiles, by the threads of a block and the largest tile; a larger one beside them,
+# tiles of two rows, custom boundaries, more tiles than blocks
+@pytest.mark.parametrize("threads,ctas", [(1024, 1), (512, 2), (256, 4)])
+@pytest.mark.parametrize("sides,ntiles", [((2, 9), 20), ((38, 43), 30), ((43, 44), 30), ((50, 60), 30), ((59, 61), 30),
+                                          ((20, 74), 160), ((24, 75), 160), ((12, 50), 310), ((12, 52), 310)])
+def test_batches_of_small_tiles(cuda, threads, ctas, sides, ntiles):
+    """Against single grids, and every launch shape and the graph alike."""
+    torch = cuda
+    from pyfastflow_b200.flow import FlowRouter, RaggedRouter
+
+    rng = np.random.default_rng(ntiles)
+    shapes = [tuple(int(v) for v in rng.integers(sides[0], sides[1] + 1, 2)) for _ in range(ntiles)]
+    shapes[0] = (sides[1], sides[1])
+    names = ["normal", "periodic_EW", "periodic_NS", "custom"]
+    modes = [names[k % 4] for k in range(ntiles)]
+    codes = [codes_like(3, nx, ny, k) if k % 4 == 3 else None for k, (ny, nx) in enumerate(shapes)]
+    kinds = ["int", "spectral", "zeros"]
+    zs = [surface(kinds[k % 3] if min(shapes[k]) > 4 else "int", nx, ny, k) for k, (ny, nx) in enumerate(shapes)]
+    rr = RaggedRouter(shapes, 30.0, modes, codes=codes)
+    rr.threads, rr.ctas_per_sm = threads, ctas
+    rr.set_z(zs)
+    rr.seed_weights(synthetic.lognormal_weights(rr.total, 4))
+    rr.route()
+    got = [t.clone() for t in (rr.receivers, rr.gradient, rr.Q, rr.counts)]
+    for graph in (True, True, False):
+        rr.route(graph=graph)
+        for a, b in zip(got, (rr.receivers, rr.gradient, rr.Q, rr.counts)):
+            assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    for t in [0] + list(range(1, ntiles, ntiles // 8)):
+        ny, nx = shapes[t]
+        f = FlowRouter(nx, ny, 30.0, modes[t], boundaries=codes[t])
+        f.set_z(zs[t])
+        f.compute_receivers()
+        f.reroute_flow()
+        f.accumulate_weighted_Q(rr._slice(rr.seed, t), exact_order=True)
+        torch.cuda.synchronize()
+        assert np.array_equal(rr.get_receivers(t), f.get_receivers()), t
+        assert np.array_equal(rr.get_counts(t), f.get_counts()), t
+        assert np.array_equal(rr.get_Q(t).view(np.uint32), f.get_Q().view(np.uint32)), t
+
+
 def batch_shape(graphflood, total, ntiles, threads, ctas):
     from pyfastflow_b200 import _lib
 
