@@ -16,8 +16,7 @@ reference itself is Python on Taichi, which is not installable here) on the
 same full workload with all host threads, one chain per step.
 
 roofline: the kernel with the largest event time per step among the probed
-kernels (library-side CUDA events around each launch, in a separate pass with
-the reroute loop driven from the host so that its kernels launch one by one).
+kernels (library-side CUDA events around each launch, in a separate pass).
 """
 from __future__ import annotations
 
@@ -46,8 +45,9 @@ ALG_BYTES = {"receivers": 12, "reroute": 16, "accumulate": 16}
 KERNELS = {
     "k_receivers": (12, 152.3e6),           # z in; receivers + gradient out
     "k_tile_terminal<grid>": (8, None),     # receivers in; tile terminals out
-    "k_tile_terminal<list>": (None, None),  # the tiles a carve changed
+    "k_reroute_labels": (8, None),          # tile terminals in; labels out
     "k_saddle_p12_strip": (13, None),       # labels + z in; is_border + z' out (the border lists are extra)
+    "k_reroute_loop": (16, 2049.1e6),       # the reroute's own bytes: receivers + z in; receivers + basin ids out
     "k_tree_tile<up>": (8, 421.0e6),        # receivers + seeds in (in-tile totals are kept: 12 B out)
     "k_tree_tile<down>": (16, 464.2e6),     # receivers + seeds in; Q + counts out (totals read back)
 }
@@ -329,7 +329,6 @@ def main():
     # ---- per-kernel event times (separate pass, probes armed) -> roofline ----
     import ctypes
 
-    prev_graphs = lib.pff_reroute_use_graphs(0)
     lib.pff_probe_enable(1)
     for s in range(args.steps):
         flush.fill_(s & 0xFF)
@@ -349,7 +348,6 @@ def main():
             k["traffic"] = traffic * (n * n) / 16777216.0 if traffic else None
         kernels[name] = k
     lib.pff_probe_enable(0)
-    lib.pff_reroute_use_graphs(prev_graphs)
     timed = [k for k in kernels if "alg_bytes_per_launch" in kernels[k]]
     dom = max(timed, key=lambda k: kernels[k]["ms_per_step"])
     kd = kernels[dom]
@@ -900,8 +898,9 @@ def graphflood_main(args):
 GF_KERNELS = {
     "k_receivers": 12,            # zh in; receivers + gradient out
     "k_tile_terminal<grid>": 8,   # receivers in; tile terminals out
-    "k_tile_terminal<list>": None,
-    "k_relabel_jump_block": None,  # one CTA: the basin chains of a short pit list
+    "k_reroute_labels": 8,        # tile terminals in; labels out
+    "k_saddle_p12_strip": 13,     # labels + z in; is_border + z' out
+    "k_reroute_loop": 16,         # the reroute's own bytes: receivers + z in; receivers + basin ids out
     "k_fill_round_packed": 16,    # one 8-byte {pointer, z} record in and out per round (the gather at the pointer is extra)
     "k_fill_round_late": 16,      # the same rounds from the tenth on (a round after a settled one returns at once)
     "k_diffuse_fused": 12,        # zh + Q in; Q after all sweeps out
@@ -923,7 +922,7 @@ def graphflood_kernel_probe(router, fl, reset, n, iters):
     pk, pk_kind = peak_hbm()
     reset()
     torch.cuda.synchronize()
-    prev_graphs, prev_fl = lib.pff_reroute_use_graphs(0), fl.graphs
+    prev_fl = fl.graphs
     fl.graphs = False
     lib.pff_probe_enable(1)
     for _ in range(iters):
@@ -942,7 +941,6 @@ def graphflood_kernel_probe(router, fl, reset, n, iters):
             k["frac"] = k["achieved_gbs"] / pk
         res[name] = k
     lib.pff_probe_enable(0)
-    lib.pff_reroute_use_graphs(prev_graphs)
     fl.graphs = prev_fl
     return res
 

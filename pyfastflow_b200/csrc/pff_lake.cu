@@ -1798,12 +1798,12 @@ static void l_strip(const LoopArgs &A, cudaStream_t st)
     int *na = A.it_ctr + LC_NA;
     if (MODE != 3 && vec) {
         const long long warps = (long long)((g.nx + 127) / 128) * ((g.ny + SAD4_ROWS - 1) / SAD4_ROWS);
-        k_saddle_p12_strip4<MODE == 3 ? 0 : MODE><<<div_up(warps, 4), 128, 0, st>>>(
-            A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr, A.alist[0], na, A.info);
+        PFF_PROBED("k_saddle_p12_strip", st, k_saddle_p12_strip4<MODE == 3 ? 0 : MODE><<<div_up(warps, 4), 128, 0, st>>>(
+            A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr, A.alist[0], na, A.info));
     } else {
         const long long warps = (long long)((g.nx + 31) / 32) * ((g.ny + SAD_ROWS - 1) / SAD_ROWS);
-        k_saddle_p12_strip<MODE><<<div_up(warps, 4), 128, 0, st>>>(A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr,
-                                                                   A.alist[0], na, A.info);
+        PFF_PROBED("k_saddle_p12_strip", st, k_saddle_p12_strip<MODE><<<div_up(warps, 4), 128, 0, st>>>(
+            A.bid, A.isb, A.zp, A.sad, A.z, g, nullptr, nullptr, A.alist[0], na, A.info));
     }
     count_launch();
 }
@@ -1826,12 +1826,15 @@ static void l_loop(const LoopArgs &A, int32_t *R, int blocks, bool whole, int nz
     }
     l_tile_terminal<MODE>(a.rec, a.J, R, a.pit0, a.info, a.g, a.rec_, st);  // :491, :493
     void *largs[] = {&a, &R};
-    cudaError_t e = cudaLaunchCooperativeKernel((void *)k_reroute_labels<MODE>, blocks, LOOP_THREADS, largs, 0, st);
+    cudaError_t e = cudaSuccess;
+    PFF_PROBED("k_reroute_labels", st,
+               e = cudaLaunchCooperativeKernel((void *)k_reroute_labels<MODE>, blocks, LOOP_THREADS, largs, 0, st));
     if (e == cudaSuccess) {
         count_launch();
         l_strip<MODE>(a, st);
         void *args[] = {&a};
-        e = cudaLaunchCooperativeKernel((void *)k_reroute_loop<MODE>, blocks, LOOP_THREADS, args, LOOP_SMEM, st);
+        PFF_PROBED("k_reroute_loop", st,
+                   e = cudaLaunchCooperativeKernel((void *)k_reroute_loop<MODE>, blocks, LOOP_THREADS, args, LOOP_SMEM, st));
         count_launch();
     }
     if (e != cudaSuccess) {
