@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(ACC_THREADS, 1) k_acc_rounds(AccRounds a)
 // hops.  The initial state of a cell needs the receivers of its neighbours, one
 // more cell.  So one CTA loads a tile plus a halo of 2^FR cells (receivers and
 // seeds), builds the initial states in shared memory, and runs the rounds with
-// k_acc_round's per-node rule: round r only over the cells within
+// the rule of acc_node and acc_node_many: round r only over the cells within
 // 2^FR - 2^(r+1) of the tile (what the later rounds of the tile's cells read),
 // the last round in registers for the tile's cells alone.
 //
@@ -646,7 +646,7 @@ struct Front {
     static_assert((TW * TH) % BS == 0, "uniform output trips");
 };
 
-// One node's round on shared-memory snapshots (k_acc_round's rule; local ids).
+// One node's round on shared-memory snapshots (the rule of acc_node and acc_node_many; local ids).
 struct FrontNode {
     int todo;
     float p;

@@ -8,7 +8,7 @@
 // exponent's rounding d = 5.0f/3.0f - 5/3 (about -4e-8) multiplies by exp(d ln h) =
 // 1 + g + g^2/2, whose error is at most 1e-12 (log2's absolute error of 2.4e-5 times d).
 // A result within 2^-36 of halfway between two floats, where that error could decide the
-// rounding (about one in 2000), and arguments outside [2^-70, 2^70] (zero, negative, NaN
+// rounding (one in 4096), and arguments outside [2^-70, 2^70] (zero, negative, NaN
 // among them) take pow.  pff_pow53_selfcheck compares the two over ranges of floats.
 #pragma once
 #include <cuda_runtime.h>

@@ -446,3 +446,12 @@ def test_small_ops_16_byte_forms(cuda, C_, B, H, W):
     # f32 sums of n values in two orders: each within n 2^-24 of the sum of magnitudes
     mag = (fine.double().abs() * (fine2.double() > 0)).sum(0)
     assert ((db[0] - db[1]).abs() <= 2 * B * H * W * 2.0 ** -24 * mag + 1e-30).all()
+
+
+def test_pow53_is_the_double_power_over_its_whole_range(cuda):
+    """Every float of [2^-70, 2^70], where the short form is taken, and an octave beyond: 1.2 G values."""
+    from pyfastflow_b200 import _lib
+
+    bad = C.c_longlong(-1)
+    _lib.call("pff_pow53_selfcheck", 0x1C000000, 0x63000000, C.byref(bad))
+    assert bad.value == 0
