@@ -361,7 +361,17 @@ __global__ void __launch_bounds__(DF_THREADS) k_diffuse_fused(const float *__res
     for (int sw = 1; sw <= H; ++sw) {
         const int bw = RX - 2 * sw, bh = RY - 2 * sw;
         if (inner) {  // every cell inside the grid, off its edges: summation order top, left, right, bottom
-            for (int t = threadIdx.x; t < PX / 4 * bh; t += blockDim.x) {
+            if (H == 2) {  // 578 and 544 groups of four would leave the second trip of 512 threads nearly empty
+                for (int t = threadIdx.x; t < bw * bh; t += blockDim.x) {
+                    const int i = (sw + t / bw) * PX + sw + t % bw;
+                    float acc = prec_dx2;
+                    acc = df_add(acc, w0[i], qc[i - PX]);
+                    acc = df_add(acc, w1[i], qc[i - 1]);
+                    acc = df_add(acc, w2[i], qc[i + 1]);
+                    qn[i] = df_add(acc, w3[i], qc[i + PX]);
+                }
+            }
+            for (int t = threadIdx.x; H != 2 && t < PX / 4 * bh; t += blockDim.x) {
                 const int i = (sw + t / (PX / 4)) * PX + t % (PX / 4) * 4;
                 auto ld = [](const float *p) { return *reinterpret_cast<const float4 *>(p); };
                 const float4 a0 = ld(w0 + i), a1 = ld(w1 + i), a2 = ld(w2 + i), a3 = ld(w3 + i);
