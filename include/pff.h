@@ -37,7 +37,7 @@ extern "C" {
 #define PFF_ERR_CUDA 2       /* CUDA runtime error (launch or copy) */
 #define PFF_ERR_NOCONV 3     /* iteration cap reached before convergence */
 #define PFF_ERR_WORKSPACE 4  /* workspace too small */
-#define PFF_ERR_UNAVAILABLE 5 /* this path is not available here (e.g. CUDA graphs switched off) */
+#define PFF_ERR_UNAVAILABLE 5 /* this path is not available here (e.g. the device-driven reroute loop switched off) */
 
 /* Library version (major*10000 + minor*100 + patch). */
 int pff_version(void);
@@ -62,9 +62,10 @@ int pff_barrier_test(int kernels, int absent, int limit_us);
  * in milliseconds and the number of probed launches (0 if it never ran). */
 int pff_probe_enable(int on);
 int pff_probe_read(const char *name, double *total_ms, int *launches);
-/* Whether pff_reroute_flow drives its outer loop from a device-side CUDA graph
- * (1, the default) or from the host (0: one synchronisation per outer iteration;
- * its kernels can then be profiled and probed one by one).  The environment
+/* Whether pff_reroute_flow runs its outer loop in a persistent cooperative kernel
+ * (1, the default) or drives it from the host (0: one synchronisation per outer
+ * iteration; its kernels can then be profiled and probed one by one).  The name is
+ * kept from an earlier form that used a CUDA graph.  The environment
  * variable PFF_REROUTE_NO_GRAPH makes 0 the default.  Returns the previous
  * setting.  No reference counterpart. */
 int pff_reroute_use_graphs(int on);
