@@ -819,15 +819,6 @@ __device__ __noinline__ void tile_reroute(const BatchTile &T, const BatchArrays 
     const int N = g.nx * g.ny;
     const long long o = T.off, ob = T.boff;
     int32_t *R = reinterpret_cast<int32_t *>(A.p_) + o;  // later the segment list
-    if (N <= GF_SMALL) {
-        if (Tm.r == 0) {
-            FOR_CELLS(i, N) A.rec_[o + i] = A.rcv[o + i];
-            __syncthreads();
-            tile_reroute_steps<MODE>(g, T, A, z, sh, 0, -1);
-        }
-        Tm.sync();
-        return;
-    }
     if (Tm.r == 0)
         for (int k = threadIdx.x; k < 64 + LOOP_ITS * LOOP_CTR; k += blockDim.x) sh.loop[k] = 0;
     if (threadIdx.x == 0) {
@@ -1153,7 +1144,16 @@ __device__ __forceinline__ void gf_tile(const BatchTile &T, const BatchArrays &A
     float rmax = 0.f, rmean = 0.f;
     for (; it < P.niter; ++it) {
         tile_receivers<MODE>(g, dx, zh, rec, nullptr, Tm);
-        tile_reroute<MODE>(T, A, zh, sh, Tm, smem);
+        if (N <= GF_SMALL) {
+            if (Tm.r == 0) {
+                FOR_CELLS(i, N) A.rec_[o + i] = rec[i];
+                __syncthreads();
+                tile_reroute_steps<MODE>(g, T, A, zh, sh, 0, -1);
+            }
+            Tm.sync();
+        } else {
+            tile_reroute<MODE>(T, A, zh, sh, Tm, smem);
+        }
         const int2 *a = gf_fill(N, fa, fb, rec, zh, h, href, nr, P.eps, sh, Tm);
         gf_weights<MODE>(g, dx, zh, w, Tm);
         const float *qa = gf_sweeps<MODE>(g, w, Q, temp, prec_dx2, Tm);
@@ -1365,16 +1365,17 @@ static int batch_team(long long total, int ntiles, int slots)
 // take 900 and 1150; 48 x 48: 205 and 250, but 2000 of them 2198 and 2126, and 40 of 56 x 56
 // with 512 threads 264 and 259; with 256 threads 40 of 40 x 40 237 and 239.  Mixed batches go by their
 // largest tile, the last to end: 40 of 24 to 60 cells a side 219 and 234, of 24 to 75 289 and
-// 275.  Where blocks of 1024 threads have two tiles each, the smaller ones make up for
-// it: 200 of 24 to 75 384 and 476 (but of 64 x 64 567 and 503).
+// 275.  Where tiles outnumber the SMs the smaller ones make up for it: 200 of 24 to 75 384 and
+// 476 (but of 64 x 64 567 and 503), with 512 threads 280 of 37 to 60 328 and
+// 367 (220 of 40 to 66 368 and 344).
 constexpr int SMALL_CLASSES = 3;
 static int small_class(int threads) { return threads == 1024 ? 0 : (threads == 512 ? 1 : 2); }
 static int small_cells(int cls, int ntiles, long long total)
 {
     if (cls == 2) return 1900;
     if (ntiles > 300) return 2600;
-    if (cls == 1) return 3100;
-    return ntiles > 148 && total <= 2600LL * ntiles ? 5600 : 3600;
+    const bool many = ntiles > 148 && total <= (cls == 0 ? 2800LL : 2400LL) * ntiles;
+    return cls == 0 ? (many ? 5600 : 3600) : (many ? 4400 : 3100);
 }
 
 struct BatchShape {
